@@ -693,16 +693,47 @@ int llg_apply_matrix(llg_state* st, int k, const int* qubits, const double* m) {
         bd.k = ++k;
         m = mx;
     }
-    if (block_tc_eligible(st->P, st->n, k)) {
-        const size_t wb = block_tc_weight_bytes(st->P, k);
+    if (k == 5 && gate_block_eligible(st->P, st->n)) {
         if (!st->d_block_tc) {
-            // the largest weight set of any precision (the eight-slice FP64 one)
-            const size_t cap = std::max(block_tc_weight_bytes(LLG_DF64, kMaxBlockQubits),
-                                        block_tc_weight_bytes(LLG_F64, kMaxBlockQubits));
+            const size_t cap = gate_block_weight_bytes(LLG_F64);
             LLG_CUDA(cudaMalloc(&st->d_block_tc, cap), "cudaMalloc(block weights)");
             LLG_CUDA(cudaHostAlloc((void**)&st->h_block_tc, cap, cudaHostAllocDefault), "cudaHostAlloc(block weights)");
         }
-        if (wb > std::max(block_tc_weight_bytes(LLG_DF64, kMaxBlockQubits), block_tc_weight_bytes(LLG_F64, kMaxBlockQubits)))
+        // the targets in increasing order; the matrix follows them
+        int ord[5] = {0, 1, 2, 3, 4};
+        std::sort(ord, ord + 5, [&](int a, int b) { return bd.q[a] < bd.q[b]; });
+        int from[32];  // sorted index -> caller's index
+        for (int i = 0; i < 32; ++i) {
+            from[i] = 0;
+            for (int b = 0; b < 5; ++b) from[i] |= ((i >> b) & 1) << ord[b];
+        }
+        double* hm = reinterpret_cast<double*>(st->h_block);
+        for (int r = 0; r < 32; ++r)
+            for (int c = 0; c < 32; ++c)
+                for (int p = 0; p < 2; ++p) hm[2 * (r * 32 + c) + p] = m[2 * (from[r] * 32 + from[c]) + p];
+        BlockDesc sd = bd;
+        for (int b = 0; b < 5; ++b) sd.q[b] = bd.q[ord[b]];
+        LLG_CUDA(cudaMemcpyAsync(st->d_block, hm, slots * sizeof(double), cudaMemcpyHostToDevice, st->stream),
+                 "cudaMemcpyAsync(block)");
+        LLG_CUDA(cudaEventRecord(st->block_done, st->stream), "cudaEventRecord");
+        st->block_pending = true;
+        st->block_tc_launched = true;
+        return traced(st, LLG_PROF_GATE, 2, "block kernel (tensor cores)", [&] {
+            const cudaError_t e =
+                launch_gate_block_matrix(st->P, reinterpret_cast<const double*>(st->d_block), st->d_block_tc, st->stream);
+            if (e != cudaSuccess) return e;
+            return launch_gate_block(st->P, st->d_psi, st->n, sd, st->d_block_tc, true, st->d_flags + 1, st->stream);
+        });
+    }
+    if (block_tc_eligible(st->P, st->n, k)) {
+        const size_t wb = block_tc_weight_bytes(st->P, k);
+        if (!st->d_block_tc) {
+            // the largest weight set of any block (the 5-qubit FP64 one)
+            const size_t cap = gate_block_weight_bytes(LLG_F64);
+            LLG_CUDA(cudaMalloc(&st->d_block_tc, cap), "cudaMalloc(block weights)");
+            LLG_CUDA(cudaHostAlloc((void**)&st->h_block_tc, cap, cudaHostAllocDefault), "cudaHostAlloc(block weights)");
+        }
+        if (wb > gate_block_weight_bytes(LLG_F64))
             return set_error(LLG_ERUNTIME, "apply_matrix: block weights larger than their staging buffer");
         block_tc_prepare(st->P, k, m, st->h_block_tc);
         LLG_CUDA(cudaMemcpyAsync(st->d_block_tc, st->h_block_tc, wb, cudaMemcpyHostToDevice, st->stream),
@@ -711,7 +742,7 @@ int llg_apply_matrix(llg_state* st, int k, const int* qubits, const double* m) {
         st->block_pending = true;
         st->block_tc_launched = true;
         return traced(st, LLG_PROF_GATE, 1, "block kernel (tensor cores)",
-                      [&] { return launch_block_tc(st->P, st->d_psi, st->n, bd, st->d_block_tc, st->d_flags, st->stream); });
+                      [&] { return launch_block_tc(st->P, st->d_psi, st->n, bd, st->d_block_tc, st->d_flags + 1, st->stream); });
     }
     for (int i = 0; i < slots; ++i) st->h_block[i] = pack_coef(st->P, m[i]);
     LLG_CUDA(cudaMemcpyAsync(st->d_block, st->h_block, slots * sizeof(uint64_t), cudaMemcpyHostToDevice, st->stream),

@@ -1,0 +1,696 @@
+// llg_gateblock.cu -- dense 5-qubit blocks of 16-byte states (IEEE complex128, double-float) on the
+// fifth-generation tensor cores, as a warp-specialised pipeline.
+//
+// A block maps every group of 32 amplitudes that differ only in its five target qubits through a
+// 32 x 32 complex matrix.  Over reals, a tile of 128 groups is one product D[g][r] = sum_c X[g][c]
+// W[r][c] with W the 64 x 64 real form.  Both operands are cut into S balanced 8-bit digits (the
+// Ozaki scheme: Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 2012), exact in fp16:
+//     x = 2^(e_g - 1084) sum_i x_i 2^(56 - 8 i),   w = 2^(e_r - 6) sum_j w_j 2^(-8 j),
+// where e_g is the group's largest biased exponent (the digits are the bytes of the 62-bit integer
+// X = m 2^(9 - e_g + e) plus a bias), |x_0|, |w_0| <= 64 and the other digits at most 128 in size.
+// The products with i + j <= S - 1 are accumulated by diagonal d = i + j in fp32: a diagonal is a
+// sum of at most 64 (d + 1) products of integers, below 2^24, so every diagonal is exact.  The
+// epilogue adds the diagonals in a 64-bit integer (D_0 .. D_4 exactly, the rest rounded at 2^-57 of
+// the full scale) and converts once.  The error against the group's largest amplitude is that one
+// rounding plus dropped products near 2^-58 (S = 8) or 2^-50 (S = 7, for double-float states, whose
+// own significand has about 48 bits).
+//
+// What bounds it: 32 bytes of HBM per amplitude (5.1 ms per 2^30) against 36 slice products of
+// M128 N64 K64 per tile (4608 clocks of the tensor pipe, 4.2 ms per 2^30).  Both need every phase to
+// run at the same time, so the CTA (one per SM, persistent) has three roles:
+//   * 8 slicer warps: load the tile into registers, agree on e_g, cut the amplitudes into digits and
+//     write them in the no-swizzle K-major core-matrix layout.  A tile is 4 chunks of 8 amplitudes
+//     per group (K = 16); a ring of 5 chunks lets the slicing run ahead of the products.  The next
+//     tile's loads reuse a chunk's registers as soon as it is sliced.
+//   * one MMA warp: D is computed in two halves of 16 output amplitudes, each with its own
+//     accumulator set, so one half is recombined while the other is computed.  The gate's S slices
+//     are stacked along N: X_i times [W_0 .. W_(S-1-i)] is one instruction whose columns are the
+//     diagonals i .. S-1, so a state slice is read once per K step instead of S - i times (N = 64
+//     products were bound by shared-memory reads, 48 clocks for 32 of tensor work).
+//   * 8 epilogue warps: tcgen05.ld, recombination, stores.
+// The serial form that this replaced (one set of accumulators, load - slice - multiply - recombine
+// one after the other on 16 warps) took 25k clocks per tile.
+//
+// Digits without integer work: the bytes u of X + 0x8080..80 are d + 128, and the fp16 with bits
+// 0x6400 | u is 1024 + u, so a byte permute and one packed subtraction of 1152 make two digits.
+// fp32 to integer without conversions (16 per clock and SM): diagonals 0 .. 4 are at most 2^22 in
+// size, so adding 1.5 2^23 leaves the integer in the low bits of the float.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <cstring>
+
+#include "llg_common.cuh"
+#include "llg_internal.h"
+#include "llg_launch.h"
+
+namespace llg {
+
+namespace {
+
+constexpr int kGroups = 128;     // groups per tile (the MMA's M)
+constexpr int kAmps = 32;        // amplitudes per group
+constexpr int kChunks = 4;       // K steps of 16 reals (8 amplitudes) per tile
+constexpr int kRing = 5;         // chunk buffers
+constexpr int kSlicerWarps = 8, kEpiWarps = 8;
+constexpr int kMmaWarp = kSlicerWarps + kEpiWarps;
+constexpr int kThreads = (kSlicerWarps + kEpiWarps + 4) * 32;  // five warpgroups; the last one's first warp issues the MMAs
+// registers a thread by role (setmaxnreg): 96 at launch, 2 * 112 + 2 * 104 + 40 <= 5 * 96 per scheduler
+constexpr int kSlicerRegs = 112, kEpiRegs = 104, kMmaRegs = 40;
+constexpr int kSliceBytes = kGroups * 16 * 2;  // one digit of one chunk
+constexpr int kTmemCols = 512;                 // two accumulator sets
+constexpr long kWaitLimit = 1L << 22;          // mbarrier polls before the kernel reports a timeout
+
+template <int P>
+struct Shape {
+    static constexpr int S = P == LLG_F64 ? 8 : 7;             // digits per operand
+    static constexpr int kChunkBytes = S * kSliceBytes;
+    static constexpr int kWHalfBytes = S * 32 * 64 * 2;        // 32 S rows (digit, output) of 64 columns
+    static constexpr int kSetStride = 256;                     // columns between the accumulator sets (32 S used)
+    static constexpr size_t kSmem = (size_t)kRing * kChunkBytes + 2 * kWHalfBytes;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// tcgen05 shared-memory descriptor, no swizzle (start, leading and stride byte offsets, version 1)
+__device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)((lbo >> 4) & 0x3FFF) << 16 | (uint64_t)((sbo >> 4) & 0x3FFF) << 32 |
+           (uint64_t)1 << 46;
+}
+
+// byte offset of element (row, c) of a rows x kreals fp16 operand: 8x8 cores of 128 bytes,
+// K-direction cores adjacent, 8-row groups kreals / 8 cores apart
+__device__ __forceinline__ uint32_t core_off(int row, int c, int kreals) {
+    return (uint32_t)((row >> 3) * (kreals / 8) * 128 + (c >> 3) * 128 + (row & 7) * 16 + (c & 7) * 2);
+}
+
+// column (K index) of part `part` (0 real, 1 imaginary) of amplitude j: chunks of 8 amplitudes; a
+// slicer thread's four amplitudes (j bit 0 fixed) fill one 8-wide core row
+__device__ __forceinline__ int col_of(int j, int part) { return 16 * (j >> 3) + 8 * (j & 1) + 2 * ((j >> 1) & 3) + part; }
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait for the completion of phase `ph`; false when the limit ran out here or in another
+// role (then *abort_s is set).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t ph, volatile int* abort_s) {
+    for (long it = 0; it < kWaitLimit; ++it) {
+        uint32_t done;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(bar), "r"(ph)
+                     : "memory");
+        if (done) return true;
+        if ((it & 255) == 255 && *abort_s) return false;
+    }
+    *abort_s = 1;
+    return false;
+}
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t ph, volatile int* abort_s) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_s));
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// X = the 62-bit fixed-point integer of |x| against the group exponent eg (eg20 = eg 2^20 + 2^20 - 1;
+// a shift by 64 or more gives zero), plus the digit bias.  eg > 64: zeros and subnormals need no
+// care, their X is zero.
+__device__ __forceinline__ uint64_t fixed_f64(double x, uint32_t eg20) {
+    const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x);
+    const uint32_t s = (eg20 - (h & 0x7FFFFFFFu)) >> 20;
+    const uint32_t mh = (__funnelshift_l(l, h, 9) & 0x1FFFFFFFu) | 0x20000000u;
+    uint64_t X = ((uint64_t)mh << 32) | (l << 9);
+    asm("shr.u64 %0, %0, %1;" : "+l"(X) : "r"(s));
+    return X + 0x8080808080808080ULL;
+}
+// the same for any group exponent: a zero or subnormal has no hidden bit and exponent 1
+__device__ __noinline__ uint64_t fixed_f64_any(double x, int eg) {
+    const uint64_t b = (uint64_t)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFULL;
+    const int ex = (int)(b >> 52);
+    const uint64_t m = (b & 0xFFFFFFFFFFFFFULL) | (ex ? 1ULL << 52 : 0ULL);
+    return ((m << 9) >> min(eg - max(ex, 1), 63)) + 0x8080808080808080ULL;
+}
+
+__device__ __forceinline__ uint32_t h2_bits(__half2 v) {
+    uint32_t b;
+    memcpy(&b, &v, 4);
+    return b;
+}
+__device__ __forceinline__ __half2 h2_of(uint32_t b) {
+    __half2 v;
+    memcpy(&v, &b, 4);
+    return v;
+}
+
+// Four digits (bytes 3 .. 0 of the biased words) of eight reals as fp16, one 16-byte core row each;
+// sgn: +-1 of each pair of reals, bias: -1152 sgn
+__device__ __forceinline__ void digits4(const uint32_t (&w)[8], const __half2 (&sgn)[4], const __half2 (&bias)[4],
+                                        unsigned char* dst) {
+    uint32_t v[4][4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const uint32_t t = __byte_perm(w[2 * p], w[2 * p + 1], 0x6273);
+        const uint32_t u = __byte_perm(w[2 * p], w[2 * p + 1], 0x4051);
+        v[0][p] = h2_bits(__hfma2(h2_of(__byte_perm(t, 0x64646464u, 0x4140)), sgn[p], bias[p]));
+        v[1][p] = h2_bits(__hfma2(h2_of(__byte_perm(t, 0x64646464u, 0x4342)), sgn[p], bias[p]));
+        v[2][p] = h2_bits(__hfma2(h2_of(__byte_perm(u, 0x64646464u, 0x4140)), sgn[p], bias[p]));
+        v[3][p] = h2_bits(__hfma2(h2_of(__byte_perm(u, 0x64646464u, 0x4342)), sgn[p], bias[p]));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        *reinterpret_cast<uint4*>(dst + k * kSliceBytes) = make_uint4(v[k][0], v[k][1], v[k][2], v[k][3]);
+}
+
+// 2^e as a float for e in [-126, 127]
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
+
+// r 2^e for a result outside the range of the exponent-field addition
+__device__ __noinline__ double scale_slow(double r, int e) { return ldexp(r, e); }
+
+// element offset of every amplitude of a group (a kernel parameter: constant-bank operands)
+struct TargetOffsets {
+    uint64_t o[kAmps];
+};
+
+template <int P>
+struct Elem;
+template <>
+struct Elem<LLG_F64> {
+    using S = double2;
+};
+template <>
+struct Elem<LLG_DF64> {
+    using S = float4;
+};
+
+// `mirror` (nullptr: none): the device address of a mapped host buffer that also receives the
+// output as FP64.
+// kRows: the gate's rows have exponents of their own (any matrix); else all have exponent 1 (a product
+// of unitary gates, entries at most 1).
+template <int P, bool kRows>
+__global__ void __launch_bounds__(kThreads, 1)
+    k_gate_block(typename Elem<P>::S* __restrict__ psi, int n, const __grid_constant__ TargetOffsets to, uint64_t tmask,
+                 const uint4* __restrict__ weights, int* __restrict__ err_flag, double2* __restrict__ mirror) {
+    using T = Shape<P>;
+    constexpr int S = T::S;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char* sA = smem;                            // kRing chunks of S digits
+    unsigned char* sW = smem + kRing * T::kChunkBytes;   // two halves of the gate's digits
+    __shared__ uint64_t toff[kAmps];
+    __shared__ int32_t eg_s[3][kGroups];  // group exponents, three tiles in turn
+    __shared__ __align__(16) int32_t er_s[64];
+    __shared__ __align__(8) uint64_t bars[2 * kRing + 8];
+    __shared__ uint32_t tmem_s;
+    __shared__ int abort_flag;
+    volatile int* abort_s = &abort_flag;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kRing]);
+    const uint32_t accfull0 = smem_u32(&bars[2 * kRing]), accempty0 = smem_u32(&bars[2 * kRing + 2]);
+    const uint32_t egfull0 = smem_u32(&bars[2 * kRing + 4]), drain = smem_u32(&bars[2 * kRing + 7]);
+
+    if (tid < kAmps) toff[tid] = to.o[tid];
+    {
+        uint4* dst = reinterpret_cast<uint4*>(sW);
+        for (int i = tid; i < 2 * T::kWHalfBytes / 16; i += kThreads) dst[i] = weights[i];
+        if (tid < 16) reinterpret_cast<uint4*>(er_s)[tid] = weights[2 * T::kWHalfBytes / 16 + tid];
+    }
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < kRing; ++i) {
+            mbar_init(full0 + 8 * i, kSlicerWarps);
+            mbar_init(empty0 + 8 * i, 1);
+        }
+        for (int h = 0; h < 2; ++h) {
+            mbar_init(accfull0 + 8 * h, 1);
+            mbar_init(accempty0 + 8 * h, kEpiWarps);
+        }
+        for (int i = 0; i < 3; ++i) mbar_init(egfull0 + 8 * i, kSlicerWarps);
+        mbar_init(drain, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)),
+                     "r"(kTmemCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the gate's digits are read by the MMAs
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_s;
+    const uint64_t ntiles = (1ULL << (n - 5)) / kGroups;
+
+    if (warp < kSlicerWarps) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSlicerRegs));
+        // ---- slicers: group g = 16 warp + (lane & 15), amplitudes j = 8 ks + 2 i + h with h = lane / 16:
+        // a warp reads whole 32-byte sectors when the lowest target is qubit 0 (j and j + 1 adjacent),
+        // and eight neighbouring lanes store one 128-byte core ----
+        const int g = 16 * warp + (lane & 15), h = lane >> 4;
+        // a tile is runs of 2^cl contiguous amplitudes (at least 2 KB); lane j of warp 0 asks for the run
+        // that starts at target offset j, two tiles ahead, so that the loads of the last chunk, which are
+        // waited for at once, come from L2
+        const uint64_t in_tile = insert0_mask(kGroups - 1, tmask) | tmask;
+        const int cl = __ffsll((long long)~in_tile) - 1;
+        const bool run_start = warp == 0 && (toff[lane] & ((1ULL << cl) - 1)) == 0;
+        auto prefetch_l2 = [&](uint64_t t) {
+            if (run_start && t < ntiles)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(psi + (insert0_mask(t * kGroups, tmask) | toff[lane])),
+                             "r"(16u << cl)
+                             : "memory");
+        };
+        prefetch_l2(blockIdx.x + (uint64_t)gridDim.x);
+        typename Elem<P>::S a[16];
+        uint64_t tile = blockIdx.x;
+        if (tile < ntiles) {
+            const auto* pb = psi + (insert0_mask(tile * kGroups + (uint64_t)g, tmask) | (h ? to.o[1] : 0));
+#pragma unroll
+            for (int k = 0; k < 16; ++k) a[k] = __ldcg(pb + to.o[2 * k]);
+        }
+        int slot = 0, egb = 0;
+        uint32_t phase = 1;  // of the slot's previous release: the first round needs no wait
+        bool first = true, ok = true;
+        for (; tile < ntiles && ok; tile += gridDim.x, egb = egb == 2 ? 0 : egb + 1) {
+            int eg;
+            if constexpr (P == LLG_F64) {
+                uint32_t mx = 0;
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                    mx = max(mx, max((uint32_t)__double2hiint(a[k].x) & 0x7FFFFFFFu, (uint32_t)__double2hiint(a[k].y) & 0x7FFFFFFFu));
+                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                eg = (int)(mx >> 20);
+                if (eg == 0) {  // zeros (any scale gives zero) or subnormals
+                    uint32_t any = 0;
+#pragma unroll
+                    for (int k = 0; k < 16; ++k)
+                        any |= (uint32_t)__double2hiint(a[k].x) << 1 | (uint32_t)__double2loint(a[k].x) |
+                               (uint32_t)__double2hiint(a[k].y) << 1 | (uint32_t)__double2loint(a[k].y);
+                    eg = any ? 1 : 1023;
+                }
+                eg = min(eg, __shfl_xor_sync(0xffffffffu, eg, 16));  // one half zero, the other subnormal
+            } else {
+                // stored pairs may be unnormalised: TwoSum makes the high part the leading one
+                float mx = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const df re = two_sum(a[k].x, a[k].z), im = two_sum(a[k].y, a[k].w);
+                    a[k] = make_float4(re.hi, im.hi, re.lo, im.lo);
+                    mx = fmaxf(mx, fmaxf(fabsf(re.hi), fabsf(im.hi)));
+                }
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                // clamped so that the scale factor 2^(132 - e) below stays a normal float
+                eg = max((int)(__float_as_uint(mx) >> 23), 8);
+            }
+            const uint64_t next = tile + gridDim.x;
+            prefetch_l2(next + gridDim.x);
+            const auto* pb = psi + ((next < ntiles ? insert0_mask(next * kGroups + (uint64_t)g, tmask) : 0) | (h ? to.o[1] : 0));
+#pragma unroll
+            for (int ks = 0; ks < kChunks; ++ks) {
+                if (!first && !warp_wait(empty0 + 8 * slot, phase, abort_s)) {
+                    ok = false;
+                    break;
+                }
+                if (ks == 0) {
+                    // the slot's last reader, the epilogue three tiles back, ended before the products
+                    // that freed this chunk were issued
+                    if (h == 0) eg_s[egb][g] = eg;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(egfull0 + 8 * egb);
+                }
+                unsigned char* dst = sA + slot * T::kChunkBytes + core_off(g, 8 * h, 16);
+                if constexpr (P == LLG_F64) {
+                    uint32_t wh[8], wl[8];
+                    __half2 sgn[4], bias[4];
+                    const uint32_t eg20 = ((uint32_t)eg << 20) | 0xFFFFFu;
+                    const bool small = __any_sync(0xffffffffu, eg <= 64);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const double2 v = a[4 * ks + i];
+                        const uint64_t xr = small ? fixed_f64_any(v.x, eg) : fixed_f64(v.x, eg20);
+                        const uint64_t xi = small ? fixed_f64_any(v.y, eg) : fixed_f64(v.y, eg20);
+                        wh[2 * i] = (uint32_t)(xr >> 32);
+                        wl[2 * i] = (uint32_t)xr;
+                        wh[2 * i + 1] = (uint32_t)(xi >> 32);
+                        wl[2 * i + 1] = (uint32_t)xi;
+                        const uint32_t sg = __byte_perm((uint32_t)__double2hiint(v.x), (uint32_t)__double2hiint(v.y), 0x7733);
+                        sgn[i] = h2_of((sg & 0x80008000u) | 0x3C003C00u);
+                        bias[i] = __hmul2(sgn[i], __half2half2(__ushort_as_half(0xE480)));  // -1152
+                    }
+                    digits4(wh, sgn, bias, dst);
+                    digits4(wl, sgn, bias, dst + 4 * kSliceBytes);
+                } else {
+                    // nearest-integer digits by the magic addition, from the high part and (from the
+                    // fourth digit on) the low part added to what is left of it
+                    const float sc = pow2f(132 - eg);  // the largest high part becomes 2^5 .. 2^6
+#pragma unroll
+                    for (int hv2 = 0; hv2 < 2; ++hv2) {  // four reals at a time: half a core row
+                        float dg[S][4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float4 v = a[4 * ks + 2 * hv2 + (q >> 1)];
+                            float r = ((q & 1) ? v.y : v.x) * sc, rest = 0.0f;
+                            const float lo = ((q & 1) ? v.w : v.z) * sc * 16777216.0f;
+#pragma unroll
+                            for (int s = 0; s < S; ++s) {
+                                if (s == 3) {
+                                    const df t = two_sum(r, lo);
+                                    r = t.hi;
+                                    rest = t.lo;
+                                }
+                                if (s == 6) r = fmaf(rest, 16777216.0f, r);
+                                dg[s][q] = __fsub_rn(__fadd_rn(r, 12582912.0f), 12582912.0f);
+                                r = __fsub_rn(r, dg[s][q]) * 256.0f;
+                            }
+                        }
+#pragma unroll
+                        for (int s = 0; s < S; ++s) {
+                            const __half2 h0 = __floats2half2_rn(dg[s][0], dg[s][1]), h1 = __floats2half2_rn(dg[s][2], dg[s][3]);
+                            uint2 o;
+                            memcpy(&o.x, &h0, 4);
+                            memcpy(&o.y, &h1, 4);
+                            *reinterpret_cast<uint2*>(dst + s * kSliceBytes + 8 * hv2) = o;
+                        }
+                    }
+                }
+                if (next < ntiles) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) a[4 * ks + i] = __ldcg(pb + to.o[2 * (4 * ks + i)]);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full0 + 8 * slot);
+                if (++slot == kRing) {
+                    slot = 0;
+                    phase ^= 1;
+                    first = false;
+                }
+            }
+        }
+    } else if (warp < kMmaWarp) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
+        // ---- epilogue: tensor-memory lanes 32 (warp & 3) .. +31 (the groups), amplitudes
+        // 16 half + 8 e + 4 p .. +3 ----
+        const int row = 32 * (warp & 3) + lane, e = (warp - kSlicerWarps) >> 2;
+        const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        const bool pair32 = to.o[1] == 1;  // amplitudes j and j + 1 (j even) are adjacent
+        int erm = 1;
+        if (kRows)
+            for (int r = 0; r < 64; ++r) erm = max(erm, abs(er_s[r]));
+        int egb = 0;
+        uint32_t phase = 0, egphase = 0;
+        bool ok = true;
+        for (uint64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, phase ^= 1) {
+            const uint64_t base = insert0_mask(tile * kGroups + (uint64_t)row, tmask) | toff[8 * e];
+            if (!warp_wait(egfull0 + 8 * egb, egphase, abort_s)) break;
+            const int eg = eg_s[egb][row];
+            if (++egb == 3) {
+                egb = 0;
+                egphase ^= 1;
+            }
+            // the exponent-field addition is safe (results normal or zero)
+            const bool all_fast = __all_sync(0xffffffffu, erm <= 32 && eg >= 128 && eg <= 1984);
+#pragma unroll 1
+            for (int half = 0; half < 2; ++half) {
+                if (!warp_wait(accfull0 + 8 * half, phase, abort_s)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+                for (int p = 0; p < 2; ++p) {
+                    uint32_t v[S][8];
+#pragma unroll
+                    for (int d = 0; d < S; ++d) {
+                        const uint32_t taddr = tlane + (uint32_t)(half * T::kSetStride + 32 * d + 16 * e + 8 * p);
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                                     : "=r"(v[d][0]), "=r"(v[d][1]), "=r"(v[d][2]), "=r"(v[d][3]), "=r"(v[d][4]),
+                                       "=r"(v[d][5]), "=r"(v[d][6]), "=r"(v[d][7])
+                                     : "r"(taddr));
+                    }
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (p == 1) {  // this warp has read the set
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(accempty0 + 8 * half);
+                    }
+                    const uint64_t pos = base | toff[16 * half + 4 * p];
+                    typename Elem<P>::S out[4];
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const int er = kRows ? er_s[32 * half + 16 * e + 8 * p + c] : 1;
+                        if constexpr (P == LLG_F64) {
+                            // 2^44 sum_d 2^(-8 d) D_d: D_0 .. D_4 exact, D_5 .. D_7 rounded to an integer
+                            const float magic = 12582912.0f;
+                            const uint32_t b0 = __float_as_uint(__fadd_rn(__uint_as_float(v[0][c]), magic));
+                            const uint32_t b1 = __float_as_uint(__fadd_rn(__uint_as_float(v[1][c]), magic));
+                            const uint32_t b2 = __float_as_uint(__fadd_rn(__uint_as_float(v[2][c]), magic));
+                            const uint32_t b3 = __float_as_uint(__fadd_rn(__uint_as_float(v[3][c]), magic));
+                            const uint32_t b4 = __float_as_uint(__fadd_rn(__uint_as_float(v[4][c]), magic));
+                            const float low = fmaf(__uint_as_float(v[7][c]), 0x1p-12f,
+                                                   fmaf(__uint_as_float(v[6][c]), 0x1p-4f, __uint_as_float(v[5][c]) * 16.0f));
+                            constexpr uint64_t kM = 0x4B400000ULL;
+                            constexpr uint64_t kC = kM * ((1ULL << 28) + (1ULL << 20) + (1ULL << 12)) +
+                                                    (kM * ((1ULL << 12) + (1ULL << 4)) << 32);
+                            uint64_t acc = (uint64_t)(int64_t)__float2int_rn(low) - kC;
+                            asm("mad.wide.u32 %0, %1, 4096, %0;" : "+l"(acc) : "r"(b4));
+                            asm("mad.wide.u32 %0, %1, 1048576, %0;" : "+l"(acc) : "r"(b3));
+                            asm("mad.wide.u32 %0, %1, 268435456, %0;" : "+l"(acc) : "r"(b2));
+                            acc += (uint64_t)((b0 << 12) + (b1 << 4)) << 32;
+                            double r = __ll2double_rn((long long)acc);
+                            const int et = eg + er - 1078;
+                            if (all_fast) {
+                                const int hi = __double2hiint(r);
+                                r = __hiloint2double(hi ? hi + (et << 20) : hi, __double2loint(r));
+                            } else if (eg == 2047) {
+                                r = __longlong_as_double(0x7FF8000000000000LL);  // an Inf or a NaN in the group
+                            } else {
+                                r = scale_slow(r, et);
+                            }
+                            if (c & 1) out[c >> 1].y = r;
+                            else out[c >> 1].x = r;
+                        } else {
+                            // D_0 + 2^-8 D_1 + 2^-16 D_2 exactly, then 2^-24 (D_3 + ..) rounded
+                            const float d0 = __uint_as_float(v[0][c]), d1 = __uint_as_float(v[1][c]) * 0x1p-8f;
+                            const float d2 = __uint_as_float(v[2][c]) * 0x1p-16f, d3 = __uint_as_float(v[3][c]) * 0x1p-24f;
+                            const float t = fmaf(__uint_as_float(v[6][c]), 0x1p-16f,
+                                                 fmaf(__uint_as_float(v[5][c]), 0x1p-8f, __uint_as_float(v[4][c]))) * 0x1p-32f;
+                            const df s1 = two_sum(d0, d1), s2 = two_sum(s1.hi, d2);
+                            const df s3 = two_sum(__fadd_rn(s1.lo, s2.lo), d3);
+                            const df s4 = two_sum(s2.hi, s3.hi);
+                            const df acc = fast_two_sum(s4.hi, __fadd_rn(s4.lo, __fadd_rn(s3.lo, t)));
+                            const int et = eg + er - 138;  // x = 2^(e_g - 132) .., w = 2^(e_r - 6) ..
+                            const int e1 = max(min(et, 100), -100), e2 = max(min(et - e1, 100), -126);
+                            const float f1 = pow2f(e1), f2 = pow2f(e2);
+                            const float oh = acc.hi * f1 * f2, ol = acc.lo * f1 * f2;
+                            if (c & 1) {
+                                out[c >> 1].y = oh;
+                                out[c >> 1].w = ol;
+                            } else {
+                                out[c >> 1].x = oh;
+                                out[c >> 1].z = ol;
+                            }
+                        }
+                    }
+                    if (pair32) {
+#pragma unroll
+                        for (int c = 0; c < 4; c += 2) {
+                            uint64_t w[4];
+                            memcpy(w, &out[c], 32);
+                            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(psi + pos + to.o[c]), "l"(w[0]), "l"(w[1]),
+                                         "l"(w[2]), "l"(w[3])
+                                         : "memory");
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) psi[pos + to.o[c]] = out[c];
+                    }
+                    if (mirror) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            if constexpr (P == LLG_F64) mirror[pos + to.o[c]] = out[c];
+                            else
+                                mirror[pos + to.o[c]] = make_double2((double)out[c].x + (double)out[c].z,
+                                                                           (double)out[c].y + (double)out[c].w);
+                        }
+                    }
+                }
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegs));
+        if (warp == kMmaWarp) {
+            // ---- the MMA warp: the whole warp walks the loop (so that the descriptors are uniform), one
+            // elected thread issues ----
+            constexpr uint32_t idesc0 = (1u << 4) | ((uint32_t)(kGroups >> 4) << 24);  // fp32 from fp16, M = 128
+            const uint64_t dA = tc_desc(smem_u32(sA), 128, 256), dW = tc_desc(smem_u32(sW), 128, 1024);
+            uint32_t leader;
+            asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(leader));
+            int slot0 = 0;  // ring slot of the tile's first chunk
+            uint32_t fphase = 0, aphase = 1;
+            bool ok = true, any = false;
+            for (uint64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, aphase ^= 1) {
+#pragma unroll 1
+                for (int half = 0; half < 2 && ok; ++half) {
+                    if (any && !warp_wait(accempty0 + 8 * half, aphase, abort_s)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    int slot = slot0;
+                    uint32_t fp = fphase;
+#pragma unroll 1
+                    for (int ks = 0; ks < kChunks; ++ks) {
+                        if (half == 0) {
+                            if (!warp_wait(full0 + 8 * slot, fp, abort_s)) {
+                                ok = false;
+                                break;
+                            }
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
+                        const uint64_t da = dA + (uint64_t)((uint32_t)(slot * T::kChunkBytes) >> 4);
+                        const uint64_t dw = dW + (uint64_t)((uint32_t)(half * T::kWHalfBytes + ks * 256) >> 4);
+                        const uint32_t dcol = tmem + (uint32_t)(half * T::kSetStride);
+                        if (leader) {
+#pragma unroll
+                            for (int i = 0; i < S; ++i) {
+                                const uint32_t acc = (ks > 0 || i > 0) ? 1u : 0u;
+                                asm volatile(
+                                    "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, "
+                                    "p;\n}" ::"r"(dcol + (uint32_t)(32 * i)),
+                                    "l"(da + (uint64_t)(i * (kSliceBytes >> 4))), "l"(dw),
+                                    "r"(idesc0 | ((uint32_t)(32 * (S - i) >> 3) << 17)), "r"(acc)
+                                    : "memory");
+                            }
+                            if (half == 1) tc_commit(empty0 + 8 * slot);
+                            if (ks == kChunks - 1) tc_commit(accfull0 + 8 * half);
+                        }
+                        __syncwarp();
+                        if (++slot == kRing) {
+                            slot = 0;
+                            fp ^= 1;
+                        }
+                    }
+                    if (half == 1) {
+                        slot0 = slot;
+                        fphase = fp;
+                    }
+                }
+                any = true;
+            }
+            // every product has ended before the columns are freed, after a timeout too
+            if (leader) tc_commit(drain);
+            for (long it = 0; it < kWaitLimit; ++it) {
+                uint32_t done;
+                asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                             : "=r"(done)
+                             : "r"(drain), "r"(0u)
+                             : "memory");
+                if (done) break;
+            }
+        }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0 && abort_flag) atomicExch(err_flag, 1);
+    if (warp == kMmaWarp)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+}
+
+// ---- the gate's digits -------------------------------------------------------------------------
+// Device layout of a block's weights: two halves (outputs 0-15 and 16-31) of 32 S rows (digit-major)
+// by 64 columns in core-matrix order, then 64 row exponents.
+
+// The digits of W[out][in] = w against the row exponent eg (biased) into the layout above.
+template <int S>
+__device__ __forceinline__ void put_digits(unsigned char* wt, int jo, int po, int ji, int pi, double w, int eg) {
+    const uint64_t X = fixed_f64_any(w, eg);
+    const int col = col_of(ji, pi), row = 2 * (jo & 15) + po;
+    unsigned char* half = wt + (jo >> 4) * (S * 32 * 64 * 2);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int u = (int)((X >> (56 - 8 * s)) & 0xFF) - 128, d = w < 0.0 ? -u : u;
+        *reinterpret_cast<__half*>(half + core_off(32 * s + row, col, 64)) = __int2half_rn(d);
+    }
+}
+
+// One matrix (row-major, in the order of the sorted targets), any finite entries: one CTA.
+template <int S>
+__global__ void __launch_bounds__(1024) k_weights_matrix(const double2* __restrict__ m, unsigned char* __restrict__ wt) {
+    __shared__ int eg_s[kAmps];
+    const int tid = threadIdx.x, r = tid >> 5, c = tid & 31;
+    const double2 v = m[tid];
+    // both real rows of output r hold the same magnitudes
+    uint32_t mx = max((uint32_t)__double2hiint(v.x) & 0x7FFFFFFFu, (uint32_t)__double2hiint(v.y) & 0x7FFFFFFFu);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (c == 0) {
+        const int eg = max((int)(mx >> 20), 1);
+        eg_s[r] = eg;
+        int32_t* er = reinterpret_cast<int32_t*>(wt + 2 * (S * 32 * 64 * 2));
+        for (int po = 0; po < 2; ++po) er[32 * (r >> 4) + 2 * (r & 15) + po] = eg - 1022;
+    }
+    __syncwarp();
+    const int eg = eg_s[r];
+    put_digits<S>(wt, r, 0, c, 0, v.x, eg);
+    put_digits<S>(wt, r, 0, c, 1, -v.y, eg);
+    put_digits<S>(wt, r, 1, c, 0, v.y, eg);
+    put_digits<S>(wt, r, 1, c, 1, v.x, eg);
+}
+
+int sm_count() {
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+template <int P, bool kRows>
+cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, int* err, cudaStream_t s, double* mirror) {
+    using T = Shape<P>;
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_gate_block<P, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmem);
+    if (attr != cudaSuccess) return attr;
+    TargetOffsets to;
+    for (int j = 0; j < kAmps; ++j) {
+        to.o[j] = 0;
+        for (int b = 0; b < 5; ++b)
+            if ((j >> b) & 1) to.o[j] |= 1ULL << bd.q[b];
+    }
+    const uint64_t ntiles = (1ULL << (n - 5)) / kGroups, sms = (uint64_t)sm_count();
+    k_gate_block<P, kRows><<<(unsigned)(ntiles < sms ? ntiles : sms), kThreads, T::kSmem, s>>>(
+        static_cast<typename Elem<P>::S*>(psi), n, to, bd.tmask, static_cast<const uint4*>(w), err,
+        reinterpret_cast<double2*>(mirror));
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+bool gate_block_eligible(int P, int n) { return (P == LLG_F64 || P == LLG_DF64) && n >= 12; }
+
+size_t gate_block_weight_bytes(int P) {
+    return (P == LLG_F64 ? 2 * Shape<LLG_F64>::kWHalfBytes : 2 * Shape<LLG_DF64>::kWHalfBytes) + 64 * sizeof(int32_t);
+}
+
+cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weights, cudaStream_t s) {
+    unsigned char* w = static_cast<unsigned char*>(d_weights);
+    const double2* m = reinterpret_cast<const double2*>(d_matrix);
+    if (P == LLG_F64) k_weights_matrix<Shape<LLG_F64>::S><<<1, 1024, 0, s>>>(m, w);
+    else k_weights_matrix<Shape<LLG_DF64>::S><<<1, 1024, 0, s>>>(m, w);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, int* err_flag,
+                              cudaStream_t s, double* mirror) {
+    if (P == LLG_F64)
+        return rows ? launch<LLG_F64, true>(psi, n, bd, d_weights, err_flag, s, mirror)
+                    : launch<LLG_F64, false>(psi, n, bd, d_weights, err_flag, s, mirror);
+    return rows ? launch<LLG_DF64, true>(psi, n, bd, d_weights, err_flag, s, mirror)
+                : launch<LLG_DF64, false>(psi, n, bd, d_weights, err_flag, s, mirror);
+}
+
+}  // namespace llg

@@ -84,7 +84,7 @@ struct BlockSparsity {
 cudaError_t launch_block_sparse(int P, void* psi, int n, const BlockDesc& bd, const uint64_t* d_mat,
                                 const BlockSparsity& nz, cudaStream_t s);
 
-// 4- and 5-qubit blocks on double-float states of at least k + 7 qubits on the tensor cores
+// 4-qubit blocks on double-float and 3- and 4-qubit blocks on FP64 states of k + 7 or more qubits on the tensor cores
 // (llg_block_tc.cu): the host slices the matrix (2 * 4^k doubles, row-major re/im) into
 // block_tc_weight_bytes(k) of device input; a kernel whose products do not arrive within its
 // wait limit sets *err_flag (a device int of the caller's) to 1
@@ -93,6 +93,17 @@ size_t block_tc_weight_bytes(int P, int k);
 void block_tc_prepare(int P, int k, const double* m, void* weights);
 cudaError_t launch_block_tc(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, int* err_flag,
                             cudaStream_t s);
+
+// dense 5-qubit blocks of 16-byte states on the tensor cores (llg_gateblock.cu): n >= 12, bd.q in
+// increasing order.  d_weights: gate_block_weight_bytes of device memory, filled by
+// launch_gate_block_matrix (d_matrix: 32 x 32 row-major (re, im) doubles on the device, bit b of an
+// index is bd.q[b]).  rows: the weights have row exponents of their own (launch_gate_block_matrix).  mirror: nullptr, or the device address of a mapped host buffer that also
+// receives the output as FP64.  A kernel whose waits run out sets *err_flag to 1.
+bool gate_block_eligible(int P, int n);
+size_t gate_block_weight_bytes(int P);
+cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weights, cudaStream_t s);
+cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, int* err_flag,
+                              cudaStream_t s, double* mirror = nullptr);
 
 // process-wide tuning cache (llg_tune.cu), keyed by an FNV-1a hash of the workload's shape
 uint64_t tune_hash(uint64_t h, uint64_t v);
