@@ -528,6 +528,24 @@ int llg_diag_export(int n, int nterms, const int* a, const int* b, const double*
 int llg_plan_export_tables(int n, const llg_op* ops, int nops, int tile_qubits, int flags, double* tables,
                            int64_t max_doubles, int64_t* ndoubles);
 
+/* The plan of dense 5-qubit blocks that a flush of a complex128 or double-float state of 12 and more
+ * qubits may take: steps in order, each either a block (gates on bits 0..4 of its index, bit b is
+ * qubit q[b], q increasing) or one CNOT / sign flip on global qubits.  Writes at most max_steps /
+ * max_gates records and the true counts.  LLG_EINVAL when the list has no block plan. */
+typedef struct {
+    int32_t is_block;
+    int32_t q[5];
+    int32_t gate_begin, ngates;
+} llg_block_step;
+typedef struct {
+    int32_t kind; /* 0: 2x2 matrix m on q0; 1: CNOT, control q0, target q1; 2: sign flip where all of mask is set */
+    int32_t q0, q1, pad;
+    uint64_t mask;
+    double m[8];
+} llg_block_gate;
+int llg_block_plan_export(int n, const llg_op* ops, int nops, llg_block_step* steps, int max_steps, int* nsteps,
+                          llg_block_gate* gates, int max_gates, int* ngates);
+
 #ifdef __cplusplus
 }
 #endif

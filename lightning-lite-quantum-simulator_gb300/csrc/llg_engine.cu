@@ -76,6 +76,15 @@ struct llg_state {
     void* d_block_tc = nullptr;
     unsigned char* h_block_tc = nullptr;
     bool block_tc_launched = false;
+    // block plans: gates and steps (device, pinned staging) and the blocks' weights
+    unsigned char* d_bplan = nullptr;
+    unsigned char* h_bplan = nullptr;
+    size_t d_bplan_cap = 0;  // of both
+    void* d_bweights = nullptr;
+    size_t d_bweights_cap = 0;
+    // log2 of a bound on the state's 2-norm (infinite: not known to be finite); block plans hold
+    // their amplitudes as integers against each group's largest, so they run on finite states only
+    double log2_norm = 0.0;
     bool tiles_launched = false;  // a tile pass ran since the last sync (its load-timeout flag to check)
     // this state's timeout flags on the device: [0] a bulk tile load, [1] tensor-core products
     int* d_flags = nullptr;
@@ -313,6 +322,171 @@ int run_tiles(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
     return LLG_OK;
 }
 
+// A flush as dense 5-qubit blocks on the tensor cores (llg_blockplan.cpp, llg_gateblock.cu), the rest
+// of the plan made while the first blocks run.  nops: the flush's gates (bounds the plan's size).
+// mirror / mirrored: as for run_tiles.
+int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
+    constexpr int kGroup = 16;   // blocks planned, uploaded and launched at a time
+    constexpr int kSlots = 128;  // blocks whose weights are held at once
+    static_assert(kSlots % kGroup == 0, "a group's weights are contiguous");
+    const size_t wb = gate_block_weight_bytes(st->P);
+    const size_t slots = nops <= kSlots ? (std::max<size_t>(nops, 1) + kGroup - 1) / kGroup * kGroup : kSlots;
+    // a group's upload: its blocks' steps and its gates; every group has its own part of the buffers
+    const size_t bytes = (nops / kGroup + 2) * (kGroup * sizeof(BlockStep) + 512) + nops * sizeof(BlockGate);
+    if (bytes > st->d_bplan_cap || slots * wb > st->d_bweights_cap)
+        LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
+    if (bytes > st->d_bplan_cap) {
+        if (st->d_bplan) cudaFree(st->d_bplan);
+        if (st->h_bplan) cudaFreeHost(st->h_bplan);
+        st->d_bplan = st->h_bplan = nullptr;
+        st->d_bplan_cap = 0;
+        LLG_CUDA(cudaMalloc(&st->d_bplan, bytes), "cudaMalloc(block plan)");
+        LLG_CUDA(cudaHostAlloc((void**)&st->h_bplan, bytes, cudaHostAllocDefault), "cudaHostAlloc(block plan)");
+        st->d_bplan_cap = bytes;
+    }
+    if (slots * wb > st->d_bweights_cap) {
+        if (st->d_bweights) cudaFree(st->d_bweights);
+        st->d_bweights = nullptr;
+        st->d_bweights_cap = 0;
+        LLG_CUDA(cudaMalloc(&st->d_bweights, slots * wb), "cudaMalloc(block weights)");
+        st->d_bweights_cap = slots * wb;
+    }
+    LLG_CUDA(cudaEventSynchronize(st->ops_done), "cudaEventSynchronize");  // the staging buffer's last copies
+    st->block_tc_launched = true;
+    const BlockPlan& plan = planner.plan;
+    size_t from = 0, gates_from = 0, off = 0;
+    int slot = 0;
+    std::vector<BlockStep> bs;
+    bool rest = planner.advance(0);  // gates that are not planned yet
+    while (from < plan.steps.size() || rest) {
+        if (from == plan.steps.size()) rest = planner.advance(kGroup);
+        // the steps planned so far, at most kGroup blocks of them
+        size_t to = from, gates_to = gates_from;
+        bs.clear();
+        for (; to < plan.steps.size() && (int)bs.size() < kGroup; ++to) {
+            BlockStep p = plan.steps[to];
+            gates_to = (size_t)p.gate_begin + p.ngates;
+            p.gate_begin -= (int)gates_from;
+            if (p.is_block) bs.push_back(p);
+        }
+        const bool last_group = !rest && to == plan.steps.size();
+        int done = 0;
+        const unsigned char* w = static_cast<const unsigned char*>(st->d_bweights) + wb * slot;
+        if (!bs.empty()) {
+            const size_t sbytes = (bs.size() * sizeof(BlockStep) + 255) / 256 * 256;
+            const size_t gbytes = (gates_to - gates_from) * sizeof(BlockGate);
+            std::memcpy(st->h_bplan + off, bs.data(), bs.size() * sizeof(BlockStep));
+            std::memcpy(st->h_bplan + off + sbytes, plan.gates.data() + gates_from, gbytes);
+            LLG_CUDA(cudaMemcpyAsync(st->d_bplan + off, st->h_bplan + off, sbytes + gbytes, cudaMemcpyHostToDevice, st->stream),
+                     "cudaMemcpyAsync(block plan)");
+            const int rc = traced(st, LLG_PROF_TILE, 1, "block weights", [&] {
+                return launch_gate_block_weights(st->P, reinterpret_cast<const BlockGate*>(st->d_bplan + off + sbytes),
+                                                 reinterpret_cast<const BlockStep*>(st->d_bplan + off), (int)bs.size(),
+                                                 static_cast<unsigned char*>(st->d_bweights) + wb * slot, st->stream);
+            });
+            if (rc) return rc;
+            off += (sbytes + gbytes + 255) / 256 * 256;
+            slot = (slot + kGroup) % (int)slots;
+        }
+        for (size_t i = from; i < to; ++i) {
+            const BlockStep& p = plan.steps[i];
+            int rc;
+            if (!p.is_block) {
+                const BlockGate& g = plan.gates[p.gate_begin];
+                ExecOp e;
+                std::memset(&e, 0, sizeof(e));
+                e.kind = g.kind == 1 ? EX_CNOT : EX_MCZ;
+                e.q0 = g.q0;
+                e.q1 = g.q1;
+                e.mask = g.mask;
+                rc = traced(st, LLG_PROF_GATE, 1, "gate kernel",
+                            [&] { return launch_exec_op(st->P, st->d_psi, st->n, e, st->stream); });
+                if (rc) return rc;
+                continue;
+            }
+            BlockDesc bd;
+            std::memset(&bd, 0, sizeof(bd));
+            bd.k = 5;
+            for (int b = 0; b < 5; ++b) {
+                bd.q[b] = p.q[b];
+                bd.tmask |= 1ULL << p.q[b];
+            }
+            const bool last = mirror && last_group && i + 1 == to;
+            rc = traced(st, LLG_PROF_TILE, 1, "gate block", [&] {
+                return launch_gate_block(st->P, st->d_psi, st->n, bd, w + wb * done, false, st->d_flags + 1, st->stream,
+                                         last ? mirror : nullptr);
+            });
+            if (rc) return rc;
+            if (last && mirrored) *mirrored = true;
+            ++done;
+        }
+        from = to;
+        gates_from = gates_to;
+    }
+    LLG_CUDA(cudaEventRecord(st->ops_done, st->stream), "cudaEventRecord");
+    return LLG_OK;
+}
+
+// log2 of the state's norm into st->log2_norm (waits for the stream)
+int measure_norm(llg_state* st) {
+    ZTerms z;
+    std::memset(&z, 0, sizeof(z));
+    int rc = traced(st, LLG_PROF_READOUT, 2, "reduce",
+                    [&] { return launch_reduce_z(st->P, st->d_psi, st->n, z, st->d_partials, st->d_red, st->stream); });
+    if (rc) return rc;
+    double v = 0.0;
+    LLG_CUDA(cudaMemcpyAsync(&v, st->d_red, sizeof(v), cudaMemcpyDeviceToHost, st->stream), "cudaMemcpyAsync(norm)");
+    LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
+    st->log2_norm = !std::isfinite(v) ? HUGE_VAL : (v > 0.0 ? 0.5 * std::log2(v) : 0.0);
+    return LLG_OK;
+}
+
+// Which plan a flush of 16-byte states takes when the caller has left the tile width and CTA size
+// to the engine: blocks when their passes cost less than tile passes with the same gates (judged on
+// the blocks planned so far).  Measured on this GPU: a block 9.2 ms (FP64) / 12.5 ms (double-float)
+// per 2^30 amplitudes and at least 12 us; a CNOT or sign-flip pass 2.6 ms per 2^30.  Tile passes
+// take 3.2 FP64 multiply-adds per amplitude for a merged one-qubit gate that mixes and 4 for a
+// diagonal one, at 0.56 T a second (double-float: 2.0 ms per 2^30 for either); no less than 2.6 us
+// a gate, however small the register (a CTA's latency); and one read and write of the state.
+bool blocks_pay(int P, int n, const BlockPlan& plan) {
+    const double amps = std::ldexp(1.0, n);
+    const double block = std::max(12e-6, amps * (P == LLG_F64 ? 8.6e-12 : 11.6e-12));
+    const double single = 3e-6 + amps * 2.4e-12;
+    const double t_blocks = plan.blocks * block + ((double)plan.steps.size() - plan.blocks) * single + 10e-6;
+    const double arith = P == LLG_F64 ? (3.2 * plan.mixing_1q + 4.0 * plan.diag_1q) / 0.56e12
+                                      : 1.9e-12 * (plan.mixing_1q + plan.diag_1q);
+    const double t_tiles = std::max(std::max(arith * amps, 2.6e-6 * (double)plan.gates.size()), amps * 4.8e-12);
+    return t_blocks < t_tiles;
+}
+
+// growth of the norm bound over a queue (2x2s that are not unitary)
+void note_growth(llg_state* st, const std::vector<llg_op>& q) {
+    for (const llg_op& op : q)
+        if (op.kind == LLG_OP_U2) {
+            const double s = spectral_norm_2x2(op.m);
+            if (!(s <= kBlockNormLimit)) st->log2_norm += std::log2(s);
+        }
+    if (std::isnan(st->log2_norm)) st->log2_norm = HUGE_VAL;
+}
+
+// the queue as fused passes (blocks, shared-memory tiles or register tiles)
+int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = nullptr, bool* mirrored = nullptr) {
+    if (!gate_block_eligible(st->P, st->n)) return run_tiles(st, q, mirror, mirrored);
+    // amplitudes stay below 2^(limit + 10) within a flush
+    const double limit = st->P == LLG_F64 ? 900.0 : 90.0;
+    if (st->log2_norm > limit && st->log2_norm < HUGE_VAL)
+        if (int rc = measure_norm(st)) return rc;
+    if (st->fuse_mode == LLG_FUSE_TILE && st->tile_qubits == 0 && st->tile_threads == 0 && st->log2_norm <= limit) {
+        if (has_block_plan(st->n, q.data(), (int)q.size())) {
+            BlockPlanner planner(st->n, q.data(), (int)q.size());
+            planner.advance(8);
+            if (blocks_pay(st->P, st->n, planner.plan)) return run_blocks(st, planner, q.size(), mirror, mirrored);
+        }
+    }
+    note_growth(st, q);
+    return run_tiles(st, q, mirror, mirrored);
+}
+
 int enqueue(llg_state* st, const llg_op& op) {
     st->queue.push_back(op);
     if (st->queue.size() >= kQueueFlushAt) return llg_flush(st);
@@ -463,6 +637,9 @@ int llg_destroy(llg_state* st) {
     if (st->d_block_tc) cudaFree(st->d_block_tc);
     if (st->h_block_tc) cudaFreeHost(st->h_block_tc);
     if (st->block_done) cudaEventDestroy(st->block_done);
+    if (st->d_bplan) cudaFree(st->d_bplan);
+    if (st->h_bplan) cudaFreeHost(st->h_bplan);
+    if (st->d_bweights) cudaFree(st->d_bweights);
     for (auto& r : st->prof_recs) {
         cudaEventDestroy(r.a);
         cudaEventDestroy(r.b);
@@ -480,6 +657,7 @@ int llg_reset(llg_state* st, int n_qubits) {
     st->queue.clear();
     int rc = alloc_state(st, n_qubits);
     if (rc) return rc;
+    st->log2_norm = 0.0;
     return traced(st, LLG_PROF_INIT, 1, "init", [&] { return launch_init_basis(st->P, st->d_psi, st->size, 0, st->stream); });
 }
 
@@ -642,6 +820,22 @@ int llg_apply_matrix(llg_state* st, int k, const int* qubits, const double* m) {
         if (!std::isfinite(m[i])) return set_error(LLG_EINVAL, "apply_matrix: non-finite matrix entry");
     int rc = llg_flush(st);  // earlier gates first
     if (rc) return rc;
+    {
+        // the 2-norm is at most the geometric mean of the largest column and row sums
+        double rows = 0.0, cols[kMaxBlockDim] = {0.0}, col = 0.0;
+        for (int r = 0; r < 1 << k; ++r) {
+            double sum = 0.0;
+            for (int c = 0; c < 1 << k; ++c) {
+                const double v = std::hypot(m[2 * ((r << k) + c)], m[2 * ((r << k) + c) + 1]);
+                sum += v;
+                cols[c] += v;
+            }
+            rows = std::max(rows, sum);
+        }
+        for (int c = 0; c < 1 << k; ++c) col = std::max(col, cols[c]);
+        st->log2_norm += std::max(0.0, 0.5 * (std::log2(rows) + std::log2(col)));
+        if (std::isnan(st->log2_norm)) st->log2_norm = HUGE_VAL;
+    }
     const size_t cap = (size_t)2 * kMaxBlockDim * kMaxBlockDim;
     if (!st->d_block) {
         LLG_CUDA(cudaMalloc(&st->d_block, cap * sizeof(uint64_t)), "cudaMalloc(block)");
@@ -826,7 +1020,9 @@ int llg_flush(llg_state* st) {
     std::vector<llg_op> q;
     q.swap(st->queue);
     if (st->n == 0) return LLG_OK;
-    return st->fuse_mode != LLG_FUSE_NONE ? run_tiles(st, q) : run_streaming(st, q);
+    if (st->fuse_mode != LLG_FUSE_NONE) return run_fused(st, q);
+    note_growth(st, q);
+    return run_streaming(st, q);
 }
 
 // After the state's stream has drained: the timeout flags of the kernels that wait on the
@@ -872,7 +1068,7 @@ int llg_copy_to_host(llg_state* st, double* out) {
         std::vector<llg_op> q;
         q.swap(st->queue);
         bool mirrored = false;
-        if ((rc = run_tiles(st, q, static_cast<double*>(dev_out), &mirrored))) return rc;
+        if ((rc = run_fused(st, q, static_cast<double*>(dev_out), &mirrored))) return rc;
         if (mirrored) {
             LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
             return device_checks(st);
@@ -918,6 +1114,7 @@ int llg_copy_from_host(llg_state* st, const double* amps) {
     st->queue.clear();  // overwritten anyway
     if (st->P == LLG_F64) {
         LLG_CUDA(cudaMemcpyAsync(st->d_psi, amps, st->size * 16, cudaMemcpyHostToDevice, st->stream), "cudaMemcpyAsync(H2D)");
+        if (gate_block_eligible(st->P, st->n)) return measure_norm(st);
         LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
         return LLG_OK;
     }
@@ -936,6 +1133,7 @@ int llg_copy_from_host(llg_state* st, const double* amps) {
         if (rc) return rc;
         LLG_CUDA(cudaEventRecord(st->stage_ev[which], st->stream), "cudaEventRecord");
     }
+    if (gate_block_eligible(st->P, st->n)) return measure_norm(st);
     LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
     return LLG_OK;
 }
@@ -1173,6 +1371,7 @@ int llg_renormalize(llg_state* st) {
     int rc = llg_norm2(st, &nrm);
     if (rc) return rc;
     if (!(nrm > 0.0) || !std::isfinite(nrm)) return set_error(LLG_ERUNTIME, "renormalize: state norm vanished");
+    st->log2_norm = 0.0;
     return traced(st, LLG_PROF_READOUT, 1, "scale",
                   [&] { return launch_scale(st->P, st->d_psi, st->size, 1.0 / std::sqrt(nrm), st->stream); });
 }
@@ -1305,6 +1504,27 @@ int llg_diag_export(int n, int nterms, const int* a, const int* b, const double*
     std::string err;
     if (!build_diag_obs(n, nterms, a, b, coeff, h, err)) return set_error(LLG_EINVAL, "diag_export: " + err);
     diag_obs_eval_host(h, out);
+    return LLG_OK;
+}
+
+int llg_block_plan_export(int n, const llg_op* ops, int nops, llg_block_step* steps, int max_steps, int* nsteps,
+                          llg_block_gate* gates, int max_gates, int* ngates) {
+    if (n < 1 || n > kMaxQubits || nops < 0 || (nops > 0 && !ops) || !nsteps || !ngates)
+        return set_error(LLG_EINVAL, "block_plan_export: bad argument");
+    llg_state tmp;
+    tmp.n = n;
+    for (int i = 0; i < nops; ++i)
+        if (int rc = validate_op(&tmp, ops[i], "block_plan_export")) return rc;
+    if (!has_block_plan(n, ops, nops))
+        return set_error(LLG_EINVAL, "block_plan_export: no block plan (fewer than 12 qubits, or a 2x2 gate of norm above 1)");
+    BlockPlanner planner(n, ops, nops);
+    while (planner.advance(1 << 20)) {}
+    const BlockPlan& plan = planner.plan;
+    static_assert(sizeof(llg_block_step) == sizeof(BlockStep) && sizeof(llg_block_gate) == sizeof(BlockGate), "exported layouts");
+    *nsteps = (int)plan.steps.size();
+    *ngates = (int)plan.gates.size();
+    if (steps) std::memcpy(steps, plan.steps.data(), std::min<size_t>(std::max(max_steps, 0), plan.steps.size()) * sizeof(BlockStep));
+    if (gates) std::memcpy(gates, plan.gates.data(), std::min<size_t>(std::max(max_gates, 0), plan.gates.size()) * sizeof(BlockGate));
     return LLG_OK;
 }
 

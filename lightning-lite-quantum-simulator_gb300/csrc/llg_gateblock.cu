@@ -147,8 +147,9 @@ __device__ __forceinline__ __half2 h2_of(uint32_t b) {
     return v;
 }
 
-// Four digits (bytes 3 .. 0 of the biased words) of eight reals as fp16, one 16-byte core row each;
-// sgn: +-1 of each pair of reals, bias: -1152 sgn
+// The first kCount of four digits (bytes 3 .. 0 of the biased words) of eight reals as fp16, one
+// 16-byte core row each; sgn: +-1 of each pair of reals, bias: -1152 sgn
+template <int kCount>
 __device__ __forceinline__ void digits4(const uint32_t (&w)[8], const __half2 (&sgn)[4], const __half2 (&bias)[4],
                                         unsigned char* dst) {
     uint32_t v[4][4];
@@ -162,7 +163,7 @@ __device__ __forceinline__ void digits4(const uint32_t (&w)[8], const __half2 (&
         v[3][p] = h2_bits(__hfma2(h2_of(__byte_perm(u, 0x64646464u, 0x4342)), sgn[p], bias[p]));
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < kCount; ++k)
         *reinterpret_cast<uint4*>(dst + k * kSliceBytes) = make_uint4(v[k][0], v[k][1], v[k][2], v[k][3]);
 }
 
@@ -340,8 +341,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                         sgn[i] = h2_of((sg & 0x80008000u) | 0x3C003C00u);
                         bias[i] = __hmul2(sgn[i], __half2half2(__ushort_as_half(0xE480)));  // -1152
                     }
-                    digits4(wh, sgn, bias, dst);
-                    digits4(wl, sgn, bias, dst + 4 * kSliceBytes);
+                    digits4<4>(wh, sgn, bias, dst);
+                    digits4<4>(wl, sgn, bias, dst + 4 * kSliceBytes);
                 } else {
                     // nearest-integer digits by the magic addition, from the high part and (from the
                     // fourth digit on) the low part added to what is left of it
@@ -606,40 +607,80 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Device layout of a block's weights: two halves (outputs 0-15 and 16-31) of 32 S rows (digit-major)
 // by 64 columns in core-matrix order, then 64 row exponents.
 
-// The digits of W[out][in] = w against the row exponent eg (biased) into the layout above.
-template <int S>
-__device__ __forceinline__ void put_digits(unsigned char* wt, int jo, int po, int ji, int pi, double w, int eg) {
-    const uint64_t X = fixed_f64_any(w, eg);
-    const int col = col_of(ji, pi), row = 2 * (jo & 15) + po;
-    unsigned char* half = wt + (jo >> 4) * (S * 32 * 64 * 2);
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-        const int u = (int)((X >> (56 - 8 * s)) & 0xFF) - 128, d = w < 0.0 ? -u : u;
-        *reinterpret_cast<__half*>(half + core_off(32 * s + row, col, 64)) = __int2half_rn(d);
-    }
-}
-
-// One matrix (row-major, in the order of the sorted targets), any finite entries: one CTA.
-template <int S>
-__global__ void __launch_bounds__(1024) k_weights_matrix(const double2* __restrict__ m, unsigned char* __restrict__ wt) {
+// A CTA cuts the eight input amplitudes (16 columns) of one K chunk, blockIdx.y, of one block,
+// blockIdx.x.  kMatrix: the matrix m (row-major, in the order of the sorted targets), any finite
+// entries; else the product of the block's gates, run on the identity's columns in shared memory.
+template <int S, bool kMatrix>
+__global__ void __launch_bounds__(128)
+    k_weights(const double2* __restrict__ m, const BlockGate* __restrict__ gates, const BlockStep* __restrict__ steps,
+              unsigned char* __restrict__ wt, size_t stride) {
+    __shared__ double2 M[kAmps][9];
     __shared__ int eg_s[kAmps];
-    const int tid = threadIdx.x, r = tid >> 5, c = tid & 31;
-    const double2 v = m[tid];
-    // both real rows of output r hold the same magnitudes
-    uint32_t mx = max((uint32_t)__double2hiint(v.x) & 0x7FFFFFFFu, (uint32_t)__double2hiint(v.y) & 0x7FFFFFFFu);
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if (c == 0) {
-        const int eg = max((int)(mx >> 20), 1);
-        eg_s[r] = eg;
-        int32_t* er = reinterpret_cast<int32_t*>(wt + 2 * (S * 32 * 64 * 2));
-        for (int po = 0; po < 2; ++po) er[32 * (r >> 4) + 2 * (r & 15) + po] = eg - 1022;
+    const int tid = threadIdx.x, ks = blockIdx.y, c = tid & 7, p = tid >> 3;
+    wt += blockIdx.x * stride;
+    if constexpr (kMatrix) {
+        for (int r = p; r < kAmps; r += 16) M[r][c] = m[r * kAmps + 8 * ks + c];
+        if (tid < kAmps) {
+            // both real rows of an output hold the same magnitudes
+            uint32_t mx = 0;
+            for (int j = 0; j < kAmps; ++j) {
+                const double2 v = m[tid * kAmps + j];
+                mx = max(mx, max((uint32_t)__double2hiint(v.x) & 0x7FFFFFFFu, (uint32_t)__double2hiint(v.y) & 0x7FFFFFFFu));
+            }
+            eg_s[tid] = max((int)(mx >> 20), 1);
+        }
+    } else {
+        for (int r = p; r < kAmps; r += 16) M[r][c] = make_double2(r == 8 * ks + c ? 1.0 : 0.0, 0.0);
+        if (tid < kAmps) eg_s[tid] = 1023;  // entries below 2
+        __syncthreads();
+        const BlockStep st = steps[blockIdx.x];
+        for (int g = 0; g < st.ngates; ++g) {
+            const BlockGate& o = gates[st.gate_begin + g];
+            if (o.kind == 0) {
+                const int b = o.q0, r0 = ((p >> b) << (b + 1)) | (p & ((1 << b) - 1)), r1 = r0 | 1 << b;
+                const double2 x = M[r0][c], y = M[r1][c];
+                M[r0][c] = make_double2(fma(o.m[0], x.x, fma(-o.m[1], x.y, fma(o.m[2], y.x, -o.m[3] * y.y))),
+                                        fma(o.m[0], x.y, fma(o.m[1], x.x, fma(o.m[2], y.y, o.m[3] * y.x))));
+                M[r1][c] = make_double2(fma(o.m[4], x.x, fma(-o.m[5], x.y, fma(o.m[6], y.x, -o.m[7] * y.y))),
+                                        fma(o.m[4], x.y, fma(o.m[5], x.x, fma(o.m[6], y.y, o.m[7] * y.x))));
+            } else if (o.kind == 1) {
+                if (p < 8) {
+                    const int r = (int)insert0_mask((uint64_t)p, 1ULL << o.q0 | 1ULL << o.q1) | 1 << o.q0, r1 = r | 1 << o.q1;
+                    const double2 x = M[r][c];
+                    M[r][c] = M[r1][c];
+                    M[r1][c] = x;
+                }
+            } else {
+                for (int r = p; r < kAmps; r += 16)
+                    if ((r & (int)o.mask) == (int)o.mask) M[r][c] = make_double2(-M[r][c].x, -M[r][c].y);
+            }
+            __syncthreads();
+        }
     }
-    __syncwarp();
-    const int eg = eg_s[r];
-    put_digits<S>(wt, r, 0, c, 0, v.x, eg);
-    put_digits<S>(wt, r, 0, c, 1, -v.y, eg);
-    put_digits<S>(wt, r, 1, c, 0, v.y, eg);
-    put_digits<S>(wt, r, 1, c, 1, v.x, eg);
+    __syncthreads();
+    // this thread: real output row `row` (2 jo + po), one core row of inputs j = 8 ks + 2 i + h
+    const int row = tid >> 1, h = tid & 1, jo = row >> 1, po = row & 1, eg = eg_s[jo];
+    uint32_t wh[8], wl[8];
+    __half2 sgn[4], bias[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double2 v = M[jo][2 * i + h];
+        const double w[2] = {po ? v.y : v.x, po ? v.x : -v.y};  // real part in, imaginary part in
+#pragma unroll
+        for (int pi = 0; pi < 2; ++pi) {
+            const uint64_t X = fixed_f64_any(w[pi], eg);
+            wh[2 * i + pi] = (uint32_t)(X >> 32);
+            wl[2 * i + pi] = (uint32_t)X;
+        }
+        const uint32_t sg = __byte_perm((uint32_t)__double2hiint(w[0]), (uint32_t)__double2hiint(w[1]), 0x7733);
+        sgn[i] = h2_of((sg & 0x80008000u) | 0x3C003C00u);
+        bias[i] = __hmul2(sgn[i], __half2half2(__ushort_as_half(0xE480)));
+    }
+    unsigned char* dst = wt + (row >> 5) * (S * 32 * 64 * 2) + core_off(row & 31, 16 * ks + 8 * h, 64);
+    static_assert(kSliceBytes == 32 * 64 * 2, "a digit's 32 rows are kSliceBytes apart");
+    digits4<4>(wh, sgn, bias, dst);
+    digits4<S - 4>(wl, sgn, bias, dst + 4 * kSliceBytes);
+    if (ks == 0 && h == 0) reinterpret_cast<int32_t*>(wt + 2 * (S * 32 * 64 * 2))[row] = eg - 1022;
 }
 
 int sm_count() {
@@ -679,8 +720,18 @@ size_t gate_block_weight_bytes(int P) {
 cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weights, cudaStream_t s) {
     unsigned char* w = static_cast<unsigned char*>(d_weights);
     const double2* m = reinterpret_cast<const double2*>(d_matrix);
-    if (P == LLG_F64) k_weights_matrix<Shape<LLG_F64>::S><<<1, 1024, 0, s>>>(m, w);
-    else k_weights_matrix<Shape<LLG_DF64>::S><<<1, 1024, 0, s>>>(m, w);
+    if (P == LLG_F64) k_weights<Shape<LLG_F64>::S, true><<<dim3(1, kChunks), 128, 0, s>>>(m, nullptr, nullptr, w, 0);
+    else k_weights<Shape<LLG_DF64>::S, true><<<dim3(1, kChunks), 128, 0, s>>>(m, nullptr, nullptr, w, 0);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const BlockStep* d_steps, int nblocks, void* d_weights,
+                                      cudaStream_t s) {
+    unsigned char* w = static_cast<unsigned char*>(d_weights);
+    const size_t stride = gate_block_weight_bytes(P);
+    const dim3 grid((unsigned)nblocks, kChunks);
+    if (P == LLG_F64) k_weights<Shape<LLG_F64>::S, false><<<grid, 128, 0, s>>>(nullptr, d_gates, d_steps, w, stride);
+    else k_weights<Shape<LLG_DF64>::S, false><<<grid, 128, 0, s>>>(nullptr, d_gates, d_steps, w, stride);
     return cudaGetLastError();
 }
 

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -186,6 +187,45 @@ enum RegCode : int32_t {
     RC_LAYOUT = 75,
 };
 int32_t reg_dispatch_code(const ExecOp& x);
+
+// A plan of dense 5-qubit blocks (llg_blockplan.cpp) for 16-byte states of 12 and more qubits.
+struct BlockGate {
+    int32_t kind;  // 0: 2x2 matrix m on q0; 1: CNOT, control q0, target q1; 2: sign flip where all of `mask` is set
+    int32_t q0, q1, pad;
+    uint64_t mask;
+    double m[8];
+};
+static_assert(sizeof(BlockGate) == 88, "BlockGate layout");
+struct BlockStep {
+    int32_t is_block;    // 1: gates on bits 0..4 of the block's index, bit b is qubit q[b] (increasing);
+                         // 0: one CNOT or sign flip on global qubits, run as a streaming pass
+    int32_t q[5];
+    int32_t gate_begin, ngates;
+};
+struct BlockPlan {
+    std::vector<BlockStep> steps;
+    std::vector<BlockGate> gates;
+    int blocks = 0;
+    int mixing_1q = 0, diag_1q = 0;  // merged one-qubit gates among `gates`, for the cost of other plans
+};
+// 2x2 gates of a block have spectral norm at most this, so that its entries stay below 2
+constexpr double kBlockNormLimit = 1.0 + 1e-6;
+double spectral_norm_2x2(const double* m);
+// false: no block plan (fewer than 12 qubits, or a 2x2 beyond the norm limit)
+bool has_block_plan(int n, const llg_op* ops, int nops);
+// Plans block by block, so that the first ones can run while the rest is planned.  `ops` is read by
+// the constructor only.
+class BlockPlanner {
+public:
+    BlockPlanner(int n, const llg_op* ops, int nops);
+    ~BlockPlanner();
+    bool advance(int blocks);  // appends up to `blocks` blocks to `plan`; false: the list is done
+    BlockPlan plan;
+
+private:
+    class Impl;
+    std::unique_ptr<Impl> impl_;
+};
 
 // Lower one gate record to executor ops with GLOBAL qubit indices (streaming path).
 bool lower_op(int n, const llg_op& op, int precision, std::vector<ExecOp>& out, std::string& err);

@@ -102,6 +102,9 @@ cudaError_t launch_block_tc(int P, void* psi, int n, const BlockDesc& bd, const 
 bool gate_block_eligible(int P, int n);
 size_t gate_block_weight_bytes(int P);
 cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weights, cudaStream_t s);
+// the weights of `nblocks` blocks of a plan (d_steps: their steps, in order), one after the other
+cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const BlockStep* d_steps, int nblocks, void* d_weights,
+                                      cudaStream_t s);
 cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, int* err_flag,
                               cudaStream_t s, double* mirror = nullptr);
 

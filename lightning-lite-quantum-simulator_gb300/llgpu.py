@@ -46,6 +46,11 @@ XOP_DTYPE = np.dtype([("kind", np.int32), ("q0", np.int32), ("q1", np.int32), ("
                       ("mask", np.uint64), ("nl_mask", np.uint64), ("c", np.float64, (8,))])
 
 
+BLOCK_STEP_DTYPE = np.dtype([("is_block", np.int32), ("q", np.int32, (5,)), ("gate_begin", np.int32), ("ngates", np.int32)])
+BLOCK_GATE_DTYPE = np.dtype([("kind", np.int32), ("q0", np.int32), ("q1", np.int32), ("pad", np.int32),
+                             ("mask", np.uint64), ("m", np.float64, (8,))])
+
+
 class LLGError(RuntimeError):
     pass
 
@@ -117,6 +122,7 @@ def lib() -> ctypes.CDLL:
             "llg_plan_export": (i, [i, vp, i, i, vp, i, P(i), vp, i, P(i)]),
             "llg_plan_export_ex": (i, [i, vp, i, i, i, vp, i, P(i), vp, i, P(i)]),
             "llg_plan_export_tables": (i, [i, vp, i, i, i, vp, ctypes.c_int64, P(ctypes.c_int64)]),
+            "llg_block_plan_export": (i, [i, vp, i, vp, i, P(i), vp, i, P(i)]),
             "llg_profile": (i, [vp, i]),
             "llg_profile_read": (i, [vp, vp, vp, i]),
             "llg_kernel_launches": (ctypes.c_int64, []),
@@ -450,6 +456,19 @@ def plan_export(n: int, ops: np.ndarray, tile_qubits: int, zyz: bool = False, ta
     check(lib().llg_plan_export_tables(n, _ptr(ops) if ops.size else None, ops.size, tile_qubits, flags, _ptr(tab),
                                        tab.size, ctypes.byref(nd)))
     return passes, xops[: nx.value], tab[: nd.value].view(np.complex128)
+
+
+def block_plan_export(n: int, ops: np.ndarray):
+    """The plan of dense 5-qubit blocks for `ops` on n >= 12 qubits: (steps, gates)."""
+    ops = np.ascontiguousarray(ops, dtype=OP_DTYPE)
+    p = _ptr(ops) if ops.size else None
+    ns, ng = ctypes.c_int(), ctypes.c_int()
+    check(lib().llg_block_plan_export(n, p, ops.size, None, 0, ctypes.byref(ns), None, 0, ctypes.byref(ng)))
+    steps = np.zeros(max(ns.value, 1), dtype=BLOCK_STEP_DTYPE)
+    gates = np.zeros(max(ng.value, 1), dtype=BLOCK_GATE_DTYPE)
+    check(lib().llg_block_plan_export(n, p, ops.size, _ptr(steps), steps.size, ctypes.byref(ns), _ptr(gates),
+                                      gates.size, ctypes.byref(ng)))
+    return steps[: ns.value], gates[: ng.value]
 
 
 def fp64_fma_rate(iters: int = 1 << 16) -> float:

@@ -68,3 +68,80 @@ def test_small_and_special_groups():
         bound = max(TOL["complex128"] * np.max(np.abs(want[sl])), 2.0 ** -1073)
         assert np.max(np.abs(got[sl] - want[sl])) <= bound, g
     st.close()
+
+
+def _circuit(n, depth, seed):
+    """Every gate kind, with sign flips on more than five qubits and lone CNOTs between layers."""
+    rng = np.random.default_rng(seed)
+    recs = []
+    for d in range(depth):
+        for q in range(n):
+            u = np.linalg.qr(rng.normal(size=(2, 2)) + 1j * rng.normal(size=(2, 2)))[0]
+            recs.append((llgpu.OP_U2, q, 0, 0.0, None, u) if d % 2 else (llgpu.OP_RY, q, 0, rng.uniform(0, 6)))
+            recs.append((llgpu.OP_RZ, q, 0, rng.uniform(0, 6)))
+        for _ in range(n // 2):
+            a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+            recs.append((int(rng.choice([llgpu.OP_CNOT, llgpu.OP_CZ])), a, b))
+        recs.append((llgpu.OP_MCZ, 0, 0, 0.0, (1 << 7) - 1))
+    return llgpu.make_ops(recs)
+
+
+@pytest.mark.parametrize("precision", ["complex128", "df64"])
+@pytest.mark.parametrize("n,depth", [(12, 12), (13, 8), (17, 6), (20, 4)])
+def test_fused_blocks_match_oracle(precision, n, depth):
+    ops = _circuit(n, depth, n)
+    want = oracle.run_ops(n, ops)
+    st = llgpu.State(n, precision)
+    st.profile(True)
+    st.apply_ops(ops)
+    assert np.max(np.abs(st.state() - want)) <= 1e-12
+    # the same gates as tile passes
+    st.set_fusion("tile", 11)
+    st.reset(n)
+    st.apply_ops(ops)
+    assert np.max(np.abs(st.state() - want)) <= 1e-12
+    st.close()
+
+
+def test_block_plans_over_many_weights():
+    # more blocks than weights are held at once, in one flush
+    n = 12
+    ops = np.concatenate([_circuit(n, 40, 5)] * 2)
+    st = llgpu.State(n, "complex128")
+    st.apply_ops(ops)
+    assert np.max(np.abs(st.state() - oracle.run_ops(n, ops))) <= 1e-12
+    st.close()
+
+
+def test_states_that_are_not_finite_keep_to_the_tile_passes():
+    # a block would spread an infinity over its 32 amplitudes; the gates alone reach half of the pairs
+    n = 12
+    psi = np.zeros(1 << n, dtype=complex)
+    psi[0], psi[5] = 1.0, np.inf
+    ops = llgpu.make_ops([(llgpu.OP_RY, 3, 0, 0.7), (llgpu.OP_CNOT, 3, 4)] * 30)
+    st = llgpu.State(precision="complex128", amps=psi)
+    st.apply_ops(ops)
+    got = st.state()
+    ref = llgpu.State(precision="complex128", amps=psi)
+    ref.set_fusion("tile", 12)
+    ref.apply_ops(ops)
+    want = ref.state()
+    assert np.array_equal(np.isfinite(got), np.isfinite(want)) and np.isfinite(got).sum() > (1 << n) - 32
+    st.close()
+    ref.close()
+
+
+def test_gates_of_norm_above_one_grow_the_state():
+    # 2x2s that double the norm, far past what integers against a group's largest could hold
+    n = 12
+    grow = llgpu.make_ops([(llgpu.OP_U2, q % n, 0, 0.0, None, [[4.0, 0], [0, 4.0]]) for q in range(300)])
+    mix = _circuit(n, 6, 3)
+    st = llgpu.State(n, "complex128")
+    st.apply_ops(mix)
+    st.apply_ops(grow)
+    st.flush()
+    st.apply_ops(mix)
+    got = np.ldexp(st.state().view(np.float64), -600).view(np.complex128)
+    want = oracle.run_ops(n, np.concatenate([mix, mix]))
+    assert np.max(np.abs(got - want)) <= 1e-12
+    st.close()
