@@ -413,7 +413,7 @@ int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror
             }
             const bool last = mirror && last_group && i + 1 == to;
             rc = traced(st, LLG_PROF_TILE, 1, "gate block", [&] {
-                return launch_gate_block(st->P, st->d_psi, st->n, bd, w + wb * done, false, st->d_flags + 1, st->stream,
+                return launch_gate_block(st->P, st->d_psi, st->n, bd, w + wb * done, false, done > 0, st->d_flags + 1, st->stream,
                                          last ? mirror : nullptr);
             });
             if (rc) return rc;
@@ -916,7 +916,7 @@ int llg_apply_matrix(llg_state* st, int k, const int* qubits, const double* m) {
             const cudaError_t e =
                 launch_gate_block_matrix(st->P, reinterpret_cast<const double*>(st->d_block), st->d_block_tc, st->stream);
             if (e != cudaSuccess) return e;
-            return launch_gate_block(st->P, st->d_psi, st->n, sd, st->d_block_tc, true, st->d_flags + 1, st->stream);
+            return launch_gate_block(st->P, st->d_psi, st->n, sd, st->d_block_tc, true, false, st->d_flags + 1, st->stream);
         });
     }
     if (block_tc_eligible(st->P, st->n, k)) {

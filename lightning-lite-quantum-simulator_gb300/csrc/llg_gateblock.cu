@@ -196,7 +196,7 @@ struct Elem<LLG_DF64> {
 template <int P, bool kRows>
 __global__ void __launch_bounds__(kThreads, 1)
     k_gate_block(typename Elem<P>::S* __restrict__ psi, int n, const __grid_constant__ TargetOffsets to, uint64_t tmask,
-                 const uint4* __restrict__ weights, int* __restrict__ err_flag, double2* __restrict__ mirror) {
+                 const uint4* __restrict__ weights, bool weights_ready, int* __restrict__ err_flag, double2* __restrict__ mirror) {
     using T = Shape<P>;
     constexpr int S = T::S;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -215,6 +215,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t egfull0 = smem_u32(&bars[2 * kRing + 4]), drain = smem_u32(&bars[2 * kRing + 7]);
 
     if (tid < kAmps) toff[tid] = to.o[tid];
+    // Launched while the previous kernel of the stream runs: everything up to the wait below touches
+    // nothing that it writes (the weights only if they were ready before it began).
+    if (!weights_ready) asm volatile("griddepcontrol.wait;" ::: "memory");
     {
         uint4* dst = reinterpret_cast<uint4*>(sW);
         for (int i = tid; i < 2 * T::kWHalfBytes / 16; i += kThreads) dst[i] = weights[i];
@@ -245,6 +248,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_s;
     const uint64_t ntiles = (1ULL << (n - 5)) / kGroups;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp < kSlicerWarps) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSlicerRegs));
@@ -691,7 +696,7 @@ int sm_count() {
 }
 
 template <int P, bool kRows>
-cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, int* err, cudaStream_t s, double* mirror) {
+cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool ready, int* err, cudaStream_t s, double* mirror) {
     using T = Shape<P>;
     static const cudaError_t attr =
         cudaFuncSetAttribute(k_gate_block<P, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmem);
@@ -703,10 +708,20 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, int* er
             if ((j >> b) & 1) to.o[j] |= 1ULL << bd.q[b];
     }
     const uint64_t ntiles = (1ULL << (n - 5)) / kGroups, sms = (uint64_t)sm_count();
-    k_gate_block<P, kRows><<<(unsigned)(ntiles < sms ? ntiles : sms), kThreads, T::kSmem, s>>>(
-        static_cast<typename Elem<P>::S*>(psi), n, to, bd.tmask, static_cast<const uint4*>(w), err,
-        reinterpret_cast<double2*>(mirror));
-    return cudaGetLastError();
+    // programmatic dependent launch: the CTA's set-up (barriers, tensor memory, the gate's digits)
+    // runs under the end of the stream's previous kernel
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ntiles < sms ? ntiles : sms));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = T::kSmem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_gate_block<P, kRows>, static_cast<typename Elem<P>::S*>(psi), n, to, bd.tmask,
+                              static_cast<const uint4*>(w), ready, err, reinterpret_cast<double2*>(mirror));
 }
 
 }  // namespace
@@ -735,13 +750,13 @@ cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const Blo
     return cudaGetLastError();
 }
 
-cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, int* err_flag,
-                              cudaStream_t s, double* mirror) {
+cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, bool ready,
+                              int* err_flag, cudaStream_t s, double* mirror) {
     if (P == LLG_F64)
-        return rows ? launch<LLG_F64, true>(psi, n, bd, d_weights, err_flag, s, mirror)
-                    : launch<LLG_F64, false>(psi, n, bd, d_weights, err_flag, s, mirror);
-    return rows ? launch<LLG_DF64, true>(psi, n, bd, d_weights, err_flag, s, mirror)
-                : launch<LLG_DF64, false>(psi, n, bd, d_weights, err_flag, s, mirror);
+        return rows ? launch<LLG_F64, true>(psi, n, bd, d_weights, ready, err_flag, s, mirror)
+                    : launch<LLG_F64, false>(psi, n, bd, d_weights, ready, err_flag, s, mirror);
+    return rows ? launch<LLG_DF64, true>(psi, n, bd, d_weights, ready, err_flag, s, mirror)
+                : launch<LLG_DF64, false>(psi, n, bd, d_weights, ready, err_flag, s, mirror);
 }
 
 }  // namespace llg

@@ -97,7 +97,8 @@ cudaError_t launch_block_tc(int P, void* psi, int n, const BlockDesc& bd, const 
 // dense 5-qubit blocks of 16-byte states on the tensor cores (llg_gateblock.cu): n >= 12, bd.q in
 // increasing order.  d_weights: gate_block_weight_bytes of device memory, filled by
 // launch_gate_block_matrix (d_matrix: 32 x 32 row-major (re, im) doubles on the device, bit b of an
-// index is bd.q[b]).  rows: the weights have row exponents of their own (launch_gate_block_matrix).  mirror: nullptr, or the device address of a mapped host buffer that also
+// index is bd.q[b]).  rows: the weights have row exponents of their own (launch_gate_block_matrix).  ready:
+// the weights were complete before the stream's previous kernel began.  mirror: nullptr, or the device address of a mapped host buffer that also
 // receives the output as FP64.  A kernel whose waits run out sets *err_flag to 1.
 bool gate_block_eligible(int P, int n);
 size_t gate_block_weight_bytes(int P);
@@ -105,8 +106,8 @@ cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weig
 // the weights of `nblocks` blocks of a plan (d_steps: their steps, in order), one after the other
 cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const BlockStep* d_steps, int nblocks, void* d_weights,
                                       cudaStream_t s);
-cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, int* err_flag,
-                              cudaStream_t s, double* mirror = nullptr);
+cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, bool ready,
+                              int* err_flag, cudaStream_t s, double* mirror = nullptr);
 
 // process-wide tuning cache (llg_tune.cu), keyed by an FNV-1a hash of the workload's shape
 uint64_t tune_hash(uint64_t h, uint64_t v);
