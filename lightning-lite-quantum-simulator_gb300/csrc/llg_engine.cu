@@ -441,21 +441,22 @@ int measure_norm(llg_state* st) {
     return LLG_OK;
 }
 
-// Which plan a flush of 16-byte states takes when the caller has left the tile width and CTA size
-// to the engine: blocks when their passes cost less than tile passes with the same gates (judged on
-// the blocks planned so far).  Measured on this GPU: a block 9.2 ms (FP64) / 12.5 ms (double-float)
-// per 2^30 amplitudes and at least 12 us; a CNOT or sign-flip pass 2.6 ms per 2^30.  Tile passes
-// take 3.2 FP64 multiply-adds per amplitude for a merged one-qubit gate that mixes and 4 for a
-// diagonal one, at 0.56 T a second (double-float: 2.0 ms per 2^30 for either); no less than 2.6 us
-// a gate, however small the register (a CTA's latency); and one read and write of the state.
+// Which plan a flush takes when the caller has left the tile width and CTA size to the engine:
+// blocks when their passes cost less than tile passes with the same gates (judged on the blocks
+// planned so far).  Measured on this GPU, per 2^30 amplitudes: a block 8.6 (FP64) or 10.3 ms
+// (double-float), and at least 9.5 us; a CNOT or sign-flip pass 2.6 ms.  Tile passes take 3.2 FP64
+// multiply-adds per amplitude for a merged one-qubit gate that mixes and 4 for a diagonal one, at
+// 0.56 T a second (double-float: 2.0 ms per 2^30 for either); no less than 2.6 (FP64) or 2 us a
+// gate, however small the register (a CTA's latency); and one read and write of the state.
 bool blocks_pay(int P, int n, const BlockPlan& plan) {
+    const bool f64 = P == LLG_F64;
     const double amps = std::ldexp(1.0, n);
-    const double block = std::max(12e-6, amps * (P == LLG_F64 ? 8.6e-12 : 11.6e-12));
+    const double block = std::max(9.5e-6, amps * (f64 ? 8.0e-12 : 9.6e-12));
     const double single = 3e-6 + amps * 2.4e-12;
-    const double t_blocks = plan.blocks * block + ((double)plan.steps.size() - plan.blocks) * single + 10e-6;
-    const double arith = P == LLG_F64 ? (3.2 * plan.mixing_1q + 4.0 * plan.diag_1q) / 0.56e12
-                                      : 1.9e-12 * (plan.mixing_1q + plan.diag_1q);
-    const double t_tiles = std::max(std::max(arith * amps, 2.6e-6 * (double)plan.gates.size()), amps * 4.8e-12);
+    const double t_blocks = plan.blocks * block + ((double)plan.steps.size() - plan.blocks) * single + 20e-6;
+    const double arith = f64 ? (3.2 * plan.mixing_1q + 4.0 * plan.diag_1q) / 0.56e12 : 1.9e-12 * (plan.mixing_1q + plan.diag_1q);
+    const double latency = f64 ? 2.6e-6 : 2.0e-6;
+    const double t_tiles = std::max(std::max(arith * amps, latency * (double)plan.gates.size()), amps * 4.8e-12);
     return t_blocks < t_tiles;
 }
 

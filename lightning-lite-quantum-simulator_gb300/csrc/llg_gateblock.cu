@@ -27,12 +27,18 @@
 //     are stacked along N: X_i times [W_0 .. W_(S-1-i)] is one instruction whose columns are the
 //     diagonals i .. S-1, so a state slice is read once per K step instead of S - i times (N = 64
 //     products were bound by shared-memory reads, 48 clocks for 32 of tensor work).
-//   * 8 epilogue warps: tcgen05.ld, recombination, stores.
-// The serial form that this replaced (one set of accumulators, load - slice - multiply - recombine
-// one after the other on 16 warps) took 25k clocks per tile.
+//   * 16 (FP64) or 8 epilogue warps: tcgen05.ld, recombination, stores.
+//   * one warp that prefetches into L2.
+// Measured at 26 qubits, ms per 2^30 amplitudes, targets (5, 9, 13, 17, 25) / (0, 1, 2, 3, 4): FP64 8.3 /
+// 12.6 (9.0k clocks per tile: the MMAs take 6.7k of them, sharing shared memory with the slicers'
+// stores; FP64 pipe 41 % busy with the conversions), double-float 10.1 / 13.0 (bound by slicing).
+// With the lowest five qubits a warp's 32 accesses go to 32 lines.  The serial form that this replaced
+// (one set of accumulators, load - slice - multiply - recombine one after the other on 16 warps)
+// took 25k clocks per tile, 22 / 26 and 14 / 19 ms.
 //
-// Digits without integer work: the bytes u of X + 0x8080..80 are d + 128, and the fp16 with bits
-// 0x6400 | u is 1024 + u, so a byte permute and one packed subtraction of 1152 make two digits.
+// Digits without integer work: the bytes u of |X| + 0x8080..80 are d + 128, and the fp16 with bits
+// 0x6400 | u is 1024 + u, so a byte permute and one packed multiply-add (by the sign, minus 1152) make
+// two digits.
 // fp32 to integer without conversions (16 per clock and SM): diagonals 0 .. 4 are at most 2^22 in
 // size, so adding 1.5 2^23 leaves the integer in the low bits of the float.
 #include <cuda_fp16.h>
@@ -40,6 +46,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #include "llg_common.cuh"
 #include "llg_internal.h"
@@ -53,11 +60,7 @@ constexpr int kGroups = 128;     // groups per tile (the MMA's M)
 constexpr int kAmps = 32;        // amplitudes per group
 constexpr int kChunks = 4;       // K steps of 16 reals (8 amplitudes) per tile
 constexpr int kRing = 5;         // chunk buffers
-constexpr int kSlicerWarps = 8, kEpiWarps = 8;
-constexpr int kMmaWarp = kSlicerWarps + kEpiWarps;
-constexpr int kThreads = (kSlicerWarps + kEpiWarps + 4) * 32;  // five warpgroups; the last one's first warp issues the MMAs
-// registers a thread by role (setmaxnreg): 96 at launch, 2 * 112 + 2 * 104 + 40 <= 5 * 96 per scheduler
-constexpr int kSlicerRegs = 112, kEpiRegs = 104, kMmaRegs = 40;
+constexpr int kSlicerWarps = 8;
 constexpr int kSliceBytes = kGroups * 16 * 2;  // one digit of one chunk
 constexpr int kTmemCols = 512;                 // two accumulator sets
 constexpr long kWaitLimit = 1L << 22;          // mbarrier polls before the kernel reports a timeout
@@ -69,7 +72,28 @@ struct Shape {
     static constexpr int kWHalfBytes = S * 32 * 64 * 2;        // 32 S rows (digit, output) of 64 columns
     static constexpr int kSetStride = 256;                     // columns between the accumulator sets (32 S used)
     static constexpr size_t kSmem = (size_t)kRing * kChunkBytes + 2 * kWHalfBytes;
+    // FP64: the conversion of the 64-bit sums (2 a clock and SM) leaves its warps waiting, so twice as
+    // many with half the registers (8.54 -> 8.30 ms per 2^30; double-float loses 4 %)
+    static constexpr int kEpiWarps = P == LLG_F64 ? 16 : 8;
+    static constexpr int kStep = P == LLG_F64 ? 4 : 8;         // reals that an epilogue thread recombines at a time
+    // the MMA warp, the prefetching warp and two more fill the last warpgroup
+    static constexpr int kMmaWarp = kSlicerWarps + kEpiWarps;
+    static constexpr int kThreads = (kMmaWarp + 4) * 32;
+    // registers a thread at launch and by role (setmaxnreg): the roles' sum over the warps of a
+    // scheduler is at most the launch's
+    static constexpr int kLaunchRegs = P == LLG_F64 ? 72 : 96;
+    static constexpr int kSlicerRegs = 112, kEpiRegs = P == LLG_F64 ? 64 : 104, kMmaRegs = P == LLG_F64 ? 24 : 40;
+    static_assert(kSlicerWarps / 4 * kSlicerRegs + kEpiWarps / 4 * kEpiRegs + kMmaRegs <= kThreads / 128 * kLaunchRegs,
+                  "the roles' registers come out of the launch's");
+    static_assert(kThreads / 128 * kLaunchRegs * 128 <= 65536, "one CTA's registers");
 };
+
+// setmaxnreg to kTo registers from kFrom (an increase must not name fewer than there are)
+template <int kFrom, int kTo>
+__device__ __forceinline__ void set_registers() {
+    if constexpr (kTo > kFrom) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTo));
+    else if constexpr (kTo < kFrom) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTo));
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -85,9 +109,8 @@ __device__ __forceinline__ uint32_t core_off(int row, int c, int kreals) {
     return (uint32_t)((row >> 3) * (kreals / 8) * 128 + (c >> 3) * 128 + (row & 7) * 16 + (c & 7) * 2);
 }
 
-// column (K index) of part `part` (0 real, 1 imaginary) of amplitude j: chunks of 8 amplitudes; a
-// slicer thread's four amplitudes (j bit 0 fixed) fill one 8-wide core row
-__device__ __forceinline__ int col_of(int j, int part) { return 16 * (j >> 3) + 8 * (j & 1) + 2 * ((j >> 1) & 3) + part; }
+// Column (K index) of part p (0 real, 1 imaginary) of amplitude j: 16 (j >> 3) + 8 (j & 1) + 2 ((j >> 1) & 3) + p,
+// so that a slicer thread's four amplitudes of a chunk (j bit 0 fixed) fill one 8-wide core row.
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
@@ -194,7 +217,7 @@ struct Elem<LLG_DF64> {
 // kRows: the gate's rows have exponents of their own (any matrix); else all have exponent 1 (a product
 // of unitary gates, entries at most 1).
 template <int P, bool kRows>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Shape<P>::kThreads, 1)
     k_gate_block(typename Elem<P>::S* __restrict__ psi, int n, const __grid_constant__ TargetOffsets to, uint64_t tmask,
                  const uint4* __restrict__ weights, bool weights_ready, int* __restrict__ err_flag, double2* __restrict__ mirror) {
     using T = Shape<P>;
@@ -207,8 +230,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     __shared__ __align__(16) int32_t er_s[64];
     __shared__ __align__(8) uint64_t bars[2 * kRing + 8];
     __shared__ uint32_t tmem_s;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, progress;
     volatile int* abort_s = &abort_flag;
+    volatile int* progress_s = &progress;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[kRing]);
     const uint32_t accfull0 = smem_u32(&bars[2 * kRing]), accempty0 = smem_u32(&bars[2 * kRing + 2]);
@@ -220,24 +244,25 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (!weights_ready) asm volatile("griddepcontrol.wait;" ::: "memory");
     {
         uint4* dst = reinterpret_cast<uint4*>(sW);
-        for (int i = tid; i < 2 * T::kWHalfBytes / 16; i += kThreads) dst[i] = weights[i];
+        for (int i = tid; i < 2 * T::kWHalfBytes / 16; i += T::kThreads) dst[i] = weights[i];
         if (tid < 16) reinterpret_cast<uint4*>(er_s)[tid] = weights[2 * T::kWHalfBytes / 16 + tid];
     }
     if (tid == 0) {
         abort_flag = 0;
+        progress = 0;
         for (int i = 0; i < kRing; ++i) {
             mbar_init(full0 + 8 * i, kSlicerWarps);
             mbar_init(empty0 + 8 * i, 1);
         }
         for (int h = 0; h < 2; ++h) {
             mbar_init(accfull0 + 8 * h, 1);
-            mbar_init(accempty0 + 8 * h, kEpiWarps);
+            mbar_init(accempty0 + 8 * h, T::kEpiWarps);
         }
         for (int i = 0; i < 3; ++i) mbar_init(egfull0 + 8 * i, kSlicerWarps);
         mbar_init(drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == kMmaWarp) {
+    if (warp == T::kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)),
                      "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -252,24 +277,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp < kSlicerWarps) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSlicerRegs));
+        set_registers<T::kLaunchRegs, T::kSlicerRegs>();
         // ---- slicers: group g = 16 warp + (lane & 15), amplitudes j = 8 ks + 2 i + h with h = lane / 16:
         // a warp reads whole 32-byte sectors when the lowest target is qubit 0 (j and j + 1 adjacent),
         // and eight neighbouring lanes store one 128-byte core ----
         const int g = 16 * warp + (lane & 15), h = lane >> 4;
-        // a tile is runs of 2^cl contiguous amplitudes (at least 2 KB); lane j of warp 0 asks for the run
-        // that starts at target offset j, two tiles ahead, so that the loads of the last chunk, which are
-        // waited for at once, come from L2
-        const uint64_t in_tile = insert0_mask(kGroups - 1, tmask) | tmask;
-        const int cl = __ffsll((long long)~in_tile) - 1;
-        const bool run_start = warp == 0 && (toff[lane] & ((1ULL << cl) - 1)) == 0;
-        auto prefetch_l2 = [&](uint64_t t) {
-            if (run_start && t < ntiles)
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(psi + (insert0_mask(t * kGroups, tmask) | toff[lane])),
-                             "r"(16u << cl)
-                             : "memory");
-        };
-        prefetch_l2(blockIdx.x + (uint64_t)gridDim.x);
+        int seen = 0;  // tiles begun, for the prefetching warp
         typename Elem<P>::S a[16];
         uint64_t tile = blockIdx.x;
         if (tile < ntiles) {
@@ -312,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 eg = max((int)(__float_as_uint(mx) >> 23), 8);
             }
             const uint64_t next = tile + gridDim.x;
-            prefetch_l2(next + gridDim.x);
+            if (tid == 0) *progress_s = ++seen;
             const auto* pb = psi + ((next < ntiles ? insert0_mask(next * kGroups + (uint64_t)g, tmask) : 0) | (h ? to.o[1] : 0));
 #pragma unroll
             for (int ks = 0; ks < kChunks; ++ks) {
@@ -396,10 +409,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             }
         }
-    } else if (warp < kMmaWarp) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
+    } else if (warp < T::kMmaWarp) {
+        set_registers<T::kLaunchRegs, T::kEpiRegs>();
         // ---- epilogue: tensor-memory lanes 32 (warp & 3) .. +31 (the groups), amplitudes
-        // 16 half + 8 e + 4 p .. +3 ----
+        // kStep / 2 of the half's 16 at a time ----
         const int row = 32 * (warp & 3) + lane, e = (warp - kSlicerWarps) >> 2;
         const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
         const bool pair32 = to.o[1] == 1;  // amplitudes j and j + 1 (j even) are adjacent
@@ -410,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t phase = 0, egphase = 0;
         bool ok = true;
         for (uint64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, phase ^= 1) {
-            const uint64_t base = insert0_mask(tile * kGroups + (uint64_t)row, tmask) | toff[8 * e];
+            const uint64_t base = insert0_mask(tile * kGroups + (uint64_t)row, tmask) | toff[T::kStep * e];
             if (!warp_wait(egfull0 + 8 * egb, egphase, abort_s)) break;
             const int eg = eg_s[egb][row];
             if (++egb == 3) {
@@ -428,14 +441,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
                 for (int p = 0; p < 2; ++p) {
-                    uint32_t v[S][8];
+                    const int col = T::kStep * (2 * e + p);  // within each diagonal's 32 columns
+                    uint32_t v[S][T::kStep];
 #pragma unroll
                     for (int d = 0; d < S; ++d) {
-                        const uint32_t taddr = tlane + (uint32_t)(half * T::kSetStride + 32 * d + 16 * e + 8 * p);
-                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                                     : "=r"(v[d][0]), "=r"(v[d][1]), "=r"(v[d][2]), "=r"(v[d][3]), "=r"(v[d][4]),
-                                       "=r"(v[d][5]), "=r"(v[d][6]), "=r"(v[d][7])
-                                     : "r"(taddr));
+                        const uint32_t taddr = tlane + (uint32_t)(half * T::kSetStride + 32 * d + col);
+                        if constexpr (T::kStep == 4)
+                            asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                                         : "=r"(v[d][0]), "=r"(v[d][1]), "=r"(v[d][2]), "=r"(v[d][3])
+                                         : "r"(taddr));
+                        else
+                            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                                         : "=r"(v[d][0]), "=r"(v[d][1]), "=r"(v[d][2]), "=r"(v[d][3]), "=r"(v[d][4]),
+                                           "=r"(v[d][5]), "=r"(v[d][6]), "=r"(v[d][7])
+                                         : "r"(taddr));
                     }
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (p == 1) {  // this warp has read the set
@@ -443,11 +462,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                         __syncwarp();
                         if (lane == 0) mbar_arrive(accempty0 + 8 * half);
                     }
-                    const uint64_t pos = base | toff[16 * half + 4 * p];
-                    typename Elem<P>::S out[4];
+                    const uint64_t pos = base | toff[16 * half + T::kStep / 2 * p];
+                    typename Elem<P>::S out[T::kStep / 2];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const int er = kRows ? er_s[32 * half + 16 * e + 8 * p + c] : 1;
+                    for (int c = 0; c < T::kStep; ++c) {
+                        const int er = kRows ? er_s[32 * half + col + c] : 1;
                         if constexpr (P == LLG_F64) {
                             // 2^44 sum_d 2^(-8 d) D_d: D_0 .. D_4 exact, D_5 .. D_7 rounded to an integer
                             const float magic = 12582912.0f;
@@ -503,7 +522,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                     if (pair32) {
 #pragma unroll
-                        for (int c = 0; c < 4; c += 2) {
+                        for (int c = 0; c < T::kStep / 2; c += 2) {
                             uint64_t w[4];
                             memcpy(w, &out[c], 32);
                             asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(psi + pos + to.o[c]), "l"(w[0]), "l"(w[1]),
@@ -512,11 +531,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                         }
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) psi[pos + to.o[c]] = out[c];
+                        for (int c = 0; c < T::kStep / 2; ++c) psi[pos + to.o[c]] = out[c];
                     }
                     if (mirror) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
+                        for (int c = 0; c < T::kStep / 2; ++c) {
                             if constexpr (P == LLG_F64) mirror[pos + to.o[c]] = out[c];
                             else
                                 mirror[pos + to.o[c]] = make_double2((double)out[c].x + (double)out[c].z,
@@ -527,8 +546,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
     } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegs));
-        if (warp == kMmaWarp) {
+        set_registers<T::kLaunchRegs, T::kMmaRegs>();
+        if (warp == T::kMmaWarp) {
             // ---- the MMA warp: the whole warp walks the loop (so that the descriptors are uniform), one
             // elected thread issues ----
             constexpr uint32_t idesc0 = (1u << 4) | ((uint32_t)(kGroups >> 4) << 24);  // fp32 from fp16, M = 128
@@ -597,6 +616,21 @@ __global__ void __launch_bounds__(kThreads, 1)
                              : "memory");
                 if (done) break;
             }
+        } else if (warp == T::kMmaWarp + 1) {
+            // ---- a tile is runs of 2^cl contiguous amplitudes (at least 2 KB); lane j asks for the run that
+            // starts at target offset j, two tiles ahead of the slicers, so that their loads come from L2
+            // (issued by a slicer warp, the same instructions held it up for 3000 clocks a tile) ----
+            const uint64_t in_tile = insert0_mask(kGroups - 1, tmask) | tmask;
+            const int cl = __ffsll((long long)~in_tile) - 1;
+            const bool run_start = (toff[lane] & ((1ULL << cl) - 1)) == 0;
+            int begun = 0;
+            for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x; t < ntiles && !*abort_s; t += gridDim.x, ++begun) {
+                for (int it = 0; it < 100000 && *progress_s < begun && !*abort_s; ++it) __nanosleep(200);
+                if (run_start)
+                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(psi + (insert0_mask(t * kGroups, tmask) | toff[lane])),
+                                 "r"((uint32_t)sizeof(typename Elem<P>::S) << cl)
+                                 : "memory");
+            }
         }
     }
     __syncwarp();
@@ -604,7 +638,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (tid == 0 && abort_flag) atomicExch(err_flag, 1);
-    if (warp == kMmaWarp)
+    if (warp == T::kMmaWarp)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
@@ -715,7 +749,7 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool re
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(ntiles < sms ? ntiles : sms));
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(T::kThreads);
     cfg.dynamicSmemBytes = T::kSmem;
     cfg.stream = s;
     cfg.attrs = &at;
@@ -728,35 +762,43 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool re
 
 bool gate_block_eligible(int P, int n) { return (P == LLG_F64 || P == LLG_DF64) && n >= 12; }
 
+namespace {
+// f with the precision as a compile-time constant
+template <class F>
+auto by_precision(int P, F&& f) {
+    if (P == LLG_F64) return f(std::integral_constant<int, LLG_F64>());
+    return f(std::integral_constant<int, LLG_DF64>());
+}
+}  // namespace
+
 size_t gate_block_weight_bytes(int P) {
-    return (P == LLG_F64 ? 2 * Shape<LLG_F64>::kWHalfBytes : 2 * Shape<LLG_DF64>::kWHalfBytes) + 64 * sizeof(int32_t);
+    return by_precision(P, [](auto p) { return (size_t)2 * Shape<decltype(p)::value>::kWHalfBytes + 64 * sizeof(int32_t); });
 }
 
 cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weights, cudaStream_t s) {
-    unsigned char* w = static_cast<unsigned char*>(d_weights);
-    const double2* m = reinterpret_cast<const double2*>(d_matrix);
-    if (P == LLG_F64) k_weights<Shape<LLG_F64>::S, true><<<dim3(1, kChunks), 128, 0, s>>>(m, nullptr, nullptr, w, 0);
-    else k_weights<Shape<LLG_DF64>::S, true><<<dim3(1, kChunks), 128, 0, s>>>(m, nullptr, nullptr, w, 0);
-    return cudaGetLastError();
+    return by_precision(P, [&](auto p) {
+        k_weights<Shape<decltype(p)::value>::S, true><<<dim3(1, kChunks), 128, 0, s>>>(
+            reinterpret_cast<const double2*>(d_matrix), nullptr, nullptr, static_cast<unsigned char*>(d_weights), 0);
+        return cudaGetLastError();
+    });
 }
 
 cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const BlockStep* d_steps, int nblocks, void* d_weights,
                                       cudaStream_t s) {
-    unsigned char* w = static_cast<unsigned char*>(d_weights);
-    const size_t stride = gate_block_weight_bytes(P);
-    const dim3 grid((unsigned)nblocks, kChunks);
-    if (P == LLG_F64) k_weights<Shape<LLG_F64>::S, false><<<grid, 128, 0, s>>>(nullptr, d_gates, d_steps, w, stride);
-    else k_weights<Shape<LLG_DF64>::S, false><<<grid, 128, 0, s>>>(nullptr, d_gates, d_steps, w, stride);
-    return cudaGetLastError();
+    return by_precision(P, [&](auto p) {
+        k_weights<Shape<decltype(p)::value>::S, false><<<dim3((unsigned)nblocks, kChunks), 128, 0, s>>>(
+            nullptr, d_gates, d_steps, static_cast<unsigned char*>(d_weights), gate_block_weight_bytes(P));
+        return cudaGetLastError();
+    });
 }
 
 cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, bool ready,
                               int* err_flag, cudaStream_t s, double* mirror) {
-    if (P == LLG_F64)
-        return rows ? launch<LLG_F64, true>(psi, n, bd, d_weights, ready, err_flag, s, mirror)
-                    : launch<LLG_F64, false>(psi, n, bd, d_weights, ready, err_flag, s, mirror);
-    return rows ? launch<LLG_DF64, true>(psi, n, bd, d_weights, ready, err_flag, s, mirror)
-                : launch<LLG_DF64, false>(psi, n, bd, d_weights, ready, err_flag, s, mirror);
+    return by_precision(P, [&](auto p) {
+        constexpr int PP = decltype(p)::value;
+        return rows ? launch<PP, true>(psi, n, bd, d_weights, ready, err_flag, s, mirror)
+                    : launch<PP, false>(psi, n, bd, d_weights, ready, err_flag, s, mirror);
+    });
 }
 
 }  // namespace llg
