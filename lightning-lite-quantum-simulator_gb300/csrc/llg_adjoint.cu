@@ -14,6 +14,10 @@
 // array and summed in a fixed order, so gradients are deterministic.  Forward states can be
 // checkpointed every C passes; the backward sweep then restarts psi from each checkpoint instead
 // of relying on uncomputation alone (deep circuits).
+//
+// IEEE complex128 circuits on 12 to 26 qubits run as dense 5-qubit blocks on the tensor cores where
+// that costs less (llg_gateblock.cu; the gradients of a block from one 32 x 32 matrix,
+// llg_adjblock.cu); not with checkpoints or a set CTA size.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -23,7 +27,9 @@
 #include <cuda_runtime.h>
 
 #include "../../include/llgpu.h"
+#include "llg_adjblock.h"
 #include "llg_common.cuh"
+#include "llg_common_host.h"
 #include "llg_internal.h"
 #include "llg_diag_launch.h"
 #include "llg_launch.h"
@@ -567,6 +573,20 @@ struct llg_adjoint {
     double* d_shift_val = nullptr;
     std::vector<void*> ckpt;
     size_t state_bytes = 0;  // one batch element
+    // the block form: plan, its device copy, and the workspace for `bsets` parameter sets at a time
+    // (0: no block plan or no room for it)
+    std::vector<BlockStep> bsteps;
+    std::vector<BlockGate> bgates;
+    std::vector<char> bparams;  // per step: has parametrised gates
+    BlockStep* d_bsteps = nullptr;
+    BlockGate* d_bgates = nullptr;
+    int bsets = -1;             // -1: not allocated yet
+    unsigned char* d_bweights = nullptr;  // [step][set], the blocks, then their inverses
+    double2* d_angles = nullptr;          // [batch][occurrence]
+    double2* d_bR = nullptr;              // [step][set]
+    double2* d_bpart = nullptr;
+    uint32_t* d_bexps = nullptr;          // [step + 1][2 sets]
+    int* d_bflag = nullptr;
 };
 
 namespace {
@@ -680,6 +700,135 @@ int run_backward(llg_adjoint* h, int batch, int C) {
     k_grad_finish<<<(total + 255) / 256, 256, 0, s>>>(h->d_gpart, batch, h->nocc, h->tiles, h->nparams, h->d_csr_ptr,
                                                       h->d_csr_occ, h->d_grad);
     ADJ_CUDA(cudaGetLastError(), "gradient finish");
+    return LLG_OK;
+}
+
+// Time of a batch in the two forms.  Measured on this GPU in IEEE complex128: tile passes 10 ps per gate and
+// amplitude (2.8 ps forward only), and no less than 6 us (2.5) a gate; a block 8.0 ps per amplitude and at
+// least 9.5 us, the 32 x 32 sums 9.5 ps and at least 20 us.
+bool blocks_pay(const llg_adjoint* h, int batch, bool grads) {
+    const double amps = std::ldexp((double)batch, h->n);
+    const double tiles = (double)h->fwd.ops.size() * std::max(grads ? 6e-6 : 2.5e-6, amps * (grads ? 1.0e-11 : 2.8e-12));
+    const double fwd = std::max(9.5e-6, amps * 8.0e-12);
+    const double bwd = std::max(20e-6, amps * 9.5e-12) + std::max(9.5e-6, amps * 16e-12);
+    return (double)h->bsteps.size() * (fwd + (grads ? bwd : 0.0)) + 50e-6 < tiles;
+}
+
+// Allocates the block form's workspace once; h->bsets = 0 when there is no room (the tile passes run).
+void ensure_blocks(llg_adjoint* h) {
+    if (h->bsets >= 0) return;
+    h->bsets = 0;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // sets at a time: 512 MB each for the weights and the CTAs' sums
+    constexpr size_t kCap = (size_t)512 << 20;
+    const size_t steps = h->bsteps.size(), wb = gate_block_weight_bytes(LLG_F64);
+    int sets = (int)std::min<size_t>(h->max_batch, kCap / (2 * steps * wb));
+    size_t part = 0;
+    for (int k = 1; k <= sets; ++k) {
+        const size_t need = (size_t)k * cross_ctas(h->n, k, sms) * 1024 * sizeof(double2);
+        if (need > kCap) {
+            sets = k - 1;
+            break;
+        }
+        part = std::max(part, need);
+    }
+    if (sets < 1) return;
+    bool ok = cudaMalloc((void**)&h->d_bsteps, steps * sizeof(BlockStep)) == cudaSuccess;
+    ok = ok && cudaMalloc((void**)&h->d_bgates, h->bgates.size() * sizeof(BlockGate)) == cudaSuccess;
+    ok = ok && cudaMalloc((void**)&h->d_bweights, 2 * steps * sets * wb) == cudaSuccess;
+    ok = ok && cudaMalloc((void**)&h->d_angles, std::max<size_t>(1, (size_t)h->max_batch * h->nocc) * sizeof(double2)) == cudaSuccess;
+    ok = ok && cudaMalloc((void**)&h->d_bR, steps * sets * 1024 * sizeof(double2)) == cudaSuccess;
+    ok = ok && cudaMalloc((void**)&h->d_bpart, part) == cudaSuccess;
+    ok = ok && cudaMalloc((void**)&h->d_bexps, (steps + 1) * 2 * sets * sizeof(uint32_t)) == cudaSuccess;
+    ok = ok && cudaMalloc((void**)&h->d_bflag, sizeof(int)) == cudaSuccess;
+    ok = ok && cudaMemcpy(h->d_bsteps, h->bsteps.data(), steps * sizeof(BlockStep), cudaMemcpyHostToDevice) == cudaSuccess;
+    ok = ok && cudaMemcpy(h->d_bgates, h->bgates.data(), h->bgates.size() * sizeof(BlockGate), cudaMemcpyHostToDevice) == cudaSuccess;
+    if (!ok) {
+        cudaGetLastError();
+        void** all[] = {(void**)&h->d_bsteps, (void**)&h->d_bgates, (void**)&h->d_bweights, (void**)&h->d_angles,
+                        (void**)&h->d_bR, (void**)&h->d_bpart, (void**)&h->d_bexps, (void**)&h->d_bflag};
+        for (void** p : all) {
+            if (*p) cudaFree(*p);
+            *p = nullptr;
+        }
+        return;
+    }
+    h->bsets = sets;
+}
+
+// energies and, with grads, the gradients of a batch in blocks
+int run_blocks(llg_adjoint* h, int batch, bool grads) {
+    cudaStream_t s = h->stream;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int steps = (int)h->bsteps.size(), n = h->n;
+    const size_t wb = gate_block_weight_bytes(LLG_F64);
+    const uint64_t size = 1ULL << n, tiles = size >> 12;
+    ADJ_CUDA(cudaMemsetAsync(h->d_bflag, 0, sizeof(int), s), "memset flag");
+    if (h->nocc)
+        ADJ_CUDA(launch_angles(h->d_params, h->nparams, h->d_occ_param, h->nocc, batch, h->d_angles, s), "angles");
+    int first = steps;  // the earliest step with parametrised gates
+    for (int j = steps - 1; j >= 0; --j)
+        if (h->bparams[j]) first = j;
+    for (int s0 = 0; s0 < batch; s0 += h->bsets) {
+        const int sets = std::min(h->bsets, batch - s0);
+        double2* psi = static_cast<double2*>(h->d_psi) + (size_t)s0 * size;
+        double2* lam = static_cast<double2*>(h->d_lam) + (size_t)s0 * size;
+        const double2* ang = h->d_angles + (size_t)s0 * h->nocc;
+        unsigned char* inverse = h->d_bweights + (size_t)steps * sets * wb;
+        auto desc = [&](int j) {
+            BlockDesc bd;
+            std::memset(&bd, 0, sizeof(bd));
+            bd.k = 5;
+            for (int b = 0; b < 5; ++b) {
+                bd.q[b] = h->bsteps[j].q[b];
+                bd.tmask |= 1ULL << bd.q[b];
+            }
+            return bd;
+        };
+        ADJ_CUDA(launch_gate_block_weights(LLG_F64, h->d_bgates, h->d_bsteps, steps, h->d_bweights, s, ang, h->nocc, sets, false),
+                 "block weights");
+        if (grads)
+            ADJ_CUDA(launch_gate_block_weights(LLG_F64, h->d_bgates, h->d_bsteps, steps, inverse, s, ang, h->nocc, sets, true),
+                     "block weights");
+        ADJ_CUDA(cudaMemsetAsync(psi, 0, (size_t)sets * h->state_bytes, s), "memset psi");
+        k_set_rows<PolF64><<<(sets + 255) / 256, 256, 0, s>>>(psi, n, sets);
+        ADJ_CUDA(cudaGetLastError(), "init rows");
+        const int fwd_ctas = block_ctas(tiles, sets, sms, 1), bwd_ctas = block_ctas(tiles, 2 * sets, sms, 1);
+        for (int j = 0; j < steps; ++j)
+            ADJ_CUDA(launch_gate_block_batch(psi, nullptr, sets, fwd_ctas, n, desc(j), h->d_bweights + (size_t)j * sets * wb,
+                                             true, nullptr, h->d_bflag, s),
+                     "block");
+        const int eblocks = (int)std::min<uint64_t>(kEBlocksPerState, size >> h->obs.L);
+        ADJ_CUDA(launch_lambda_diag(h->P, psi, grads ? lam : nullptr, diag_obs_view(h->obs, h->d_obs), sets, eblocks,
+                                    h->d_epart, h->d_energy + s0, s),
+                 "energy");
+        if (!grads) continue;
+        ADJ_CUDA(cudaMemsetAsync(h->d_bexps, 0, (size_t)(steps + 1) * 2 * sets * sizeof(uint32_t), s), "memset exponents");
+        ADJ_CUDA(launch_max_exponent(psi, lam, n, sets, h->d_bexps + (size_t)steps * 2 * sets, s), "exponents");
+        for (int j = steps - 1; j >= first; --j) {
+            if (h->bparams[j])
+                ADJ_CUDA(launch_cross(psi, lam, n, sets, cross_ctas(n, sets, sms), desc(j), h->d_bexps + (size_t)(j + 1) * 2 * sets,
+                                      h->d_bpart, h->d_bR + (size_t)j * sets * 1024, h->d_bflag, s),
+                         "block sums");
+            if (j > first)
+                ADJ_CUDA(launch_gate_block_batch(psi, lam, sets, bwd_ctas, n, desc(j), inverse + (size_t)j * sets * wb, true,
+                                                 h->d_bexps + (size_t)j * 2 * sets, h->d_bflag, s),
+                         "inverse block");
+        }
+        ADJ_CUDA(launch_block_grads(h->d_bR, h->d_bsteps, steps, h->d_bgates, ang, h->nocc, sets, h->d_gpart + (size_t)s0 * h->nocc, s),
+                 "block gradients");
+    }
+    if (grads) {
+        const int total = batch * h->nparams;
+        if (total > 0)
+            k_grad_finish<<<(total + 255) / 256, 256, 0, s>>>(h->d_gpart, batch, h->nocc, 1, h->nparams, h->d_csr_ptr,
+                                                              h->d_csr_occ, h->d_grad);
+        ADJ_CUDA(cudaGetLastError(), "gradient finish");
+    }
     return LLG_OK;
 }
 
@@ -812,6 +961,21 @@ int llg_adjoint_create(int n, const llg_op* ops, int nops, int nparams, int max_
         return set_error(LLG_EINVAL, "adjoint_create: " + err);
     }
     h->tiles = 1 << (n - t);
+    if (precision == LLG_F64 && n <= 26 && has_block_plan(n, ops, nops)) {
+        bool fits = true;  // sign flips on more than five qubits have no block
+        for (int i = 0; i < nops; ++i) fits = fits && !(ops[i].kind == LLG_OP_MCZ && popcount64(ops[i].mask) > 5);
+        if (fits) {
+            BlockPlanner planner(n, ops, nops, true);
+            while (planner.advance(1 << 20)) {}
+            h->bsteps = planner.plan.steps;
+            h->bgates = planner.plan.gates;
+            for (const BlockStep& b : h->bsteps) {
+                char has = 0;
+                for (int k = 0; k < b.ngates; ++k) has |= h->bgates[b.gate_begin + k].kind == 3;
+                h->bparams.push_back(has);
+            }
+        }
+    }
     // backward plan: passes reversed, ops reversed and inverted, parametrised ops flagged
     for (int j = (int)h->fwd.passes.size() - 1; j >= 0; --j) {
         PassDesc pd = h->fwd.passes[j];
@@ -879,7 +1043,8 @@ int llg_adjoint_destroy(llg_adjoint* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     void* ptrs[] = {h->d_psi, h->d_lam, h->d_fwd_ops, h->d_bwd_ops, h->d_table, h->d_form, h->d_occ_param, h->d_csr_ptr,
                     h->d_csr_occ, h->d_params, h->d_gpart, h->d_epart, h->d_energy, h->d_grad, h->d_row_set,
-                    h->d_shift_occ, h->d_shift_val, h->d_obs};
+                    h->d_shift_occ, h->d_shift_val, h->d_obs, h->d_bsteps, h->d_bgates, h->d_bweights, h->d_angles,
+                    h->d_bR, h->d_bpart, h->d_bexps, h->d_bflag};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (void* p : h->ckpt) cudaFree(p);
@@ -910,6 +1075,17 @@ int llg_adjoint_run(llg_adjoint* h, const double* params, int batch, double* ene
         return set_error(LLG_EINVAL, "adjoint_run: batch must be in [1, " + std::to_string(h->max_batch) + "]");
     if (checkpoint_every < 0) return set_error(LLG_EINVAL, "adjoint_run: checkpoint_every must be >= 0");
     int rc = load_params(h, params, batch);
+    if (!h->bsteps.empty() && h->threads == 0 && checkpoint_every == 0 && blocks_pay(h, batch, grads != nullptr)) ensure_blocks(h);
+    if (!rc && h->bsets > 0 && h->threads == 0 && checkpoint_every == 0 && blocks_pay(h, batch, grads != nullptr)) {
+        rc = run_blocks(h, batch, grads != nullptr);
+        int flag = 0;
+        if (!rc) rc = store_out(h, energies, h->d_energy, batch);
+        if (!rc && grads) rc = store_out(h, grads, h->d_grad, (size_t)batch * h->nparams);
+        if (!rc) ADJ_CUDA(cudaMemcpyAsync(&flag, h->d_bflag, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "flag");
+        if (!rc) ADJ_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+        if (!rc && flag) rc = set_error(LLG_ECUDA, "adjoint: a tensor-core kernel timed out waiting for its products");
+        return rc;
+    }
     if (!rc) rc = build_table(h, batch, false);
     if (!rc && grads) rc = ensure_checkpoints(h, checkpoint_every);
     if (!rc) rc = forward_dispatch(h, batch, grads != nullptr, grads ? &checkpoint_every : nullptr);

@@ -27,7 +27,8 @@ namespace {
 struct Node {
     uint64_t mask = 0;  // its qubits
     int kind = 0;       // BlockGate kinds
-    int mat = -1;       // kind 0: its 2x2 matrix; kind 1: the target
+    int mat = -1;       // kind 0: its 2x2 matrix; kind 1: the target; kind 3: its occurrence
+    int axis = 0;       // kind 3
     int seg_begin = 0;  // its qubits in increasing order: segments seg_of_[seg_begin ..]
     float weight = 0.f;
 };
@@ -47,7 +48,7 @@ void matmul(const double* a, const double* b, double* out) {
 
 class BlockPlanner::Impl {
 public:
-    Impl(int n, const llg_op* ops, int nops, BlockPlan& out) : n_(n), out_(out) { build(ops, nops); }
+    Impl(int n, const llg_op* ops, int nops, bool params, BlockPlan& out) : n_(n), params_(params), out_(out) { build(ops, nops); }
 
     bool advance(int blocks) {
         const int goal = out_.blocks + blocks;
@@ -96,8 +97,20 @@ private:
             add_node(v, pdiag[q] ? v.mask : 0);
             pend[q] = -1;
         };
+        int occ = 0;
         for (int i = 0; i < nops; ++i) {
             const llg_op& op = ops[i];
+            if (params_ && op.param >= 0) {
+                flush(op.q0);
+                Node v;
+                v.kind = 3;
+                v.mask = 1ULL << op.q0;
+                v.mat = occ++;
+                v.axis = op.kind == LLG_OP_RX ? 0 : (op.kind == LLG_OP_RY ? 1 : 2);
+                v.weight = v.axis == 2 ? 0.5f : 1.0f;
+                add_node(v, v.axis == 2 ? v.mask : 0);
+                continue;
+            }
             if (is_single_qubit(op.kind)) {
                 M8 g;
                 op_matrix(op, g.m);
@@ -297,7 +310,11 @@ private:
         std::memset(&g, 0, sizeof(g));
         g.kind = v.kind;
         auto local = [&](int q) { return to_local ? to_local[q] : q; };
-        if (v.kind == 0) {
+        if (v.kind == 3) {
+            g.q0 = local(__builtin_ctzll(v.mask));
+            g.q1 = v.mat;
+            g.pad = v.axis;
+        } else if (v.kind == 0) {
             if (v.weight < 1.0f) ++out_.diag_1q;
             else ++out_.mixing_1q;
             g.q0 = local(__builtin_ctzll(v.mask));
@@ -329,8 +346,8 @@ private:
         for (int id : got_) finish(id);
         // up to three gates that only move amplitudes or signs run on their own: a CNOT or CZ pass
         // takes 2.6 ms at 30 qubits, a block 8.8
-        bool moves = got_.size() <= 3;
-        for (int id : got_) moves &= nodes_[id].kind != 0;
+        bool moves = !params_ && got_.size() <= 3;
+        for (int id : got_) moves = moves && nodes_[id].kind != 0;
         if (moves) {
             for (int id : got_) single(nodes_[id]);
             return;
@@ -355,6 +372,7 @@ private:
 
     static constexpr int kSeeds = 4;
     int n_;
+    bool params_;
     BlockPlan& out_;
     std::vector<M8> mats_;
     std::vector<Node> nodes_;
@@ -369,7 +387,7 @@ private:
     size_t first_ = 0;
 };
 
-BlockPlanner::BlockPlanner(int n, const llg_op* ops, int nops) : impl_(new Impl(n, ops, nops, plan)) {}
+BlockPlanner::BlockPlanner(int n, const llg_op* ops, int nops, bool params) : impl_(new Impl(n, ops, nops, params, plan)) {}
 BlockPlanner::~BlockPlanner() = default;
 bool BlockPlanner::advance(int blocks) { return impl_->advance(blocks); }
 

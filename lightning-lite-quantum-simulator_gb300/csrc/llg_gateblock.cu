@@ -41,7 +41,6 @@
 // two digits.
 // fp32 to integer without conversions (16 per clock and SM): diagonals 0 .. 4 are at most 2^22 in
 // size, so adding 1.5 2^23 leaves the integer in the low bits of the float.
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -49,21 +48,13 @@
 #include <type_traits>
 
 #include "llg_common.cuh"
+#include "llg_gateblock.cuh"
 #include "llg_internal.h"
 #include "llg_launch.h"
 
 namespace llg {
 
 namespace {
-
-constexpr int kGroups = 128;     // groups per tile (the MMA's M)
-constexpr int kAmps = 32;        // amplitudes per group
-constexpr int kChunks = 4;       // K steps of 16 reals (8 amplitudes) per tile
-constexpr int kRing = 5;         // chunk buffers
-constexpr int kSlicerWarps = 8;
-constexpr int kSliceBytes = kGroups * 16 * 2;  // one digit of one chunk
-constexpr int kTmemCols = 512;                 // two accumulator sets
-constexpr long kWaitLimit = 1L << 22;          // mbarrier polls before the kernel reports a timeout
 
 template <int P>
 struct Shape {
@@ -87,108 +78,6 @@ struct Shape {
                   "the roles' registers come out of the launch's");
     static_assert(kThreads / 128 * kLaunchRegs * 128 <= 65536, "one CTA's registers");
 };
-
-// setmaxnreg to kTo registers from kFrom (an increase must not name fewer than there are)
-template <int kFrom, int kTo>
-__device__ __forceinline__ void set_registers() {
-    if constexpr (kTo > kFrom) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTo));
-    else if constexpr (kTo < kFrom) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTo));
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// tcgen05 shared-memory descriptor, no swizzle (start, leading and stride byte offsets, version 1)
-__device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)((lbo >> 4) & 0x3FFF) << 16 | (uint64_t)((sbo >> 4) & 0x3FFF) << 32 |
-           (uint64_t)1 << 46;
-}
-
-// byte offset of element (row, c) of a rows x kreals fp16 operand: 8x8 cores of 128 bytes,
-// K-direction cores adjacent, 8-row groups kreals / 8 cores apart
-__device__ __forceinline__ uint32_t core_off(int row, int c, int kreals) {
-    return (uint32_t)((row >> 3) * (kreals / 8) * 128 + (c >> 3) * 128 + (row & 7) * 16 + (c & 7) * 2);
-}
-
-// Column (K index) of part p (0 real, 1 imaginary) of amplitude j: 16 (j >> 3) + 8 (j & 1) + 2 ((j >> 1) & 3) + p,
-// so that a slicer thread's four amplitudes of a chunk (j bit 0 fixed) fill one 8-wide core row.
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// Bounded wait for the completion of phase `ph`; false when the limit ran out here or in another
-// role (then *abort_s is set).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t ph, volatile int* abort_s) {
-    for (long it = 0; it < kWaitLimit; ++it) {
-        uint32_t done;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(done)
-                     : "r"(bar), "r"(ph)
-                     : "memory");
-        if (done) return true;
-        if ((it & 255) == 255 && *abort_s) return false;
-    }
-    *abort_s = 1;
-    return false;
-}
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t ph, volatile int* abort_s) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_s));
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// X = the 62-bit fixed-point integer of |x| against the group exponent eg (eg20 = eg 2^20 + 2^20 - 1;
-// a shift by 64 or more gives zero), plus the digit bias.  eg > 64: zeros and subnormals need no
-// care, their X is zero.
-__device__ __forceinline__ uint64_t fixed_f64(double x, uint32_t eg20) {
-    const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x);
-    const uint32_t s = (eg20 - (h & 0x7FFFFFFFu)) >> 20;
-    const uint32_t mh = (__funnelshift_l(l, h, 9) & 0x1FFFFFFFu) | 0x20000000u;
-    uint64_t X = ((uint64_t)mh << 32) | (l << 9);
-    asm("shr.u64 %0, %0, %1;" : "+l"(X) : "r"(s));
-    return X + 0x8080808080808080ULL;
-}
-// the same for any group exponent: a zero or subnormal has no hidden bit and exponent 1
-__device__ __noinline__ uint64_t fixed_f64_any(double x, int eg) {
-    const uint64_t b = (uint64_t)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFULL;
-    const int ex = (int)(b >> 52);
-    const uint64_t m = (b & 0xFFFFFFFFFFFFFULL) | (ex ? 1ULL << 52 : 0ULL);
-    return ((m << 9) >> min(eg - max(ex, 1), 63)) + 0x8080808080808080ULL;
-}
-
-__device__ __forceinline__ uint32_t h2_bits(__half2 v) {
-    uint32_t b;
-    memcpy(&b, &v, 4);
-    return b;
-}
-__device__ __forceinline__ __half2 h2_of(uint32_t b) {
-    __half2 v;
-    memcpy(&v, &b, 4);
-    return v;
-}
-
-// The first kCount of four digits (bytes 3 .. 0 of the biased words) of eight reals as fp16, one
-// 16-byte core row each; sgn: +-1 of each pair of reals, bias: -1152 sgn
-template <int kCount>
-__device__ __forceinline__ void digits4(const uint32_t (&w)[8], const __half2 (&sgn)[4], const __half2 (&bias)[4],
-                                        unsigned char* dst) {
-    uint32_t v[4][4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        const uint32_t t = __byte_perm(w[2 * p], w[2 * p + 1], 0x6273);
-        const uint32_t u = __byte_perm(w[2 * p], w[2 * p + 1], 0x4051);
-        v[0][p] = h2_bits(__hfma2(h2_of(__byte_perm(t, 0x64646464u, 0x4140)), sgn[p], bias[p]));
-        v[1][p] = h2_bits(__hfma2(h2_of(__byte_perm(t, 0x64646464u, 0x4342)), sgn[p], bias[p]));
-        v[2][p] = h2_bits(__hfma2(h2_of(__byte_perm(u, 0x64646464u, 0x4140)), sgn[p], bias[p]));
-        v[3][p] = h2_bits(__hfma2(h2_of(__byte_perm(u, 0x64646464u, 0x4342)), sgn[p], bias[p]));
-    }
-#pragma unroll
-    for (int k = 0; k < kCount; ++k)
-        *reinterpret_cast<uint4*>(dst + k * kSliceBytes) = make_uint4(v[k][0], v[k][1], v[k][2], v[k][3]);
-}
 
 // 2^e as a float for e in [-126, 127]
 __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
@@ -214,12 +103,24 @@ struct Elem<LLG_DF64> {
 
 // `mirror` (nullptr: none): the device address of a mapped host buffer that also receives the
 // output as FP64.
-// kRows: the gate's rows have exponents of their own (any matrix); else all have exponent 1 (a product
+// A batch of states: row y of the grid is set y mod `sets`, whose state is 2^n elements from the
+// first one's (the next `sets` rows: from `second`) and whose weights are `wstride` 16-byte words from
+// the first set's.  max_exp (nullptr: none): per row, raised to the largest biased exponent stored (FP64).
+template <int P>
+struct BlockBatch {
+    typename Elem<P>::S* second;
+    int sets;
+    uint64_t wstride;
+    uint32_t* max_exp;
+};
+
+// kRows: the gate's rows have exponents of their own (any matrix); else all have exponent 0 (a product
 // of unitary gates, entries at most 1).
 template <int P, bool kRows>
 __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
     k_gate_block(typename Elem<P>::S* __restrict__ psi, int n, const __grid_constant__ TargetOffsets to, uint64_t tmask,
-                 const uint4* __restrict__ weights, bool weights_ready, int* __restrict__ err_flag, double2* __restrict__ mirror) {
+                 const uint4* __restrict__ weights, bool weights_ready, int* __restrict__ err_flag, double2* __restrict__ mirror,
+                 BlockBatch<P> batch) {
     using T = Shape<P>;
     constexpr int S = T::S;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -238,6 +139,9 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
     const uint32_t accfull0 = smem_u32(&bars[2 * kRing]), accempty0 = smem_u32(&bars[2 * kRing + 2]);
     const uint32_t egfull0 = smem_u32(&bars[2 * kRing + 4]), drain = smem_u32(&bars[2 * kRing + 7]);
 
+    const int row_y = blockIdx.y, set_y = row_y % batch.sets;
+    psi = (row_y < batch.sets ? psi : batch.second) + ((uint64_t)set_y << n);
+    weights += set_y * batch.wstride;
     if (tid < kAmps) toff[tid] = to.o[tid];
     // Launched while the previous kernel of the stream runs: everything up to the wait below touches
     // nothing that it writes (the weights only if they were ready before it began).
@@ -420,7 +324,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
         if (kRows)
             for (int r = 0; r < 64; ++r) erm = max(erm, abs(er_s[r]));
         int egb = 0;
-        uint32_t phase = 0, egphase = 0;
+        uint32_t phase = 0, egphase = 0, largest = 0;
         bool ok = true;
         for (uint64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, phase ^= 1) {
             const uint64_t base = insert0_mask(tile * kGroups + (uint64_t)row, tmask) | toff[T::kStep * e];
@@ -466,7 +370,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                     typename Elem<P>::S out[T::kStep / 2];
 #pragma unroll
                     for (int c = 0; c < T::kStep; ++c) {
-                        const int er = kRows ? er_s[32 * half + col + c] : 1;
+                        const int er = kRows ? er_s[32 * half + col + c] : 0;
                         if constexpr (P == LLG_F64) {
                             // 2^44 sum_d 2^(-8 d) D_d: D_0 .. D_4 exact, D_5 .. D_7 rounded to an integer
                             const float magic = 12582912.0f;
@@ -495,6 +399,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                             } else {
                                 r = scale_slow(r, et);
                             }
+                            if (batch.max_exp) largest = max(largest, (uint32_t)__double2hiint(r) & 0x7FFFFFFFu);
                             if (c & 1) out[c >> 1].y = r;
                             else out[c >> 1].x = r;
                         } else {
@@ -544,6 +449,10 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                     }
                 }
             }
+        }
+        if (batch.max_exp) {
+            largest = __reduce_max_sync(0xffffffffu, largest);
+            if (lane == 0) atomicMax(batch.max_exp + row_y, largest >> 20);
         }
     } else {
         set_registers<T::kLaunchRegs, T::kMmaRegs>();
@@ -647,71 +556,28 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
 // by 64 columns in core-matrix order, then 64 row exponents.
 
 // A CTA cuts the eight input amplitudes (16 columns) of one K chunk, blockIdx.y, of one block,
-// blockIdx.x.  kMatrix: the matrix m (row-major, in the order of the sorted targets), any finite
-// entries; else the product of the block's gates, run on the identity's columns in shared memory.
-template <int S, bool kMatrix>
-__global__ void __launch_bounds__(128)
-    k_weights(const double2* __restrict__ m, const BlockGate* __restrict__ gates, const BlockStep* __restrict__ steps,
-              unsigned char* __restrict__ wt, size_t stride) {
-    __shared__ double2 M[kAmps][9];
-    __shared__ int eg_s[kAmps];
-    const int tid = threadIdx.x, ks = blockIdx.y, c = tid & 7, p = tid >> 3;
-    wt += blockIdx.x * stride;
-    if constexpr (kMatrix) {
-        for (int r = p; r < kAmps; r += 16) M[r][c] = m[r * kAmps + 8 * ks + c];
-        if (tid < kAmps) {
-            // both real rows of an output hold the same magnitudes
-            uint32_t mx = 0;
-            for (int j = 0; j < kAmps; ++j) {
-                const double2 v = m[tid * kAmps + j];
-                mx = max(mx, max((uint32_t)__double2hiint(v.x) & 0x7FFFFFFFu, (uint32_t)__double2hiint(v.y) & 0x7FFFFFFFu));
-            }
-            eg_s[tid] = max((int)(mx >> 20), 1);
-        }
-    } else {
-        for (int r = p; r < kAmps; r += 16) M[r][c] = make_double2(r == 8 * ks + c ? 1.0 : 0.0, 0.0);
-        if (tid < kAmps) eg_s[tid] = 1023;  // entries below 2
-        __syncthreads();
-        const BlockStep st = steps[blockIdx.x];
-        for (int g = 0; g < st.ngates; ++g) {
-            const BlockGate& o = gates[st.gate_begin + g];
-            if (o.kind == 0) {
-                const int b = o.q0, r0 = ((p >> b) << (b + 1)) | (p & ((1 << b) - 1)), r1 = r0 | 1 << b;
-                const double2 x = M[r0][c], y = M[r1][c];
-                M[r0][c] = make_double2(fma(o.m[0], x.x, fma(-o.m[1], x.y, fma(o.m[2], y.x, -o.m[3] * y.y))),
-                                        fma(o.m[0], x.y, fma(o.m[1], x.x, fma(o.m[2], y.y, o.m[3] * y.x))));
-                M[r1][c] = make_double2(fma(o.m[4], x.x, fma(-o.m[5], x.y, fma(o.m[6], y.x, -o.m[7] * y.y))),
-                                        fma(o.m[4], x.y, fma(o.m[5], x.x, fma(o.m[6], y.y, o.m[7] * y.x))));
-            } else if (o.kind == 1) {
-                if (p < 8) {
-                    const int r = (int)insert0_mask((uint64_t)p, 1ULL << o.q0 | 1ULL << o.q1) | 1 << o.q0, r1 = r | 1 << o.q1;
-                    const double2 x = M[r][c];
-                    M[r][c] = M[r1][c];
-                    M[r1][c] = x;
-                }
-            } else {
-                for (int r = p; r < kAmps; r += 16)
-                    if ((r & (int)o.mask) == (int)o.mask) M[r][c] = make_double2(-M[r][c].x, -M[r][c].y);
-            }
-            __syncthreads();
-        }
-    }
-    __syncthreads();
-    // this thread: real output row `row` (2 jo + po), one core row of inputs j = 8 ks + 2 i + h
-    const int row = tid >> 1, h = tid & 1, jo = row >> 1, po = row & 1, eg = eg_s[jo];
+// blockIdx.x.  k_weights_matrix: the matrix m (row-major, in the order of the sorted targets), any finite
+// entries.  k_weights_gates: the product of the block's gates, run on the identity's columns in shared
+// memory in 64-bit fixed point (units of 2^-62, every 2x2 product rounded once from 128 bits): ten bits
+// closer than FP64 where an error would repeat in every group, and faster here than FP64's two
+// multiply-adds a clock and SM.  Gates of kind 3 take (cos, sin) of their half angle from `angles`, nocc
+// entries a set, blockIdx.z the set; inverse: the inverse product (the gates' inverses, last first).
+
+// Thread tid's core row: real output row tid / 2 (2 jo + po), inputs j = 8 ks + 2 i + h with h = tid & 1.
+// x: the biased fixed-point magnitudes of its eight reals, neg: their signs in bit 31
+template <int S>
+__device__ __forceinline__ void put_core_row(unsigned char* wt, int ks, const uint64_t (&x)[8], const uint32_t (&neg)[8], int er) {
+    const int row = threadIdx.x >> 1, h = threadIdx.x & 1;
     uint32_t wh[8], wl[8];
     __half2 sgn[4], bias[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const double2 v = M[jo][2 * i + h];
-        const double w[2] = {po ? v.y : v.x, po ? v.x : -v.y};  // real part in, imaginary part in
+    for (int i = 0; i < 8; ++i) {
+        wh[i] = (uint32_t)(x[i] >> 32);
+        wl[i] = (uint32_t)x[i];
+    }
 #pragma unroll
-        for (int pi = 0; pi < 2; ++pi) {
-            const uint64_t X = fixed_f64_any(w[pi], eg);
-            wh[2 * i + pi] = (uint32_t)(X >> 32);
-            wl[2 * i + pi] = (uint32_t)X;
-        }
-        const uint32_t sg = __byte_perm((uint32_t)__double2hiint(w[0]), (uint32_t)__double2hiint(w[1]), 0x7733);
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t sg = __byte_perm(neg[2 * i], neg[2 * i + 1], 0x7733);
         sgn[i] = h2_of((sg & 0x80008000u) | 0x3C003C00u);
         bias[i] = __hmul2(sgn[i], __half2half2(__ushort_as_half(0xE480)));
     }
@@ -719,7 +585,99 @@ __global__ void __launch_bounds__(128)
     static_assert(kSliceBytes == 32 * 64 * 2, "a digit's 32 rows are kSliceBytes apart");
     digits4<4>(wh, sgn, bias, dst);
     digits4<S - 4>(wl, sgn, bias, dst + 4 * kSliceBytes);
-    if (ks == 0 && h == 0) reinterpret_cast<int32_t*>(wt + 2 * (S * 32 * 64 * 2))[row] = eg - 1022;
+    if (ks == 0 && h == 0) reinterpret_cast<int32_t*>(wt + 2 * (S * 32 * 64 * 2))[row] = er;
+}
+
+template <int S>
+__global__ void __launch_bounds__(128) k_weights_matrix(const double2* __restrict__ m, unsigned char* __restrict__ wt) {
+    __shared__ int eg_s[kAmps];
+    const int tid = threadIdx.x, ks = blockIdx.y;
+    if (tid < kAmps) {
+        // both real rows of an output hold the same magnitudes
+        uint32_t mx = 0;
+        for (int j = 0; j < kAmps; ++j) {
+            const double2 v = m[tid * kAmps + j];
+            mx = max(mx, max((uint32_t)__double2hiint(v.x) & 0x7FFFFFFFu, (uint32_t)__double2hiint(v.y) & 0x7FFFFFFFu));
+        }
+        eg_s[tid] = max((int)(mx >> 20), 1);
+    }
+    __syncthreads();
+    const int row = tid >> 1, h = tid & 1, jo = row >> 1, po = row & 1, eg = eg_s[jo];
+    uint64_t x[8];
+    uint32_t neg[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double2 v = m[jo * kAmps + 8 * ks + 2 * i + h];
+        const double w[2] = {po ? v.y : v.x, po ? v.x : -v.y};  // real part in, imaginary part in
+#pragma unroll
+        for (int pi = 0; pi < 2; ++pi) {
+            x[2 * i + pi] = fixed_f64_any(w[pi], eg);
+            neg[2 * i + pi] = (uint32_t)__double2hiint(w[pi]);
+        }
+    }
+    put_core_row<S>(wt, ks, x, neg, eg - 1022);
+}
+
+template <int S>
+__global__ void __launch_bounds__(128)
+    k_weights_gates(const BlockGate* __restrict__ gates, const BlockStep* __restrict__ steps, const double2* __restrict__ angles,
+                    int nocc, bool inverse, unsigned char* __restrict__ wt, size_t stride) {
+    constexpr int kStage = 32;  // gates whose coefficients are in shared memory
+    __shared__ Fixed2 M[kAmps][9];
+    __shared__ Fixed2 coef[kStage][4];  // 2x2 matrices, row-major
+    __shared__ int4 what[kStage];       // kind, q0, q1, mask
+    const int tid = threadIdx.x, ks = blockIdx.y, c = tid & 7, p = tid >> 3;
+    wt += ((size_t)blockIdx.x * gridDim.z + blockIdx.z) * stride;
+    constexpr int64_t one = (int64_t)1 << 62;
+    for (int r = p; r < kAmps; r += 16) M[r][c] = {r == 8 * ks + c ? one : 0, 0};
+    const BlockStep st = steps[blockIdx.x];
+    for (int k0 = 0; k0 < st.ngates; k0 += kStage) {
+        const int cnt = min(kStage, st.ngates - k0);
+        __syncthreads();
+        // thread: entry (tid & 3) of gate tid / 4
+        if (tid / 4 < cnt) {
+            const int k = k0 + tid / 4, e = tid & 3;
+            const BlockGate& o = gates[st.gate_begin + (inverse ? st.ngates - 1 - k : k)];
+            coef[tid / 4][e] = gate_entry(o, e, o.kind == 3 ? angles[(size_t)blockIdx.z * nocc + o.q1] : make_double2(0.0, 0.0), inverse);
+            if (e == 0) what[tid / 4] = make_int4(o.kind, o.q0, o.q1, (int)o.mask);
+        }
+        __syncthreads();
+        for (int k = 0; k < cnt; ++k) {
+            const int4 o = what[k];
+            if (o.x == 0 || o.x == 3) {
+                const int b = o.y, r0 = ((p >> b) << (b + 1)) | (p & ((1 << b) - 1)), r1 = r0 | 1 << b;
+                const Fixed2 x = M[r0][c], y = M[r1][c];
+                M[r0][c] = mix(coef[k][0], x, coef[k][1], y);
+                M[r1][c] = mix(coef[k][2], x, coef[k][3], y);
+            } else if (o.x == 1) {
+                if (p < 8) {
+                    const int r = (int)insert0_mask((uint64_t)p, 1ULL << o.y | 1ULL << o.z) | 1 << o.y, r1 = r | 1 << o.z;
+                    const Fixed2 x = M[r][c];
+                    M[r][c] = M[r1][c];
+                    M[r1][c] = x;
+                }
+            } else {
+                for (int r = p; r < kAmps; r += 16)
+                    if ((r & o.w) == o.w) M[r][c] = {-M[r][c].x, -M[r][c].y};
+            }
+            __syncthreads();
+        }
+    }
+    __syncthreads();
+    const int row = tid >> 1, h = tid & 1, jo = row >> 1, po = row & 1;
+    uint64_t x[8];
+    uint32_t neg[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const Fixed2 v = M[jo][2 * i + h];
+        const int64_t w[2] = {po ? v.y : v.x, po ? v.x : -v.y};  // real part in, imaginary part in
+#pragma unroll
+        for (int pi = 0; pi < 2; ++pi) {
+            x[2 * i + pi] = (uint64_t)(w[pi] < 0 ? -w[pi] : w[pi]) + 0x8080808080808080ULL;
+            neg[2 * i + pi] = (uint32_t)((uint64_t)w[pi] >> 32);
+        }
+    }
+    put_core_row<S>(wt, ks, x, neg, 0);
 }
 
 int sm_count() {
@@ -729,8 +687,10 @@ int sm_count() {
     return sms;
 }
 
+// ctas: CTAs a state (0: one per SM); sets states from psi and, unless nullptr, as many from `second`
 template <int P, bool kRows>
-cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool ready, int* err, cudaStream_t s, double* mirror) {
+cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool ready, int* err, cudaStream_t s, double* mirror,
+                   int ctas, void* second, int sets, uint32_t* max_exp) {
     using T = Shape<P>;
     static const cudaError_t attr =
         cudaFuncSetAttribute(k_gate_block<P, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmem);
@@ -741,21 +701,22 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool re
         for (int b = 0; b < 5; ++b)
             if ((j >> b) & 1) to.o[j] |= 1ULL << bd.q[b];
     }
-    const uint64_t ntiles = (1ULL << (n - 5)) / kGroups, sms = (uint64_t)sm_count();
+    const uint64_t ntiles = (1ULL << (n - 5)) / kGroups, most = ctas > 0 ? (uint64_t)ctas : (uint64_t)sm_count();
     // programmatic dependent launch: the CTA's set-up (barriers, tensor memory, the gate's digits)
     // runs under the end of the stream's previous kernel
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(ntiles < sms ? ntiles : sms));
+    cfg.gridDim = dim3((unsigned)(ntiles < most ? ntiles : most), (unsigned)(second ? 2 * sets : sets));
     cfg.blockDim = dim3(T::kThreads);
     cfg.dynamicSmemBytes = T::kSmem;
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_gate_block<P, kRows>, static_cast<typename Elem<P>::S*>(psi), n, to, bd.tmask,
-                              static_cast<const uint4*>(w), ready, err, reinterpret_cast<double2*>(mirror));
+                              static_cast<const uint4*>(w), ready, err, reinterpret_cast<double2*>(mirror),
+                              BlockBatch<P>{static_cast<typename Elem<P>::S*>(second), sets, gate_block_weight_bytes(P) / 16, max_exp});
 }
 
 }  // namespace
@@ -777,17 +738,17 @@ size_t gate_block_weight_bytes(int P) {
 
 cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weights, cudaStream_t s) {
     return by_precision(P, [&](auto p) {
-        k_weights<Shape<decltype(p)::value>::S, true><<<dim3(1, kChunks), 128, 0, s>>>(
-            reinterpret_cast<const double2*>(d_matrix), nullptr, nullptr, static_cast<unsigned char*>(d_weights), 0);
+        k_weights_matrix<Shape<decltype(p)::value>::S><<<dim3(1, kChunks), 128, 0, s>>>(
+            reinterpret_cast<const double2*>(d_matrix), static_cast<unsigned char*>(d_weights));
         return cudaGetLastError();
     });
 }
 
 cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const BlockStep* d_steps, int nblocks, void* d_weights,
-                                      cudaStream_t s) {
+                                      cudaStream_t s, const double2* d_angles, int nocc, int sets, bool inverse) {
     return by_precision(P, [&](auto p) {
-        k_weights<Shape<decltype(p)::value>::S, false><<<dim3((unsigned)nblocks, kChunks), 128, 0, s>>>(
-            nullptr, d_gates, d_steps, static_cast<unsigned char*>(d_weights), gate_block_weight_bytes(P));
+        k_weights_gates<Shape<decltype(p)::value>::S><<<dim3((unsigned)nblocks, kChunks, (unsigned)sets), 128, 0, s>>>(
+            d_gates, d_steps, d_angles, nocc, inverse, static_cast<unsigned char*>(d_weights), gate_block_weight_bytes(P));
         return cudaGetLastError();
     });
 }
@@ -796,9 +757,14 @@ cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, cons
                               int* err_flag, cudaStream_t s, double* mirror) {
     return by_precision(P, [&](auto p) {
         constexpr int PP = decltype(p)::value;
-        return rows ? launch<PP, true>(psi, n, bd, d_weights, ready, err_flag, s, mirror)
-                    : launch<PP, false>(psi, n, bd, d_weights, ready, err_flag, s, mirror);
+        return rows ? launch<PP, true>(psi, n, bd, d_weights, ready, err_flag, s, mirror, 0, nullptr, 1, nullptr)
+                    : launch<PP, false>(psi, n, bd, d_weights, ready, err_flag, s, mirror, 0, nullptr, 1, nullptr);
     });
+}
+
+cudaError_t launch_gate_block_batch(void* psi, void* second, int sets, int ctas, int n, const BlockDesc& bd,
+                                    const void* d_weights, bool ready, uint32_t* max_exp, int* err_flag, cudaStream_t s) {
+    return launch<LLG_F64, false>(psi, n, bd, d_weights, ready, err_flag, s, nullptr, ctas, second, sets, max_exp);
 }
 
 }  // namespace llg

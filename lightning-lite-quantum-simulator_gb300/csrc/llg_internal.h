@@ -190,7 +190,10 @@ int32_t reg_dispatch_code(const ExecOp& x);
 
 // A plan of dense 5-qubit blocks (llg_blockplan.cpp) for 16-byte states of 12 and more qubits.
 struct BlockGate {
-    int32_t kind;  // 0: 2x2 matrix m on q0; 1: CNOT, control q0, target q1; 2: sign flip where all of `mask` is set
+    // 0: 2x2 matrix m on q0; 1: CNOT, control q0, target q1; 2: sign flip where all of `mask` is set;
+    // 3 (with parameters only): rotation exp(-i theta P / 2) on q0, P = X, Y, Z for pad = 0, 1, 2, theta
+    // the q1-th parametrised gate's angle
+    int32_t kind;
     int32_t q0, q1, pad;
     uint64_t mask;
     double m[8];
@@ -208,7 +211,7 @@ struct BlockPlan {
     int blocks = 0;
     int mixing_1q = 0, diag_1q = 0;  // merged one-qubit gates among `gates`, for the cost of other plans
 };
-// 2x2 gates of a block have spectral norm at most this, so that its entries stay below 2
+// 2x2 gates of a block have spectral norm at most this, so that its entries stay well below 2
 constexpr double kBlockNormLimit = 1.0 + 1e-6;
 double spectral_norm_2x2(const double* m);
 // false: no block plan (fewer than 12 qubits, or a 2x2 beyond the norm limit)
@@ -217,7 +220,9 @@ bool has_block_plan(int n, const llg_op* ops, int nops);
 // the constructor only.
 class BlockPlanner {
 public:
-    BlockPlanner(int n, const llg_op* ops, int nops);
+    // params: rotations with param >= 0 stay gates of their own (kind 3) and every step is a block; the
+    // list must have no sign flip on more than five qubits
+    BlockPlanner(int n, const llg_op* ops, int nops, bool params = false);
     ~BlockPlanner();
     bool advance(int blocks);  // appends up to `blocks` blocks to `plan`; false: the list is done
     BlockPlan plan;
