@@ -17,8 +17,10 @@
 // two of X's digits fill the MMA's M = 128 (rows 0-63 digit 2 p, rows 64-127 digit 2 p + 1), up to four of
 // Y's its N = 256, and the columns 64 e of the accumulators collect the pairs with 2 p + j = e: diagonal
 // e in the low rows, e + 1 in the high ones.  128 groups give integers below 2^24, exact in fp32; the
-// epilogue adds them to 64-bit integers (unit 2^-52 of the two scales' product, at most 16 tiles: 2^63)
-// and converts once per CTA.  In FP64 the sum would take 128 multiply-adds per amplitude, 0.2 ms per 2^20.
+// epilogue adds them to 64-bit integers, each tile's sum rounded to what keeps the total from overflowing:
+// 2^-62 of a bound on |psi| |lambda| (by Cauchy and Schwarz no part of a sum is larger; this serves states
+// that sit in a few amplitudes) or 2^-62 of the CTA's groups at full scale, whichever is finer.  The CTAs' sums are added in 128 bits, and R is a
+// pair of doubles.  In FP64 the sum would take 128 multiply-adds per amplitude, 0.2 ms per 2^20.
 //
 // What bounds k_cross: 32 bytes per amplitude pair against 20 digit products of M128 N64 K128 per 128
 // groups (5120 clocks of the tensor pipe) and 65536 accumulators read back for each.  The accumulators
@@ -27,6 +29,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #include "llg_adjblock.h"
 #include "llg_common.cuh"
@@ -45,7 +48,6 @@ constexpr int kDigitBytes = kRGroups * 64 * 2;             // one digit of one v
 constexpr int kVecBytes = kDigits * kDigitBytes;           // 16 KB
 constexpr int kRChunkBytes = 2 * kVecBytes;                // psi, lambda
 constexpr int kTileChunks = kGroups / kRGroups;            // 8 chunks per drain of the accumulators
-constexpr int kMaxTiles = 16;                              // per CTA: the 64-bit sums hold no more
 constexpr int kDepth = 4;                                  // chunks whose loads are in flight
 constexpr int kREpiWarps = 8;
 constexpr int kRMmaWarp = kSlicerWarps + kREpiWarps;
@@ -59,11 +61,19 @@ struct CrossOffsets {
     uint64_t o[kAmps];
 };
 
+// the biased exponent that a vector's digits are cut against, from its largest one (zero vector: any scale)
+__device__ __forceinline__ uint32_t cut_exponent(uint32_t e) { return e == 0 ? 1023u : max(e, 128u); }
+// right shift of the tiles' sums (units of 2^-56 of the two scales' product), see above; `tiles` per CTA
+__device__ __forceinline__ int cross_shift(int log2_bound, int tiles, uint32_t e0, uint32_t e1) {
+    return max(min(log2_bound - 6 + 2044 - (int)e0 - (int)e1, 33 - __clz(tiles)), 0);
+}
+
 // exps: per set the largest biased exponents of psi and (sets further on) lambda.  partial: per set and
-// CTA 32 x 32 complex sums in units of 2^(e_psi + e_lambda - 2096).
+// CTA 32 x 32 complex sums in units of 2^(e_psi + e_lambda - 2100 + cross_shift).  log2_bound: of |psi| |lambda|;
+// tiles: at most this many for a CTA.
 __global__ void __launch_bounds__(kRThreads, 1)
     k_cross(const double2* __restrict__ psi, const double2* __restrict__ lam, int n, const __grid_constant__ CrossOffsets to,
-            uint64_t tmask, const uint32_t* __restrict__ exps, double2* __restrict__ partial, int* __restrict__ err_flag) {
+            uint64_t tmask, int log2_bound, int tiles, const uint32_t* __restrict__ exps, Fixed2* __restrict__ partial, int* __restrict__ err_flag) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t coff[kTileChunks];  // element offset of a tile's chunks
     __shared__ __align__(8) uint64_t bars[2 * kRRing + 3];
@@ -96,15 +106,14 @@ __global__ void __launch_bounds__(kRThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_s;
     const uint64_t ntiles = (1ULL << (n - 5)) / kGroups;
-    const int mine = (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // tiles of this CTA, 1 .. kMaxTiles
+    const int mine = (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // tiles of this CTA, at least 1
     const int chunks = mine * kTileChunks;
 
     if (warp < kSlicerWarps) {
         set_registers<kRLaunchRegs, kRSlicerRegs>();
         // ---- slicers: warps 0-3 psi, 4-7 lambda; group g of the chunk, amplitudes j = h + 2 i + 8 u ----
         const int vec = warp >> 2, u = warp & 3, g = lane & 15, h = lane >> 4;
-        const uint32_t e = exps[vec * gridDim.y + set];
-        const uint32_t eg = e == 0 ? 1023u : max(e, 128u);  // a zero vector: any scale
+        const uint32_t eg = cut_exponent(exps[vec * gridDim.y + set]);
         const uint32_t eg20 = (eg << 20) | 0xFFFFFu;
         const double2* src = (vec ? lam : psi) + ((uint64_t)set << n) +
                              (insert0_mask((uint64_t)g, tmask) | (h ? to.o[1] : 0) | (u & 1 ? to.o[8] : 0) | (u & 2 ? to.o[16] : 0));
@@ -161,17 +170,19 @@ __global__ void __launch_bounds__(kRThreads, 1)
         // ---- epilogue: rows 32 (warp & 3) + lane, columns 32 e .. +31 ----
         const int row = 32 * (warp & 3) + lane, e = (warp - kSlicerWarps) >> 2;
         const uint32_t tbase = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * e);
-        uint64_t acc[32];
+        const int shift = cross_shift(log2_bound, tiles, cut_exponent(exps[set]), cut_exponent(exps[gridDim.y + set]));
+        const int64_t half = shift ? (int64_t)1 << (shift - 1) : 0;
+        int64_t acc[32];
 #pragma unroll
         for (int c = 0; c < 32; ++c) acc[c] = 0;
-        uint32_t phase = 0;
-        bool ok = true;
-        for (int t = 0; t < mine; ++t, phase ^= 1) {
-            if (!warp_wait(accfull, phase, abort_s)) {
-                ok = false;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // a tile's sums in units of 2^-56: sum_e 2^(44 - 8 e) P_e in the low rows, 2^(36 - 8 e) in the high
+        // ones (odd digits), whose lowest terms are rounded at once.  |P_0 .. P_3| <= 2^22: the integer is in
+        // the low bits of the float plus 1.5 2^23
+        auto add_tile = [&](auto odd) {
+            constexpr bool kOdd = decltype(odd)::value;
+            constexpr uint64_t kM = 0x4B400000ULL;
+            constexpr uint64_t kC = kOdd ? kM * ((1ULL << 28) + (1ULL << 20) + (1ULL << 12)) + (kM << 36)
+                                         : kM * ((1ULL << 28) + (1ULL << 20)) + (kM * ((1ULL << 12) + (1ULL << 4)) << 32);
 #pragma unroll
             for (int cg = 0; cg < 8; ++cg) {
                 uint32_t v[kDigits][4];
@@ -188,41 +199,59 @@ __global__ void __launch_bounds__(kRThreads, 1)
                 }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    // sum_e 2^(40 - 8 e) P_e.  |P_0 .. P_3| <= 2^22: the integer is in the float's low bits
                     const float magic = 12582912.0f;
                     const uint32_t b0 = __float_as_uint(__fadd_rn(__uint_as_float(v[0][c]), magic));
                     const uint32_t b1 = __float_as_uint(__fadd_rn(__uint_as_float(v[1][c]), magic));
                     const uint32_t b2 = __float_as_uint(__fadd_rn(__uint_as_float(v[2][c]), magic));
                     const uint32_t b3 = __float_as_uint(__fadd_rn(__uint_as_float(v[3][c]), magic));
                     const int b4 = __float2int_rn(__uint_as_float(v[4][c]));
-                    const int low = __float2int_rn(fmaf(__uint_as_float(v[7][c]), 0x1p-16f,
-                                                        fmaf(__uint_as_float(v[6][c]), 0x1p-8f, __uint_as_float(v[5][c]))));
-                    constexpr uint64_t kM = 0x4B400000ULL;
-                    constexpr uint64_t kC = kM * ((1ULL << 24) + (1ULL << 16)) + (kM * ((1ULL << 8) + 1ULL) << 32);
+                    const int low = __float2int_rn(fmaf(__uint_as_float(v[7][c]), kOdd ? 0x1p-20f : 0x1p-12f,
+                                                        fmaf(__uint_as_float(v[6][c]), kOdd ? 0x1p-12f : 0x1p-4f,
+                                                             __uint_as_float(v[5][c]) * (kOdd ? 0x1p-4f : 0x1p4f))));
                     uint64_t s = (uint64_t)(int64_t)low - kC;
-                    asm("mad.wide.s32 %0, %1, 256, %0;" : "+l"(s) : "r"(b4));
-                    asm("mad.wide.u32 %0, %1, 65536, %0;" : "+l"(s) : "r"(b3));
-                    asm("mad.wide.u32 %0, %1, 16777216, %0;" : "+l"(s) : "r"(b2));
-                    s += (uint64_t)((b0 << 8) + b1) << 32;
-                    acc[4 * cg + c] += s;
+                    if constexpr (kOdd) {
+                        asm("mad.wide.s32 %0, %1, 16, %0;" : "+l"(s) : "r"(b4));
+                        asm("mad.wide.u32 %0, %1, 4096, %0;" : "+l"(s) : "r"(b3));
+                        asm("mad.wide.u32 %0, %1, 1048576, %0;" : "+l"(s) : "r"(b2));
+                        asm("mad.wide.u32 %0, %1, 268435456, %0;" : "+l"(s) : "r"(b1));
+                        s += (uint64_t)(b0 << 4) << 32;
+                    } else {
+                        asm("mad.wide.s32 %0, %1, 4096, %0;" : "+l"(s) : "r"(b4));
+                        asm("mad.wide.u32 %0, %1, 1048576, %0;" : "+l"(s) : "r"(b3));
+                        asm("mad.wide.u32 %0, %1, 268435456, %0;" : "+l"(s) : "r"(b2));
+                        s += (uint64_t)((b0 << 12) + (b1 << 4)) << 32;
+                    }
+                    // the rounding bit apart: s alone may be near 2^63
+                    acc[4 * cg + c] += ((int64_t)s >> shift) + (int64_t)(((int64_t)s & half) != 0);
                 }
             }
+        };
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int t = 0; t < mine; ++t, phase ^= 1) {
+            if (!warp_wait(accfull, phase, abort_s)) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (warp & 2) add_tile(std::true_type());
+            else add_tile(std::false_type());
         }
         // ---- the CTA's 32 x 32 sums, through the ring (every product has been read) ----
-        double* D = reinterpret_cast<double*>(smem);  // [row][64]
+        int64_t* D = reinterpret_cast<int64_t*>(smem);  // [row][64]
         if (ok) {
 #pragma unroll
-            for (int c = 0; c < 32; ++c) D[row * 64 + 32 * e + c] = (double)(long long)acc[c];
+            for (int c = 0; c < 32; ++c) D[row * 64 + 32 * e + c] = acc[c];
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kREpiWarps * 32) : "memory");
         if (ok) {
-            double2* out = partial + ((size_t)set * gridDim.x + blockIdx.x) * kAmps * kAmps;
-            auto real = [&](int r, int c) { return fma(D[(r + 64) * 64 + c], 0x1p-8, D[r * 64 + c]); };
+            Fixed2* out = partial + ((size_t)set * gridDim.x + blockIdx.x) * kAmps * kAmps;
+            auto real = [&](int r, int c) { return D[r * 64 + c] + D[(r + 64) * 64 + c]; };
             for (int k = tid - kSlicerWarps * 32; k < kAmps * kAmps; k += kREpiWarps * 32) {
                 const int ja = k >> 5, jb = k & 31;
                 const int ra = 16 * (ja >> 3) + 8 * (ja & 1) + 2 * ((ja >> 1) & 3);
                 const int cb = 16 * (jb >> 3) + 8 * (jb & 1) + 2 * ((jb >> 1) & 3);
-                out[k] = make_double2(real(ra, cb) + real(ra + 1, cb + 1), real(ra + 1, cb) - real(ra, cb + 1));
+                out[k] = {real(ra, cb) + real(ra + 1, cb + 1), real(ra + 1, cb) - real(ra, cb + 1)};
             }
         }
     } else {
@@ -295,23 +324,34 @@ __global__ void __launch_bounds__(kRThreads, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// The CTAs' sums in a fixed order, scaled: R of set blockIdx.y.  NaN where a vector held one or an infinity.
+// s 2^e as a double and what is left of it, as a double
+__device__ __forceinline__ double2 pair_of(__int128 s, int e) {
+    const double hi = (double)s;
+    return make_double2(ldexp(hi, e), ldexp((double)(int64_t)(s - (__int128)hi), e));
+}
+
+// The CTAs' sums added exactly and scaled: R of set blockIdx.y, the high parts of its 32 x 32 entries, then
+// the low ones.  NaN where a vector held one or an infinity.
 __global__ void __launch_bounds__(128)
-    k_cross_sum(const double2* __restrict__ partial, int ctas, const uint32_t* __restrict__ exps, double2* __restrict__ R) {
+    k_cross_sum(const Fixed2* __restrict__ partial, int ctas, int log2_bound, int tiles, const uint32_t* __restrict__ exps,
+                double2* __restrict__ R) {
     const int set = blockIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
-    const double2* p = partial + (size_t)set * ctas * kAmps * kAmps + k;
-    double re = 0.0, im = 0.0;
+    const longlong2* p = reinterpret_cast<const longlong2*>(partial) + (size_t)set * ctas * kAmps * kAmps + k;
+    __int128 re = 0, im = 0;
 #pragma unroll 4
     for (int c = 0; c < ctas; ++c) {
-        const double2 v = __ldcg(p + (size_t)c * kAmps * kAmps);
+        const longlong2 v = __ldcg(p + (size_t)c * kAmps * kAmps);
         re += v.x;
         im += v.y;
     }
     const uint32_t e0 = exps[set], e1 = exps[gridDim.y + set];
-    const int e = (e0 == 0 ? 1023 : (int)max(e0, 128u)) + (e1 == 0 ? 1023 : (int)max(e1, 128u)) - 2096;
-    const double nan = __longlong_as_double(0x7FF8000000000000LL);
-    const bool bad = e0 == 2047 || e1 == 2047;
-    R[(size_t)set * kAmps * kAmps + k] = bad ? make_double2(nan, nan) : make_double2(ldexp(re, e), ldexp(im, e));
+    const uint32_t c0 = cut_exponent(e0), c1 = cut_exponent(e1);
+    const int e = (int)(c0 + c1) - 2100 + cross_shift(log2_bound, tiles, c0, c1);
+    double2 a = pair_of(re, e), b = pair_of(im, e);
+    if (e0 == 2047 || e1 == 2047) a.x = b.x = __longlong_as_double(0x7FF8000000000000LL);
+    double2* out = R + (size_t)set * 2 * kAmps * kAmps + k;
+    out[0] = make_double2(a.x, b.x);
+    out[kAmps * kAmps] = make_double2(a.y, b.y);
 }
 
 // largest biased exponent of the 2^n amplitudes of each set, psi then lambda
@@ -339,33 +379,36 @@ __global__ void k_angles(const double* __restrict__ params, int nparams, const i
 }
 
 // Gradients of block blockIdx.x's parametrised gates for set blockIdx.y, from R after the block: per gate,
-// last to first, Im tr(P R), then R <- G^+ R G.  In fixed point against the largest entry (54 bits; the
-// Frobenius norm is kept, so entries and traces stay below 2^61), every product rounded once: in FP64
-// the roundings of some 25 gates on one small matrix cost 1.5e-15 of the gradients on 12 qubits, more than
-// sums over all amplitudes gate by gate.
+// last to first, Im tr(P R), then R <- G^+ R G.  In fixed point against the Frobenius norm (60 bits; the
+// norm is kept, so entries stay below 2^60 and traces below 2^63), every product rounded once: a gradient
+// is a small difference of large traces, and the roundings of some 25 gates on one matrix do not
+// average out as those of 2^n amplitudes do (in FP64 they cost 1.5e-15 of the gradients on 12 qubits).
 __global__ void __launch_bounds__(128)
     k_block_grads(const double2* __restrict__ R, const BlockStep* __restrict__ steps, const BlockGate* __restrict__ gates,
                   const double2* __restrict__ angles, int nocc, double* __restrict__ grads) {
     __shared__ Fixed2 M[kAmps][kAmps + 1];
     __shared__ Fixed2 u[2][4];  // this gate's matrix and its inverse's
-    __shared__ uint32_t mx_s;
+    __shared__ double sq_s[4];
     const int step = blockIdx.x, set = blockIdx.y, sets = gridDim.y, tid = threadIdx.x;
     const BlockStep st = steps[step];
     int first = st.ngates;  // the earliest parametrised gate: nothing before it is needed
     for (int k = st.ngates - 1; k >= 0; --k)
         if (gates[st.gate_begin + k].kind == 3) first = k;
     if (first == st.ngates) return;
-    const double2* src = R + ((size_t)step * sets + set) * kAmps * kAmps;
-    if (tid == 0) mx_s = 0;
+    const double2* src = R + ((size_t)step * sets + set) * 2 * kAmps * kAmps;
+    double sq = 0.0;
+    for (int k = tid; k < kAmps * kAmps; k += 128) sq = fma(src[k].x, src[k].x, fma(src[k].y, src[k].y, sq));
+    for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+    if ((tid & 31) == 0) sq_s[tid >> 5] = sq;
     __syncthreads();
-    uint32_t mx = 0;
-    for (int k = tid; k < kAmps * kAmps; k += 128)
-        mx = max(mx, max((uint32_t)__double2hiint(src[k].x) & 0x7FFFFFFFu, (uint32_t)__double2hiint(src[k].y) & 0x7FFFFFFFu));
-    atomicMax(&mx_s, mx);
-    __syncthreads();
-    const int ex = (int)(mx_s >> 20);  // all below 2^(ex - 1022)
-    for (int k = tid; k < kAmps * kAmps; k += 128)
-        M[k >> 5][k & 31] = {__double2ll_rn(ldexp(src[k].x, 1022 + 54 - ex)), __double2ll_rn(ldexp(src[k].y, 1022 + 54 - ex))};
+    const double norm = sqrt(sq_s[0] + sq_s[1] + sq_s[2] + sq_s[3]);
+    int ex = 0;
+    if (norm > 0.0 && norm < 1e300) frexp(norm, &ex);  // norm < 2^ex
+    for (int k = tid; k < kAmps * kAmps; k += 128) {
+        const double2 h = src[k], l = src[kAmps * kAmps + k];
+        M[k >> 5][k & 31] = {__double2ll_rn(ldexp(h.x, 60 - ex)) + __double2ll_rn(ldexp(l.x, 60 - ex)),
+                             __double2ll_rn(ldexp(h.y, 60 - ex)) + __double2ll_rn(ldexp(l.y, 60 - ex))};
+    }
     __syncthreads();
     for (int k = st.ngates - 1; k >= first; --k) {
         const BlockGate& o = gates[st.gate_begin + k];
@@ -378,7 +421,7 @@ __global__ void __launch_bounds__(128)
             for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
             if (tid == 0)
                 grads[(size_t)set * nocc + o.q1] =
-                    ex == 2047 ? __longlong_as_double(0x7FF8000000000000LL) : ldexp((double)v, ex - 1022 - 54);
+                    norm < 1e300 ? ldexp((double)v, ex - 60) : __longlong_as_double(0x7FF8000000000000LL);
         }
         if (k == first) break;
         if ((o.kind == 0 || o.kind == 3) && tid >= 32 && tid < 40)
@@ -430,14 +473,14 @@ __global__ void __launch_bounds__(128)
 
 int cross_ctas(int n, int sets, int sms) {
     const uint64_t tiles = (1ULL << (n - 5)) / kGroups;
-    return block_ctas(tiles, sets, sms, (int)((tiles + kMaxTiles - 1) / kMaxTiles));
+    return block_ctas(tiles, sets, sms);
 }
 
-int block_ctas(uint64_t tiles, int sets, int sms, int least) {
+int block_ctas(uint64_t tiles, int sets, int sms) {
     // a CTA costs about one tile to start; the CTAs beyond one per SM run in turn
-    int best = least;
+    int best = 1;
     double cost = 1e300;
-    for (uint64_t k = (uint64_t)least; k <= tiles && k <= (uint64_t)std::max(least, 4 * sms); ++k) {
+    for (uint64_t k = 1; k <= tiles && k <= (uint64_t)(4 * sms); ++k) {
         const double rounds = std::ceil((double)(k * sets) / sms), per = std::ceil((double)tiles / (double)k) + 1.0;
         if (rounds * per < cost) {
             cost = rounds * per;
@@ -447,8 +490,8 @@ int block_ctas(uint64_t tiles, int sets, int sms, int least) {
     return best;
 }
 
-cudaError_t launch_cross(const void* psi, const void* lam, int n, int sets, int ctas, const BlockDesc& bd, const uint32_t* exps,
-                         double2* partial, double2* R, int* err_flag, cudaStream_t s) {
+cudaError_t launch_cross(const void* psi, const void* lam, int n, int sets, int ctas, const BlockDesc& bd, int log2_bound,
+                         const uint32_t* exps, void* partial, double2* R, int* err_flag, cudaStream_t s) {
     static const cudaError_t attr = cudaFuncSetAttribute(k_cross, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem);
     if (attr != cudaSuccess) return attr;
     CrossOffsets to;
@@ -457,11 +500,13 @@ cudaError_t launch_cross(const void* psi, const void* lam, int n, int sets, int 
         for (int b = 0; b < 5; ++b)
             if ((j >> b) & 1) to.o[j] |= 1ULL << bd.q[b];
     }
+    const int tiles = (int)(((1ULL << (n - 5)) / kGroups + ctas - 1) / ctas);
     k_cross<<<dim3((unsigned)ctas, (unsigned)sets), kRThreads, kRSmem, s>>>(
-        static_cast<const double2*>(psi), static_cast<const double2*>(lam), n, to, bd.tmask, exps, partial, err_flag);
+        static_cast<const double2*>(psi), static_cast<const double2*>(lam), n, to, bd.tmask, log2_bound, tiles, exps,
+        static_cast<Fixed2*>(partial), err_flag);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_cross_sum<<<dim3(kAmps * kAmps / 128, (unsigned)sets), 128, 0, s>>>(partial, ctas, exps, R);
+    k_cross_sum<<<dim3(kAmps * kAmps / 128, (unsigned)sets), 128, 0, s>>>(static_cast<const Fixed2*>(partial), ctas, log2_bound, tiles, exps, R);
     return cudaGetLastError();
 }
 

@@ -13,14 +13,14 @@
 
 namespace llg {
 
-// CTAs a state for `tiles` tiles of 128 groups on each of `sets` states, at least `least`
-int block_ctas(uint64_t tiles, int sets, int sms, int least);
+// CTAs a state for `tiles` tiles of 128 groups on each of `sets` states
+int block_ctas(uint64_t tiles, int sets, int sms);
 int cross_ctas(int n, int sets, int sms);  // of launch_cross
 
-// R = sum over the groups of psi lambda^+ on the block's qubits, 32 x 32 a set.  exps: per set the
-// largest biased exponents of psi, then of lambda; partial: sets x ctas x 1024 double2
-cudaError_t launch_cross(const void* psi, const void* lam, int n, int sets, int ctas, const BlockDesc& bd, const uint32_t* exps,
-                         double2* partial, double2* R, int* err_flag, cudaStream_t s);
+// R = sum over the groups of psi lambda^+ on the block's qubits, 32 x 32 a set (high parts, then low
+// parts).  log2_bound: an integer at least log2(|psi| |lambda|); exps: per set the largest biased exponents of psi, then of lambda; partial: sets x ctas x 16 KB
+cudaError_t launch_cross(const void* psi, const void* lam, int n, int sets, int ctas, const BlockDesc& bd, int log2_bound,
+                         const uint32_t* exps, void* partial, double2* R, int* err_flag, cudaStream_t s);
 // raises exps (2 sets words, zeroed by the caller) to the largest biased exponents
 cudaError_t launch_max_exponent(const void* psi, const void* lam, int n, int sets, uint32_t* exps, cudaStream_t s);
 // (cos, sin) of half the angles; occ_code: 2 parameter + anything

@@ -578,13 +578,14 @@ struct llg_adjoint {
     std::vector<BlockStep> bsteps;
     std::vector<BlockGate> bgates;
     std::vector<char> bparams;  // per step: has parametrised gates
+    int log2_obs = 0;           // an integer above log2 of the observable's largest eigenvalue
     BlockStep* d_bsteps = nullptr;
     BlockGate* d_bgates = nullptr;
     int bsets = -1;             // -1: not allocated yet
     unsigned char* d_bweights = nullptr;  // [step][set], the blocks, then their inverses
     double2* d_angles = nullptr;          // [batch][occurrence]
     double2* d_bR = nullptr;              // [step][set]
-    double2* d_bpart = nullptr;
+    void* d_bpart = nullptr;
     uint32_t* d_bexps = nullptr;          // [step + 1][2 sets]
     int* d_bflag = nullptr;
 };
@@ -703,15 +704,15 @@ int run_backward(llg_adjoint* h, int batch, int C) {
     return LLG_OK;
 }
 
-// Time of a batch in the two forms.  Measured on this GPU in IEEE complex128: tile passes 10 ps per gate and
-// amplitude (2.8 ps forward only), and no less than 6 us (2.5) a gate; a block 8.0 ps per amplitude and at
-// least 9.5 us, the 32 x 32 sums 9.5 ps and at least 20 us.
-bool blocks_pay(const llg_adjoint* h, int batch, bool grads) {
+// Time of a batch's gradients in the two forms; energies alone take the same one, so that they are the same
+// numbers.  Measured on this GPU in IEEE complex128: tile passes 10 ps per gate and amplitude, and no less than
+// 6 us a gate; a block and its inverse on both vectors 24 ps per amplitude, and at least 19 us; the 32 x 32
+// sums 9.5 ps and at least 20 us.
+bool blocks_pay(const llg_adjoint* h, int batch) {
     const double amps = std::ldexp((double)batch, h->n);
-    const double tiles = (double)h->fwd.ops.size() * std::max(grads ? 6e-6 : 2.5e-6, amps * (grads ? 1.0e-11 : 2.8e-12));
-    const double fwd = std::max(9.5e-6, amps * 8.0e-12);
-    const double bwd = std::max(20e-6, amps * 9.5e-12) + std::max(9.5e-6, amps * 16e-12);
-    return (double)h->bsteps.size() * (fwd + (grads ? bwd : 0.0)) + 50e-6 < tiles;
+    const double tiles = (double)h->fwd.ops.size() * std::max(6e-6, amps * 1.0e-11);
+    const double step = std::max(19e-6, amps * 24e-12) + std::max(20e-6, amps * 9.5e-12);
+    return (double)h->bsteps.size() * step + 50e-6 < tiles;
 }
 
 // Allocates the block form's workspace once; h->bsets = 0 when there is no room (the tile passes run).
@@ -739,8 +740,8 @@ void ensure_blocks(llg_adjoint* h) {
     ok = ok && cudaMalloc((void**)&h->d_bgates, h->bgates.size() * sizeof(BlockGate)) == cudaSuccess;
     ok = ok && cudaMalloc((void**)&h->d_bweights, 2 * steps * sets * wb) == cudaSuccess;
     ok = ok && cudaMalloc((void**)&h->d_angles, std::max<size_t>(1, (size_t)h->max_batch * h->nocc) * sizeof(double2)) == cudaSuccess;
-    ok = ok && cudaMalloc((void**)&h->d_bR, steps * sets * 1024 * sizeof(double2)) == cudaSuccess;
-    ok = ok && cudaMalloc((void**)&h->d_bpart, part) == cudaSuccess;
+    ok = ok && cudaMalloc((void**)&h->d_bR, steps * sets * 2048 * sizeof(double2)) == cudaSuccess;
+    ok = ok && cudaMalloc(&h->d_bpart, part) == cudaSuccess;
     ok = ok && cudaMalloc((void**)&h->d_bexps, (steps + 1) * 2 * sets * sizeof(uint32_t)) == cudaSuccess;
     ok = ok && cudaMalloc((void**)&h->d_bflag, sizeof(int)) == cudaSuccess;
     ok = ok && cudaMemcpy(h->d_bsteps, h->bsteps.data(), steps * sizeof(BlockStep), cudaMemcpyHostToDevice) == cudaSuccess;
@@ -797,7 +798,7 @@ int run_blocks(llg_adjoint* h, int batch, bool grads) {
         ADJ_CUDA(cudaMemsetAsync(psi, 0, (size_t)sets * h->state_bytes, s), "memset psi");
         k_set_rows<PolF64><<<(sets + 255) / 256, 256, 0, s>>>(psi, n, sets);
         ADJ_CUDA(cudaGetLastError(), "init rows");
-        const int fwd_ctas = block_ctas(tiles, sets, sms, 1), bwd_ctas = block_ctas(tiles, 2 * sets, sms, 1);
+        const int fwd_ctas = block_ctas(tiles, sets, sms), bwd_ctas = block_ctas(tiles, 2 * sets, sms);
         for (int j = 0; j < steps; ++j)
             ADJ_CUDA(launch_gate_block_batch(psi, nullptr, sets, fwd_ctas, n, desc(j), h->d_bweights + (size_t)j * sets * wb,
                                              true, nullptr, h->d_bflag, s),
@@ -811,8 +812,8 @@ int run_blocks(llg_adjoint* h, int batch, bool grads) {
         ADJ_CUDA(launch_max_exponent(psi, lam, n, sets, h->d_bexps + (size_t)steps * 2 * sets, s), "exponents");
         for (int j = steps - 1; j >= first; --j) {
             if (h->bparams[j])
-                ADJ_CUDA(launch_cross(psi, lam, n, sets, cross_ctas(n, sets, sms), desc(j), h->d_bexps + (size_t)(j + 1) * 2 * sets,
-                                      h->d_bpart, h->d_bR + (size_t)j * sets * 1024, h->d_bflag, s),
+                ADJ_CUDA(launch_cross(psi, lam, n, sets, cross_ctas(n, sets, sms), desc(j), h->log2_obs, h->d_bexps + (size_t)(j + 1) * 2 * sets,
+                                      h->d_bpart, h->d_bR + (size_t)j * sets * 2048, h->d_bflag, s),
                          "block sums");
             if (j > first)
                 ADJ_CUDA(launch_gate_block_batch(psi, lam, sets, bwd_ctas, n, desc(j), inverse + (size_t)j * sets * wb, true,
@@ -965,6 +966,10 @@ int llg_adjoint_create(int n, const llg_op* ops, int nops, int nparams, int max_
         bool fits = true;  // sign flips on more than five qubits have no block
         for (int i = 0; i < nops; ++i) fits = fits && !(ops[i].kind == LLG_OP_MCZ && popcount64(ops[i].mask) > 5);
         if (fits) {
+            double sum = 0.0;
+            for (int k = 0; k < nterms; ++k) sum += std::fabs(zcoeff[k]);
+            std::frexp(std::max(sum, 1e-300), &h->log2_obs);
+            ++h->log2_obs;  // and the state's norm, 1 within rounding
             BlockPlanner planner(n, ops, nops, true);
             while (planner.advance(1 << 20)) {}
             h->bsteps = planner.plan.steps;
@@ -1075,8 +1080,9 @@ int llg_adjoint_run(llg_adjoint* h, const double* params, int batch, double* ene
         return set_error(LLG_EINVAL, "adjoint_run: batch must be in [1, " + std::to_string(h->max_batch) + "]");
     if (checkpoint_every < 0) return set_error(LLG_EINVAL, "adjoint_run: checkpoint_every must be >= 0");
     int rc = load_params(h, params, batch);
-    if (!h->bsteps.empty() && h->threads == 0 && checkpoint_every == 0 && blocks_pay(h, batch, grads != nullptr)) ensure_blocks(h);
-    if (!rc && h->bsets > 0 && h->threads == 0 && checkpoint_every == 0 && blocks_pay(h, batch, grads != nullptr)) {
+    const bool blocks = !h->bsteps.empty() && h->threads == 0 && checkpoint_every == 0 && blocks_pay(h, batch);
+    if (!rc && blocks) ensure_blocks(h);
+    if (!rc && blocks && h->bsets > 0) {
         rc = run_blocks(h, batch, grads != nullptr);
         int flag = 0;
         if (!rc) rc = store_out(h, energies, h->d_energy, batch);
