@@ -790,10 +790,10 @@ int run_blocks(llg_adjoint* h, int batch, bool grads) {
             }
             return bd;
         };
-        ADJ_CUDA(launch_gate_block_weights(LLG_F64, h->d_bgates, h->d_bsteps, steps, h->d_bweights, s, ang, h->nocc, sets, false),
+        ADJ_CUDA(launch_gate_block_weights(LLG_F64, h->d_bgates, h->d_bsteps, steps, h->d_bweights, s, nullptr, ang, h->nocc, sets, false),
                  "block weights");
         if (grads)
-            ADJ_CUDA(launch_gate_block_weights(LLG_F64, h->d_bgates, h->d_bsteps, steps, inverse, s, ang, h->nocc, sets, true),
+            ADJ_CUDA(launch_gate_block_weights(LLG_F64, h->d_bgates, h->d_bsteps, steps, inverse, s, nullptr, ang, h->nocc, sets, true),
                      "block weights");
         ADJ_CUDA(cudaMemsetAsync(psi, 0, (size_t)sets * h->state_bytes, s), "memset psi");
         k_set_rows<PolF64><<<(sets + 255) / 256, 256, 0, s>>>(psi, n, sets);

@@ -27,7 +27,7 @@ namespace {
 struct Node {
     uint64_t mask = 0;  // its qubits
     int kind = 0;       // BlockGate kinds
-    int mat = -1;       // kind 0: its 2x2 matrix; kind 1: the target; kind 3: its occurrence
+    int mat = -1;       // kind 0: its 2x2 matrix; kind 1: the target; kind 3: its occurrence; kind 4: its index
     int axis = 0;       // kind 3
     int seg_begin = 0;  // its qubits in increasing order: segments seg_of_[seg_begin ..]
     float weight = 0.f;
@@ -48,7 +48,10 @@ void matmul(const double* a, const double* b, double* out) {
 
 class BlockPlanner::Impl {
 public:
-    Impl(int n, const llg_op* ops, int nops, bool params, BlockPlan& out) : n_(n), params_(params), out_(out) { build(ops, nops); }
+    Impl(int n, const llg_op* ops, int nops, bool params, const std::vector<MatrixOp>* matrices, BlockPlan& out)
+        : n_(n), params_(params), mops_(matrices), out_(out) {
+        build(ops, nops);
+    }
 
     bool advance(int blocks) {
         const int goal = out_.blocks + blocks;
@@ -124,6 +127,21 @@ private:
                     matmul(g.m, p.m, p.m);
                     pdiag[op.q0] = pdiag[op.q0] && d;
                 }
+                continue;
+            }
+            if (op.kind == kOpMatrix) {
+                const MatrixOp& mo = (*mops_)[op.q0];
+                Node v;
+                v.kind = 4;
+                v.mat = op.q0;
+                for (int j = 0; j < mo.k; ++j) v.mask |= 1ULL << mo.q[j];
+                for (uint64_t s = v.mask; s; s &= s - 1) flush(__builtin_ctzll(s));
+                bool diag = true;
+                const int d = 1 << mo.k;
+                for (int e = 0; e < d * d; ++e)
+                    if (e / d != e % d) diag = diag && mo.m[2 * e] == 0.0 && mo.m[2 * e + 1] == 0.0;
+                v.weight = mo.k <= 2 ? 2.0f : 5.0f;
+                add_node(v, diag ? v.mask : 0);
                 continue;
             }
             Node v;
@@ -310,7 +328,14 @@ private:
         std::memset(&g, 0, sizeof(g));
         g.kind = v.kind;
         auto local = [&](int q) { return to_local ? to_local[q] : q; };
-        if (v.kind == 3) {
+        if (v.kind == 4) {
+            const MatrixOp& mo = (*mops_)[v.mat];
+            for (int j = 0; j < mo.k; ++j) g.q0 |= local(mo.q[j]) << (4 * j);
+            g.q1 = mo.k;
+            g.pad = (int)(out_.matrices.size() / 2);
+            out_.matrices.insert(out_.matrices.end(), mo.m.begin(), mo.m.end());
+            ++(mo.k <= 2 ? out_.small_matrices : out_.large_matrices);
+        } else if (v.kind == 3) {
             g.q0 = local(__builtin_ctzll(v.mask));
             g.q1 = v.mat;
             g.pad = v.axis;
@@ -347,7 +372,7 @@ private:
         // up to three gates that only move amplitudes or signs run on their own: a CNOT or CZ pass
         // takes 2.6 ms at 30 qubits, a block 8.8
         bool moves = !params_ && got_.size() <= 3;
-        for (int id : got_) moves = moves && nodes_[id].kind != 0;
+        for (int id : got_) moves = moves && (nodes_[id].kind == 1 || nodes_[id].kind == 2);
         if (moves) {
             for (int id : got_) single(nodes_[id]);
             return;
@@ -373,6 +398,7 @@ private:
     static constexpr int kSeeds = 4;
     int n_;
     bool params_;
+    const std::vector<MatrixOp>* mops_;
     BlockPlan& out_;
     std::vector<M8> mats_;
     std::vector<Node> nodes_;
@@ -387,7 +413,8 @@ private:
     size_t first_ = 0;
 };
 
-BlockPlanner::BlockPlanner(int n, const llg_op* ops, int nops, bool params) : impl_(new Impl(n, ops, nops, params, plan)) {}
+BlockPlanner::BlockPlanner(int n, const llg_op* ops, int nops, bool params, const std::vector<MatrixOp>* matrices)
+    : impl_(new Impl(n, ops, nops, params, matrices, plan)) {}
 BlockPlanner::~BlockPlanner() = default;
 bool BlockPlanner::advance(int blocks) { return impl_->advance(blocks); }
 

@@ -56,6 +56,7 @@ struct llg_state {
     int tile_qubits = 0;   // 0 = default
     int tile_threads = 0;  // CTA size of the tile kernel, 0 = default
     std::vector<llg_op> queue;
+    std::vector<MatrixOp> matrices;  // of the queue's kOpMatrix entries
     // op upload
     ExecOp* d_ops = nullptr;
     size_t d_ops_cap = 0;
@@ -326,13 +327,15 @@ int run_tiles(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
 // of the plan made while the first blocks run.  nops: the flush's gates (bounds the plan's size).
 // mirror / mirrored: as for run_tiles.
 int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
+    size_t mbytes = 0;
+    for (const MatrixOp& m : st->matrices) mbytes += m.m.size() * sizeof(double);
     constexpr int kGroup = 16;   // blocks planned, uploaded and launched at a time
     constexpr int kSlots = 128;  // blocks whose weights are held at once
     static_assert(kSlots % kGroup == 0, "a group's weights are contiguous");
     const size_t wb = gate_block_weight_bytes(st->P);
     const size_t slots = nops <= kSlots ? (std::max<size_t>(nops, 1) + kGroup - 1) / kGroup * kGroup : kSlots;
-    // a group's upload: its blocks' steps and its gates; every group has its own part of the buffers
-    const size_t bytes = (nops / kGroup + 2) * (kGroup * sizeof(BlockStep) + 512) + nops * sizeof(BlockGate);
+    // a group's upload: its blocks' steps, its gates, their matrices; every group has its own part of the buffers
+    const size_t bytes = (nops / kGroup + 2) * (kGroup * sizeof(BlockStep) + 1024) + nops * sizeof(BlockGate) + mbytes;
     if (bytes > st->d_bplan_cap || slots * wb > st->d_bweights_cap)
         LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
     if (bytes > st->d_bplan_cap) {
@@ -374,18 +377,30 @@ int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror
         const unsigned char* w = static_cast<const unsigned char*>(st->d_bweights) + wb * slot;
         if (!bs.empty()) {
             const size_t sbytes = (bs.size() * sizeof(BlockStep) + 255) / 256 * 256;
-            const size_t gbytes = (gates_to - gates_from) * sizeof(BlockGate);
+            const size_t gbytes = ((gates_to - gates_from) * sizeof(BlockGate) + 255) / 256 * 256;
             std::memcpy(st->h_bplan + off, bs.data(), bs.size() * sizeof(BlockStep));
-            std::memcpy(st->h_bplan + off + sbytes, plan.gates.data() + gates_from, gbytes);
-            LLG_CUDA(cudaMemcpyAsync(st->d_bplan + off, st->h_bplan + off, sbytes + gbytes, cudaMemcpyHostToDevice, st->stream),
+            BlockGate* hg = reinterpret_cast<BlockGate*>(st->h_bplan + off + sbytes);
+            std::memcpy(hg, plan.gates.data() + gates_from, (gates_to - gates_from) * sizeof(BlockGate));
+            double* hm = reinterpret_cast<double*>(st->h_bplan + off + sbytes + gbytes);
+            size_t doubles = 0;
+            for (size_t i = 0; i < gates_to - gates_from; ++i)
+                if (hg[i].kind == 4) {
+                    const size_t count = (size_t)2 << (2 * hg[i].q1);
+                    std::memcpy(hm + doubles, plan.matrices.data() + 2 * (size_t)hg[i].pad, count * sizeof(double));
+                    hg[i].pad = (int)(doubles / 2);
+                    doubles += count;
+                }
+            LLG_CUDA(cudaMemcpyAsync(st->d_bplan + off, st->h_bplan + off, sbytes + gbytes + doubles * sizeof(double),
+                                     cudaMemcpyHostToDevice, st->stream),
                      "cudaMemcpyAsync(block plan)");
             const int rc = traced(st, LLG_PROF_TILE, 1, "block weights", [&] {
                 return launch_gate_block_weights(st->P, reinterpret_cast<const BlockGate*>(st->d_bplan + off + sbytes),
                                                  reinterpret_cast<const BlockStep*>(st->d_bplan + off), (int)bs.size(),
-                                                 static_cast<unsigned char*>(st->d_bweights) + wb * slot, st->stream);
+                                                 static_cast<unsigned char*>(st->d_bweights) + wb * slot, st->stream,
+                                                 reinterpret_cast<const double2*>(st->d_bplan + off + sbytes + gbytes));
             });
             if (rc) return rc;
-            off += (sbytes + gbytes + 255) / 256 * 256;
+            off += (sbytes + gbytes + doubles * sizeof(double) + 255) / 256 * 256;
             slot = (slot + kGroup) % (int)slots;
         }
         for (size_t i = from; i < to; ++i) {
@@ -447,7 +462,8 @@ int measure_norm(llg_state* st) {
 // (double-float), and at least 9.5 us; a CNOT or sign-flip pass 2.6 ms.  Tile passes take 3.2 FP64
 // multiply-adds per amplitude for a merged one-qubit gate that mixes and 4 for a diagonal one, at
 // 0.56 T a second (double-float: 2.0 ms per 2^30 for either); no less than 2.6 (FP64) or 2 us a
-// gate, however small the register (a CTA's latency); and one read and write of the state.
+// gate, however small the register (a CTA's latency); and one read and write of the state.  A channel
+// on its own is a sparse pass: 6.2 ms per 2^30 on one qubit of a density matrix, 9 on two, at least 6 us.
 bool blocks_pay(int P, int n, const BlockPlan& plan) {
     const bool f64 = P == LLG_F64;
     const double amps = std::ldexp(1.0, n);
@@ -456,8 +472,10 @@ bool blocks_pay(int P, int n, const BlockPlan& plan) {
     const double t_blocks = plan.blocks * block + ((double)plan.steps.size() - plan.blocks) * single + 20e-6;
     const double arith = f64 ? (3.2 * plan.mixing_1q + 4.0 * plan.diag_1q) / 0.56e12 : 1.9e-12 * (plan.mixing_1q + plan.diag_1q);
     const double latency = f64 ? 2.6e-6 : 2.0e-6;
-    const double t_tiles = std::max(std::max(arith * amps, latency * (double)plan.gates.size()), amps * 4.8e-12);
-    return t_blocks < t_tiles;
+    const double gates = (double)plan.gates.size() - plan.small_matrices - plan.large_matrices;
+    const double t_tiles = gates > 0 ? std::max(std::max(arith * amps, latency * gates), amps * 4.8e-12) : 0.0;
+    const double channels = plan.small_matrices * std::max(6e-6, amps * 5.8e-12) + plan.large_matrices * std::max(6e-6, amps * 8.4e-12);
+    return t_blocks < t_tiles + channels;
 }
 
 // growth of the norm bound over a queue (2x2s that are not unitary)
@@ -470,6 +488,31 @@ void note_growth(llg_state* st, const std::vector<llg_op>& q) {
     if (std::isnan(st->log2_norm)) st->log2_norm = HUGE_VAL;
 }
 
+// growth of the norm bound by a matrix: its 2-norm is at most the geometric mean of the largest column and
+// row sums
+void note_growth(llg_state* st, int k, const double* m) {
+    double rows = 0.0, cols[kMaxBlockDim] = {0.0}, col = 0.0;
+    for (int r = 0; r < 1 << k; ++r) {
+        double sum = 0.0;
+        for (int c = 0; c < 1 << k; ++c) {
+            const double v = std::hypot(m[2 * ((r << k) + c)], m[2 * ((r << k) + c) + 1]);
+            sum += v;
+            cols[c] += v;
+        }
+        rows = std::max(rows, sum);
+    }
+    for (int c = 0; c < 1 << k; ++c) col = std::max(col, cols[c]);
+    st->log2_norm += std::max(0.0, 0.5 * (std::log2(rows) + std::log2(col)));
+    if (std::isnan(st->log2_norm)) st->log2_norm = HUGE_VAL;
+}
+
+int apply_matrix_now(llg_state* st, int k, const int* qubits, const double* m);
+
+// whether gates and channels may wait for a plan in blocks: the caller has left the passes to the engine
+bool blocks_allowed(const llg_state* st) {
+    return gate_block_eligible(st->P, st->n) && st->fuse_mode == LLG_FUSE_TILE && st->tile_qubits == 0 && st->tile_threads == 0;
+}
+
 // the queue as fused passes (blocks, shared-memory tiles or register tiles)
 int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = nullptr, bool* mirrored = nullptr) {
     if (!gate_block_eligible(st->P, st->n)) return run_tiles(st, q, mirror, mirrored);
@@ -477,15 +520,36 @@ int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
     const double limit = st->P == LLG_F64 ? 900.0 : 90.0;
     if (st->log2_norm > limit && st->log2_norm < HUGE_VAL)
         if (int rc = measure_norm(st)) return rc;
-    if (st->fuse_mode == LLG_FUSE_TILE && st->tile_qubits == 0 && st->tile_threads == 0 && st->log2_norm <= limit) {
-        if (has_block_plan(st->n, q.data(), (int)q.size())) {
-            BlockPlanner planner(st->n, q.data(), (int)q.size());
-            planner.advance(8);
-            if (blocks_pay(st->P, st->n, planner.plan)) return run_blocks(st, planner, q.size(), mirror, mirrored);
+    if (blocks_allowed(st) && st->log2_norm <= limit && has_block_plan(st->n, q.data(), (int)q.size())) {
+        BlockPlanner planner(st->n, q.data(), (int)q.size(), false, &st->matrices);
+        planner.advance(8);
+        if (blocks_pay(st->P, st->n, planner.plan)) {
+            const int rc = run_blocks(st, planner, q.size(), mirror, mirrored);
+            for (const MatrixOp& m : st->matrices) note_growth(st, m.k, m.m.data());
+            st->matrices.clear();
+            return rc;
         }
     }
     note_growth(st, q);
-    return run_tiles(st, q, mirror, mirrored);
+    if (st->matrices.empty()) return run_tiles(st, q, mirror, mirrored);
+    // channels one by one, the gates between them in tile passes
+    std::vector<MatrixOp> mats;
+    mats.swap(st->matrices);
+    std::vector<llg_op> part;
+    for (size_t i = 0; i <= q.size(); ++i) {
+        if (i < q.size() && q[i].kind != kOpMatrix) {
+            part.push_back(q[i]);
+            continue;
+        }
+        if (!part.empty())
+            if (int rc = run_tiles(st, part)) return rc;
+        part.clear();
+        if (i < q.size()) {
+            const MatrixOp& m = mats[q[i].q0];
+            if (int rc = apply_matrix_now(st, m.k, m.q, m.m.data())) return rc;
+        }
+    }
+    return LLG_OK;
 }
 
 int enqueue(llg_state* st, const llg_op& op) {
@@ -656,6 +720,7 @@ int llg_reset(llg_state* st, int n_qubits) {
     if (n_qubits < 1 || n_qubits > kMaxQubits)
         return set_error(LLG_EINVAL, "llg_reset: n_qubits must be in [1, " + std::to_string(kMaxQubits) + "]");
     st->queue.clear();
+    st->matrices.clear();
     int rc = alloc_state(st, n_qubits);
     if (rc) return rc;
     st->log2_norm = 0.0;
@@ -804,6 +869,14 @@ int llg_expect_diag_zz(llg_state* st, int nterms, const int* a, const int* b, co
 
 int llg_apply_matrix(llg_state* st, int k, const int* qubits, const double* m) {
     if (!st || !qubits || !m) return set_error(LLG_EINVAL, "apply_matrix: NULL argument");
+    return apply_matrix_now(st, k, qubits, m);
+}
+
+}  // extern "C"
+
+namespace {
+// a dense matrix on up to five qubits after the queued gates
+int apply_matrix_now(llg_state* st, int k, const int* qubits, const double* m) {
     if (k < 1 || k > kMaxBlockQubits || k > st->n)
         return set_error(LLG_EINVAL, "apply_matrix: k must be in [1, 5] and at most the register size");
     BlockDesc bd;
@@ -821,22 +894,7 @@ int llg_apply_matrix(llg_state* st, int k, const int* qubits, const double* m) {
         if (!std::isfinite(m[i])) return set_error(LLG_EINVAL, "apply_matrix: non-finite matrix entry");
     int rc = llg_flush(st);  // earlier gates first
     if (rc) return rc;
-    {
-        // the 2-norm is at most the geometric mean of the largest column and row sums
-        double rows = 0.0, cols[kMaxBlockDim] = {0.0}, col = 0.0;
-        for (int r = 0; r < 1 << k; ++r) {
-            double sum = 0.0;
-            for (int c = 0; c < 1 << k; ++c) {
-                const double v = std::hypot(m[2 * ((r << k) + c)], m[2 * ((r << k) + c) + 1]);
-                sum += v;
-                cols[c] += v;
-            }
-            rows = std::max(rows, sum);
-        }
-        for (int c = 0; c < 1 << k; ++c) col = std::max(col, cols[c]);
-        st->log2_norm += std::max(0.0, 0.5 * (std::log2(rows) + std::log2(col)));
-        if (std::isnan(st->log2_norm)) st->log2_norm = HUGE_VAL;
-    }
+    note_growth(st, k, m);
     const size_t cap = (size_t)2 * kMaxBlockDim * kMaxBlockDim;
     if (!st->d_block) {
         LLG_CUDA(cudaMalloc(&st->d_block, cap * sizeof(uint64_t)), "cudaMalloc(block)");
@@ -947,6 +1005,9 @@ int llg_apply_matrix(llg_state* st, int k, const int* qubits, const double* m) {
     return traced(st, LLG_PROF_GATE, 1, "block kernel",
                   [&] { return launch_block(st->P, st->d_psi, st->n, bd, st->d_block, st->stream); });
 }
+}  // namespace
+
+extern "C" {
 
 int llg_dm_apply_op(llg_state* st, int n, const llg_op* op) {
     if (!st || !op) return set_error(LLG_EINVAL, "dm_apply_op: NULL argument");
@@ -1012,7 +1073,16 @@ int llg_dm_apply_kraus(llg_state* st, int n, int nkraus, const double* kraus, in
         qs[j] = targets[j];
         qs[m + j] = targets[j] + n;
     }
-    return llg_apply_matrix(st, 2 * m, qs, S.data());
+    if (!blocks_allowed(st)) return llg_apply_matrix(st, 2 * m, qs, S.data());
+    // the channel waits with the gates: a block takes it together with those on its qubits.  Its entries, and
+    // those of products of channels and unitary gates, are matrix elements of maps that do not increase the
+    // trace norm: at most 1
+    MatrixOp mo;
+    mo.k = 2 * m;
+    for (int j = 0; j < 4; ++j) mo.q[j] = j < mo.k ? qs[j] : 0;
+    mo.m = S;
+    st->matrices.push_back(mo);
+    return enqueue(st, make_op(kOpMatrix, (int)st->matrices.size() - 1));
 }
 
 int llg_flush(llg_state* st) {
@@ -1113,6 +1183,7 @@ int llg_copy_to_host(llg_state* st, double* out) {
 int llg_copy_from_host(llg_state* st, const double* amps) {
     if (!st || !amps) return set_error(LLG_EINVAL, "copy_from_host: NULL argument");
     st->queue.clear();  // overwritten anyway
+    st->matrices.clear();
     if (st->P == LLG_F64) {
         LLG_CUDA(cudaMemcpyAsync(st->d_psi, amps, st->size * 16, cudaMemcpyHostToDevice, st->stream), "cudaMemcpyAsync(H2D)");
         if (gate_block_eligible(st->P, st->n)) return measure_norm(st);

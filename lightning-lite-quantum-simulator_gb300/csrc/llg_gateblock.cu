@@ -620,12 +620,13 @@ __global__ void __launch_bounds__(128) k_weights_matrix(const double2* __restric
 
 template <int S>
 __global__ void __launch_bounds__(128)
-    k_weights_gates(const BlockGate* __restrict__ gates, const BlockStep* __restrict__ steps, const double2* __restrict__ angles,
-                    int nocc, bool inverse, unsigned char* __restrict__ wt, size_t stride) {
+    k_weights_gates(const BlockGate* __restrict__ gates, const BlockStep* __restrict__ steps,
+                    const double2* __restrict__ matrices, const double2* __restrict__ angles, int nocc, bool inverse, unsigned char* __restrict__ wt, size_t stride) {
     constexpr int kStage = 32;  // gates whose coefficients are in shared memory
     __shared__ Fixed2 M[kAmps][9];
     __shared__ Fixed2 coef[kStage][4];  // 2x2 matrices, row-major
-    __shared__ int4 what[kStage];       // kind, q0, q1, mask
+    __shared__ int4 what[kStage];       // kind, q0, q1, mask (kind 4: the matrix's first entry)
+    __shared__ Fixed2 dense[256];       // a gate of kind 4
     const int tid = threadIdx.x, ks = blockIdx.y, c = tid & 7, p = tid >> 3;
     wt += ((size_t)blockIdx.x * gridDim.z + blockIdx.z) * stride;
     constexpr int64_t one = (int64_t)1 << 62;
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(128)
             const int k = k0 + tid / 4, e = tid & 3;
             const BlockGate& o = gates[st.gate_begin + (inverse ? st.ngates - 1 - k : k)];
             coef[tid / 4][e] = gate_entry(o, e, o.kind == 3 ? angles[(size_t)blockIdx.z * nocc + o.q1] : make_double2(0.0, 0.0), inverse);
-            if (e == 0) what[tid / 4] = make_int4(o.kind, o.q0, o.q1, (int)o.mask);
+            if (e == 0) what[tid / 4] = make_int4(o.kind, o.q0, o.q1, o.kind == 4 ? o.pad : (int)o.mask);
         }
         __syncthreads();
         for (int k = 0; k < cnt; ++k) {
@@ -656,6 +657,40 @@ __global__ void __launch_bounds__(128)
                     M[r][c] = M[r1][c];
                     M[r1][c] = x;
                 }
+            } else if (o.x == 4) {
+                const int dim = 1 << o.z;
+                for (int e = tid; e < dim * dim; e += 128) {
+                    const double2 v = matrices[o.w + e];
+                    dense[e] = {__double2ll_rn(v.x * 0x1p62), __double2ll_rn(v.y * 0x1p62)};
+                }
+                __syncthreads();
+                // rows p and p + 16 of column c: the matrix's row picked by the row's bits, over the rows
+                // that differ in them
+                Fixed2 out[2];
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {
+                    const int r = p + 16 * w;
+                    int mine = 0, rest = r;
+                    for (int j = 0; j < o.z; ++j) {
+                        const int b = (o.y >> (4 * j)) & 15;
+                        mine |= ((r >> b) & 1) << j;
+                        rest &= ~(1 << b);
+                    }
+                    __int128 re = (__int128)1 << 61, im = re;
+                    for (int l = 0; l < dim; ++l) {
+                        const Fixed2 d = dense[mine * dim + l];
+                        if (d.x == 0 && d.y == 0) continue;
+                        int from = rest;
+                        for (int j = 0; j < o.z; ++j) from |= ((l >> j) & 1) << ((o.y >> (4 * j)) & 15);
+                        const Fixed2 x = M[from][c];
+                        re += (__int128)d.x * x.x - (__int128)d.y * x.y;
+                        im += (__int128)d.x * x.y + (__int128)d.y * x.x;
+                    }
+                    out[w] = {(int64_t)(re >> 62), (int64_t)(im >> 62)};
+                }
+                __syncthreads();
+                M[p][c] = out[0];
+                M[p + 16][c] = out[1];
             } else {
                 for (int r = p; r < kAmps; r += 16)
                     if ((r & o.w) == o.w) M[r][c] = {-M[r][c].x, -M[r][c].y};
@@ -745,10 +780,11 @@ cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weig
 }
 
 cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const BlockStep* d_steps, int nblocks, void* d_weights,
-                                      cudaStream_t s, const double2* d_angles, int nocc, int sets, bool inverse) {
+                                      cudaStream_t s, const double2* d_matrices, const double2* d_angles, int nocc, int sets,
+                                      bool inverse) {
     return by_precision(P, [&](auto p) {
         k_weights_gates<Shape<decltype(p)::value>::S><<<dim3((unsigned)nblocks, kChunks, (unsigned)sets), 128, 0, s>>>(
-            d_gates, d_steps, d_angles, nocc, inverse, static_cast<unsigned char*>(d_weights), gate_block_weight_bytes(P));
+            d_gates, d_steps, d_matrices, d_angles, nocc, inverse, static_cast<unsigned char*>(d_weights), gate_block_weight_bytes(P));
         return cudaGetLastError();
     });
 }

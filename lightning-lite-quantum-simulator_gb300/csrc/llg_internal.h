@@ -192,7 +192,8 @@ int32_t reg_dispatch_code(const ExecOp& x);
 struct BlockGate {
     // 0: 2x2 matrix m on q0; 1: CNOT, control q0, target q1; 2: sign flip where all of `mask` is set;
     // 3 (with parameters only): rotation exp(-i theta P / 2) on q0, P = X, Y, Z for pad = 0, 1, 2, theta
-    // the q1-th parametrised gate's angle
+    // the q1-th parametrised gate's angle; 4 (with matrices only): a dense matrix on q1 qubits, bit j of its
+    // index the (q0 >> 4 j) & 15-th of the block's, row-major (re, im) from entry `pad` of the plan's matrices
     int32_t kind;
     int32_t q0, q1, pad;
     uint64_t mask;
@@ -205,10 +206,21 @@ struct BlockStep {
     int32_t q[5];
     int32_t gate_begin, ngates;
 };
+// A dense matrix on up to four qubits in a gate list: an op of kind kOpMatrix whose q0 is its index in a list
+// of these.  Entries of it, and of products with the list's other gates, are at most 1 in size (channels on
+// density matrices).
+constexpr int32_t kOpMatrix = 1000;
+struct MatrixOp {
+    int k;
+    int q[4];
+    std::vector<double> m;  // 2 * 4^k
+};
 struct BlockPlan {
     std::vector<BlockStep> steps;
     std::vector<BlockGate> gates;
+    std::vector<double> matrices;  // of the kind-4 gates
     int blocks = 0;
+    int small_matrices = 0, large_matrices = 0;  // on one or two qubits, on three or four
     int mixing_1q = 0, diag_1q = 0;  // merged one-qubit gates among `gates`, for the cost of other plans
 };
 // 2x2 gates of a block have spectral norm at most this, so that its entries stay well below 2
@@ -222,7 +234,7 @@ class BlockPlanner {
 public:
     // params: rotations with param >= 0 stay gates of their own (kind 3) and every step is a block; the
     // list must have no sign flip on more than five qubits
-    BlockPlanner(int n, const llg_op* ops, int nops, bool params = false);
+    BlockPlanner(int n, const llg_op* ops, int nops, bool params = false, const std::vector<MatrixOp>* matrices = nullptr);
     ~BlockPlanner();
     bool advance(int blocks);  // appends up to `blocks` blocks to `plan`; false: the list is done
     BlockPlan plan;

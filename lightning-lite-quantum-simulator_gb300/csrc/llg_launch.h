@@ -103,12 +103,13 @@ cudaError_t launch_block_tc(int P, void* psi, int n, const BlockDesc& bd, const 
 bool gate_block_eligible(int P, int n);
 size_t gate_block_weight_bytes(int P);
 cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weights, cudaStream_t s);
-// the weights of `nblocks` blocks of a plan (d_steps: their steps, in order), one after the other; with
+// the weights of `nblocks` blocks of a plan (d_steps: their steps, in order; d_matrices: of the kind-4
+// gates), one after the other; with
 // parametrised gates (kind 3) `sets` of them per block, d_angles holding (cos, sin) of the half angles,
 // nocc a set; inverse: of the blocks' inverses
 cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const BlockStep* d_steps, int nblocks, void* d_weights,
-                                      cudaStream_t s, const double2* d_angles = nullptr, int nocc = 0, int sets = 1,
-                                      bool inverse = false);
+                                      cudaStream_t s, const double2* d_matrices = nullptr, const double2* d_angles = nullptr,
+                                      int nocc = 0, int sets = 1, bool inverse = false);
 // a block on `sets` FP64 states side by side from psi and (unless nullptr) as many from `second`, each
 // set with its own weights, `ctas` CTAs a state.  max_exp: nullptr, or per state (2 sets) a word that is
 // raised to the largest biased exponent stored

@@ -145,3 +145,33 @@ def test_gates_of_norm_above_one_grow_the_state():
     want = oracle.run_ops(n, np.concatenate([mix, mix]))
     assert np.max(np.abs(got - want)) <= 1e-12
     st.close()
+
+
+def test_channels_join_blocks():
+    # a density matrix of 2^12 elements: dense, diagonal and complex channels between gates, one and two targets
+    # in both orders, read in the middle; the same with one pass a channel
+    n = 6
+    rng = np.random.default_rng(2)
+    k1 = np.linalg.qr(rng.normal(size=(6, 2)) + 1j * rng.normal(size=(6, 2)))[0].reshape(3, 2, 2)
+    k2 = np.linalg.qr(rng.normal(size=(12, 4)) + 1j * rng.normal(size=(12, 4)))[0].reshape(3, 4, 4)
+    want = oracle.dm_zero(n)
+    fused, plain = llgpu.DensityMatrix(n), llgpu.DensityMatrix(n)
+    plain.state.set_fusion("tile", 12)
+    for step in range(4):
+        ops = _circuit(n + 2, 1, step)  # gates of every kind on the qubits that exist
+        ops = ops[(ops["q0"] < n) & (ops["q1"] < n) & (ops["kind"] != llgpu.OP_MCZ)]
+        want = oracle.dm_apply_ops(want, n, ops)
+        channels = [(llgpu.amplitude_damping(0.1), [q]) for q in range(n)] + [(llgpu.phase_damping(0.2), [step])]
+        channels += [(k1, [5 - step]), (k2, [step, 5]), (k2, [4, 0]), (llgpu.depolarizing(0.05, 2), [3, 1])]
+        for dm in (fused, plain):
+            dm.apply_ops(ops)
+        for ks, targets in channels:
+            for dm in (fused, plain):
+                dm.kraus(ks, targets)
+            want = oracle.kraus_apply(want, n, ks, targets)
+        if step == 1:
+            assert np.max(np.abs(fused.rho() - want)) <= 1e-12
+    assert np.max(np.abs(fused.rho() - want)) <= 1e-12
+    assert np.max(np.abs(plain.rho() - want)) <= 1e-12
+    fused.close()
+    plain.close()
