@@ -705,7 +705,10 @@ size_t traj_elem() {
     return sizeof(typename P::S);
 }
 
-const void* kernel_for(int P, int cl) {
+#include "llg_traj_f64.cuh"
+
+const void* kernel_for(int P, int cl, bool fast) {
+    if (fast) return cl == 2 ? reinterpret_cast<const void*>(&k_traj_fast2) : reinterpret_cast<const void*>(&k_traj_fast1);
     switch (P) {
         case LLG_F64: return traj_kernel<PolF64>(cl);
         case LLG_F32: return traj_kernel<PolF32>(cl);
@@ -721,6 +724,7 @@ const void* kernel_for(int P, int cl) {
 struct llg_traj {
     int n = 0, P = LLG_DF64;
     int cl = 1, threads = 0, grid = 0;
+    int launch = 0;  // threads of the launch
     size_t smem = 0;
     int ngates = 0;
     int64_t sites = 0;
@@ -730,6 +734,13 @@ struct llg_traj {
     uint64_t max_traj = 0;
     uint64_t shape_key = 0;
     TrajGate* d_gates = nullptr;
+    // one-pass steps (FP64 Kraus handles with weak noise), planned by configure()
+    std::vector<TrajGate> gates;
+    bool fast = false;
+    int nsteps = 0, zpos = 0;
+    FastStep* d_steps = nullptr;  // owns the buffer that d_slow and d_tabs point into
+    TrajGate* d_slow = nullptr;
+    double* d_tabs = nullptr;
     double* d_z0 = nullptr;
     uint32_t* d_jumps = nullptr;
     double* d_margin = nullptr;
@@ -740,6 +751,14 @@ struct llg_traj {
 };
 
 namespace {
+
+void drop_fast(llg_traj* h) {
+    cudaFree(h->d_steps);
+    h->d_steps = nullptr;
+    h->d_tabs = nullptr;
+    h->d_slow = nullptr;
+    h->fast = false;
+}
 
 void drop_graph(llg_traj* h) {
     if (h->exec) cudaGraphExecDestroy(h->exec);
@@ -768,37 +787,339 @@ int resolve_threads(int n, int P, int cl, int threads, size_t* smem_out) {
     return threads;
 }
 
+// One-pass steps: FP64 Kraus trajectories whose site pairs have 1 - g^2 <= 1/8.  A jump costs two passes and the
+// general sites; 600 trajectories, 4 layers of rx, ry and a cnot chain, one pass against the general kernel:
+//     gamma + lambda    0.005           0.03           0.1            0.2
+//     8 qubits          272 / 520 us    310 / 521      434 / 519      520 / 520 us
+//     14 qubits         11.3 / 21.1 ms  12.7 / 21.2    15.5 / 21.2    21.3 / 21.3 ms
+// (At 1/8 the extra warp's five factors of 1 / (1 - x) leave 2^-64.)  512 trajectories of 14 qubits and 8 layers
+// take 19.6 ms instead of 36.9; FP64 multiply-adds alone take 14 ms at 2 a clock and SM.  3 to 13 qubits: 1.6 to
+// 2.9 times faster.
+bool fast_noise(int P, const KrausParams& kp) {
+    return P == LLG_F64 && kp.mode == NOISE_KRAUS && kp.gamma + kp.lambda - kp.gamma * kp.lambda <= kFastKappa;
+}
+
+// CTA threads of a one-pass launch: 8 amplitude pairs a thread, at most the threads asked for, and one warp
+int fast_threads(int nl, int threads) {
+    int w = 32;
+    while (2 * w <= threads && 2 * w <= (1 << nl) / 16 && 2 * w <= kFastWorkers) w *= 2;
+    return w + 32;
+}
+
+// pairs of doubles for the pending factors, which a whole circuit multiplies up
+struct Pair {
+    double h, l;
+};
+Pair pair_sum(double a, double b) {  // exact
+    const double s = a + b, t = s - a;
+    return {s, (a - (s - t)) + (b - t)};
+}
+Pair operator*(const Pair& a, const Pair& b) {
+    const double h = a.h * b.h, l = std::fma(a.h, b.h, -h) + (a.h * b.l + a.l * b.h);
+    return pair_sum(h, l);
+}
+Pair operator+(const Pair& a, const Pair& b) {
+    const Pair s = pair_sum(a.h, b.h);
+    return pair_sum(s.h, s.l + a.l + b.l);
+}
+Pair inverse(const Pair& a) {
+    const double x = 1.0 / a.h;
+    const Pair r = Pair{-a.h, -a.l} * Pair{x, 0.0} + Pair{1.0, 0.0};
+    return pair_sum(x, x * r.h);
+}
+Fix62 fixed62(const Pair& a) {  // a > 0
+    int e = 0;
+    std::frexp(a.h, &e);  // a.h in [2^(e-1), 2^e)
+    uint64_t m = (uint64_t)std::ldexp(a.h, 63 - e) + (uint64_t)(int64_t)std::ldexp(a.l, 63 - e);
+    Fix62 f{m, e - 1};
+    if (m < (1ULL << 62)) f = {m << 1, e - 2};  // a power of two less a little
+    return f;
+}
+
+// Steps and tables of a circuit on nl local positions (and a cluster's top one); false where the general kernel
+// is to run.  zpos: where qubit 0 is at the end.  slow_gates: those that keep the general code, by position.
+bool plan_fast(int n, int nl, int workers, const std::vector<TrajGate>& gates, const KrausParams& kp, std::vector<FastStep>& steps,
+               std::vector<double>& tabs, std::vector<TrajGate>& slow_gates, int& zpos) {
+    if (nl < kFastMinQubits) return false;
+    // the Kraus factors are the general kernel's (and the oracle's) rounded roots
+    const Pair one{1.0, 0.0}, g = Pair{kp.sq1mg, 0.0} * Pair{kp.sq1ml, 0.0};
+    std::vector<Pair> p(n, one);  // by position
+    std::vector<int> pos(n), who(n);
+    for (int q = 0; q < n; ++q) pos[q] = who[q] = q;
+    // each qubit's gates, for the exchanges
+    std::vector<std::vector<int>> uses(n);
+    std::vector<size_t> used(n, 0);
+    for (size_t i = 0; i < gates.size(); ++i)
+        for (int k = 0; k < gates[i].nt; ++k) uses[gates[i].q[k]].push_back((int)i);
+    auto put = [&](const std::vector<double>& v) {
+        const int at = (int)tabs.size();
+        tabs.insert(tabs.end(), v.begin(), v.end());
+        return at;
+    };
+    auto heads = [&](bool inverted) {
+        std::vector<double> v(n);
+        for (int q = 0; q < n; ++q) v[q] = inverted ? inverse(p[q]).h : p[q].h;
+        return v;
+    };
+    auto scale = [&]() {  // apply all pending factors
+        bool any = false;
+        for (const Pair& v : p) any = any || v.h != 1.0 || v.l != 0.0;
+        if (!any) return;
+        FastStep s{};
+        s.kind = FS_SCALE;
+        s.pend = put(heads(false));
+        steps.push_back(s);
+        std::fill(p.begin(), p.end(), one);
+    };
+    for (size_t i = 0; i < gates.size(); ++i) {
+        const TrajGate& G = gates[i];
+        const ExecOp& o = G.op;
+        if (o.kind == EX_U2) return false;  // need not be unitary: P(1) has no bound
+        FastStep s{};
+        double v = 0.0;
+        if (o.kind == EX_RT || o.kind == EX_RC || o.kind == EX_RXT || o.kind == EX_RXC) {
+            s.kind = o.kind == EX_RT ? FS_RT : o.kind == EX_RC ? FS_RC : o.kind == EX_RXT ? FS_RXT : FS_RXC;
+            std::memcpy(&v, &o.c[2], sizeof(v));
+        } else if (o.kind == EX_H) {  // (a + b, -(b - a)) / sqrt(2)
+            s.kind = FS_RT;
+            v = -1.0;
+        } else if (o.kind == EX_DIAG) {
+            double d[4];
+            for (int k = 0; k < 4; ++k) std::memcpy(&d[k], &o.c[k], sizeof(double));
+            // diag(d0, d1) = d0 diag(1, d1 conj(d0)) for |d0| = 1
+            s.kind = FS_PHASE;
+            s.c0 = d[2] * d[0] + d[3] * d[1];
+            s.c1 = d[3] * d[0] - d[2] * d[1];
+        } else if (o.kind == EX_CNOT) {
+            s.kind = FS_CNOT;
+        } else if (o.kind == EX_MCZ && G.nt == 2) {
+            s.kind = FS_CZ;
+        }
+        // far from their true size the amplitudes would leave the format's range
+        double spread = 0.0;
+        for (const Pair& x : p) spread += std::fabs(std::log2(std::fabs(x.h)));
+        if (spread > 60.0 || s.kind == FS_SLOW) scale();
+        if (s.kind == FS_SLOW) {
+            TrajGate m = G;
+            for (int k = 0; k < G.nt; ++k) m.q[k] = pos[G.q[k]];
+            m.op.q0 = pos[o.q0];
+            m.op.mask = 0;
+            for (int q = 0; q < n; ++q)
+                if ((o.mask >> q) & 1) m.op.mask |= 1ULL << pos[q];
+            s.gate = (int)slow_gates.size();
+            slow_gates.push_back(m);
+            steps.push_back(s);
+            continue;
+        }
+        for (int k = 0; k < G.nt; ++k) {
+            if (pos[G.q[k]] < nl) continue;
+            // the top qubit changes places with the local one that is longest without a gate
+            int out = -1;
+            long far = -1;
+            for (int q = 0; q < n; ++q) {
+                if (pos[q] >= nl || q == G.q[0] || (G.nt > 1 && q == G.q[1])) continue;
+                while (used[q] < uses[q].size() && uses[q][used[q]] < (int)i) ++used[q];
+                const long next = used[q] < uses[q].size() ? uses[q][used[q]] : (long)gates.size() + 1;
+                if (next > far) {
+                    far = next;
+                    out = q;
+                }
+            }
+            FastStep x{};
+            x.kind = FS_SWAP;
+            x.q = pos[out];
+            steps.push_back(x);
+            std::swap(p[pos[out]], p[nl]);
+            std::swap(who[pos[out]], who[nl]);
+            for (int a = 0; a < n; ++a) pos[who[a]] = a;
+        }
+        s.q = pos[G.q[0]];
+        s.t = G.nt > 1 ? pos[G.q[1]] : s.q;
+        // Factors of the positions that a pass loops over cost it a multiply-add per summed amplitude (14 % of a
+        // rotation, 25 % of a CNOT); applying them, half a rotation.  So they go first where 6 gates off those
+        // positions follow.
+        int lw = 0;
+        while (2 << lw <= workers) ++lw;
+        auto looped = [&]() {
+            int index = 0;
+            bool any = false;
+            for (int q = 0; q < nl; ++q)
+                if (q != s.q && q != s.t && index++ >= lw) any = any || p[q].h != 1.0;
+            return any;
+        };
+        bool weighed = looped();
+        if (weighed) {
+            size_t end = i;
+            auto off = [&](const TrajGate& x) {
+                for (int k = 0; k < x.nt; ++k)
+                    if (pos[x.q[k]] >= lw) return false;
+                return true;
+            };
+            while (end < gates.size() && end < i + 6 && off(gates[end])) ++end;
+            if (end == i + 6) {
+                std::vector<double> w(1, 1.0);
+                for (int q = lw; q < nl; ++q) {
+                    const size_t len = w.size();
+                    for (size_t k = 0; k < len; ++k) w.push_back(w[k] * p[q].h);
+                    p[q] = one;
+                }
+                FastStep x{};
+                x.kind = FS_SCALE;
+                x.flat = 1;
+                x.tab = put(w);
+                x.ntab = (int)w.size();
+                steps.push_back(x);
+                weighed = false;
+            }
+        }
+        s.flat = !weighed;
+        Pair &pq = p[s.q], &pt = p[s.t], f = one, f0 = one, f1 = one;
+        if (s.kind == FS_CNOT || s.kind == FS_CZ) {
+            // (c, t) held short of pc^c pt^t; a CNOT's (1, 0) becomes (1, 1), short of pc only: with the control
+            // short of pc pt from now on, that amplitude is held times pt^-2
+            if (s.kind == FS_CNOT) {
+                s.c0 = inverse(pt * pt).h;
+                pq = pq * pt;
+            }
+            f0 = pq * pq;
+            f1 = pt * pt;
+            s.k0 = f1.h;
+            s.k1 = (f0 * g * g).h;
+        } else {
+            if (s.kind != FS_PHASE) {
+                const bool tan_form = s.kind == FS_RT || s.kind == FS_RXT;
+                const Pair vp = Pair{v, 0.0} * pq, vi = Pair{v, 0.0} * inverse(pq);
+                s.c0 = tan_form ? vp.h : vi.h;
+                s.c1 = tan_form ? vi.h : vp.h;
+                // the factor that keeps the rounded matrix's determinant: 1 / (1 + c0 c1) squared, times p^2 where
+                // both rows are short of it
+                f = inverse(one + Pair{s.c0, 0.0} * Pair{s.c1, 0.0});
+                if (!tan_form) {
+                    f = f * (pq * pq);
+                    pq = inverse(pq);
+                }
+                if (o.kind == EX_H) pq = {-pq.h, -pq.l};
+            }
+            f0 = pq * pq;
+        }
+        s.f = fixed62(f);
+        s.f0 = fixed62(f * f0);
+        s.f1 = fixed62(f * f1);
+        // weights: products of the other positions' squares, in the order of the pass's index bits
+        std::vector<double> sq;
+        for (int q = 0; q < nl; ++q)
+            if (q != s.q && q != s.t) sq.push_back((p[q] * p[q]).h);
+        auto products = [&](size_t first, size_t count, size_t size, double start) {
+            std::vector<double> out(size, start);
+            size_t len = 1;
+            for (size_t b = 0; b < count && first + b < sq.size(); ++b, len *= 2)
+                for (size_t k = 0; k < len; ++k) out[len + k] = out[k] * sq[first + b];
+            return out;
+        };
+        s.tab = put(products(0, 5, kTabLanes, 1.0));
+        put(products(0, 5, kTabLanes, nl < n ? (p[nl] * p[nl]).h : 1.0));
+        const size_t rest = sq.size() > 5 ? sq.size() - 5 : 0;
+        put(products(5, rest, (size_t)1 << rest, 1.0));
+        s.ntab = (int)tabs.size() - s.tab;
+        s.pend = put(heads(false));
+        pq = pq * g;
+        if (s.kind >= FS_CNOT) pt = pt * g;
+        put(heads(true));
+        steps.push_back(s);
+        if (tabs.size() > kFastTabWords) return false;
+    }
+    scale();
+    zpos = pos[0];
+    // a gate that keeps the general code costs a pass for the factors as well: 200 random gates on 14 qubits with none
+    // of them, 1/10, 1/4, 2/5: 14.6, 16.9, 18.5, 24.7 ms against the general kernel's 28.1, 27.7, 26.6, 24.7
+    return slow_gates.size() * 4 <= gates.size();
+}
+
+constexpr int kMaxArgs = 14;
+void launch_args(llg_traj* h, KrausParams* kp, uint64_t* begin, uint64_t* count, uint8_t** log, int64_t* stride, void** args) {
+    int k = 0;
+    args[k++] = &h->n;
+    if (h->fast) {
+        args[k++] = &h->d_slow;
+        args[k++] = &h->d_steps;
+        args[k++] = &h->nsteps;
+        args[k++] = &h->d_tabs;
+        args[k++] = &h->zpos;
+        args[k++] = kp;
+    } else {
+        args[k++] = &h->d_gates;
+        args[k++] = &h->ngates;
+        args[k++] = kp;
+        args[k++] = &h->d_obs;
+    }
+    args[k++] = begin;
+    args[k++] = count;
+    args[k++] = &h->d_z0;
+    args[k++] = &h->d_jumps;
+    args[k++] = log;
+    args[k++] = stride;
+    args[k++] = &h->d_margin;
+}
+
 // Sets (cluster, threads), sizes the persistent grid from the occupancy and captures the graph.
 int configure(llg_traj* h, int cl, int threads) {
     size_t smem = 0;
     const int th = resolve_threads(h->n, h->P, cl, threads, &smem);
     if (!th) return set_error(LLG_EINVAL, "traj: cluster " + std::to_string(cl) + " with " + std::to_string(threads) +
                                               " threads cannot hold a " + std::to_string(h->n) + "-qubit state");
-    const void* fn = kernel_for(h->P, cl);
+    drop_graph(h);
+    drop_fast(h);
+    if (fast_noise(h->P, h->kp)) {
+        std::vector<FastStep> steps;
+        std::vector<double> tabs;
+        std::vector<TrajGate> slow;
+        if (plan_fast(h->n, cl == 2 ? h->n - 1 : h->n, fast_threads(cl == 2 ? h->n - 1 : h->n, th) - 32, h->gates, h->kp, steps, tabs, slow, h->zpos)) {
+            // one buffer: steps, gates, tables (both records are multiples of 8 bytes)
+            const size_t a = steps.size() * sizeof(FastStep), b = slow.size() * sizeof(TrajGate), c = tabs.size() * sizeof(double);
+            std::vector<unsigned char> all(a + b + c);
+            std::memcpy(all.data(), steps.data(), a);
+            if (b) std::memcpy(all.data() + a, slow.data(), b);
+            if (c) std::memcpy(all.data() + a + b, tabs.data(), c);
+            unsigned char* d = nullptr;
+            cudaError_t e = all.empty() ? cudaSuccess : cudaMalloc(&d, all.size());
+            if (e == cudaSuccess && d) e = cudaMemcpy(d, all.data(), all.size(), cudaMemcpyHostToDevice);
+            h->d_steps = reinterpret_cast<FastStep*>(d);
+            h->d_slow = reinterpret_cast<TrajGate*>(d + a);
+            h->d_tabs = reinterpret_cast<double*>(d + a + b);
+            h->nsteps = (int)steps.size();
+            h->fast = e == cudaSuccess;
+            if (!h->fast) {  // without room the general kernel runs
+                cudaGetLastError();
+                drop_fast(h);
+            }
+        }
+    }
+    const int launch = h->fast ? fast_threads(cl == 2 ? h->n - 1 : h->n, th) : th;
+    const void* fn = kernel_for(h->P, cl, h->fast);
     int dev = 0, sms = 1, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, th, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, launch, smem);
     if (e != cudaSuccess) return cuda_fail(e, "trajectory kernel attributes");
     if (per_sm < 1) return set_error(LLG_EINVAL, "traj: configuration does not fit an SM");
     uint64_t groups = (uint64_t)sms * per_sm / cl;
     groups = std::max<uint64_t>(1, std::min<uint64_t>(groups, h->max_traj));
     groups = std::min<uint64_t>(groups, (uint64_t)(kMaxGrid / cl));  // margin buffer holds kMaxGrid CTAs
-    drop_graph(h);
     h->cl = cl;
     h->threads = th;
+    h->launch = launch;
     h->smem = smem;
     h->grid = (int)(groups * cl);
     // capture one launch; its arguments are replaced before every replay
-    int n = h->n, ngates = h->ngates;
     uint64_t b0 = 0, c0 = 0;
     uint8_t* lg = nullptr;
     int64_t ls = 0;
-    void* args[] = {&n, &h->d_gates, &ngates, &h->kp, &h->d_obs, &b0, &c0, &h->d_z0, &h->d_jumps, &lg, &ls, &h->d_margin};
+    void* args[kMaxArgs];
+    launch_args(h, &h->kp, &b0, &c0, &lg, &ls, args);
     e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        cudaError_t le = cudaLaunchKernel(fn, dim3(h->grid), dim3(th), args, smem, h->stream);
+        cudaError_t le = cudaLaunchKernel(fn, dim3(h->grid), dim3(launch), args, smem, h->stream);
         e = cudaStreamEndCapture(h->stream, &h->graph);
         if (le != cudaSuccess) e = le;
     }
@@ -815,16 +1136,15 @@ int configure(llg_traj* h, int cl, int threads) {
 
 // Replays the graph for trajectories [begin, begin + count) (outputs stay on the device).
 int replay(llg_traj* h, uint64_t seed, uint64_t begin, uint64_t count, uint8_t* d_log, int64_t log_stride) {
-    int n = h->n, ngates = h->ngates;
     KrausParams kp = h->kp;
     kp.seed = seed;
-    void* args[] = {&n,     &h->d_gates, &ngates,     &kp,        &h->d_obs,    &begin,
-                    &count, &h->d_z0,    &h->d_jumps, &d_log,     &log_stride, &h->d_margin};
+    void* args[kMaxArgs];
+    launch_args(h, &kp, &begin, &count, &d_log, &log_stride, args);
     cudaKernelNodeParams p;
     std::memset(&p, 0, sizeof(p));
-    p.func = const_cast<void*>(kernel_for(h->P, h->cl));
+    p.func = const_cast<void*>(kernel_for(h->P, h->cl, h->fast));
     p.gridDim = dim3(h->grid);
-    p.blockDim = dim3(h->threads);
+    p.blockDim = dim3(h->launch);
     p.sharedMemBytes = (unsigned)h->smem;
     p.kernelParams = args;
     cudaError_t e = cudaGraphExecKernelNodeSetParams(h->exec, h->node, &p);
@@ -975,6 +1295,7 @@ int create_handle(int n, int precision, const std::vector<TrajGate>& gates, int6
     h->kp = kp;
     h->obs = ob;
     h->shape_key = shape_key;
+    if (fast_noise(precision, kp)) h->gates = gates;
     int rc = LLG_OK;
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_gates, std::max<size_t>(gates.size(), 1) * sizeof(TrajGate));
@@ -1014,6 +1335,7 @@ int llg_traj_destroy(llg_traj* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     drop_graph(h);
     cudaFree(h->d_gates);
+    drop_fast(h);
     cudaFree(h->d_z0);
     cudaFree(h->d_jumps);
     cudaFree(h->d_margin);
