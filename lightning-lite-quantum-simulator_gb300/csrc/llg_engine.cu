@@ -323,37 +323,57 @@ int run_tiles(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
     return LLG_OK;
 }
 
-// A flush as dense 5-qubit blocks on the tensor cores (llg_blockplan.cpp, llg_gateblock.cu), the rest
-// of the plan made while the first blocks run.  nops: the flush's gates (bounds the plan's size).
-// mirror / mirrored: as for run_tiles.
-int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
+constexpr int kBlockGroup = 16;   // blocks planned, uploaded and launched at a time
+constexpr int kBlockSlots = 128;  // blocks whose weights are held at once
+static_assert(kBlockSlots % kBlockGroup == 0, "a group's weights are contiguous");
+
+size_t block_slots(size_t nops) {
+    return nops <= kBlockSlots ? (std::max<size_t>(nops, 1) + kBlockGroup - 1) / kBlockGroup * kBlockGroup : kBlockSlots;
+}
+
+// Buffers for a flush of nops gates in blocks; *room: false where there is no memory for them (the flush then
+// takes tile passes, which need less).
+int ensure_blocks(llg_state* st, size_t nops, bool* room) {
     size_t mbytes = 0;
     for (const MatrixOp& m : st->matrices) mbytes += m.m.size() * sizeof(double);
-    constexpr int kGroup = 16;   // blocks planned, uploaded and launched at a time
-    constexpr int kSlots = 128;  // blocks whose weights are held at once
-    static_assert(kSlots % kGroup == 0, "a group's weights are contiguous");
-    const size_t wb = gate_block_weight_bytes(st->P);
-    const size_t slots = nops <= kSlots ? (std::max<size_t>(nops, 1) + kGroup - 1) / kGroup * kGroup : kSlots;
+    const size_t weights = block_slots(nops) * gate_block_weight_bytes(st->P);
     // a group's upload: its blocks' steps, its gates, their matrices; every group has its own part of the buffers
-    const size_t bytes = (nops / kGroup + 2) * (kGroup * sizeof(BlockStep) + 1024) + nops * sizeof(BlockGate) + mbytes;
-    if (bytes > st->d_bplan_cap || slots * wb > st->d_bweights_cap)
+    const size_t bytes = (nops / kBlockGroup + 2) * (kBlockGroup * sizeof(BlockStep) + 1024) + nops * sizeof(BlockGate) + mbytes;
+    *room = true;
+    if (bytes > st->d_bplan_cap || weights > st->d_bweights_cap)
         LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
     if (bytes > st->d_bplan_cap) {
         if (st->d_bplan) cudaFree(st->d_bplan);
         if (st->h_bplan) cudaFreeHost(st->h_bplan);
         st->d_bplan = st->h_bplan = nullptr;
         st->d_bplan_cap = 0;
-        LLG_CUDA(cudaMalloc(&st->d_bplan, bytes), "cudaMalloc(block plan)");
-        LLG_CUDA(cudaHostAlloc((void**)&st->h_bplan, bytes, cudaHostAllocDefault), "cudaHostAlloc(block plan)");
-        st->d_bplan_cap = bytes;
+        *room = cudaMalloc(&st->d_bplan, bytes) == cudaSuccess &&
+                cudaHostAlloc((void**)&st->h_bplan, bytes, cudaHostAllocDefault) == cudaSuccess;
+        if (*room) st->d_bplan_cap = bytes;
     }
-    if (slots * wb > st->d_bweights_cap) {
+    if (*room && weights > st->d_bweights_cap) {
         if (st->d_bweights) cudaFree(st->d_bweights);
         st->d_bweights = nullptr;
         st->d_bweights_cap = 0;
-        LLG_CUDA(cudaMalloc(&st->d_bweights, slots * wb), "cudaMalloc(block weights)");
-        st->d_bweights_cap = slots * wb;
+        *room = cudaMalloc(&st->d_bweights, weights) == cudaSuccess;
+        if (*room) st->d_bweights_cap = weights;
     }
+    if (!*room) {
+        cudaGetLastError();
+        if (!st->d_bplan_cap && st->d_bplan) {
+            cudaFree(st->d_bplan);
+            st->d_bplan = nullptr;
+        }
+    }
+    return LLG_OK;
+}
+
+// A flush as dense 5-qubit blocks on the tensor cores (llg_blockplan.cpp, llg_gateblock.cu), the rest
+// of the plan made while the first blocks run.  nops: the flush's gates, for which ensure_blocks() found room.
+// mirror / mirrored: as for run_tiles.
+int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
+    constexpr int kGroup = kBlockGroup;
+    const size_t wb = gate_block_weight_bytes(st->P), slots = block_slots(nops);
     LLG_CUDA(cudaEventSynchronize(st->ops_done), "cudaEventSynchronize");  // the staging buffer's last copies
     st->block_tc_launched = true;
     const BlockPlan& plan = planner.plan;
@@ -523,7 +543,10 @@ int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
     if (blocks_allowed(st) && st->log2_norm <= limit && has_block_plan(st->n, q.data(), (int)q.size())) {
         BlockPlanner planner(st->n, q.data(), (int)q.size(), false, &st->matrices);
         planner.advance(8);
-        if (blocks_pay(st->P, st->n, planner.plan)) {
+        bool room = blocks_pay(st->P, st->n, planner.plan);
+        if (room)
+            if (int rc = ensure_blocks(st, q.size(), &room)) return rc;
+        if (room) {
             const int rc = run_blocks(st, planner, q.size(), mirror, mirrored);
             for (const MatrixOp& m : st->matrices) note_growth(st, m.k, m.m.data());
             st->matrices.clear();
