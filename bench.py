@@ -4,20 +4,22 @@
 Workload (seeded, synthetic): a 30-qubit state from |0..0> (16 GiB of complex128), 20 layers of
 RX, RY, RZ on every qubit (angles U[0, 2pi)) plus a CNOT brickwork on (i, i+1) with alternating
 offsets -- 1800 rotations + 290 CNOTs = 2090 gates.  One step = reset the state and run the whole
-circuit through the engine: fused shared-memory tile passes with carried phases and phase tables,
-complex128 in IEEE binary64 (the reference's arithmetic).
+circuit through the engine, which fuses it into dense 5-qubit blocks on the tensor cores (exact
+products of 8-bit digits, errors no larger than IEEE binary64 arithmetic's) or, where that is
+faster, into shared-memory tile passes on the FP64 pipe; complex128 amplitudes in IEEE binary64.
 
 Printed as one JSON line:
   value        gates/s over the whole job (logical, pre-fusion gates), device-timed with CUDA
                events on the engine's stream, inputs resident in HBM;
   e2e          the same metric through the drop-in API (quantum_sim_v3.StateVector) with the
                final amplitudes read back to host memory (get_numpy_view) every step;
-  roofline     the dominant kernel (the tile pass): algorithmic bytes per launch (32 B x 2^30
-               amplitudes: one read and one write of the state) / its mean launch time, measured
+  roofline     the dominant kernel (the gate block or tile pass): algorithmic bytes per launch (32 B x
+               2^30 amplitudes: one read and one write of the state) / its mean launch time, measured
                with CUDA events around every launch inside the timed region;
-  fp64_roofline the bound that applies to IEEE complex128 on this GPU: the plan's algorithmic FP64
-               multiply-adds per step over the tile passes' time, against the FP64 FMA rate
-               measured live by a throughput kernel;
+  tensor_roofline  gate blocks: fp16 operations of the digit products over the blocks' time, against
+               the measured rate of a 16-bit library product under the power cap;
+  fp64_roofline    tile passes: the plan's algorithmic FP64 multiply-adds per step over their time,
+               against the FP64 FMA rate measured live by a throughput kernel;
   cpu_baseline the reference's CPU algorithms on the machine's host cores (the oracle's restatement,
                checked bit-exact against the reference build): the per-gate ll::StateVectorBackend
                path and the fused path (GateFuser.fuse_circuit + apply_gate_cache_optimized), each
@@ -373,6 +375,21 @@ def profile_traffic(precision: str, n: int):
     return None
 
 
+def per_block_s(ms: float, count: int) -> float:
+    return ms / count / 1e3
+
+
+def tensor_peak():
+    """(TFLOP/s of the measured 16-bit library product under the power cap, its kind)."""
+    path = os.path.join(REPO, "MEASURED_PEAKS.json")
+    if os.path.exists(path):
+        with open(path) as f:
+            v = json.load(f).get("bf16_tflops_sustained")
+        if v:
+            return float(v), "measured"
+    return 1700.0, "fallback"
+
+
 def measure_circuit(args, torch, precision, n, ops, steps, warmup, world, sampler_gpu=None, keep=False):
     """Timed steps of the layered circuit at `precision`: reset, apply, flush per step, CUDA events
     on the engine's stream, per-launch events for the tile passes.  Returns a dict (and the state
@@ -437,26 +454,44 @@ def measure_circuit(args, torch, precision, n, ops, steps, warmup, world, sample
                                          device="cuda")
     elapsed_ms = slowest_s * 1e3
     tile_ms, tile_n = prof["tile"] if prof["tile"][1] else prof["gate"]
+    # a flush that the engine planned as gate blocks launches those (and their weights) instead of the tile passes
+    blocks, upload_bytes = 0, xops.nbytes + table_bytes
+    if tuning["fuse_mode"] == "tile" and n >= 12 and prof["tile"][1] and prof["tile"][1] != len(passes) * steps:
+        bsteps, bgates = llgpu.block_plan_export(n, ops)
+        blocks, sweeps = int(np.sum(bsteps["is_block"] != 0)), len(bsteps)
+        upload_bytes, table_bytes = bsteps.nbytes + bgates.nbytes, 0
+        passes, tile_n = np.zeros(sweeps), blocks * steps
     peak, peak_kind = peaks()
     per_launch_s = (tile_ms / tile_n) / 1e3 if tile_n else float("nan")
     achieved = state_bytes * 2 / per_launch_s / 1e9 if tile_n else None
     res = {
         "value": value, "unit": "gates/s", "steps": steps, "warmup": warmup, "ms_per_step": elapsed_ms / steps,
-        "gpu_launches": launches, "tile_passes": int(len(passes)), "tile_qubits": tile_q, "fusion": tuning,
+        "gpu_launches": launches, "tile_passes": 0 if blocks else int(len(passes)), "gate_blocks": blocks,
+        "tile_qubits": tile_q, "fusion": tuning,
         "phase_table_bytes": table_bytes,
         "autotune": tune, "state_bytes": state_bytes, "clocks": clocks,
         "sweeps_per_s": len(passes) * steps * world / (elapsed_ms / 1e3),
         "hbm_gbs_algorithmic": len(passes) * 2 * state_bytes * steps * world / (elapsed_ms / 1e3) / 1e9,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": (achieved / peak) if achieved else None, "traffic": profile_traffic(precision, n),
-                     "kernel": (f"k_tile_reg<{TILE_POLICY.get(precision, precision)}> (register-tiled pass)"
+                     "frac": (achieved / peak) if achieved else None,
+                     "traffic": None if blocks else profile_traffic(precision, n),
+                     "kernel": (f"k_gate_block<{TILE_POLICY.get(precision, precision)}> (dense 5-qubit block)" if blocks else
+                                f"k_tile_reg<{TILE_POLICY.get(precision, precision)}> (register-tiled pass)"
                                 if tuning["fuse_mode"] == "reg" else f"k_tile<{TILE_POLICY.get(precision, precision)}> (tile pass)"),
                      "launches": tile_n,
                      "mean_launch_ms": tile_ms / tile_n if tile_n else None, "peak_source": f"{peak_kind} hbm_gbs"},
         "kernel_ms_per_step": {k: v[0] / steps for k, v in prof.items()},
-        "_xops": xops if tuning["fuse_mode"] != "none" else np.zeros(0, dtype=xops.dtype),
+        "_xops": np.zeros(0, dtype=xops.dtype) if blocks or tuning["fuse_mode"] == "none" else xops,
+        "_upload_bytes": int(upload_bytes),
         "_tile_ms_step": prof["tile"][0] / steps,
     }
+    if blocks:
+        # fp16 products of 8-bit digits: S (S + 1) / 2 of M128 N64 K64 per 4096 amplitudes, S = 8 (FP64) or 7
+        products = 36 if is_f64(precision) else 28
+        rate = products * 2.0 * 128 * 64 * 64 * (1 << n) / 4096 / per_block_s(tile_ms, tile_n) / 1e12
+        tpeak, tkind = tensor_peak()
+        res["tensor_roofline"] = {"bound": "fp16 tensor products", "achieved": rate, "peak": tpeak, "unit": "TFLOP/s",
+                                  "frac": rate / tpeak, "peak_source": tkind, "products_per_tile": products}
     if keep:
         return res, st
     st.close()
@@ -498,7 +533,7 @@ def run_ours(args, rank, world, local):
     head = finish_rooflines(head, args.precision, n, fma_rate)
     clocks = head.pop("clocks")
     elem = ELEM_BYTES.get(args.precision, 16)
-    _, xops_e2e, tables_e2e = plan_for(args.precision, n, ops, head["tile_qubits"], head["fusion"]["fuse_mode"] == "reg")
+    upload_e2e = head.pop("_upload_bytes")
 
     # the same circuit in the other precisions, each compared with this (FP64) final state
     variants = None
@@ -514,15 +549,15 @@ def run_ours(args, rank, world, local):
                             "max_abs_diff_rel_to_max_amp": (dmax / amax) if amax else None}
             vst.close()
             if not args.no_e2e:
-                _, vx, vtab = plan_for(prec, n, ops, v["tile_qubits"], v["fusion"]["fuse_mode"] == "reg")
-                v["e2e"] = run_e2e(args, prec, ops, vx, vtab, n, ELEM_BYTES.get(prec, 16), world, torch)
+                v["e2e"] = run_e2e(args, prec, ops, v["_upload_bytes"], n, ELEM_BYTES.get(prec, 16), world, torch)
+            v.pop("_upload_bytes")
             variants[prec] = v
     st.close()
 
     # end to end through the drop-in module: op records in, final amplitudes out, every step
     e2e = None
     if not args.no_e2e:
-        e2e = run_e2e(args, args.precision, ops, xops_e2e, tables_e2e, n, elem, world, torch)
+        e2e = run_e2e(args, args.precision, ops, upload_e2e, n, elem, world, torch)
 
     sweeps = None
     if not args.no_sweeps:
@@ -553,16 +588,21 @@ def run_ours(args, rank, world, local):
         "vs_baseline": None, "dtype": dtype,
         "data": "synthetic (seeded layered circuit)",
         "config": {"workload": f"{n}-qubit complex128 layered circuit: {args.layers} layers of RX/RY/RZ on every "
-                               f"qubit + CNOT brickwork, {ngates} gates, fused into {head['tile_passes']} shared-memory "
-                               f"tile passes of {head['tile_qubits']} qubits", "qubits": n, "layers": args.layers,
-                   "gates": ngates, "tile_passes": head["tile_passes"], "tile_qubits": head["tile_qubits"],
+                               f"qubit + CNOT brickwork, {ngates} gates, fused into " +
+                               (f"{head['gate_blocks']} dense 5-qubit blocks" if head["gate_blocks"] else
+                                f"{head['tile_passes']} shared-memory tile passes of {head['tile_qubits']} qubits"),
+                   "qubits": n, "layers": args.layers, "gates": ngates, "gate_blocks": head["gate_blocks"],
+                   "tile_passes": head["tile_passes"], "tile_qubits": head["tile_qubits"],
                    "precision": args.precision,
-                   "arithmetic": "IEEE binary64 (FP64 pipe)" if is_f64(args.precision) else args.precision,
+                   "arithmetic": args.precision if not is_f64(args.precision) else
+                                 "IEEE binary64 (exact 8-bit digit products on the tensor cores, 64-bit integer sums)"
+                                 if head["gate_blocks"] else "IEEE binary64 (FP64 pipe)",
                    "fusion": head["fusion"], "autotune": head["autotune"],
                    "l2": f"inputs larger than L2 ({head['state_bytes'] / 2**30:g} GiB state), no flush needed"},
         "sweeps_per_s": head["sweeps_per_s"], "hbm_gbs_algorithmic": head["hbm_gbs_algorithmic"],
         "roofline": head["roofline"],
         "fp64_roofline": head.get("fp64_roofline"),
+        "tensor_roofline": head.get("tensor_roofline"),
         "compute_roofline": head.get("compute_roofline"),
         "kernel_ms_per_step": head["kernel_ms_per_step"],
         "gpu_launches": head["gpu_launches"],
@@ -1005,10 +1045,10 @@ def run_dm_bench(args, torch, cpu: bool):
     qubits is a 2n-qubit state.  Amplitude damping (gamma 0.01) on every qubit is a 2-qubit block
     Sum_k K (x) conj(K) on (q, q + n); 2-qubit depolarizing (p 0.01) on (q, q + 1) a 4-qubit block.
     n = 10 is the reference's limit (MAX_DM_QUBITS, a 16 MiB state); n = 13 is a 1 GiB state, larger
-    than L2.  Algorithmic bytes per channel: 32 B x 4^n (every element read and written)."""
+    than L2.  gbs_one_sweep_per_channel: 32 B x 4^n per channel (every element read and written), of
+    which blocks that take several channels move less."""
     import llgpu
 
-    peak, _ = peaks()
     ad = llgpu.amplitude_damping(0.01)
     dp = llgpu.depolarizing(0.01, 2)
     out = {"workload": "density matrices: amplitude damping on every qubit and 2-qubit depolarizing on "
@@ -1033,12 +1073,16 @@ def run_dm_bench(args, torch, cpu: bool):
                     dm.kraus(kops, t)
             st.sync()
             wall = time.perf_counter() - t0
-            ms, cnt = st.profile_read(reset=True)["gate"]
+            prof = st.profile_read(reset=True)
             st.profile(False)
-            per = ms / max(1, cnt) / 1e3
-            gbs = 32 * (1 << (2 * n)) / per / 1e9
+            # channels on their own are "gate" launches; those that the engine joins into blocks are "tile" ones
+            # (a block's read and write of the state serves several channels, and its weights' launch counts too)
+            ms = prof["gate"][0] + prof["tile"][0]
+            per = ms / (reps * len(tg)) / 1e3
             res[name] = {"channels": reps * len(tg), "kernel_ms_per_channel": per * 1e3,
-                         "channels_per_s_wall": reps * len(tg) / wall, "gbs": gbs, "frac_of_hbm": gbs / peak,
+                         "channels_per_s_wall": reps * len(tg) / wall,
+                         "passes": {"channel": prof["gate"][1], "block": prof["tile"][1]},
+                         "gbs_one_sweep_per_channel": 32 * (1 << (2 * n)) / per / 1e9,
                          "block_qubits": 2 * len(tg[0])}
         tr = dm.trace()
         res["trace_minus_1"] = abs(tr - 1.0)
@@ -1115,7 +1159,7 @@ def run_batch_bench(args, torch, cpu: bool):
     return res
 
 
-def run_e2e(args, precision, ops, xops, table_bytes, n, elem, world, torch):
+def run_e2e(args, precision, ops, upload_bytes, n, elem, world, torch):
     import quantum_sim_v3
 
     sv = quantum_sim_v3.StateVector(n, precision)
@@ -1147,8 +1191,8 @@ def run_e2e(args, precision, ops, xops, table_bytes, n, elem, world, torch):
     del sv, view
     return {"value": len(ops) * steps * world / (t1 - t0), "unit": "gates/s", "steps": steps,
             "ms_per_step": 1e3 * (t1 - t0) / steps, "passes_alone_ms": 1e3 * (b - a), "readback_alone_ms": 1e3 * (c - b),
-            "h2d_bytes_per_step": int(xops.nbytes + table_bytes),
-            "h2d_note": "the planned executor ops and phase tables uploaded by the flush",
+            "h2d_bytes_per_step": upload_bytes,
+            "h2d_note": "what the flush uploads: the planned blocks and gates, or executor ops and phase tables",
             "d2h_bytes_per_step": int((1 << n) * 16),
             "api": "quantum_sim_v3.StateVector: reset, apply_ops, get_numpy_view (host copy of all amplitudes; "
                    "the last tile pass writes the pinned host mirror as it stores its tiles)"}

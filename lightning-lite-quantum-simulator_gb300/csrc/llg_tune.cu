@@ -146,6 +146,14 @@ int llg_autotune(llg_state* st, const llg_op* ops, int nops, int sample_ops, llg
         if (!rc) rc = llg_set_fusion(tmp, LLG_FUSE_TILE, 0);
         if (!rc) rc = llg_set_tile_threads(tmp, 0);
         if (!rc) rc = time_sample(tmp, ops, ns, s, a, b, &res.default_ms);
+        // and the first candidate: only it leaves the choice between gate blocks and tile passes to the engine
+        // (a tile width or CTA size set by hand means tile passes).  It is kept as the width that
+        // llg_get_tuning reports and no CTA size, which no other candidate has.
+        if (!rc) {
+            best = res.best_ms = res.default_ms;
+            res.fuse_mode = LLG_FUSE_TILE;
+            rc = llg_get_tuning(tmp, nullptr, &res.tile_qubits, nullptr);
+        }
         for (const Candidate& c : cands) {
             if (rc) break;
             rc = llg_set_fusion(tmp, c.mode, c.tile);
@@ -168,7 +176,8 @@ int llg_autotune(llg_state* st, const llg_op* ops, int nops, int sample_ops, llg
         if (rc) return rc;
         tune_cache_put(key, res);
     }
-    int rc = llg_set_fusion(st, res.fuse_mode, res.tile_qubits);
+    const bool engine = res.fuse_mode == LLG_FUSE_TILE && res.cta_threads == 0;
+    int rc = llg_set_fusion(st, res.fuse_mode, engine ? 0 : res.tile_qubits);
     if (!rc) rc = llg_set_tile_threads(st, res.cta_threads);
     if (rc) return rc;
     if (out) *out = res;
