@@ -29,7 +29,7 @@ Printed as one JSON line:
                largest amplitude, and 1 - fidelity).
 `--impl reference` times the CPU implementation alone as the reference arm.
 
-Beside the headline the line carries, each with its own workload description and, where the
+Beside the headline the record on stderr (the line and its details) carries, each with its own workload description and, where the
 oracle can run a sample of it, a CPU baseline: per-gate and dense-block sweeps against HBM
 (`gate_sweeps`), adjoint gradients against parameter shift (`adjoint`), noisy trajectories
 (`trajectories`), mixed circuit batches (`mixed_batch`), zero-noise extrapolation (`zne`), the
@@ -620,6 +620,13 @@ def run_ours(args, rank, world, local):
         "density_matrix": dmat,
     }
     line["summary"] = summarize(line)
+    # the whole record goes to stderr; the line on stdout stays short enough for readers that keep a few KB of it
+    print(json.dumps(line), file=sys.stderr, flush=True)
+    for form in ("variants", "gate_sweeps", "adjoint", "trajectories", "mixed_batch", "zne", "config1_12q", "trajectory_solver",
+                 "density_matrix"):
+        line.pop(form)
+    if cpu:
+        line["cpu_baseline"] = {k: cpu[k] for k in ("value", "unit", "cores", "kind", "path")}
     print(json.dumps(line), flush=True)
 
 
@@ -635,7 +642,8 @@ def summarize(line: dict) -> dict:
     return {
         "headline_gates_per_s": line["value"], "dtype": line["dtype"],
         "e2e_gates_per_s": get(line, "e2e", "value"),
-        "fp64_roofline_frac": get(line, "fp64_roofline", "frac"), "hbm_roofline_frac": get(line, "roofline", "frac"),
+        "fp64_roofline_frac": get(line, "fp64_roofline", "frac"),
+        "tensor_roofline_frac": get(line, "tensor_roofline", "frac"), "hbm_roofline_frac": get(line, "roofline", "frac"),
         "cpu_gates_per_s": get(line, "cpu_baseline", "value"),
         "df64_gates_per_s": get(line, "variants", "df64", "value"),
         "df64_one_minus_fidelity": get(line, "variants", "df64", "vs_fp64", "one_minus_fidelity"),
@@ -656,7 +664,7 @@ def summarize(line: dict) -> dict:
         "complex128_dense_block_ms": {k: round(v["ms_per_sweep"], 2) for k, v in (get(line, "gate_sweeps", "complex128") or {}).items()
                                       if k.startswith("block")} or None,
         "block5_tensor_core_hbm_frac": get(line, "gate_sweeps", "df64", "block5", "frac"),
-        "dm_depolarizing_2q_df64_hbm_frac": get(line, "density_matrix", "df64_n13", "depolarizing_2q", "frac_of_hbm"),
+        "dm_depolarizing_2q_df64_gbs": get(line, "density_matrix", "df64_n13", "depolarizing_2q", "gbs_one_sweep_per_channel"),
     }
 
 
@@ -1195,7 +1203,7 @@ def run_e2e(args, precision, ops, upload_bytes, n, elem, world, torch):
             "h2d_note": "what the flush uploads: the planned blocks and gates, or executor ops and phase tables",
             "d2h_bytes_per_step": int((1 << n) * 16),
             "api": "quantum_sim_v3.StateVector: reset, apply_ops, get_numpy_view (host copy of all amplitudes; "
-                   "the last tile pass writes the pinned host mirror as it stores its tiles)"}
+                   "the last pass writes the pinned host mirror as it stores its tiles)"}
 
 
 def main():
