@@ -540,7 +540,14 @@ int llg_batch_copy_state(llg_batch* b, int index, double* out) {
     const uint64_t size = 1ULL << cd.n;
     const size_t eb = elem_bytes(b->P);
     double* d_tmp = nullptr;
-    cudaError_t e = cudaMalloc(&d_tmp, size * 16);
+    cudaError_t e = cudaSuccess;
+    if (b->P == LLG_F64) {  // the same layout: one copy
+        e = cudaMemcpyAsync(out, (const char*)b->d_arena + cd.offset * eb, size * eb, cudaMemcpyDeviceToHost, b->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "batch_copy_state");
+        return LLG_OK;
+    }
+    e = cudaMalloc(&d_tmp, size * 16);
     if (e != cudaSuccess) return cuda_fail(e, "batch_copy_state");
     e = launch_to_f64(b->P, (const char*)b->d_arena + cd.offset * eb, d_tmp, size, b->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_tmp, size * 16, cudaMemcpyDeviceToHost, b->stream);
