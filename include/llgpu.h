@@ -404,8 +404,9 @@ int llg_tsolver_plan_export(const llg_tsolver* s, long long* steps, double* h, i
  * planned into shared-memory tile passes of tile_qubits qubits (0: default, 12 or 13 for
  * complex64; LLG_TUNE_AUTO: picked by llg_batch_autotune) and run together from |0..0> in ONE
  * persistent launch: persistent CTAs take (circuit, pass, tile) work items from a queue; a tile
- * waits, with a bounded poll, for the previous pass of its own circuit.  Each run replays a CUDA
- * graph captured at the first run (state reset + the persistent kernel).  The reference runs such
+ * waits, with a bounded poll, for the previous pass of its own circuit.  With tile_qubits 0, complex128
+ * circuits of 12 or more qubits may run as dense 5-qubit blocks on the tensor cores instead, beside the
+ * queue.  Each run replays a CUDA graph captured at the first run (state reset + the kernels).  The reference runs such
  * circuits one at a time on StateVectorBackend (src/StateVectorBackend.h). */
 typedef struct llg_batch llg_batch;
 int llg_batch_create(int count, const int* n_qubits, const llg_op* ops, const int64_t* op_offsets, int precision,
@@ -413,8 +414,8 @@ int llg_batch_create(int count, const int* n_qubits, const llg_op* ops, const in
 int llg_batch_destroy(llg_batch* b);
 /* Builds and times the batch once per (tile width from 8 qubits to the maximum) x (256 or 512
  * threads per CTA), one untimed run each, and returns the fastest in out->tile_qubits and
- * out->cta_threads (cached by the batch's shape).  Batches created with an explicit tile width
- * use 256 threads. */
+ * out->cta_threads (cached by the batch's shape; 0 threads: the default, which leaves the choice of
+ * gate blocks to the engine).  Batches created with an explicit tile width use 256 threads. */
 int llg_batch_autotune(int count, const int* n_qubits, const llg_op* ops, const int64_t* op_offsets, int precision,
                        llg_tune_result* out);
 int llg_batch_config(const llg_batch* b, int* tile_qubits, int* grid, int* cta_threads);

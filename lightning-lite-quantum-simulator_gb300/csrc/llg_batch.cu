@@ -10,6 +10,11 @@
 // later, so the waits always end; they are bounded all the same (spin_limit polls), and a wait
 // that runs out sets an error flag the host reports as LLG_ETIMEOUT instead of hanging.
 // Tiles are read with L1-bypassing loads (other SMs wrote them).
+//
+// IEEE complex128 circuits of 12 or more qubits take dense 5-qubit blocks on the tensor cores instead where
+// that is estimated to be faster (plan_blocks): block r of every circuit runs in the r-th launch, whose CTAs are
+// dealt out to the circuits by their size.  The blocks' digits are made once per batch.  The other circuits'
+// queue runs beside them on a second branch of the graph.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -190,6 +195,14 @@ size_t batch_smem(int t) {
 }  // namespace
 
 struct llg_batch {
+    // gate blocks: per round, its first entry of d_ctas and their number
+    std::vector<std::pair<int, int>> block_rounds;
+    int64_t block_tiles = 0;
+    int block_steps = 0;
+    void* d_weights = nullptr;
+    MixedCta* d_ctas = nullptr;
+    cudaStream_t side = nullptr;  // the tile queue beside the blocks
+    cudaEvent_t fork = nullptr, join = nullptr;
     int P = LLG_DF64;
     int count = 0;
     int tile = 12;
@@ -234,6 +247,8 @@ int setup_batch(llg_batch* b) {
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<P>, b->threads, b->smem)))
         return cuda_fail(e, "batch occupancy");
     b->grid = std::max(1, sms * std::max(per_sm, 1));
+    // beside blocks no CTA without an item: it would only take their shared memory
+    if (!b->block_rounds.empty()) b->grid = (int)std::min<size_t>(b->grid, std::max<size_t>(b->items.size(), 1));
     return LLG_OK;
 }
 
@@ -243,15 +258,27 @@ cudaError_t enqueue_batch(llg_batch* b, long long spin_limit) {
     cudaStream_t s = b->stream;
     cudaError_t e;
     if ((e = cudaMemsetAsync(b->d_arena, 0, b->total_amps * sizeof(typename P::S), s))) return e;
-    k_batch_init<P><<<(b->count + 255) / 256, 256, 0, s>>>(static_cast<typename P::S*>(b->d_arena), b->d_circs, b->count);
-    if ((e = cudaGetLastError())) return e;
     if ((e = cudaMemsetAsync(b->d_next, 0, sizeof(unsigned long long), s))) return e;
     if ((e = cudaMemsetAsync(b->d_completed, 0, b->count * sizeof(unsigned), s))) return e;
-    if ((e = cudaMemsetAsync(b->d_err, 0, sizeof(int), s))) return e;
-    k_batch<P><<<b->grid, b->threads, b->smem, s>>>(static_cast<typename P::S*>(b->d_arena), b->d_circs, b->d_passes,
+    if ((e = cudaMemsetAsync(b->d_err, 0, 2 * sizeof(int), s))) return e;
+    // last, since a block's early launch is an edge from a kernel
+    k_batch_init<P><<<(b->count + 255) / 256, 256, 0, s>>>(static_cast<typename P::S*>(b->d_arena), b->d_circs, b->count);
+    if ((e = cudaGetLastError())) return e;
+    const bool blocks = !b->block_rounds.empty(), both = blocks && !b->items.empty();
+    cudaStream_t q = s;
+    if (both) {
+        if ((e = cudaEventRecord(b->fork, s)) || (e = cudaStreamWaitEvent(b->side, b->fork, 0))) return e;
+        q = b->side;
+    }
+    for (const auto& r : b->block_rounds)
+        if ((e = launch_gate_block_mixed(b->d_arena, r.second, b->d_ctas + r.first, b->d_weights, b->d_err + 1, s))) return e;
+    if (blocks && !both) return cudaSuccess;
+    k_batch<P><<<b->grid, b->threads, b->smem, q>>>(static_cast<typename P::S*>(b->d_arena), b->d_circs, b->d_passes,
                                                        b->d_ops, b->d_items, (long long)b->items.size(), b->d_next,
                                                        b->d_completed, b->d_err, spin_limit, b->d_tables);
-    return cudaGetLastError();
+    if ((e = cudaGetLastError())) return e;
+    if (both && ((e = cudaEventRecord(b->join, b->side)) || (e = cudaStreamWaitEvent(s, b->join, 0)))) return e;
+    return cudaSuccess;
 }
 
 void drop_graph(llg_batch* b) {
@@ -288,16 +315,147 @@ int launch_batch(llg_batch* b, long long spin_limit) {
 
 }  // namespace
 
+namespace {
+
+constexpr int kTileAmps = 4096;  // of a gate block
+constexpr size_t kWeightsCap = (size_t)256 << 20;
+
+struct BlockSet {
+    std::vector<char> in;                          // per circuit: takes blocks
+    std::vector<BlockStep> steps;                  // of all circuits, one after the other
+    std::vector<BlockGate> gates;
+    std::vector<MixedCta> ctas;
+    std::vector<std::pair<int, int>> rounds;
+    int64_t tiles = 0;
+};
+
+// Which circuits take gate blocks, and their launches.  Blocks against tile passes for the batch as a whole, by
+// the same rates as a single state's choice: tiles 3.2 FP64 multiply-adds per amplitude and mixing gate, 4 per
+// diagonal one at 0.56 T a second, 2.6 us a gate at least; a launch of blocks 5 us and 4.5 us for every tile
+// of the CTA that has most.  Measured, tile passes / blocks, random gates: 36 circuits of 10 to 18 qubits and 200
+// gates 1048 / 335 us; 512 of 10 to 22, 152.9 / 43.6 ms; 5 of 12 and 13 qubits and 100 gates 318 / 103 us; 16 of
+// 12 to 16 and 40 gates 312 / 73 us; 200 of 12 qubits and 200 gates, each its own CTA either way, keep 950 us of
+// tile passes.
+bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_t* off, int sms, BlockSet& out) {
+    struct Circuit {
+        int c, n;
+        uint64_t offset;
+        int first;  // step
+        int blocks;
+    };
+    std::vector<Circuit> list;
+    out.in.assign(count, 0);
+    double arith = 0.0, longest = 0.0, small_arith = 0.0, small_longest = 0.0;
+    uint64_t at = 0, total = 0;
+    int alone = 0;  // circuits of one tile that keep the queue
+    for (int c = 0; c < count; ++c) total += 1ULL << n_qubits[c];
+    const size_t cap = std::max<size_t>(kWeightsCap, total * 16) / gate_block_weight_bytes(LLG_F64);
+    for (int c = 0; c < count; ++c) {
+        const int n = n_qubits[c], nops = (int)(off[c + 1] - off[c]);
+        const uint64_t offset = at;
+        const double amps = std::ldexp(1.0, n);
+        at += 1ULL << n;
+        std::vector<llg_op> mine(ops + off[c], ops + off[c + 1]);
+        bool fits = n >= 12 && nops > 0 && has_block_plan(n, mine.data(), nops);
+        for (llg_op& o : mine) {
+            o.param = -1;
+            if (o.kind == LLG_OP_MCZ && __builtin_popcountll(o.mask) > 5) fits = false;
+        }
+        if (!fits) {
+            // about three multiply-adds a gate
+            small_arith += 2.0 * nops * amps / 0.56e12;
+            small_longest = std::max(small_longest, 2.0e-6 * nops);
+            ++alone;
+            continue;
+        }
+        BlockPlanner planner(n, mine.data(), nops, true);
+        while (planner.advance(64)) {
+        }
+        const BlockPlan& p = planner.plan;
+        if (out.steps.size() + p.steps.size() > cap) {
+            small_arith += (3.2 * p.mixing_1q + 4.0 * p.diag_1q) * amps / 0.56e12;
+            continue;
+        }
+        list.push_back({c, n, offset, (int)out.steps.size(), (int)p.steps.size()});
+        for (BlockStep st : p.steps) {
+            st.gate_begin += (int)out.gates.size();
+            out.steps.push_back(st);
+        }
+        out.gates.insert(out.gates.end(), p.gates.begin(), p.gates.end());
+        arith += (3.2 * p.mixing_1q + 4.0 * p.diag_1q) * amps / 0.56e12;
+        longest = std::max(longest, 2.6e-6 * (double)p.gates.size());
+    }
+    if (list.empty()) return false;
+    // large circuits first, so that a launch does not end with one
+    std::stable_sort(list.begin(), list.end(), [](const Circuit& x, const Circuit& y) { return x.n > y.n; });
+    // SMs that the queue's circuits hold for a while are left out of the deal
+    const int budget = std::max(sms / 2, sms - std::min(alone, sms / 8));
+    double t_blocks = 0.0;
+    for (int r = 0;; ++r) {
+        uint64_t tiles = 0;
+        int active = 0;
+        for (const Circuit& k : list)
+            if (r < k.blocks) {
+                tiles += (1ULL << k.n) / kTileAmps;
+                ++active;
+            }
+        if (!active) break;
+        // tiles a CTA: the fewest for which one wave of CTAs does; with many circuits, several waves of 4 or more
+        uint64_t per = std::max<uint64_t>(1, (tiles + budget - 1) / budget);
+        auto needed = [&](uint64_t m) {
+            uint64_t ctas = 0;
+            for (const Circuit& k : list)
+                if (r < k.blocks) ctas += ((1ULL << k.n) / kTileAmps + m - 1) / m;
+            return ctas;
+        };
+        const bool one_wave = active <= budget / 2;
+        if (one_wave)
+            while (needed(per) > (uint64_t)budget) ++per;
+        else
+            per = std::max<uint64_t>(4, per / 4);
+        const int first = (int)out.ctas.size();
+        for (const Circuit& k : list) {
+            if (r >= k.blocks) continue;
+            const uint64_t t = (1ULL << k.n) / kTileAmps, share = (t + per - 1) / per;
+            const BlockStep& st = out.steps[k.first + r];
+            for (uint64_t i = 0; i < share; ++i) {
+                MixedCta m;
+                std::memset(&m, 0, sizeof(m));
+                m.offset = k.offset;
+                m.weights = (uint32_t)(k.first + r);
+                m.first = (uint32_t)i;
+                m.step = (uint32_t)share;
+                m.n = k.n;
+                for (int b = 0; b < 5; ++b) {
+                    m.q[b] = st.q[b];
+                    m.tmask |= 1ULL << st.q[b];
+                }
+                out.ctas.push_back(m);
+            }
+        }
+        out.rounds.push_back({first, (int)out.ctas.size() - first});
+        out.tiles += (int64_t)tiles;
+        t_blocks += 5e-6 + 4.5e-6 * (one_wave ? (double)per : (double)tiles / budget + per);
+    }
+    for (const Circuit& k : list) out.in[k.c] = 1;
+    return std::max(t_blocks, std::max(small_arith, small_longest)) <
+           0.9 * std::max(arith + small_arith, std::max(longest, small_longest));
+}
+
+}  // namespace
+
 extern "C" {
 
 static int batch_build(int count, const int* n_qubits, const llg_op* ops, const int64_t* op_offsets, int precision,
-                       int tile, int threads, llg_batch** out) {
+                       int tile, int threads, bool engine, llg_batch** out) {
     llg_batch* b = new llg_batch();
     b->threads = threads;
     b->P = precision;
     b->count = count;
     b->tile = tile;
     std::vector<std::vector<std::pair<int, int>>> rounds;  // per pass round j: (circuit, tiles)
+    BlockSet set;
+    set.in.assign(count, 0);
     for (int c = 0; c < count; ++c) {
         const int n = n_qubits[c];
         const int64_t o0 = op_offsets[c], o1 = op_offsets[c + 1];
@@ -316,11 +474,27 @@ static int batch_build(int count, const int* n_qubits, const llg_op* ops, const 
                 return set_error(LLG_EINVAL, "batch_create: circuit " + std::to_string(c) + " op " + std::to_string(i - o0));
             }
         }
+    }
+    if (engine && precision == LLG_F64) {
+        int dev = 0, sms = 1;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (plan_blocks(count, n_qubits, ops, op_offsets, sms, set)) {
+            b->block_rounds = set.rounds;
+            b->block_tiles = set.tiles;
+            b->block_steps = (int)set.steps.size();
+        } else {
+            set.in.assign(count, 0);
+        }
+    }
+    for (int c = 0; c < count; ++c) {
+        const int n = n_qubits[c];
+        const int64_t o0 = op_offsets[c], o1 = op_offsets[c + 1];
         Plan plan;
         std::string err;
         // 16-byte precisions gather diagonal factors into phase tables (one table buffer for the
         // batch; each circuit's EX_PTAB offsets are shifted to its part of it)
-        if (!plan_tiles(n, ops + o0, (int)(o1 - o0), tile, precision, plan, err, false, ZYZ_DEFAULT,
+        if (!set.in[c] && !plan_tiles(n, ops + o0, (int)(o1 - o0), tile, precision, plan, err, false, ZYZ_DEFAULT,
                         precision != LLG_F32)) {
             delete b;
             return set_error(LLG_EINVAL, "batch_create: " + err);
@@ -369,7 +543,34 @@ static int batch_build(int count, const int* n_qubits, const llg_op* ops, const 
     alloc((void**)&b->d_items, b->items.size() * sizeof(Item), "work queue");
     alloc((void**)&b->d_next, sizeof(unsigned long long), "queue head");
     alloc((void**)&b->d_completed, count * sizeof(unsigned), "counters");
-    alloc((void**)&b->d_err, sizeof(int), "error flag");
+    alloc((void**)&b->d_err, 2 * sizeof(int), "error flag");
+    if (!b->block_rounds.empty() && !rc) {
+        // the blocks' digits, once; without room for them the batch is built on tile passes
+        BlockGate* d_gates = nullptr;
+        BlockStep* d_steps = nullptr;
+        auto put = [&](auto*& d, const auto& v) {
+            const size_t bytes = v.size() * sizeof(v[0]);
+            if (e == cudaSuccess) e = cudaMalloc(&d, bytes);
+            if (e == cudaSuccess) e = cudaMemcpy(d, v.data(), bytes, cudaMemcpyHostToDevice);
+        };
+        put(d_gates, set.gates);
+        put(d_steps, set.steps);
+        put(b->d_ctas, set.ctas);
+        if (e == cudaSuccess) e = cudaMalloc(&b->d_weights, set.steps.size() * gate_block_weight_bytes(LLG_F64));
+        if (e == cudaSuccess)
+            e = launch_gate_block_weights(LLG_F64, d_gates, d_steps, (int)set.steps.size(), b->d_weights, b->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming);
+        cudaFree(d_gates);
+        cudaFree(d_steps);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            llg_batch_destroy(b);
+            return batch_build(count, n_qubits, ops, op_offsets, precision, tile, threads, false, out);
+        }
+    }
     auto up = [&](void* dst, const void* src, size_t bytes) {
         if (rc || bytes == 0) return;
         if (cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) rc = set_error(LLG_ECUDA, "batch_create: upload");
@@ -400,12 +601,13 @@ int llg_batch_create(int count, const int* n_qubits, const llg_op* ops, const in
     if (tile_qubits != LLG_TUNE_AUTO) {
         const int tile = tile_qubits > 0 ? std::min(tile_qubits, tmax) : (precision == LLG_F32 ? 13 : 12);
         if (tile < 2) return set_error(LLG_EINVAL, "batch_create: tile_qubits too small");
-        return batch_build(count, n_qubits, ops, op_offsets, precision, tile, 256, out);
+        return batch_build(count, n_qubits, ops, op_offsets, precision, tile, 256, tile_qubits == 0, out);
     }
     llg_tune_result res;
     int rc = llg_batch_autotune(count, n_qubits, ops, op_offsets, precision, &res);
     if (rc) return rc;
-    return batch_build(count, n_qubits, ops, op_offsets, precision, res.tile_qubits, res.cta_threads, out);
+    const bool engine = res.cta_threads == 0;
+    return batch_build(count, n_qubits, ops, op_offsets, precision, res.tile_qubits, engine ? 256 : res.cta_threads, engine, out);
 }
 
 int llg_batch_autotune(int count, const int* n_qubits, const llg_op* ops, const int64_t* op_offsets, int precision,
@@ -439,10 +641,13 @@ int llg_batch_autotune(int count, const int* n_qubits, const llg_op* ops, const 
     if (e != cudaSuccess) return cuda_fail(e, "batch autotune events");
     int rc = LLG_OK;
     for (int t = std::min(8, tmax); t <= tmax && !rc; ++t)
-        for (int th : {256, 512}) {
+        for (int th : {0, 256, 512}) {
             if (rc) break;
+            // no CTA size: the default, which may take gate blocks (complex128 alone)
+            const bool engine = th == 0;
+            if (engine && (precision != LLG_F64 || t != tdef)) continue;
             llg_batch* b = nullptr;
-            rc = batch_build(count, n_qubits, ops, op_offsets, precision, t, th, &b);
+            rc = batch_build(count, n_qubits, ops, op_offsets, precision, t, engine ? 256 : th, engine, &b);
             if (rc) break;
             rc = llg_batch_run(b, 0);  // untimed (captures the graph)
             if (!rc) {
@@ -457,7 +662,7 @@ int llg_batch_autotune(int count, const int* n_qubits, const llg_op* ops, const 
                 if (!rc && e != cudaSuccess) rc = cuda_fail(e, "batch autotune timing");
                 if (!rc) {
                     ++res.candidates;
-                    if (t == tdef && th == 256) res.default_ms = ms;
+                    if (t == tdef && (engine || (th == 256 && precision != LLG_F64))) res.default_ms = ms;
                     if (ms < best) {
                         best = ms;
                         res.best_ms = ms;
@@ -489,9 +694,12 @@ int llg_batch_destroy(llg_batch* b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     drop_graph(b);
     void* ptrs[] = {b->d_arena, b->d_circs, b->d_passes, b->d_ops, b->d_tables, b->d_items, b->d_next, b->d_completed,
-                    b->d_err};
+                    b->d_err, b->d_weights, b->d_ctas};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    if (b->fork) cudaEventDestroy(b->fork);
+    if (b->join) cudaEventDestroy(b->join);
+    if (b->side) cudaStreamDestroy(b->side);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return LLG_OK;
@@ -499,9 +707,9 @@ int llg_batch_destroy(llg_batch* b) {
 
 int llg_batch_info(const llg_batch* b, int64_t* work_items, int64_t* total_amps, int* total_passes) {
     if (!b) return set_error(LLG_EINVAL, "batch_info: NULL handle");
-    if (work_items) *work_items = (int64_t)b->items.size();
+    if (work_items) *work_items = (int64_t)b->items.size() + b->block_tiles;
     if (total_amps) *total_amps = (int64_t)b->total_amps;
-    if (total_passes) *total_passes = (int)b->passes.size();
+    if (total_passes) *total_passes = (int)b->passes.size() + b->block_steps;
     return LLG_OK;
 }
 
@@ -515,11 +723,12 @@ int llg_batch_run(llg_batch* b, int64_t spin_limit) {
         default: rc = launch_batch<PolDF64>(b, lim); break;
     }
     if (rc) return rc;
-    int err = 0;
-    cudaError_t e = cudaMemcpyAsync(&err, b->d_err, sizeof(int), cudaMemcpyDeviceToHost, b->stream);
+    int err[2] = {0, 0};
+    cudaError_t e = cudaMemcpyAsync(err, b->d_err, sizeof(err), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) return cuda_fail(e, "batch kernel");
-    if (err) return set_error(LLG_ETIMEOUT, "batch_run: a tile waited past its limit for its circuit's previous pass");
+    if (err[1]) return set_error(LLG_ECUDA, "batch_run: a tensor-core block kernel timed out waiting for its products");
+    if (err[0]) return set_error(LLG_ETIMEOUT, "batch_run: a tile waited past its limit for its circuit's previous pass");
     return LLG_OK;
 }
 

@@ -106,17 +106,21 @@ struct Elem<LLG_DF64> {
 // A batch of states: row y of the grid is set y mod `sets`, whose state is 2^n elements from the
 // first one's (the next `sets` rows: from `second`) and whose weights are `wstride` 16-byte words from
 // the first set's.  max_exp (nullptr: none): per row, raised to the largest biased exponent stored (FP64).
+// mixed (nullptr: none): blocks of different states in one launch, each CTA's given by its entry.
 template <int P>
 struct BlockBatch {
     typename Elem<P>::S* second;
     int sets;
     uint64_t wstride;
     uint32_t* max_exp;
+    const MixedCta* mixed;
 };
 
 // kRows: the gate's rows have exponents of their own (any matrix); else all have exponent 0 (a product
 // of unitary gates, entries at most 1).
-template <int P, bool kRows>
+// kMixed: the state, its block and the CTA's tiles come from batch.mixed, and the targets' offsets from shared
+// memory instead of the parameters.
+template <int P, bool kRows, bool kMixed>
 __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
     k_gate_block(typename Elem<P>::S* __restrict__ psi, int n, const __grid_constant__ TargetOffsets to, uint64_t tmask,
                  const uint4* __restrict__ weights, bool weights_ready, int* __restrict__ err_flag, double2* __restrict__ mirror,
@@ -139,10 +143,32 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
     const uint32_t accfull0 = smem_u32(&bars[2 * kRing]), accempty0 = smem_u32(&bars[2 * kRing + 2]);
     const uint32_t egfull0 = smem_u32(&bars[2 * kRing + 4]), drain = smem_u32(&bars[2 * kRing + 7]);
 
-    const int row_y = blockIdx.y, set_y = row_y % batch.sets;
-    psi = (row_y < batch.sets ? psi : batch.second) + ((uint64_t)set_y << n);
-    weights += set_y * batch.wstride;
-    if (tid < kAmps) toff[tid] = to.o[tid];
+    const int row_y = blockIdx.y;
+    uint64_t tile0 = blockIdx.x, step = gridDim.x;  // this CTA's tiles
+    if constexpr (kMixed) {
+        const MixedCta& m = batch.mixed[blockIdx.x];
+        psi += m.offset;
+        weights += m.weights * batch.wstride;
+        n = m.n;
+        tmask = m.tmask;
+        tile0 = m.first;
+        step = m.step;
+        if (tid < kAmps) {
+            uint64_t o = 0;
+            for (int b = 0; b < 5; ++b)
+                if ((tid >> b) & 1) o |= 1ULL << m.q[b];
+            toff[tid] = o;
+        }
+    } else {
+        const int set_y = row_y % batch.sets;
+        psi = (row_y < batch.sets ? psi : batch.second) + ((uint64_t)set_y << n);
+        weights += set_y * batch.wstride;
+        if (tid < kAmps) toff[tid] = to.o[tid];
+    }
+    auto off = [&](int j) {
+        if constexpr (kMixed) return toff[j];
+        else return to.o[j];
+    };
     // Launched while the previous kernel of the stream runs: everything up to the wait below touches
     // nothing that it writes (the weights only if they were ready before it began).
     if (!weights_ready) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -188,16 +214,16 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
         const int g = 16 * warp + (lane & 15), h = lane >> 4;
         int seen = 0;  // tiles begun, for the prefetching warp
         typename Elem<P>::S a[16];
-        uint64_t tile = blockIdx.x;
+        uint64_t tile = tile0;
         if (tile < ntiles) {
-            const auto* pb = psi + (insert0_mask(tile * kGroups + (uint64_t)g, tmask) | (h ? to.o[1] : 0));
+            const auto* pb = psi + (insert0_mask(tile * kGroups + (uint64_t)g, tmask) | (h ? off(1) : 0));
 #pragma unroll
-            for (int k = 0; k < 16; ++k) a[k] = __ldcg(pb + to.o[2 * k]);
+            for (int k = 0; k < 16; ++k) a[k] = __ldcg(pb + off(2 * k));
         }
         int slot = 0, egb = 0;
         uint32_t phase = 1;  // of the slot's previous release: the first round needs no wait
         bool first = true, ok = true;
-        for (; tile < ntiles && ok; tile += gridDim.x, egb = egb == 2 ? 0 : egb + 1) {
+        for (; tile < ntiles && ok; tile += step, egb = egb == 2 ? 0 : egb + 1) {
             int eg;
             if constexpr (P == LLG_F64) {
                 uint32_t mx = 0;
@@ -228,9 +254,9 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                 // clamped so that the scale factor 2^(132 - e) below stays a normal float
                 eg = max((int)(__float_as_uint(mx) >> 23), 8);
             }
-            const uint64_t next = tile + gridDim.x;
+            const uint64_t next = tile + step;
             if (tid == 0) *progress_s = ++seen;
-            const auto* pb = psi + ((next < ntiles ? insert0_mask(next * kGroups + (uint64_t)g, tmask) : 0) | (h ? to.o[1] : 0));
+            const auto* pb = psi + ((next < ntiles ? insert0_mask(next * kGroups + (uint64_t)g, tmask) : 0) | (h ? off(1) : 0));
 #pragma unroll
             for (int ks = 0; ks < kChunks; ++ks) {
                 if (!first && !warp_wait(empty0 + 8 * slot, phase, abort_s)) {
@@ -301,7 +327,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                 }
                 if (next < ntiles) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) a[4 * ks + i] = __ldcg(pb + to.o[2 * (4 * ks + i)]);
+                    for (int i = 0; i < 4; ++i) a[4 * ks + i] = __ldcg(pb + off(2 * (4 * ks + i)));
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
@@ -319,14 +345,14 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
         // kStep / 2 of the half's 16 at a time ----
         const int row = 32 * (warp & 3) + lane, e = (warp - kSlicerWarps) >> 2;
         const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-        const bool pair32 = to.o[1] == 1;  // amplitudes j and j + 1 (j even) are adjacent
+        const bool pair32 = off(1) == 1;  // amplitudes j and j + 1 (j even) are adjacent
         int erm = 1;
         if (kRows)
             for (int r = 0; r < 64; ++r) erm = max(erm, abs(er_s[r]));
         int egb = 0;
         uint32_t phase = 0, egphase = 0, largest = 0;
         bool ok = true;
-        for (uint64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, phase ^= 1) {
+        for (uint64_t tile = tile0; tile < ntiles && ok; tile += step, phase ^= 1) {
             const uint64_t base = insert0_mask(tile * kGroups + (uint64_t)row, tmask) | toff[T::kStep * e];
             if (!warp_wait(egfull0 + 8 * egb, egphase, abort_s)) break;
             const int eg = eg_s[egb][row];
@@ -430,20 +456,20 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                         for (int c = 0; c < T::kStep / 2; c += 2) {
                             uint64_t w[4];
                             memcpy(w, &out[c], 32);
-                            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(psi + pos + to.o[c]), "l"(w[0]), "l"(w[1]),
+                            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(psi + pos + off(c)), "l"(w[0]), "l"(w[1]),
                                          "l"(w[2]), "l"(w[3])
                                          : "memory");
                         }
                     } else {
 #pragma unroll
-                        for (int c = 0; c < T::kStep / 2; ++c) psi[pos + to.o[c]] = out[c];
+                        for (int c = 0; c < T::kStep / 2; ++c) psi[pos + off(c)] = out[c];
                     }
                     if (mirror) {
 #pragma unroll
                         for (int c = 0; c < T::kStep / 2; ++c) {
-                            if constexpr (P == LLG_F64) mirror[pos + to.o[c]] = out[c];
+                            if constexpr (P == LLG_F64) mirror[pos + off(c)] = out[c];
                             else
-                                mirror[pos + to.o[c]] = make_double2((double)out[c].x + (double)out[c].z,
+                                mirror[pos + off(c)] = make_double2((double)out[c].x + (double)out[c].z,
                                                                            (double)out[c].y + (double)out[c].w);
                         }
                     }
@@ -466,7 +492,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
             int slot0 = 0;  // ring slot of the tile's first chunk
             uint32_t fphase = 0, aphase = 1;
             bool ok = true, any = false;
-            for (uint64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, aphase ^= 1) {
+            for (uint64_t tile = tile0; tile < ntiles && ok; tile += step, aphase ^= 1) {
 #pragma unroll 1
                 for (int half = 0; half < 2 && ok; ++half) {
                     if (any && !warp_wait(accempty0 + 8 * half, aphase, abort_s)) {
@@ -533,7 +559,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
             const int cl = __ffsll((long long)~in_tile) - 1;
             const bool run_start = (toff[lane] & ((1ULL << cl) - 1)) == 0;
             int begun = 0;
-            for (uint64_t t = blockIdx.x + (uint64_t)gridDim.x; t < ntiles && !*abort_s; t += gridDim.x, ++begun) {
+            for (uint64_t t = tile0 + step; t < ntiles && !*abort_s; t += step, ++begun) {
                 for (int it = 0; it < 100000 && *progress_s < begun && !*abort_s; ++it) __nanosleep(200);
                 if (run_start)
                     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(psi + (insert0_mask(t * kGroups, tmask) | toff[lane])),
@@ -723,12 +749,12 @@ int sm_count() {
 }
 
 // ctas: CTAs a state (0: one per SM); sets states from psi and, unless nullptr, as many from `second`
-template <int P, bool kRows>
+template <int P, bool kRows, bool kMixed = false>
 cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool ready, int* err, cudaStream_t s, double* mirror,
-                   int ctas, void* second, int sets, uint32_t* max_exp) {
+                   int ctas, void* second, int sets, uint32_t* max_exp, const MixedCta* mixed = nullptr) {
     using T = Shape<P>;
     static const cudaError_t attr =
-        cudaFuncSetAttribute(k_gate_block<P, kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmem);
+        cudaFuncSetAttribute(k_gate_block<P, kRows, kMixed>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmem);
     if (attr != cudaSuccess) return attr;
     TargetOffsets to;
     for (int j = 0; j < kAmps; ++j) {
@@ -736,7 +762,8 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool re
         for (int b = 0; b < 5; ++b)
             if ((j >> b) & 1) to.o[j] |= 1ULL << bd.q[b];
     }
-    const uint64_t ntiles = (1ULL << (n - 5)) / kGroups, most = ctas > 0 ? (uint64_t)ctas : (uint64_t)sm_count();
+    const uint64_t most = ctas > 0 ? (uint64_t)ctas : (uint64_t)sm_count();
+    const uint64_t ntiles = kMixed ? most : (1ULL << (n - 5)) / kGroups;
     // programmatic dependent launch: the CTA's set-up (barriers, tensor memory, the gate's digits)
     // runs under the end of the stream's previous kernel
     cudaLaunchAttribute at;
@@ -749,9 +776,9 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool re
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_gate_block<P, kRows>, static_cast<typename Elem<P>::S*>(psi), n, to, bd.tmask,
+    return cudaLaunchKernelEx(&cfg, k_gate_block<P, kRows, kMixed>, static_cast<typename Elem<P>::S*>(psi), n, to, bd.tmask,
                               static_cast<const uint4*>(w), ready, err, reinterpret_cast<double2*>(mirror),
-                              BlockBatch<P>{static_cast<typename Elem<P>::S*>(second), sets, gate_block_weight_bytes(P) / 16, max_exp});
+                              BlockBatch<P>{static_cast<typename Elem<P>::S*>(second), sets, gate_block_weight_bytes(P) / 16, max_exp, mixed});
 }
 
 }  // namespace
@@ -801,6 +828,12 @@ cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, cons
 cudaError_t launch_gate_block_batch(void* psi, void* second, int sets, int ctas, int n, const BlockDesc& bd,
                                     const void* d_weights, bool ready, uint32_t* max_exp, int* err_flag, cudaStream_t s) {
     return launch<LLG_F64, false>(psi, n, bd, d_weights, ready, err_flag, s, nullptr, ctas, second, sets, max_exp);
+}
+
+cudaError_t launch_gate_block_mixed(void* arena, int ctas, const MixedCta* d_ctas, const void* d_weights, int* err_flag,
+                                    cudaStream_t s) {
+    const BlockDesc none = {};
+    return launch<LLG_F64, false, true>(arena, 12, none, d_weights, true, err_flag, s, nullptr, ctas, nullptr, 1, nullptr, d_ctas);
 }
 
 }  // namespace llg

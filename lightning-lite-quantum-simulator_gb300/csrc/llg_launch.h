@@ -115,6 +115,19 @@ cudaError_t launch_gate_block_weights(int P, const BlockGate* d_gates, const Blo
 // raised to the largest biased exponent stored
 cudaError_t launch_gate_block_batch(void* psi, void* second, int sets, int ctas, int n, const BlockDesc& bd,
                                     const void* d_weights, bool ready, uint32_t* max_exp, int* err_flag, cudaStream_t s);
+// One FP64 launch of blocks of different states: CTA i takes d_ctas[i] (device memory that was complete before the stream's
+// previous kernel began, as the weights).
+struct MixedCta {
+    uint64_t offset;       // the state's first element
+    uint64_t tmask;        // its five targets q, increasing
+    uint32_t weights;      // index of the block's weights
+    uint32_t first, step;  // tiles of 4096 amplitudes: first, first + step, ..
+    int32_t n;
+    int32_t q[5];
+    int32_t pad;
+};
+cudaError_t launch_gate_block_mixed(void* arena, int ctas, const MixedCta* d_ctas, const void* d_weights, int* err_flag,
+                                    cudaStream_t s);
 cudaError_t launch_gate_block(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, bool rows, bool ready,
                               int* err_flag, cudaStream_t s, double* mirror = nullptr);
 
