@@ -750,6 +750,7 @@ int llg_batch_copy_state(llg_batch* b, int index, double* out) {
     const size_t eb = elem_bytes(b->P);
     double* d_tmp = nullptr;
     cudaError_t e = cudaSuccess;
+    map_destination(out, size * 16);
     if (b->P == LLG_F64) {  // the same layout: one copy
         e = cudaMemcpyAsync(out, (const char*)b->d_arena + cd.offset * eb, size * eb, cudaMemcpyDeviceToHost, b->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

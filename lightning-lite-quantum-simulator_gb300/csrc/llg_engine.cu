@@ -3,6 +3,7 @@
 // flush into fused tile passes or per-gate streaming kernels, and chunked host transfers.
 #include <algorithm>
 #include <atomic>
+#include <cerrno>
 #include <cmath>
 #include <complex>
 #include <cstdio>
@@ -11,6 +12,8 @@
 #include <vector>
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "../../include/llgpu.h"
 #include "llg_common_host.h"
@@ -24,6 +27,23 @@ using namespace llg;
 namespace llg {
 
 thread_local std::string g_last_error;
+
+void map_destination(void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    constexpr int kPopulate = MADV_POPULATE_WRITE;
+#else
+    constexpr int kPopulate = 23;  // Linux 5.14
+#endif
+    if (bytes < ((size_t)64 << 10)) return;  // the allocator's own small blocks
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), first = (uintptr_t)p / page * page;
+    const int was = errno;
+    // memory in use before is mapped throughout, a fresh array nowhere but at its ends: its middle page tells
+    unsigned char there = 0;
+    const uintptr_t middle = ((uintptr_t)p + bytes / 2) / page * page;
+    if (mincore((void*)middle, page, &there) == 0 && !(there & 1))
+        (void)madvise((void*)first, (uintptr_t)p + bytes - first, kPopulate);
+    errno = was;
+}
 
 int set_error(int code, const std::string& msg) {
     g_last_error = msg;
@@ -1180,6 +1200,7 @@ int llg_copy_to_host(llg_state* st, double* out) {
         LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
         return device_checks(st);
     }
+    map_destination(out, st->size * 16);  // while the passes run
     if (st->P == LLG_F64) {  // pageable destination, same layout: one copy
         LLG_CUDA(cudaMemcpyAsync(out, st->d_psi, st->size * 16, cudaMemcpyDeviceToHost, st->stream), "cudaMemcpyAsync(D2H)");
         LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
@@ -1238,6 +1259,7 @@ int llg_probabilities(llg_state* st, double* out) {
     int rc = llg_flush(st);
     if (rc) return rc;
     if ((rc = stage_buffers(st))) return rc;
+    map_destination(out, st->size * 8);
     const size_t eb = elem_bytes(st->P);
     const uint64_t chunk = kStageAmps * 2;  // doubles per staging buffer
     int which = 0;
