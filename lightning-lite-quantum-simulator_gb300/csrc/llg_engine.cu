@@ -83,10 +83,7 @@ struct llg_state {
     ExecOp* h_ops = nullptr;
     size_t h_ops_cap = 0;
     // phase tables of the plan (device, pinned staging), uploaded with the ops
-    uint64_t* d_tables = nullptr;
-    size_t d_tables_cap = 0;
-    uint64_t* h_tables = nullptr;
-    size_t h_tables_cap = 0;
+    uint64_t* d_tables = nullptr;  // in d_ops' buffer
     cudaEvent_t ops_done = nullptr;
     // dense-block matrix upload (pinned staging, reused once the previous copy has finished)
     uint64_t* d_block = nullptr;
@@ -109,9 +106,12 @@ struct llg_state {
     bool tiles_launched = false;  // a tile pass ran since the last sync (its load-timeout flag to check)
     // this state's timeout flags on the device: [0] a bulk tile load, [1] tensor-core products
     int* d_flags = nullptr;
-    // reductions
+    // reductions: partial sums, the diagonal observable's result, the finishing block's ticket (one buffer, with the
+    // flags), and the host's copies
     double* d_partials = nullptr;
     double* d_red = nullptr;
+    unsigned* d_ticket = nullptr;
+    Readout* h_out = nullptr;  // pinned
     // the last general diagonal observable (llg_diag.h), its device copy, and a full diagonal
     DiagObsHost obs;
     void* d_obs = nullptr;
@@ -190,12 +190,14 @@ int ensure_device_buffers(llg_state* st) {
     if (!st->stream) LLG_CUDA(cudaStreamCreateWithFlags(&st->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     if (!st->ops_done) LLG_CUDA(cudaEventCreateWithFlags(&st->ops_done, cudaEventDisableTiming), "cudaEventCreate");
     if (!st->d_partials) {
-        LLG_CUDA(cudaMalloc(&st->d_partials, sizeof(double) * kRedBlocks * kPartialSlots), "cudaMalloc(partials)");
-        LLG_CUDA(cudaMalloc(&st->d_red, sizeof(double) * kRedSlots), "cudaMalloc(red)");
-    }
-    if (!st->d_flags) {
-        LLG_CUDA(cudaMalloc(&st->d_flags, 2 * sizeof(int)), "cudaMalloc(flags)");
-        LLG_CUDA(cudaMemsetAsync(st->d_flags, 0, 2 * sizeof(int), st->stream), "cudaMemsetAsync(flags)");
+        constexpr size_t kPart = sizeof(double) * kRedBlocks * kPartialSlots, kRed = sizeof(double) * kRedSlots;
+        constexpr size_t kWords = 4 * sizeof(int);
+        LLG_CUDA(cudaHostAlloc((void**)&st->h_out, sizeof(Readout), cudaHostAllocDefault), "cudaHostAlloc(readout)");
+        LLG_CUDA(cudaMalloc(&st->d_partials, kPart + kWords + kRed), "cudaMalloc(partials)");
+        st->d_flags = reinterpret_cast<int*>(st->d_partials + kRedBlocks * kPartialSlots);
+        st->d_ticket = reinterpret_cast<unsigned*>(st->d_flags + 2);
+        st->d_red = reinterpret_cast<double*>(st->d_flags + 4);
+        LLG_CUDA(cudaMemsetAsync(st->d_flags, 0, kWords, st->stream), "cudaMemsetAsync(flags)");
     }
     return LLG_OK;
 }
@@ -255,52 +257,35 @@ int run_streaming(llg_state* st, const std::vector<llg_op>& q) {
     return LLG_OK;
 }
 
-int upload_ops(llg_state* st, const std::vector<ExecOp>& ops, const std::vector<uint64_t>* tables = nullptr) {
-    const size_t count = std::max<size_t>(ops.size(), 1);
-    if (count > st->d_ops_cap) {
+int upload_ops(llg_state* st, const std::vector<ExecOp>& ops, const std::vector<uint64_t>& tables) {
+    // one buffer and one copy: the ops, then the tables
+    const size_t obytes = (ops.size() * sizeof(ExecOp) + 255) / 256 * 256, tbytes = tables.size() * sizeof(uint64_t);
+    const size_t bytes = obytes + tbytes;
+    if (bytes > st->d_ops_cap) {
         if (st->d_ops) {
             cudaStreamSynchronize(st->stream);
             cudaFree(st->d_ops);
+            st->d_ops = nullptr;
+            st->d_ops_cap = 0;
         }
-        const size_t cap = std::max<size_t>(count, 1024);
-        LLG_CUDA(cudaMalloc(&st->d_ops, cap * sizeof(ExecOp)), "cudaMalloc(ops)");
+        const size_t cap = std::max<size_t>(bytes, 1024 * sizeof(ExecOp));
+        LLG_CUDA(cudaMalloc(&st->d_ops, cap), "cudaMalloc(ops)");
         st->d_ops_cap = cap;
     }
     // the pinned staging buffer may still feed an earlier copy
     LLG_CUDA(cudaEventSynchronize(st->ops_done), "cudaEventSynchronize");
-    if (count > st->h_ops_cap) {
+    if (bytes > st->h_ops_cap) {
         if (st->h_ops) cudaFreeHost(st->h_ops);
-        const size_t cap = std::max<size_t>(count, 1024);
-        LLG_CUDA(cudaHostAlloc((void**)&st->h_ops, cap * sizeof(ExecOp), cudaHostAllocDefault), "cudaHostAlloc(ops)");
+        st->h_ops = nullptr;
+        st->h_ops_cap = 0;
+        const size_t cap = std::max<size_t>(bytes, 1024 * sizeof(ExecOp));
+        LLG_CUDA(cudaHostAlloc((void**)&st->h_ops, cap, cudaHostAllocDefault), "cudaHostAlloc(ops)");
         st->h_ops_cap = cap;
     }
-    if (!ops.empty()) {
-        std::memcpy(st->h_ops, ops.data(), ops.size() * sizeof(ExecOp));
-        LLG_CUDA(cudaMemcpyAsync(st->d_ops, st->h_ops, ops.size() * sizeof(ExecOp), cudaMemcpyHostToDevice, st->stream),
-                 "cudaMemcpyAsync(ops)");
-    }
-    if (tables && !tables->empty()) {
-        const size_t words = tables->size();
-        if (words > st->d_tables_cap) {
-            if (st->d_tables) {
-                cudaStreamSynchronize(st->stream);
-                cudaFree(st->d_tables);
-                st->d_tables = nullptr;
-            }
-            LLG_CUDA(cudaMalloc(&st->d_tables, words * sizeof(uint64_t)), "cudaMalloc(tables)");
-            st->d_tables_cap = words;
-        }
-        if (words > st->h_tables_cap) {
-            if (st->h_tables) cudaFreeHost(st->h_tables);
-            st->h_tables = nullptr;
-            LLG_CUDA(cudaHostAlloc((void**)&st->h_tables, words * sizeof(uint64_t), cudaHostAllocDefault),
-                     "cudaHostAlloc(tables)");
-            st->h_tables_cap = words;
-        }
-        std::memcpy(st->h_tables, tables->data(), words * sizeof(uint64_t));
-        LLG_CUDA(cudaMemcpyAsync(st->d_tables, st->h_tables, words * sizeof(uint64_t), cudaMemcpyHostToDevice, st->stream),
-                 "cudaMemcpyAsync(tables)");
-    }
+    if (!ops.empty()) std::memcpy(st->h_ops, ops.data(), ops.size() * sizeof(ExecOp));
+    if (tbytes) std::memcpy(reinterpret_cast<char*>(st->h_ops) + obytes, tables.data(), tbytes);
+    if (bytes) LLG_CUDA(cudaMemcpyAsync(st->d_ops, st->h_ops, bytes, cudaMemcpyHostToDevice, st->stream), "cudaMemcpyAsync(ops)");
+    st->d_tables = reinterpret_cast<uint64_t*>(reinterpret_cast<char*>(st->d_ops) + obytes);
     LLG_CUDA(cudaEventRecord(st->ops_done, st->stream), "cudaEventRecord");
     return LLG_OK;
 }
@@ -321,7 +306,7 @@ int run_tiles(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
                     plan, err, false, f32_tiles ? ZYZ_OFF : ZYZ_ON, !reg && st->P != LLG_F32, f32_tiles))
         return set_error(LLG_EINVAL, err);
     if (reg) to_register_program(plan);
-    int rc = upload_ops(st, plan.ops, &plan.tables);
+    int rc = upload_ops(st, plan.ops, plan.tables);
     if (rc) return rc;
     st->tiles_launched = true;
     size_t last = plan.passes.size();
@@ -486,12 +471,12 @@ int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror
 int measure_norm(llg_state* st) {
     ZTerms z;
     std::memset(&z, 0, sizeof(z));
-    int rc = traced(st, LLG_PROF_READOUT, 2, "reduce",
-                    [&] { return launch_reduce_z(st->P, st->d_psi, st->n, z, st->d_partials, st->d_red, st->stream); });
+    int rc = traced(st, LLG_PROF_READOUT, 1, "reduce", [&] {
+        return launch_reduce_z(st->P, st->d_psi, st->n, z, st->d_partials, st->d_ticket, st->d_flags, st->h_out, st->stream);
+    });
     if (rc) return rc;
-    double v = 0.0;
-    LLG_CUDA(cudaMemcpyAsync(&v, st->d_red, sizeof(v), cudaMemcpyDeviceToHost, st->stream), "cudaMemcpyAsync(norm)");
     LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
+    const double v = st->h_out->red[0];
     st->log2_norm = !std::isfinite(v) ? HUGE_VAL : (v > 0.0 ? 0.5 * std::log2(v) : 0.0);
     return LLG_OK;
 }
@@ -728,11 +713,8 @@ int llg_destroy(llg_state* st) {
     if (st->d_psi) cudaFree(st->d_psi);
     if (st->d_ops) cudaFree(st->d_ops);
     if (st->h_ops) cudaFreeHost(st->h_ops);
-    if (st->d_tables) cudaFree(st->d_tables);
-    if (st->h_tables) cudaFreeHost(st->h_tables);
     if (st->d_partials) cudaFree(st->d_partials);
-    if (st->d_red) cudaFree(st->d_red);
-    if (st->d_flags) cudaFree(st->d_flags);
+    if (st->h_out) cudaFreeHost(st->h_out);
     if (st->d_obs) cudaFree(st->d_obs);
     if (st->d_diag) cudaFree(st->d_diag);
     for (int i = 0; i < 2; ++i) {
@@ -1139,27 +1121,29 @@ int llg_flush(llg_state* st) {
     return run_streaming(st, q);
 }
 
-// After the state's stream has drained: the timeout flags of the kernels that wait on the
-// asynchronous units (tensor-core products, bulk tile loads), for the launches since the last check.
-// The flags are this state's own, read and cleared on its own stream.
-static int device_checks(llg_state* st) {
-    if (!st->block_tc_launched && !st->tiles_launched) return LLG_OK;
+// The end of a call that reads back: waits for the state's stream and looks at the timeout flags of the kernels that
+// wait on the asynchronous units (tensor-core products, bulk tile loads), for the launches since the last check.  The flags
+// are this state's own, and come with the stream's last work (`here`: a readout kernel has brought them), so that one
+// wait does.
+static int finish(llg_state* st, bool here = false) {
     const bool tc = st->block_tc_launched, tiles = st->tiles_launched;
     st->block_tc_launched = st->tiles_launched = false;
-    int h[2] = {0, 0};
-    LLG_CUDA(cudaMemcpyAsync(h, st->d_flags, sizeof(h), cudaMemcpyDeviceToHost, st->stream), "cudaMemcpyAsync(flags)");
+    int* const h = st->h_out->flags;
+    if ((tc || tiles) && !here)
+        LLG_CUDA(cudaMemcpyAsync(h, st->d_flags, sizeof(st->h_out->flags), cudaMemcpyDeviceToHost, st->stream), "cudaMemcpyAsync(flags)");
     LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-    if (h[0] || h[1]) LLG_CUDA(cudaMemsetAsync(st->d_flags, 0, sizeof(h), st->stream), "cudaMemsetAsync(flags)");
-    if (tc && h[1]) return set_error(LLG_ECUDA, "apply_matrix: a tensor-core block kernel timed out waiting for its products");
-    if (tiles && h[0]) return set_error(LLG_ECUDA, "tile pass: a bulk tile load timed out");
+    if (!tc && !tiles) return LLG_OK;
+    const bool late_products = tc && h[1], late_load = tiles && h[0];
+    if (h[0] || h[1]) LLG_CUDA(cudaMemsetAsync(st->d_flags, 0, sizeof(st->h_out->flags), st->stream), "cudaMemsetAsync(flags)");
+    if (late_products) return set_error(LLG_ECUDA, "apply_matrix: a tensor-core block kernel timed out waiting for its products");
+    if (late_load) return set_error(LLG_ECUDA, "tile pass: a bulk tile load timed out");
     return LLG_OK;
 }
 
 int llg_sync(llg_state* st) {
     int rc = llg_flush(st);
     if (rc) return rc;
-    LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-    return device_checks(st);
+    return finish(st);
 }
 
 // Device address of pinned, mapped host memory (cudaHostAlloc / cudaHostRegister), else nullptr.
@@ -1184,8 +1168,7 @@ int llg_copy_to_host(llg_state* st, double* out) {
         bool mirrored = false;
         if ((rc = run_fused(st, q, static_cast<double*>(dev_out), &mirrored))) return rc;
         if (mirrored) {
-            LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-            return device_checks(st);
+            return finish(st);
         }
     }
     rc = llg_flush(st);
@@ -1197,14 +1180,12 @@ int llg_copy_to_host(llg_state* st, double* out) {
         rc = traced(st, LLG_PROF_READOUT, 1, "to_f64",
                     [&] { return launch_to_f64(st->P, st->d_psi, static_cast<double*>(dev_out), st->size, st->stream); });
         if (rc) return rc;
-        LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-        return device_checks(st);
+        return finish(st);
     }
     map_destination(out, st->size * 16);  // while the passes run
     if (st->P == LLG_F64) {  // pageable destination, same layout: one copy
         LLG_CUDA(cudaMemcpyAsync(out, st->d_psi, st->size * 16, cudaMemcpyDeviceToHost, st->stream), "cudaMemcpyAsync(D2H)");
-        LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-        return device_checks(st);
+        return finish(st);
     }
     if ((rc = stage_buffers(st))) return rc;
     const size_t eb = elem_bytes(st->P);
@@ -1220,8 +1201,7 @@ int llg_copy_to_host(llg_state* st, double* out) {
                  "cudaMemcpyAsync(D2H)");
         LLG_CUDA(cudaEventRecord(st->stage_ev[which], st->stream), "cudaEventRecord");
     }
-    LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-    return device_checks(st);
+    return finish(st);
 }
 
 int llg_copy_from_host(llg_state* st, const double* amps) {
@@ -1274,8 +1254,7 @@ int llg_probabilities(llg_state* st, double* out) {
                  "cudaMemcpyAsync(D2H)");
         LLG_CUDA(cudaEventRecord(st->stage_ev[which], st->stream), "cudaEventRecord");
     }
-    LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-    return device_checks(st);
+    return finish(st);
 }
 
 // The class-counting kernel takes up to kMaxZTerms terms with up to kMaxZClasses distinct
@@ -1323,13 +1302,14 @@ static int build_zterms(int nterms, const int* a, const int* b, const double* co
 static int reduce(llg_state* st, const ZTerms& z, double* slots) {
     int rc = llg_flush(st);
     if (rc) return rc;
-    rc = traced(st, LLG_PROF_READOUT, 2, "reduce",
-                [&] { return launch_reduce_z(st->P, st->d_psi, st->n, z, st->d_partials, st->d_red, st->stream); });
+    if ((rc = ensure_device_buffers(st))) return rc;
+    rc = traced(st, LLG_PROF_READOUT, 1, "reduce", [&] {
+        return launch_reduce_z(st->P, st->d_psi, st->n, z, st->d_partials, st->d_ticket, st->d_flags, st->h_out, st->stream);
+    });
     if (rc) return rc;
-    LLG_CUDA(cudaMemcpyAsync(slots, st->d_red, sizeof(double) * kRedSlots, cudaMemcpyDeviceToHost, st->stream),
-             "cudaMemcpyAsync(D2H)");
-    LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-    return device_checks(st);
+    rc = finish(st, true);
+    std::memcpy(slots, st->h_out->red, sizeof(st->h_out->red));
+    return rc;
 }
 
 int llg_compare(llg_state* a, llg_state* b, double* fidelity, double* max_abs_diff) {
@@ -1350,7 +1330,7 @@ int llg_compare_ex(llg_state* a, llg_state* b, double* fidelity, double* max_abs
     LLG_CUDA(cudaMemcpyAsync(part.data(), a->d_partials, part.size() * sizeof(double), cudaMemcpyDeviceToHost, a->stream),
              "cudaMemcpyAsync(D2H)");
     LLG_CUDA(cudaStreamSynchronize(a->stream), "cudaStreamSynchronize");
-    if ((rc = device_checks(a)) || (rc = device_checks(b))) return rc;
+    if ((rc = finish(a)) || (rc = finish(b))) return rc;
     double re = 0.0, im = 0.0, na = 0.0, nb = 0.0, mx = 0.0, mb = 0.0;
     for (int k = 0; k < nblocks; ++k) {  // fixed order
         re += part[(size_t)k * kCmpSlots];
@@ -1385,10 +1365,11 @@ static int reduce_diag(llg_state* st, const DiagObs& o, double* out2) {
     rc = traced(st, LLG_PROF_READOUT, 2, "diagonal observable",
                 [&] { return launch_expect_diag(st->P, st->d_psi, o, st->d_partials, st->d_red, st->stream); });
     if (rc) return rc;
-    LLG_CUDA(cudaMemcpyAsync(out2, st->d_red, 2 * sizeof(double), cudaMemcpyDeviceToHost, st->stream),
+    LLG_CUDA(cudaMemcpyAsync(st->h_out->red, st->d_red, 2 * sizeof(double), cudaMemcpyDeviceToHost, st->stream),
              "cudaMemcpyAsync(D2H)");
-    LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
-    return device_checks(st);
+    rc = finish(st);
+    std::memcpy(out2, st->h_out->red, 2 * sizeof(double));
+    return rc;
 }
 
 // The observable's layout on the device (rebuilt and uploaded only when the terms change).

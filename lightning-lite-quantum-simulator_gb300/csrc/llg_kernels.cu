@@ -447,10 +447,15 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return r;
 }
 
+// The sums, by blocks and then by the block that finishes last (one warp a slot, the blocks' sums in a fixed order),
+// which also hands them and the state's timeout flags to the host: bound by launches and copies on small registers, where
+// a second kernel, a copy of the sums and one of the flags took 20 of an 8-qubit energy's 106 us.
 template <class P>
 __global__ void __launch_bounds__(kThreads) k_reduce_z(const typename P::S* __restrict__ psi, uint64_t size, ZTerms z,
-                                                      double* __restrict__ partials) {
+                                                      double* __restrict__ partials, unsigned* __restrict__ ticket,
+                                                      const int* __restrict__ flags, Readout* __restrict__ out) {
     __shared__ double sh[kThreads / 32];
+    __shared__ bool last;
     typename P::Acc acc[kRedSlots];
 #pragma unroll
     for (int s = 0; s < kRedSlots; ++s) acc[s] = P::acc_zero();
@@ -472,8 +477,26 @@ __global__ void __launch_bounds__(kThreads) k_reduce_z(const typename P::S* __re
     }
 #pragma unroll
     for (int s = 0; s < kRedSlots; ++s) {
+        if (s > z.nclass) break;
         const double v = block_sum(P::acc_to_double(acc[s]), sh);
         if (threadIdx.x == 0) partials[(size_t)blockIdx.x * kRedSlots + s] = v;
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;  // back at zero for the next launch
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    const int slot = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (slot < kRedSlots) {
+        double r = 0.0;
+        if (slot <= z.nclass)
+            for (int b = lane; b < (int)gridDim.x; b += 32) r += __ldcg(partials + (size_t)b * kRedSlots + slot);
+        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        if (lane == 0) out->red[slot] = r;
+    } else if (slot == kRedSlots && lane < 2) {
+        out->flags[lane] = flags[lane];
     }
 }
 
@@ -516,15 +539,6 @@ __global__ void __launch_bounds__(kThreads) k_compare(const typename PA::S* __re
     if (threadIdx.x == 0) partials[(size_t)blockIdx.x * kCmpSlots + 4] = m;
     const double m2 = block_max(mb, sh);
     if (threadIdx.x == 0) partials[(size_t)blockIdx.x * kCmpSlots + 5] = m2;
-}
-
-__global__ void k_finish(const double* __restrict__ partials, int nblocks, double* __restrict__ out) {
-    // one thread per slot, fixed order: deterministic
-    const int s = threadIdx.x;
-    if (s >= kRedSlots) return;
-    double r = 0.0;
-    for (int b = 0; b < nblocks; ++b) r += partials[(size_t)b * kRedSlots + s];
-    out[s] = r;
 }
 
 // FP64 FMA throughput probe: eight independent dependency chains per thread keep the FP64
@@ -710,14 +724,15 @@ cudaError_t launch_scale(int P, void* psi, uint64_t count, double factor, cudaSt
                  return cudaGetLastError());
 }
 
-cudaError_t launch_reduce_z(int P, const void* psi, int n, const ZTerms& terms, double* d_partials, double* d_out,
-                            cudaStream_t s) {
+cudaError_t launch_reduce_z(int P, const void* psi, int n, const ZTerms& terms, double* d_partials, unsigned* d_ticket,
+                            const int* d_flags, Readout* host, cudaStream_t s) {
     const uint64_t size = 1ULL << n;
     unsigned g = grid_for(size, 4);
     if (g > (unsigned)kRedBlocks) g = kRedBlocks;
-    LLG_DISPATCH(P, k_reduce_z<Pol><<<g, kThreads, 0, s>>>(static_cast<const typename Pol::S*>(psi), size, terms, d_partials);
-                 cudaError_t e = cudaGetLastError(); if (e != cudaSuccess) return e;
-                 k_finish<<<1, 32, 0, s>>>(d_partials, (int)g, d_out); return cudaGetLastError());
+    static_assert(kRedSlots < kThreads / 32, "a warp a slot and one for the flags");
+    LLG_DISPATCH(P, k_reduce_z<Pol><<<g, kThreads, 0, s>>>(static_cast<const typename Pol::S*>(psi), size, terms, d_partials, d_ticket,
+                                                         d_flags, host);
+                 return cudaGetLastError());
 }
 
 }  // namespace llg

@@ -45,10 +45,15 @@ cudaError_t launch_from_f64(int P, const double* src, void* dst, uint64_t count,
 cudaError_t launch_to_f64(int P, const void* src, double* dst, uint64_t count, cudaStream_t s);
 cudaError_t launch_probabilities(int P, const void* psi, double* out, uint64_t count, cudaStream_t s);
 cudaError_t launch_scale(int P, void* psi, uint64_t count, double factor, cudaStream_t s);
-// Writes [norm2, W_0 .. W_{nclass-1}] (W_c = sum_i |a_i|^2 * #odd-parity terms of class c in i)
-// to d_out (device, kRedSlots doubles), via d_partials (device, kRedBlocks * kRedSlots doubles).
-cudaError_t launch_reduce_z(int P, const void* psi, int n, const ZTerms& terms, double* d_partials, double* d_out,
-                            cudaStream_t s);
+// What a readout kernel leaves in pinned host memory: [norm2, W_0 .. W_{nclass-1}] (W_c = sum_i |a_i|^2 * #odd-parity terms of
+// class c in i) and the state's timeout flags.
+struct Readout {
+    double red[kRedSlots];
+    int flags[2];
+};
+// d_partials: device, kRedBlocks * kRedSlots doubles; d_ticket: a device word that is zero between launches
+cudaError_t launch_reduce_z(int P, const void* psi, int n, const ZTerms& terms, double* d_partials, unsigned* d_ticket,
+                            const int* d_flags, Readout* host, cudaStream_t s);
 
 // Two states of equal size, any precisions: per block (kCmpSlots doubles each) Re <a|b>, Im <a|b>,
 // <a|a>, <b|b>, max |a_i - b_i| and max |b_i| (over re and im parts); *nblocks = blocks written
