@@ -447,32 +447,111 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return r;
 }
 
+// What the terms of a class count on the 256 amplitudes of a row: base + sum over the row's bits x_a of weight_a x_a (bytes of
+// w0 and w1), plus what the terms inside the row count.
+struct RowCount {
+    int base, w0, w1;
+};
+
 // The sums, by blocks and then by the block that finishes last (one warp a slot, the blocks' sums in a fixed order),
 // which also hands them and the state's timeout flags to the host: bound by launches and copies on small registers, where
 // a second kernel, a copy of the sums and one of the flags took 20 of an 8-qubit energy's 106 us.
+// On large ones bound by the FP64 pipe (four operations an amplitude; counting 34 terms bit by bit took 190 us on 23
+// qubits): a thread keeps its place in rows of 256 amplitudes, the terms inside a row are counted once, and a term across
+// (x_a ^ x_b = x_a, or 1 - x_a where the row's bit is set) is a weight of the row, so an amplitude takes two byte dot
+// products a class.
 template <class P>
 __global__ void __launch_bounds__(kThreads) k_reduce_z(const typename P::S* __restrict__ psi, uint64_t size, ZTerms z,
                                                       double* __restrict__ partials, unsigned* __restrict__ ticket,
                                                       const int* __restrict__ flags, Readout* __restrict__ out) {
     __shared__ double sh[kThreads / 32];
     __shared__ bool last;
+    __shared__ RowCount rows[kMaxZClasses][kThreads];
+    static_assert(kThreads == 256 && kMaxZTerms <= 127, "eight bits a row, weights in bytes");
     typename P::Acc acc[kRedSlots];
 #pragma unroll
     for (int s = 0; s < kRedSlots; ++s) acc[s] = P::acc_zero();
-    const uint64_t step = (uint64_t)gridDim.x * kThreads;
-    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < size; i += step) {
-        const auto a = P::load(psi[i]);
-        acc[0] = P::acc_norm(acc[0], a);
-        if (z.nterms > 0) {
-            int cnt[kMaxZClasses] = {0, 0, 0, 0};
-            for (int k = 0; k < z.nterms; ++k) {
-                int par = (int)((i >> z.a[k]) & 1);
-                if (z.b[k] >= 0) par ^= (int)((i >> z.b[k]) & 1);
-                cnt[z.cls[k]] += par;
-            }
+    const int tid = threadIdx.x;
+    const uint64_t nrows = (size + kThreads - 1) / kThreads, step = gridDim.x;
+    const uint64_t mine = blockIdx.x < nrows ? (nrows - blockIdx.x + step - 1) / step : 0;  // this block's rows
+    if (z.nterms > 0) {
+        int inside[kMaxZClasses] = {0, 0, 0, 0};
+        for (int k = 0; k < z.nterms; ++k)
+            if (z.a[k] < 8 && z.b[k] < 8) {
+                int par = (tid >> z.a[k]) & 1;
+                if (z.b[k] >= 0) par ^= (tid >> z.b[k]) & 1;
 #pragma unroll
-            for (int c = 0; c < kMaxZClasses; ++c)
-                if (c < z.nclass && cnt[c]) acc[1 + c] = P::acc_norm_w(acc[1 + c], a, (float)cnt[c]);
+                for (int c = 0; c < kMaxZClasses; ++c)
+                    if (c == z.cls[k]) inside[c] += par;
+            }
+        // the bits as bytes
+        const int x0 = (tid & 1) | (tid & 2) << 7 | (tid & 4) << 14 | (tid & 8) << 21;
+        const int x1 = (tid >> 4 & 1) | (tid >> 4 & 2) << 7 | (tid >> 4 & 4) << 14 | (tid >> 4 & 8) << 21;
+        for (uint64_t r0 = 0; r0 < mine; r0 += kThreads) {
+            const int count = (int)min((uint64_t)kThreads, mine - r0);
+            if (r0 > 0) __syncthreads();
+            if (tid < count && size <= kThreads) {  // one row: all terms are inside it
+#pragma unroll
+                for (int c = 0; c < kMaxZClasses; ++c) rows[c][0] = {0, 0, 0};
+            } else if (tid < count) {
+                const uint64_t h = (blockIdx.x + (r0 + tid) * step) << 8;
+                RowCount rc[kMaxZClasses];
+#pragma unroll
+                for (int c = 0; c < kMaxZClasses; ++c) rc[c] = {0, 0, 0};
+                for (int k = 0; k < z.nterms; ++k) {
+                    const int lo = z.b[k] < 0 ? -1 : min(z.a[k], z.b[k]), hi = max(z.a[k], z.b[k]);  // lo -1: Z alone
+                    if (hi < 8) continue;
+                    const int xh = (int)(h >> hi) & 1;
+                    int base = 0, w0 = 0, w1 = 0;
+                    base = lo < 8 ? xh : xh ^ ((int)(h >> lo) & 1);
+                    if (lo >= 0 && lo < 8) {
+                        const uint32_t w = xh ? 0xFFu : 1u;  // a byte: -1 or 1
+                        if (lo < 4) w0 = (int)(w << (8 * lo));
+                        else w1 = (int)(w << (8 * lo - 32));
+                    }
+#pragma unroll
+                    for (int c = 0; c < kMaxZClasses; ++c)
+                        if (c == z.cls[k]) {
+                            rc[c].base += base;
+                            rc[c].w0 = __vadd4(rc[c].w0, w0);
+                            rc[c].w1 = __vadd4(rc[c].w1, w1);
+                        }
+                }
+#pragma unroll
+                for (int c = 0; c < kMaxZClasses; ++c)
+                    if (c < z.nclass) rows[c][tid] = rc[c];
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (int r = 0; r < count; ++r) {
+                const uint64_t i = (blockIdx.x + (r0 + r) * step) * kThreads + tid;
+                if (i >= size) break;
+                const auto a = P::load(psi[i]);
+                if constexpr (P::kPrecision == LLG_F64) {
+                    const double n = fma(a.re, a.re, a.im * a.im);
+                    acc[0] += n;
+#pragma unroll
+                    for (int c = 0; c < kMaxZClasses; ++c)
+                        if (c < z.nclass) {
+                            const RowCount rc = rows[c][r];
+                            acc[1 + c] = fma((double)__dp4a(rc.w0, x0, __dp4a(rc.w1, x1, rc.base + inside[c])), n, acc[1 + c]);
+                        }
+                } else {
+                    acc[0] = P::acc_norm(acc[0], a);
+#pragma unroll
+                    for (int c = 0; c < kMaxZClasses; ++c)
+                        if (c < z.nclass) {
+                            const RowCount rc = rows[c][r];
+                            const int cnt = __dp4a(rc.w0, x0, __dp4a(rc.w1, x1, rc.base + inside[c]));
+                            if (cnt) acc[1 + c] = P::acc_norm_w(acc[1 + c], a, (float)cnt);
+                        }
+                }
+            }
+        }
+    } else {
+        for (uint64_t r = blockIdx.x; r < nrows; r += step) {
+            const uint64_t i = r * kThreads + tid;
+            if (i < size) acc[0] = P::acc_norm(acc[0], P::load(psi[i]));
         }
     }
 #pragma unroll
