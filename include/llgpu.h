@@ -405,7 +405,7 @@ int llg_tsolver_plan_export(const llg_tsolver* s, long long* steps, double* h, i
  * complex64; LLG_TUNE_AUTO: picked by llg_batch_autotune) and run together from |0..0> in ONE
  * persistent launch: persistent CTAs take (circuit, pass, tile) work items from a queue; a tile
  * waits, with a bounded poll, for the previous pass of its own circuit.  With tile_qubits 0, complex128
- * circuits of 12 or more qubits may run as dense 5-qubit blocks on the tensor cores instead, beside the
+ * circuits of 10 or more qubits may run as dense 5-qubit blocks on the tensor cores instead, beside the
  * queue.  Each run replays a CUDA graph captured at the first run (state reset + the kernels).  The reference runs such
  * circuits one at a time on StateVectorBackend (src/StateVectorBackend.h). */
 typedef struct llg_batch llg_batch;

@@ -11,7 +11,7 @@
 // that runs out sets an error flag the host reports as LLG_ETIMEOUT instead of hanging.
 // Tiles are read with L1-bypassing loads (other SMs wrote them).
 //
-// IEEE complex128 circuits of 12 or more qubits take dense 5-qubit blocks on the tensor cores instead where
+// IEEE complex128 circuits of 10 or more qubits take dense 5-qubit blocks on the tensor cores instead where
 // that is estimated to be faster (plan_blocks): block r of every circuit runs in the r-th launch, whose CTAs are
 // dealt out to the circuits by their size.  The blocks' digits are made once per batch.  The other circuits'
 // queue runs beside them on a second branch of the graph.
@@ -317,7 +317,9 @@ int launch_batch(llg_batch* b, long long spin_limit) {
 
 namespace {
 
-constexpr int kTileAmps = 4096;  // of a gate block
+// a gate block's tiles of 4096 amplitudes (a smaller state fills a part of one)
+uint64_t block_tiles(int n) { return n > 12 ? 1ULL << (n - 12) : 1; }
+constexpr int kBatchBlockQubits = 10;
 constexpr size_t kWeightsCap = (size_t)256 << 20;
 
 struct BlockSet {
@@ -356,7 +358,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
         const double amps = std::ldexp(1.0, n);
         at += 1ULL << n;
         std::vector<llg_op> mine(ops + off[c], ops + off[c + 1]);
-        bool fits = n >= 12 && nops > 0 && has_block_plan(n, mine.data(), nops);
+        bool fits = n >= kBatchBlockQubits && nops > 0 && has_block_plan(n, mine.data(), nops);
         for (llg_op& o : mine) {
             o.param = -1;
             if (o.kind == LLG_OP_MCZ && __builtin_popcountll(o.mask) > 5) fits = false;
@@ -396,7 +398,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
         int active = 0;
         for (const Circuit& k : list)
             if (r < k.blocks) {
-                tiles += (1ULL << k.n) / kTileAmps;
+                tiles += block_tiles(k.n);
                 ++active;
             }
         if (!active) break;
@@ -405,7 +407,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
         auto needed = [&](uint64_t m) {
             uint64_t ctas = 0;
             for (const Circuit& k : list)
-                if (r < k.blocks) ctas += ((1ULL << k.n) / kTileAmps + m - 1) / m;
+                if (r < k.blocks) ctas += (block_tiles(k.n) + m - 1) / m;
             return ctas;
         };
         const bool one_wave = active <= budget / 2;
@@ -416,7 +418,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
         const int first = (int)out.ctas.size();
         for (const Circuit& k : list) {
             if (r >= k.blocks) continue;
-            const uint64_t t = (1ULL << k.n) / kTileAmps, share = (t + per - 1) / per;
+            const uint64_t t = block_tiles(k.n), share = (t + per - 1) / per;
             const BlockStep& st = out.steps[k.first + r];
             for (uint64_t i = 0; i < share; ++i) {
                 MixedCta m;

@@ -428,7 +428,7 @@ double spectral_norm_2x2(const double* m) {
 }
 
 bool has_block_plan(int n, const llg_op* ops, int nops) {
-    if (n < 12) return false;
+    if (n < kBlockMinQubits) return false;
     for (int i = 0; i < nops; ++i)
         if (ops[i].kind == LLG_OP_U2 && !(spectral_norm_2x2(ops[i].m) <= kBlockNormLimit)) return false;
     return true;

@@ -467,6 +467,9 @@ int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror
     return LLG_OK;
 }
 
+// of a state that came from the host: measured before the first flush that may take blocks
+constexpr double kNormUnknown = 1e300;
+
 // log2 of the state's norm into st->log2_norm (waits for the stream)
 int measure_norm(llg_state* st) {
     ZTerms z;
@@ -481,26 +484,74 @@ int measure_norm(llg_state* st) {
     return LLG_OK;
 }
 
+// Microseconds that tile passes take for a gate on 6 .. 12 and more qubits, where a CTA's latency and not the arithmetic
+// counts (fits of seven circuits a size): merged gates that mix, H (cheaper in double-float), others.
+struct TileLatency {
+    double mixing, h, other;
+};
+TileLatency tile_latency(int P, int n) {
+    static const TileLatency f64[7] = {{1.15, 1.15, 0.4}, {1.35, 1.35, 0.4}, {1.4, 1.4, 0.4}, {1.6, 1.6, 0.4}, {2.45, 2.45, 0.6},
+                                      {4.0, 4.0, 0.5}, {7.0, 7.0, 0.75}};
+    static const TileLatency df64[7] = {{1.0, 1.0, 0.15}, {1.05, 1.0, 0.15}, {1.25, 1.1, 0.15}, {1.6, 1.2, 0.15}, {2.7, 1.6, 0.5},
+                                       {4.1, 2.0, 0.5}, {7.0, 3.0, 0.5}};
+    const int i = std::min(std::max(n, 6), 12) - 6;
+    return P == LLG_F64 ? f64[i] : df64[i];
+}
+
 // Which plan a flush takes when the caller has left the tile width and CTA size to the engine:
 // blocks when their passes cost less than tile passes with the same gates (judged on the blocks
-// planned so far).  Measured on this GPU, per 2^30 amplitudes: a block 8.6 (FP64) or 10.3 ms
-// (double-float), and at least 9.5 us; a CNOT or sign-flip pass 2.6 ms.  Tile passes take 3.2 FP64
-// multiply-adds per amplitude for a merged one-qubit gate that mixes and 4 for a diagonal one, at
-// 0.56 T a second (double-float: 2.0 ms per 2^30 for either); no less than 2.6 (FP64) or 2 us a
-// gate, however small the register (a CTA's latency); and one read and write of the state.  A channel
+// planned so far).  Measured on this GPU, per 2^30 amplitudes: a block 8.3 (FP64) or 10.1 ms
+// (double-float), and at least 10 us (11.5 with its planning on fewer than 12 qubits, whose passes end sooner than the
+// host); a CNOT or sign-flip pass 2.6 ms.  Tile passes take 3.2 FP64 multiply-adds per amplitude for a merged one-qubit gate
+// that mixes and 4 for a diagonal one, at 0.56 T a second (double-float: 2.0 ms per 2^30 for either); no less than
+// tile_latency's; and one read and write of the state.  A channel
 // on its own is a sparse pass: 6.2 ms per 2^30 on one qubit of a density matrix, 9 on two, at least 6 us.
-bool blocks_pay(int P, int n, const BlockPlan& plan) {
+// Tile passes / blocks, host included, us: 20 layers of rotations and CNOTs on 6, 8, 10, 11, 12 qubits 175 / 130, 244 /
+// 197, 501 / 245, 833 / 252, 1646 / 316; 1000 H and CNOT on 8, 10, 11, 12 547 / 899, 890 / 976, 1461 / 1035, 2400 / 1137.
+// h_share: of the gates that mix.
+bool blocks_pay(int P, int n, const BlockPlan& plan, double h_share) {
     const bool f64 = P == LLG_F64;
     const double amps = std::ldexp(1.0, n);
-    const double block = std::max(9.5e-6, amps * (f64 ? 8.0e-12 : 9.6e-12));
+    const double block = std::max(n < 12 ? 11.5e-6 : 10e-6, amps * (f64 ? 8.0e-12 : 9.6e-12));
     const double single = 3e-6 + amps * 2.4e-12;
-    const double t_blocks = plan.blocks * block + ((double)plan.steps.size() - plan.blocks) * single + 20e-6;
+    const double t_blocks = plan.blocks * block + ((double)plan.steps.size() - plan.blocks) * single + 5e-6;
     const double arith = f64 ? (3.2 * plan.mixing_1q + 4.0 * plan.diag_1q) / 0.56e12 : 1.9e-12 * (plan.mixing_1q + plan.diag_1q);
-    const double latency = f64 ? 2.6e-6 : 2.0e-6;
     const double gates = (double)plan.gates.size() - plan.small_matrices - plan.large_matrices;
-    const double t_tiles = gates > 0 ? std::max(std::max(arith * amps, latency * gates), amps * 4.8e-12) : 0.0;
+    const TileLatency l = tile_latency(P, n);
+    const double latency = 1e-6 * ((l.h * h_share + l.mixing * (1.0 - h_share)) * plan.mixing_1q + l.other * (gates - plan.mixing_1q));
+    const double t_tiles = gates > 0 ? std::max(std::max(arith * amps, latency), amps * 4.8e-12) : 0.0;
     const double channels = plan.small_matrices * std::max(6e-6, amps * 5.8e-12) + plan.large_matrices * std::max(6e-6, amps * 8.4e-12);
-    return t_blocks < t_tiles + channels;
+    return t_blocks < (n < 10 && channels == 0.0 ? 0.85 : 1.0) * (t_tiles + channels);  // the fits are within 15 %
+}
+
+// Whether a queue is worth the planning of blocks, by a count of its gates: planning that comes to nothing costs 10 to 60
+// us.  On fewer than 12 qubits tile passes have to take a while (without channels, which cost them 6 us each), and on
+// fewer than 10, where two-qubit gates cost them next to nothing, few gates may be of those.  H and as many CNOTs fill a block
+// with some ten gates: tile passes are faster in double-float, and on 10 qubits and fewer.
+bool worth_planning(int P, int n, const std::vector<llg_op>& q, double* h_share) {
+    double one = 0.0, two = 0.0, us = 0.0, mixing = 0.0, h = 0.0;
+    bool channels = false;
+    const TileLatency l = tile_latency(P, n);
+    for (const llg_op& o : q) {
+        if (o.kind == LLG_OP_H) {
+            us += l.h;
+            h += 1.0;
+            mixing += 1.0;
+        } else if (o.kind == LLG_OP_RX || o.kind == LLG_OP_RY || o.kind == LLG_OP_U2) {
+            us += l.mixing;
+            mixing += 1.0;
+        } else {
+            channels = channels || o.kind == kOpMatrix;
+            us += o.kind == kOpMatrix ? 6.0 : l.other;
+        }
+        if (o.kind == LLG_OP_CNOT || o.kind == LLG_OP_CZ || o.kind == LLG_OP_MCZ) two += 1.0;
+        else one += 1.0;
+    }
+    *h_share = mixing > 0.0 ? h / mixing : 0.0;
+    if (channels) return n >= 12 || us >= 45.0;
+    if ((P != LLG_F64 || n <= 10) && *h_share > 0.8 && two > 0.7 * one) return false;
+    if (n >= 12) return true;
+    return us >= (n < 9 ? 150.0 : n < 11 ? 100.0 : 80.0) && (n >= 10 || two <= 0.3 * one);
 }
 
 // growth of the norm bound over a queue (2x2s that are not unitary)
@@ -543,12 +594,17 @@ int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
     if (!gate_block_eligible(st->P, st->n)) return run_tiles(st, q, mirror, mirrored);
     // amplitudes stay below 2^(limit + 10) within a flush
     const double limit = st->P == LLG_F64 ? 900.0 : 90.0;
-    if (st->log2_norm > limit && st->log2_norm < HUGE_VAL)
+    double h_share = 0.0;
+    bool blocks = blocks_allowed(st) && worth_planning(st->P, st->n, q, &h_share) && has_block_plan(st->n, q.data(), (int)q.size());
+    if (blocks && st->log2_norm > limit && st->log2_norm < HUGE_VAL)
         if (int rc = measure_norm(st)) return rc;
-    if (blocks_allowed(st) && st->log2_norm <= limit && has_block_plan(st->n, q.data(), (int)q.size())) {
+    blocks = blocks && st->log2_norm <= limit;
+    if (blocks) {
         BlockPlanner planner(st->n, q.data(), (int)q.size(), false, &st->matrices);
-        planner.advance(8);
-        bool room = blocks_pay(st->P, st->n, planner.plan);
+        // a first look on few qubits, where the planning counts
+        const bool hopeless = st->n < 12 && planner.advance(3) && !blocks_pay(st->P, st->n, planner.plan, h_share);
+        if (!hopeless) planner.advance(8);
+        bool room = !hopeless && blocks_pay(st->P, st->n, planner.plan, h_share);
         if (room)
             if (int rc = ensure_blocks(st, q.size(), &room)) return rc;
         if (room) {
@@ -971,7 +1027,7 @@ int apply_matrix_now(llg_state* st, int k, const int* qubits, const double* m) {
         bd.k = ++k;
         m = mx;
     }
-    if (k == 5 && gate_block_eligible(st->P, st->n)) {
+    if (k == 5 && st->n >= 12 && gate_block_eligible(st->P, st->n)) {
         if (!st->d_block_tc) {
             const size_t cap = gate_block_weight_bytes(LLG_F64);
             LLG_CUDA(cudaMalloc(&st->d_block_tc, cap), "cudaMalloc(block weights)");
@@ -1210,7 +1266,7 @@ int llg_copy_from_host(llg_state* st, const double* amps) {
     st->matrices.clear();
     if (st->P == LLG_F64) {
         LLG_CUDA(cudaMemcpyAsync(st->d_psi, amps, st->size * 16, cudaMemcpyHostToDevice, st->stream), "cudaMemcpyAsync(H2D)");
-        if (gate_block_eligible(st->P, st->n)) return measure_norm(st);
+        st->log2_norm = kNormUnknown;
         LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
         return LLG_OK;
     }
@@ -1229,7 +1285,7 @@ int llg_copy_from_host(llg_state* st, const double* amps) {
         if (rc) return rc;
         LLG_CUDA(cudaEventRecord(st->stage_ev[which], st->stream), "cudaEventRecord");
     }
-    if (gate_block_eligible(st->P, st->n)) return measure_norm(st);
+    st->log2_norm = kNormUnknown;
     LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
     return LLG_OK;
 }
@@ -1613,7 +1669,7 @@ int llg_block_plan_export(int n, const llg_op* ops, int nops, llg_block_step* st
     tmp.n = n;
     for (int i = 0; i < nops; ++i)
         if (int rc = validate_op(&tmp, ops[i], "block_plan_export")) return rc;
-    if (!has_block_plan(n, ops, nops))
+    if (n < 12 || !has_block_plan(n, ops, nops))
         return set_error(LLG_EINVAL, "block_plan_export: no block plan (fewer than 12 qubits, or a 2x2 gate of norm above 1)");
     BlockPlanner planner(n, ops, nops);
     while (planner.advance(1 << 20)) {}

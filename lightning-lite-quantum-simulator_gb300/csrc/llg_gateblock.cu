@@ -202,7 +202,9 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_s;
-    const uint64_t ntiles = (1ULL << (n - 5)) / kGroups;
+    // registers of fewer than 12 qubits fill a part of their one tile: the other groups are zeros that nobody stores
+    const int groups = n >= 12 ? kGroups : 1 << (n - 5);
+    const uint64_t ntiles = n >= 12 ? (1ULL << (n - 5)) / kGroups : 1;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
         if (tile < ntiles) {
             const auto* pb = psi + (insert0_mask(tile * kGroups + (uint64_t)g, tmask) | (h ? off(1) : 0));
 #pragma unroll
-            for (int k = 0; k < 16; ++k) a[k] = __ldcg(pb + off(2 * k));
+            for (int k = 0; k < 16; ++k) a[k] = g < groups ? __ldcg(pb + off(2 * k)) : typename Elem<P>::S{};
         }
         int slot = 0, egb = 0;
         uint32_t phase = 1;  // of the slot's previous release: the first round needs no wait
@@ -451,6 +453,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                             }
                         }
                     }
+                    if (row >= groups) continue;
                     if (pair32) {
 #pragma unroll
                         for (int c = 0; c < T::kStep / 2; c += 2) {
@@ -763,7 +766,7 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool re
             if ((j >> b) & 1) to.o[j] |= 1ULL << bd.q[b];
     }
     const uint64_t most = ctas > 0 ? (uint64_t)ctas : (uint64_t)sm_count();
-    const uint64_t ntiles = kMixed ? most : (1ULL << (n - 5)) / kGroups;
+    const uint64_t ntiles = kMixed ? most : n >= 12 ? (1ULL << (n - 5)) / kGroups : 1;
     // programmatic dependent launch: the CTA's set-up (barriers, tensor memory, the gate's digits)
     // runs under the end of the stream's previous kernel
     cudaLaunchAttribute at;
@@ -783,7 +786,7 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool re
 
 }  // namespace
 
-bool gate_block_eligible(int P, int n) { return (P == LLG_F64 || P == LLG_DF64) && n >= 12; }
+bool gate_block_eligible(int P, int n) { return (P == LLG_F64 || P == LLG_DF64) && n >= kBlockMinQubits; }
 
 namespace {
 // f with the precision as a compile-time constant

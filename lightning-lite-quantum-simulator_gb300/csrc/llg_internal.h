@@ -226,7 +226,8 @@ struct BlockPlan {
 // 2x2 gates of a block have spectral norm at most this, so that its entries stay well below 2
 constexpr double kBlockNormLimit = 1.0 + 1e-6;
 double spectral_norm_2x2(const double* m);
-// false: no block plan (fewer than 12 qubits, or a 2x2 beyond the norm limit)
+constexpr int kBlockMinQubits = 6;
+// false: no block plan (fewer than kBlockMinQubits, or a 2x2 beyond the norm limit)
 bool has_block_plan(int n, const llg_op* ops, int nops);
 // Plans block by block, so that the first ones can run while the rest is planned.  `ops` is read by
 // the constructor only.

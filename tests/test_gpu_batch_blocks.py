@@ -43,6 +43,7 @@ def batch(sizes, depths, seed, wide=()):
 
 @pytest.mark.parametrize("sizes,wide", [
     ([12], ()),
+    ([10, 11, 12, 11, 10, 13], ()),
     ([12, 13, 12, 14, 16, 12], ()),
     ([3, 17, 12, 2, 15, 13, 8, 10, 14, 12], (4,)),
     ([12] * 90 + [13] * 80 + [5] * 20, ()),
