@@ -501,18 +501,18 @@ TileLatency tile_latency(int P, int n) {
 // Which plan a flush takes when the caller has left the tile width and CTA size to the engine:
 // blocks when their passes cost less than tile passes with the same gates (judged on the blocks
 // planned so far).  Measured on this GPU, per 2^30 amplitudes: a block 8.3 (FP64) or 10.1 ms
-// (double-float), and at least 10 us (11.5 with its planning on fewer than 12 qubits, whose passes end sooner than the
+// (double-float), and at least 8.5 us (10 with its planning on fewer than 12 qubits, whose passes end sooner than the
 // host); a CNOT or sign-flip pass 2.6 ms.  Tile passes take 3.2 FP64 multiply-adds per amplitude for a merged one-qubit gate
 // that mixes and 4 for a diagonal one, at 0.56 T a second (double-float: 2.0 ms per 2^30 for either); no less than
 // tile_latency's; and one read and write of the state.  A channel
 // on its own is a sparse pass: 6.2 ms per 2^30 on one qubit of a density matrix, 9 on two, at least 6 us.
-// Tile passes / blocks, host included, us: 20 layers of rotations and CNOTs on 6, 8, 10, 11, 12 qubits 175 / 130, 244 /
-// 197, 501 / 245, 833 / 252, 1646 / 316; 1000 H and CNOT on 8, 10, 11, 12 547 / 899, 890 / 976, 1461 / 1035, 2400 / 1137.
+// Tile passes / blocks, host included, us: 20 layers of rotations and CNOTs on 6, 8, 10, 11, 12 qubits 175 / 115, 237 /
+// 163, 498 / 231, 818 / 237, 1624 / 275; 1000 H and CNOT on 8, 10, 11, 12 547 / 899, 890 / 951, 1458 / 880, 2391 / 978.
 // h_share: of the gates that mix.
 bool blocks_pay(int P, int n, const BlockPlan& plan, double h_share) {
     const bool f64 = P == LLG_F64;
     const double amps = std::ldexp(1.0, n);
-    const double block = std::max(n < 12 ? 11.5e-6 : 10e-6, amps * (f64 ? 8.0e-12 : 9.6e-12));
+    const double block = std::max(n < 12 ? 10e-6 : 8.5e-6, amps * (f64 ? 8.0e-12 : 9.6e-12));
     const double single = 3e-6 + amps * 2.4e-12;
     const double t_blocks = plan.blocks * block + ((double)plan.steps.size() - plan.blocks) * single + 5e-6;
     const double arith = f64 ? (3.2 * plan.mixing_1q + 4.0 * plan.diag_1q) / 0.56e12 : 1.9e-12 * (plan.mixing_1q + plan.diag_1q);
