@@ -99,8 +99,8 @@ void block_tc_prepare(int P, int k, const double* m, void* weights);
 cudaError_t launch_block_tc(int P, void* psi, int n, const BlockDesc& bd, const void* d_weights, int* err_flag,
                             cudaStream_t s);
 
-// dense 5-qubit blocks of 16-byte states on the tensor cores (llg_gateblock.cu): n >= 12, bd.q in
-// increasing order.  d_weights: gate_block_weight_bytes of device memory, filled by
+// dense 5-qubit blocks of 16-byte states on the tensor cores (llg_gateblock.cu): n >= kBlockMinQubits, bd.q
+// in increasing order.  d_weights: gate_block_weight_bytes of device memory, filled by
 // launch_gate_block_matrix (d_matrix: 32 x 32 row-major (re, im) doubles on the device, bit b of an
 // index is bd.q[b]).  rows: the weights have row exponents of their own (launch_gate_block_matrix).  ready:
 // the weights were complete before the stream's previous kernel began.  mirror: nullptr, or the device address of a mapped host buffer that also

@@ -186,7 +186,7 @@ struct FastTraj {
                 d = make_double2(f * x.x, f * x.y);
                 s[j | cb] = c;
             } else {
-                d = make_double2(-d.x, -d.y);
+                d = make_double2(PolF64::neg(d.x), PolF64::neg(d.y));  // not on the FP64 pipe
             }
             s[j | cb | tb] = d;
         };

@@ -30,6 +30,15 @@ def tile_f64():
     st.close()
 
 
+def gate_block_f64():
+    """IEEE complex128 gate blocks: the same circuit at 26 qubits under the engine's own choice."""
+    n = 26
+    st = llgpu.State(n, "complex128")
+    st.apply_ops(workloads.layered_rotations(n, 4))
+    st.sync()
+    st.close()
+
+
 def tile_reg_c64():
     """complex64 register-tiled passes, 27 qubits (1 GiB), 13-qubit tiles."""
     n = 27
@@ -174,7 +183,7 @@ def adjoint_f64():
     adj.close()
 
 
-CASES = {"tile_f64": tile_f64, "traj_f64": traj_f64, "adjoint_f64": adjoint_f64, "block_tc": block_tc, "block_tc_f64": block_tc_f64, "dm_sparse": dm_sparse, "tile_reg_c64": tile_reg_c64, "tile_c64": tile_c64, "streaming": streaming,
+CASES = {"tile_f64": tile_f64, "gate_block_f64": gate_block_f64, "traj_f64": traj_f64, "adjoint_f64": adjoint_f64, "block_tc": block_tc, "block_tc_f64": block_tc_f64, "dm_sparse": dm_sparse, "tile_reg_c64": tile_reg_c64, "tile_c64": tile_c64, "streaming": streaming,
          "reductions": reductions, "readback": readback, "tsolve": tsolve}
 
 if __name__ == "__main__":
