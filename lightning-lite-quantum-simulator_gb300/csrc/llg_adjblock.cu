@@ -24,7 +24,9 @@
 //
 // What bounds k_cross: 32 bytes per amplitude pair against 20 digit products of M128 N64 K128 per 128
 // groups (5120 clocks of the tensor pipe) and 65536 accumulators read back for each.  The accumulators
-// fill tensor memory (512 columns), so products and epilogue of one CTA alternate.
+// fill tensor memory (512 columns), so products and epilogue of one CTA alternate.  Cutting both vectors into
+// digits takes most instructions: two teams of eight warps take the chunks in turn, since two warps a
+// scheduler issued on half of its cycles only (8 sets of 20 qubits: 173 us a block, with the two teams 115).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -48,13 +50,15 @@ constexpr int kDigitBytes = kRGroups * 64 * 2;             // one digit of one v
 constexpr int kVecBytes = kDigits * kDigitBytes;           // 16 KB
 constexpr int kRChunkBytes = 2 * kVecBytes;                // psi, lambda
 constexpr int kTileChunks = kGroups / kRGroups;            // 8 chunks per drain of the accumulators
-constexpr int kDepth = 4;                                  // chunks whose loads are in flight
+constexpr int kTeams = 2;                                  // of kSlicerWarps warps, which take the chunks in turn
+constexpr int kRSlicers = kTeams * kSlicerWarps;
 constexpr int kREpiWarps = 8;
-constexpr int kRMmaWarp = kSlicerWarps + kREpiWarps;
+constexpr int kRMmaWarp = kRSlicers + kREpiWarps;
 constexpr int kRThreads = (kRMmaWarp + 4) * 32;
 constexpr size_t kRSmem = (size_t)kRRing * kRChunkBytes;
-constexpr int kRLaunchRegs = 96, kRSlicerRegs = 96, kREpiRegs = 120, kRMmaRegs = 40;
-static_assert(2 * kRSlicerRegs + 2 * kREpiRegs + kRMmaRegs <= 5 * kRLaunchRegs, "the roles' registers come out of the launch's");
+constexpr int kRLaunchRegs = 72, kRSlicerRegs = 64, kREpiRegs = 104, kRMmaRegs = 40;
+static_assert(4 * kRSlicerRegs + 2 * kREpiRegs + kRMmaRegs <= 7 * kRLaunchRegs, "the roles' registers come out of the launch's");
+static_assert(kRRing % kTeams == 0, "a team keeps its slots");
 static_assert(kRSmem >= 128 * 64 * sizeof(double), "the sums pass through the ring at the end");
 
 struct CrossOffsets {
@@ -109,66 +113,61 @@ __global__ void __launch_bounds__(kRThreads, 1)
     const int mine = (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // tiles of this CTA, at least 1
     const int chunks = mine * kTileChunks;
 
-    if (warp < kSlicerWarps) {
+    if (warp < kRSlicers) {
         set_registers<kRLaunchRegs, kRSlicerRegs>();
-        // ---- slicers: warps 0-3 psi, 4-7 lambda; group g of the chunk, amplitudes j = h + 2 i + 8 u ----
-        const int vec = warp >> 2, u = warp & 3, g = lane & 15, h = lane >> 4;
+        // ---- slicers: of a team, warps 0-3 psi, 4-7 lambda; group g of the chunk, amplitudes j = h + 2 i + 8 u ----
+        const int team = warp / kSlicerWarps, vec = (warp >> 2) & 1, u = warp & 3, g = lane & 15, h = lane >> 4;
         const uint32_t eg = cut_exponent(exps[vec * gridDim.y + set]);
         const uint32_t eg20 = (eg << 20) | 0xFFFFFu;
         const double2* src = (vec ? lam : psi) + ((uint64_t)set << n) +
                              (insert0_mask((uint64_t)g, tmask) | (h ? to.o[1] : 0) | (u & 1 ? to.o[8] : 0) | (u & 2 ? to.o[16] : 0));
         const uint32_t at = (uint32_t)(vec * kVecBytes + (h + 2 * u) * 256 + (g >> 3) * 128 + (g & 7) * 16);
-        double2 a[kDepth][4];
-        auto load = [&](int q, double2 (&d)[4]) {
+        double2 a[4];
+        auto load = [&](int q) {
             const uint64_t tile = blockIdx.x + (uint64_t)(q >> 3) * gridDim.x;
             const double2* p = src + (insert0_mask(tile * kGroups, tmask) | coff[q & 7]);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) d[i] = __ldcg(p + to.o[2 * i]);
+            for (int i = 0; i < 4; ++i) a[i] = __ldcg(p + to.o[2 * i]);
         };
-#pragma unroll
-        for (int k = 0; k < kDepth; ++k) load(k, a[k]);  // chunks is a multiple of 8
-        int slot = 0;
+        load(team);  // chunks is a multiple of 8
+        int slot = team;
         uint32_t phase = 1;
-        bool first = true, ok = true;
-        for (int q0 = 0; q0 < chunks && ok; q0 += kDepth) {
+        bool first = true;
+#pragma unroll 1
+        for (int q = team; q < chunks; q += kTeams) {
+            uint32_t wh[8], wl[8];
+            __half2 sgn[4], bias[4];
 #pragma unroll
-            for (int k = 0; k < kDepth; ++k) {
-                if (!first && !warp_wait(empty0 + 8 * slot, phase, abort_s)) {
-                    ok = false;
-                    break;
-                }
-                uint32_t wh[8], wl[8];
-                __half2 sgn[4], bias[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const double2 v = a[k][i];
-                    const uint64_t xr = fixed_f64(v.x, eg20), xi = fixed_f64(v.y, eg20);
-                    wh[2 * i] = (uint32_t)(xr >> 32);
-                    wl[2 * i] = (uint32_t)xr;
-                    wh[2 * i + 1] = (uint32_t)(xi >> 32);
-                    wl[2 * i + 1] = (uint32_t)xi;
-                    const uint32_t sg = __byte_perm((uint32_t)__double2hiint(v.x), (uint32_t)__double2hiint(v.y), 0x7733);
-                    sgn[i] = h2_of((sg & 0x80008000u) | 0x3C003C00u);
-                    bias[i] = __hmul2(sgn[i], __half2half2(__ushort_as_half(0xE480)));  // -1152
-                }
-                unsigned char* dst = smem + slot * kRChunkBytes + at;
-                digits4<4, kDigitBytes>(wh, sgn, bias, dst);
-                digits4<4, kDigitBytes>(wl, sgn, bias, dst + 4 * kDigitBytes);
-                if (q0 + k + kDepth < chunks) load(q0 + k + kDepth, a[k]);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full0 + 8 * slot);
-                if (++slot == kRRing) {
-                    slot = 0;
-                    phase ^= 1;
-                    first = false;
-                }
+            for (int i = 0; i < 4; ++i) {
+                const double2 v = a[i];
+                const uint64_t xr = fixed_f64(v.x, eg20), xi = fixed_f64(v.y, eg20);
+                wh[2 * i] = (uint32_t)(xr >> 32);
+                wl[2 * i] = (uint32_t)xr;
+                wh[2 * i + 1] = (uint32_t)(xi >> 32);
+                wl[2 * i + 1] = (uint32_t)xi;
+                const uint32_t sg = __byte_perm((uint32_t)__double2hiint(v.x), (uint32_t)__double2hiint(v.y), 0x7733);
+                sgn[i] = h2_of((sg & 0x80008000u) | 0x3C003C00u);
+                bias[i] = __hmul2(sgn[i], __half2half2(__ushort_as_half(0xE480)));  // -1152
+            }
+            if (q + kTeams < chunks) load(q + kTeams);  // under the digits and the wait for a slot
+            if (!first && !warp_wait(empty0 + 8 * slot, phase, abort_s)) break;
+            unsigned char* dst = smem + slot * kRChunkBytes + at;
+            digits4<4, kDigitBytes>(wh, sgn, bias, dst);
+            digits4<4, kDigitBytes>(wl, sgn, bias, dst + 4 * kDigitBytes);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full0 + 8 * slot);
+            slot += kTeams;
+            if (slot >= kRRing) {
+                slot = team;
+                phase ^= 1;
+                first = false;
             }
         }
     } else if (warp < kRMmaWarp) {
         set_registers<kRLaunchRegs, kREpiRegs>();
         // ---- epilogue: rows 32 (warp & 3) + lane, columns 32 e .. +31 ----
-        const int row = 32 * (warp & 3) + lane, e = (warp - kSlicerWarps) >> 2;
+        const int row = 32 * (warp & 3) + lane, e = (warp - kRSlicers) >> 2;
         const uint32_t tbase = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * e);
         const int shift = cross_shift(log2_bound, tiles, cut_exponent(exps[set]), cut_exponent(exps[gridDim.y + set]));
         const int64_t half = shift ? (int64_t)1 << (shift - 1) : 0;
@@ -247,7 +246,7 @@ __global__ void __launch_bounds__(kRThreads, 1)
         if (ok) {
             Fixed2* out = partial + ((size_t)set * gridDim.x + blockIdx.x) * kAmps * kAmps;
             auto real = [&](int r, int c) { return D[r * 64 + c] + D[(r + 64) * 64 + c]; };
-            for (int k = tid - kSlicerWarps * 32; k < kAmps * kAmps; k += kREpiWarps * 32) {
+            for (int k = tid - kRSlicers * 32; k < kAmps * kAmps; k += kREpiWarps * 32) {
                 const int ja = k >> 5, jb = k & 31;
                 const int ra = 16 * (ja >> 3) + 8 * (ja & 1) + 2 * ((ja >> 1) & 3);
                 const int cb = 16 * (jb >> 3) + 8 * (jb & 1) + 2 * ((jb >> 1) & 3);
