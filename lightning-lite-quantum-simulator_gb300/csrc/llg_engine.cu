@@ -525,7 +525,7 @@ TileLatency tile_latency(int P, int n) {
 // tile_latency's; and one read and write of the state.  A channel
 // on its own is a sparse pass: 6.2 ms per 2^30 on one qubit of a density matrix, 9 on two, at least 6 us.
 // Tile passes / blocks, host included, us: 20 layers of rotations and CNOTs on 6, 8, 10, 11, 12 qubits 175 / 115, 237 /
-// 163, 498 / 231, 818 / 237, 1624 / 275; 1000 H and CNOT on 8, 10, 11, 12 547 / 899, 890 / 951, 1458 / 880, 2391 / 978.
+// 163, 498 / 231, 818 / 237, 1624 / 275; 1000 H and CNOT on 8, 10, 11, 12 547 / 899, 890 / 951, 1458 / 825, 2391 / 908.
 // h_share: of the gates that mix.
 bool blocks_pay(int P, int n, const BlockPlan& plan, double h_share) {
     const bool f64 = P == LLG_F64;
