@@ -851,15 +851,20 @@ bool plan_fast(int n, int nl, int workers, const std::vector<TrajGate>& gates, c
     std::vector<size_t> used(n, 0);
     for (size_t i = 0; i < gates.size(); ++i)
         for (int k = 0; k < gates[i].nt; ++k) uses[gates[i].q[k]].push_back((int)i);
-    auto put = [&](const std::vector<double>& v) {
+    auto put_heads = [&](bool inverted) {
         const int at = (int)tabs.size();
-        tabs.insert(tabs.end(), v.begin(), v.end());
+        for (int q = 0; q < n; ++q) tabs.push_back(inverted ? 1.0 / p[q].h : p[q].h);
         return at;
     };
-    auto heads = [&](bool inverted) {
-        std::vector<double> v(n);
-        for (int q = 0; q < n; ++q) v[q] = inverted ? inverse(p[q]).h : p[q].h;
-        return v;
+    // the products of subsets of f[0 .. count), `size` of them, from `start`
+    auto put_products = [&](const double* f, int count, size_t size, double start) {
+        const size_t at = tabs.size();
+        tabs.resize(at + size, start);
+        double* out = tabs.data() + at;
+        size_t len = 1;
+        for (int b = 0; b < count; ++b, len *= 2)
+            for (size_t k = 0; k < len; ++k) out[len + k] = out[k] * f[b];
+        return (int)at;
     };
     auto scale = [&]() {  // apply all pending factors
         bool any = false;
@@ -867,7 +872,7 @@ bool plan_fast(int n, int nl, int workers, const std::vector<TrajGate>& gates, c
         if (!any) return;
         FastStep s{};
         s.kind = FS_SCALE;
-        s.pend = put(heads(false));
+        s.pend = put_heads(false);
         steps.push_back(s);
         std::fill(p.begin(), p.end(), one);
     };
@@ -895,9 +900,12 @@ bool plan_fast(int n, int nl, int workers, const std::vector<TrajGate>& gates, c
         } else if (o.kind == EX_MCZ && G.nt == 2) {
             s.kind = FS_CZ;
         }
-        // far from their true size the amplitudes would leave the format's range
+        // far from their true size the amplitudes would leave the format's range (log2 of the factors, summed: 60)
         double spread = 0.0;
-        for (const Pair& x : p) spread += std::fabs(std::log2(std::fabs(x.h)));
+        bool wide = false;  // else 14 factors of at most 2^4 stay below the limit
+        for (const Pair& x : p) wide = wide || !(std::fabs(x.h) < 16.0 && std::fabs(x.h) > 1.0 / 16.0);
+        if (wide)
+            for (const Pair& x : p) spread += std::fabs(std::log2(std::fabs(x.h)));
         if (spread > 60.0 || s.kind == FS_SLOW) scale();
         if (s.kind == FS_SLOW) {
             TrajGate m = G;
@@ -957,17 +965,16 @@ bool plan_fast(int n, int nl, int workers, const std::vector<TrajGate>& gates, c
             };
             while (end < gates.size() && end < i + 6 && off(gates[end])) ++end;
             if (end == i + 6) {
-                std::vector<double> w(1, 1.0);
+                double f[16];
                 for (int q = lw; q < nl; ++q) {
-                    const size_t len = w.size();
-                    for (size_t k = 0; k < len; ++k) w.push_back(w[k] * p[q].h);
+                    f[q - lw] = p[q].h;
                     p[q] = one;
                 }
                 FastStep x{};
                 x.kind = FS_SCALE;
                 x.flat = 1;
-                x.tab = put(w);
-                x.ntab = (int)w.size();
+                x.ntab = 1 << (nl - lw);
+                x.tab = put_products(f, nl - lw, (size_t)x.ntab, 1.0);
                 steps.push_back(x);
                 weighed = false;
             }
@@ -1006,25 +1013,19 @@ bool plan_fast(int n, int nl, int workers, const std::vector<TrajGate>& gates, c
         s.f0 = fixed62(f * f0);
         s.f1 = fixed62(f * f1);
         // weights: products of the other positions' squares, in the order of the pass's index bits
-        std::vector<double> sq;
+        double sq[16];
+        int count = 0;
         for (int q = 0; q < nl; ++q)
-            if (q != s.q && q != s.t) sq.push_back((p[q] * p[q]).h);
-        auto products = [&](size_t first, size_t count, size_t size, double start) {
-            std::vector<double> out(size, start);
-            size_t len = 1;
-            for (size_t b = 0; b < count && first + b < sq.size(); ++b, len *= 2)
-                for (size_t k = 0; k < len; ++k) out[len + k] = out[k] * sq[first + b];
-            return out;
-        };
-        s.tab = put(products(0, 5, kTabLanes, 1.0));
-        put(products(0, 5, kTabLanes, nl < n ? (p[nl] * p[nl]).h : 1.0));
-        const size_t rest = sq.size() > 5 ? sq.size() - 5 : 0;
-        put(products(5, rest, (size_t)1 << rest, 1.0));
+            if (q != s.q && q != s.t) sq[count++] = (p[q] * p[q]).h;
+        const int low = std::min(count, 5), rest = count - low;
+        s.tab = put_products(sq, low, kTabLanes, 1.0);
+        put_products(sq, low, kTabLanes, nl < n ? (p[nl] * p[nl]).h : 1.0);
+        put_products(sq + low, rest, (size_t)1 << rest, 1.0);
         s.ntab = (int)tabs.size() - s.tab;
-        s.pend = put(heads(false));
+        s.pend = put_heads(false);
         pq = pq * g;
         if (s.kind >= FS_CNOT) pt = pt * g;
-        put(heads(true));
+        put_heads(true);
         steps.push_back(s);
         if (tabs.size() > kFastTabWords) return false;
     }

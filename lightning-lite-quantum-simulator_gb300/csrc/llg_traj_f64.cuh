@@ -52,7 +52,9 @@ constexpr int kFastWorkers = 512;
 constexpr int kFastThreads = kFastWorkers + 32;
 constexpr int kFastPairs = kUChunk / 2;
 constexpr int kTabLanes = 32;
-constexpr int kTabMax = 2 * kTabLanes + 128;       // 13 local qubits: 12 index bits of a pass
+// 13 local qubits: 12 index bits of a pass, or 8 loop bits of 32 threads in an FS_SCALE
+constexpr int kTabMax = 256;
+static_assert(kTabMax >= 2 * kTabLanes + 128 && kTabMax >= (1 << 13) / 32, "a step's table");
 constexpr size_t kFastTabWords = (size_t)4 << 20;  // 32 MB of tables at most
 constexpr double kFastKappa = 0.125;
 constexpr int kFastMinQubits = 3;

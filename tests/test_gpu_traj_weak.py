@@ -69,6 +69,22 @@ def test_shapes_agree(n, cluster, threads):
     assert np.array_equal(j, j2) and np.max(np.abs(z - z2)) <= 1e-10
 
 
+@pytest.mark.parametrize("n,threads", [(13, 32), (13, 64), (12, 32), (9, 256)])
+def test_factors_of_looped_qubits_are_applied(n, threads):
+    # all qubits first, then runs of gates on the lowest ones: the others' factors go before each run
+    rng = np.random.default_rng(n)
+    recs = []
+    for _ in range(3):
+        for q in range(n):
+            recs += [(OP_RX, q, 0, float(rng.uniform(0, 6.28))), (OP_CNOT, q, (q + 1) % n)]
+        for _ in range(12):
+            recs += [(OP_RY, int(rng.integers(3)), 0, float(rng.uniform(0, 6.28))), (OP_CNOT, 0, 2)]
+    ops = make_ops(recs)
+    z, j, _ = llgpu.Traj(n, ops, 0.03, 0.02, 24, "fp64", 1, threads).launch(6, 24)
+    zo, jo, _, margin_o = oracle.traj_run(n, ops, 0.03, 0.02, 6, 0, 24, log_sites=llgpu.noise_sites(ops))
+    assert margin_o > 1e-12 and np.array_equal(j, jo) and np.max(np.abs(z - zo)) <= 1e-10
+
+
 def test_many_gates_on_few_qubits():
     # the factors of two qubits grow for 700 gates, past the spread that the planner allows
     n = 6
