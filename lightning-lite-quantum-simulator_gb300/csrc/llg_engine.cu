@@ -194,7 +194,7 @@ int ensure_device_buffers(llg_state* st) {
     if (!st->d_partials) {
         constexpr size_t kPart = sizeof(double) * kRedBlocks * kPartialSlots, kRed = sizeof(double) * kRedSlots;
         constexpr size_t kWords = 4 * sizeof(int);
-        LLG_CUDA(cudaHostAlloc((void**)&st->h_out, sizeof(Readout), cudaHostAllocDefault), "cudaHostAlloc(readout)");
+        if (!st->h_out) LLG_CUDA(cudaHostAlloc((void**)&st->h_out, sizeof(Readout), cudaHostAllocDefault), "cudaHostAlloc(readout)");
         LLG_CUDA(cudaMalloc(&st->d_partials, kPart + kWords + kRed), "cudaMalloc(partials)");
         st->d_flags = reinterpret_cast<int*>(st->d_partials + kRedBlocks * kPartialSlots);
         st->d_ticket = reinterpret_cast<unsigned*>(st->d_flags + 2);
