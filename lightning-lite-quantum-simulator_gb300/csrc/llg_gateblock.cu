@@ -394,6 +394,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                 for (int p = 0; p < 2; ++p) {
                     const int col = T::kStep * (2 * e + p);  // within each diagonal's 32 columns
                     uint32_t v[S][T::kStep];
+                    __syncwarp();  // the loads are of the whole warp: lanes part in the scaling and where a tile is partly filled
 #pragma unroll
                     for (int d = 0; d < S; ++d) {
                         const uint32_t taddr = tlane + (uint32_t)(half * T::kSetStride + 32 * d + col);
@@ -473,8 +474,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                         }
                     }
                     meet();
-                    if (row >= groups) continue;
-                    if (pair32) {
+                    if (row < groups && pair32) {
 #pragma unroll
                         for (int c = 0; c < T::kStep / 2; c += 2) {
                             uint64_t w[4];
@@ -483,11 +483,11 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                                          "l"(w[2]), "l"(w[3])
                                          : "memory");
                         }
-                    } else {
+                    } else if (row < groups) {
 #pragma unroll
                         for (int c = 0; c < T::kStep / 2; ++c) psi[pos + off(c)] = out[c];
                     }
-                    if (mirror) {
+                    if (mirror && row < groups) {
 #pragma unroll
                         for (int c = 0; c < T::kStep / 2; ++c) {
                             if constexpr (P == LLG_F64) mirror[pos + off(c)] = out[c];
