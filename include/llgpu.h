@@ -447,6 +447,9 @@ int llg_profile(llg_state* st, int on);
 int llg_profile_read(llg_state* st, double* ms, int64_t* launches, int reset);
 /* Process-wide number of kernels the engine has launched (all states). */
 int64_t llg_kernel_launches(void);
+/* Process-wide number of gate-block launches (states, batches when their graph is captured, adjoint sweeps): whether a
+ * list ran as dense 5-qubit blocks or as tile passes, which the engine decides. */
+int64_t llg_gate_block_launches(void);
 /* The state's CUDA stream (a cudaStream_t), for callers that order their own work after it. */
 int llg_get_stream(const llg_state* st, void** out);
 /* Measurement aid with no counterpart in the reference: the current device's FP64 fused

@@ -1595,6 +1595,8 @@ int llg_profile_read(llg_state* st, double* ms, int64_t* launches, int reset) {
 
 int64_t llg_kernel_launches(void) { return g_launches.load(); }
 
+int64_t llg_gate_block_launches(void) { return gate_block_launches(); }
+
 int llg_fp64_fma_rate(int iters, double* fma_per_s) {
     if (!fma_per_s || iters < 1) return set_error(LLG_EINVAL, "fp64_fma_rate: bad argument");
     LLG_CUDA(fp64_fma_rate(iters, fma_per_s), "fp64_fma_rate");

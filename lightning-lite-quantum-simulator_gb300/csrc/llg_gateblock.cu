@@ -43,6 +43,7 @@
 // size, so adding 1.5 2^23 leaves the integer in the low bits of the float.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include <type_traits>
@@ -773,6 +774,8 @@ int sm_count() {
     return sms;
 }
 
+std::atomic<int64_t> g_block_launches{0};
+
 // ctas: CTAs a state (0: one per SM); sets states from psi and, unless nullptr, as many from `second`
 template <int P, bool kRows, bool kMixed = false, bool kSplit = false>
 cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool ready, int* err, cudaStream_t s, double* mirror,
@@ -804,12 +807,15 @@ cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool re
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = kSplit ? 2 : 1;
+    ++g_block_launches;
     return cudaLaunchKernelEx(&cfg, k_gate_block<P, kRows, kMixed, kSplit>, static_cast<typename Elem<P>::S*>(psi), n, to, bd.tmask,
                               static_cast<const uint4*>(w), ready, err, reinterpret_cast<double2*>(mirror),
                               BlockBatch<P>{static_cast<typename Elem<P>::S*>(second), sets, gate_block_weight_bytes(P) / 16, max_exp, mixed});
 }
 
 }  // namespace
+
+int64_t gate_block_launches() { return g_block_launches.load(); }
 
 bool gate_block_eligible(int P, int n) { return (P == LLG_F64 || P == LLG_DF64) && n >= kBlockMinQubits; }
 

@@ -106,6 +106,7 @@ cudaError_t launch_block_tc(int P, void* psi, int n, const BlockDesc& bd, const 
 // the weights were complete before the stream's previous kernel began.  mirror: nullptr, or the device address of a mapped host buffer that also
 // receives the output as FP64.  A kernel whose waits run out sets *err_flag to 1.
 bool gate_block_eligible(int P, int n);
+int64_t gate_block_launches();  // of this process, all forms
 size_t gate_block_weight_bytes(int P);
 cudaError_t launch_gate_block_matrix(int P, const double* d_matrix, void* d_weights, cudaStream_t s);
 // the weights of `nblocks` blocks of a plan (d_steps: their steps, in order; d_matrices: of the kind-4

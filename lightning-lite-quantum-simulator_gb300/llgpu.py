@@ -126,6 +126,7 @@ def lib() -> ctypes.CDLL:
             "llg_profile": (i, [vp, i]),
             "llg_profile_read": (i, [vp, vp, vp, i]),
             "llg_kernel_launches": (ctypes.c_int64, []),
+            "llg_gate_block_launches": (ctypes.c_int64, []),
             "llg_fp64_fma_rate": (i, [i, P(d)]),
             "llg_get_stream": (i, [vp, P(vp)]),
             "llg_expect_zz_noalloc": (i, [vp, i, i, i, vp, vp, vp, vp, vp]),
@@ -205,6 +206,10 @@ def device_count() -> int:
 
 def kernel_launches() -> int:
     return int(lib().llg_kernel_launches())
+
+
+def gate_block_launches() -> int:
+    return int(lib().llg_gate_block_launches())
 
 
 def _ptr(a: np.ndarray) -> int:
