@@ -962,7 +962,7 @@ int llg_adjoint_create(int n, const llg_op* ops, int nops, int nparams, int max_
         return set_error(LLG_EINVAL, "adjoint_create: " + err);
     }
     h->tiles = 1 << (n - t);
-    if (precision == LLG_F64 && n >= 12 && n <= 26 && has_block_plan(n, ops, nops)) {
+    if (precision == LLG_F64 && n >= 12 && n <= 26 && has_block_plan(n, ops, nops) && keeps_norms(ops, nops)) {
         bool fits = true;  // sign flips on more than five qubits have no block
         for (int i = 0; i < nops; ++i) fits = fits && !(ops[i].kind == LLG_OP_MCZ && popcount64(ops[i].mask) > 5);
         if (fits) {

@@ -358,7 +358,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
         const double amps = std::ldexp(1.0, n);
         at += 1ULL << n;
         std::vector<llg_op> mine(ops + off[c], ops + off[c + 1]);
-        bool fits = n >= kBatchBlockQubits && nops > 0 && has_block_plan(n, mine.data(), nops);
+        bool fits = n >= kBatchBlockQubits && nops > 0 && has_block_plan(n, mine.data(), nops) && keeps_norms(mine.data(), nops);
         for (llg_op& o : mine) {
             o.param = -1;
             if (o.kind == LLG_OP_MCZ && __builtin_popcountll(o.mask) > 5) fits = false;

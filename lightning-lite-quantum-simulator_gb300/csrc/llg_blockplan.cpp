@@ -434,4 +434,20 @@ bool has_block_plan(int n, const llg_op* ops, int nops) {
     return true;
 }
 
+bool keeps_norms(const llg_op* ops, int nops) {
+    double drift = 0.0;
+    for (int i = 0; i < nops; ++i) {
+        if (ops[i].kind != LLG_OP_U2) continue;
+        const double* m = ops[i].m;
+        const double largest = spectral_norm_2x2(m);
+        const std::complex<double> det = std::complex<double>(m[0], m[1]) * std::complex<double>(m[6], m[7]) -
+                                         std::complex<double>(m[2], m[3]) * std::complex<double>(m[4], m[5]);
+        if (!(largest > 0.0)) return false;
+        const double off = std::max(largest - 1.0, 1.0 - std::abs(det) / largest);  // of both singular values
+        if (!(off <= kBlockNormLimit - 1.0)) return false;
+        drift += off;
+    }
+    return drift <= 0.25;
+}
+
 }  // namespace llg

@@ -613,7 +613,8 @@ int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
     // amplitudes stay below 2^(limit + 10) within a flush
     const double limit = st->P == LLG_F64 ? 900.0 : 90.0;
     double h_share = 0.0;
-    bool blocks = blocks_allowed(st) && worth_planning(st->P, st->n, q, &h_share) && has_block_plan(st->n, q.data(), (int)q.size());
+    bool blocks = blocks_allowed(st) && worth_planning(st->P, st->n, q, &h_share) && has_block_plan(st->n, q.data(), (int)q.size()) &&
+                  keeps_norms(q.data(), (int)q.size());
     if (blocks && st->log2_norm > limit && st->log2_norm < HUGE_VAL)
         if (int rc = measure_norm(st)) return rc;
     blocks = blocks && st->log2_norm <= limit;

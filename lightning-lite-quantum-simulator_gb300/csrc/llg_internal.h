@@ -229,6 +229,11 @@ double spectral_norm_2x2(const double* m);
 constexpr int kBlockMinQubits = 6;
 // false: no block plan (fewer than kBlockMinQubits, or a 2x2 beyond the norm limit)
 bool has_block_plan(int n, const llg_op* ops, int nops);
+// Whether the 2x2s of a list are unitary within the norm limit, and all of them together within a quarter.  A block's weights are
+// whole numbers in units of 2^-62 of 1, whatever the size of the product: five gates 0.01 U leave it 1e-10 and
+// 7e-9 of relative error, five gates 1e-4 U nothing at all.  Lists with other 2x2s (scaled gates, Kraus operators, projectors)
+// run as tile passes, which are FP64 throughout.
+bool keeps_norms(const llg_op* ops, int nops);
 // Plans block by block, so that the first ones can run while the rest is planned.  `ops` is read by
 // the constructor only.
 class BlockPlanner {
