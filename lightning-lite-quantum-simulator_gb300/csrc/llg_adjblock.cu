@@ -377,6 +377,17 @@ __global__ void k_angles(const double* __restrict__ params, int nparams, const i
     out[i] = make_double2(c, s);
 }
 
+// |0..0> in set blockIdx.x (its amplitudes were zeroed).  A set with an angle that is not finite starts from NaN, which
+// the blocks carry to its energy and gradients: in the integers of its weights the angle would look like any other.
+__global__ void __launch_bounds__(128)
+    k_block_init(double2* __restrict__ psi, int n, const double2* __restrict__ angles, int nocc) {
+    const int set = blockIdx.x;
+    bool bad = false;
+    for (int k = threadIdx.x; k < nocc; k += 128) bad = bad || !isfinite(angles[(size_t)set * nocc + k].x);
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x == 0) psi[(uint64_t)set << n] = make_double2(bad ? __longlong_as_double(0x7FF8000000000000LL) : 1.0, 0.0);
+}
+
 // Gradients of block blockIdx.x's parametrised gates for set blockIdx.y, from R after the block: per gate,
 // last to first, Im tr(P R), then R <- G^+ R G.  In fixed point against the Frobenius norm (60 bits; the
 // norm is kept, so entries stay below 2^60 and traces below 2^63), every product rounded once: a gradient
@@ -518,6 +529,11 @@ cudaError_t launch_max_exponent(const void* psi, const void* lam, int n, int set
 
 cudaError_t launch_angles(const double* params, int nparams, const int* occ_code, int nocc, int sets, double2* out, cudaStream_t s) {
     k_angles<<<(sets * nocc + 255) / 256, 256, 0, s>>>(params, nparams, occ_code, nocc, sets, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_block_init(double2* psi, int n, const double2* angles, int nocc, int sets, cudaStream_t s) {
+    k_block_init<<<sets, 128, 0, s>>>(psi, n, angles, nocc);
     return cudaGetLastError();
 }
 

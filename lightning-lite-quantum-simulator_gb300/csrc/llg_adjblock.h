@@ -25,6 +25,8 @@ cudaError_t launch_cross(const void* psi, const void* lam, int n, int sets, int 
 cudaError_t launch_max_exponent(const void* psi, const void* lam, int n, int sets, uint32_t* exps, cudaStream_t s);
 // (cos, sin) of half the angles; occ_code: 2 parameter + anything
 cudaError_t launch_angles(const double* params, int nparams, const int* occ_code, int nocc, int sets, double2* out, cudaStream_t s);
+// |0..0> in every set (zeroed before); NaN in one whose angles are not all finite
+cudaError_t launch_block_init(double2* psi, int n, const double2* angles, int nocc, int sets, cudaStream_t s);
 // dE/dtheta of every parametrised gate, grads[set][occurrence], from R[step][set]
 cudaError_t launch_block_grads(const double2* R, const BlockStep* steps, int nsteps, const BlockGate* gates, const double2* angles,
                                int nocc, int sets, double* grads, cudaStream_t s);

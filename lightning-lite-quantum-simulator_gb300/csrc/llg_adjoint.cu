@@ -796,8 +796,7 @@ int run_blocks(llg_adjoint* h, int batch, bool grads) {
             ADJ_CUDA(launch_gate_block_weights(LLG_F64, h->d_bgates, h->d_bsteps, steps, inverse, s, nullptr, ang, h->nocc, sets, true),
                      "block weights");
         ADJ_CUDA(cudaMemsetAsync(psi, 0, (size_t)sets * h->state_bytes, s), "memset psi");
-        k_set_rows<PolF64><<<(sets + 255) / 256, 256, 0, s>>>(psi, n, sets);
-        ADJ_CUDA(cudaGetLastError(), "init rows");
+        ADJ_CUDA(launch_block_init(psi, n, ang, h->nocc, sets, s), "init rows");
         const int fwd_ctas = block_ctas(tiles, sets, sms), bwd_ctas = block_ctas(tiles, 2 * sets, sms);
         for (int j = 0; j < steps; ++j)
             ADJ_CUDA(launch_gate_block_batch(psi, nullptr, sets, fwd_ctas, n, desc(j), h->d_bweights + (size_t)j * sets * wb,
