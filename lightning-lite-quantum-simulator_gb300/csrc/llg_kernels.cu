@@ -12,6 +12,7 @@
 //    (fixed grid, per-block partials, one FP64 pass over the partials).
 #include <atomic>
 #include <cstdio>
+#include <type_traits>
 
 #include "llg_common.cuh"
 #include "llg_launch.h"
@@ -522,30 +523,47 @@ __global__ void __launch_bounds__(kThreads) k_reduce_z(const typename P::S* __re
                     if (c < z.nclass) rows[c][tid] = rc[c];
             }
             __syncthreads();
+            // kAll: counts of 0 are multiplied as well (7 of 105 us at 23 qubits less than leaving them out), which an infinite
+            // |a|^2 would turn into NaN
+            auto add_rows = [&](auto all) {
+                constexpr bool kAll = decltype(all)::value;
 #pragma unroll 4
-            for (int r = 0; r < count; ++r) {
-                const uint64_t i = (blockIdx.x + (r0 + r) * step) * kThreads + tid;
-                if (i >= size) break;
-                const auto a = P::load(psi[i]);
-                if constexpr (P::kPrecision == LLG_F64) {
-                    const double n = fma(a.re, a.re, a.im * a.im);
-                    acc[0] += n;
-#pragma unroll
-                    for (int c = 0; c < kMaxZClasses; ++c)
-                        if (c < z.nclass) {
-                            const RowCount rc = rows[c][r];
-                            acc[1 + c] = fma((double)__dp4a(rc.w0, x0, __dp4a(rc.w1, x1, rc.base + inside[c])), n, acc[1 + c]);
-                        }
-                } else {
-                    acc[0] = P::acc_norm(acc[0], a);
+                for (int r = 0; r < count; ++r) {
+                    const uint64_t i = (blockIdx.x + (r0 + r) * step) * kThreads + tid;
+                    if (i >= size) break;
+                    const auto a = P::load(psi[i]);
+                    [[maybe_unused]] double n = 0.0;
+                    if constexpr (P::kPrecision == LLG_F64) {
+                        n = fma(a.re, a.re, a.im * a.im);
+                        acc[0] += n;
+                    } else {
+                        acc[0] = P::acc_norm(acc[0], a);
+                    }
 #pragma unroll
                     for (int c = 0; c < kMaxZClasses; ++c)
                         if (c < z.nclass) {
                             const RowCount rc = rows[c][r];
                             const int cnt = __dp4a(rc.w0, x0, __dp4a(rc.w1, x1, rc.base + inside[c]));
-                            if (cnt) acc[1 + c] = P::acc_norm_w(acc[1 + c], a, (float)cnt);
+                            if constexpr (P::kPrecision == LLG_F64) {
+                                if (kAll || cnt) acc[1 + c] = fma((double)cnt, n, acc[1 + c]);
+                            } else {
+                                if (cnt) acc[1 + c] = P::acc_norm_w(acc[1 + c], a, (float)cnt);
+                            }
                         }
                 }
+            };
+            if constexpr (P::kPrecision == LLG_F64) {
+                double before[kRedSlots];
+#pragma unroll
+                for (int s = 0; s < kRedSlots; ++s) before[s] = acc[s];
+                add_rows(std::true_type());
+                if (!isfinite(acc[0])) {
+#pragma unroll
+                    for (int s = 0; s < kRedSlots; ++s) acc[s] = before[s];
+                    add_rows(std::false_type());
+                }
+            } else {
+                add_rows(std::false_type());
             }
         }
     } else {
