@@ -380,10 +380,7 @@ int ensure_blocks(llg_state* st, size_t nops, bool* room) {
     return LLG_OK;
 }
 
-// A flush as dense 5-qubit blocks on the tensor cores (llg_blockplan.cpp, llg_gateblock.cu), the rest
-// of the plan made while the first blocks run.  nops: the flush's gates, for which ensure_blocks() found room.
-// mirror / mirrored: as for run_tiles.
-int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
+int run_block_groups(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
     constexpr int kGroup = kBlockGroup;
     const size_t wb = gate_block_weight_bytes(st->P), slots = block_slots(nops);
     LLG_CUDA(cudaEventSynchronize(st->ops_done), "cudaEventSynchronize");  // the staging buffer's last copies
@@ -483,6 +480,20 @@ int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror
     }
     LLG_CUDA(cudaEventRecord(st->ops_done, st->stream), "cudaEventRecord");
     return LLG_OK;
+}
+
+// A flush as dense 5-qubit blocks on the tensor cores (llg_blockplan.cpp, llg_gateblock.cu), the rest
+// of the plan made while the first blocks run.  nops: the flush's gates, for which ensure_blocks() found room.
+// mirror / mirrored: as for run_tiles.
+int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
+    const int rc = run_block_groups(st, planner, nops, mirror, mirrored);
+    if (rc) {
+        // the streams may have parted: no upload may still read the staging buffer that the next flush fills, and no kernel
+        // the weights
+        cudaStreamSynchronize(st->side);
+        cudaStreamSynchronize(st->stream);
+    }
+    return rc;
 }
 
 // of a state that came from the host: measured before the first flush that may take blocks
