@@ -25,6 +25,7 @@
 
 #include "../../include/llgpu.h"
 #include "llg_common.cuh"
+#include "llg_cost.h"
 #include "llg_internal.h"
 #include "llg_launch.h"
 #include "llg_tile.cuh"
@@ -322,6 +323,9 @@ uint64_t block_tiles(int n) { return n > 12 ? 1ULL << (n - 12) : 1; }
 constexpr int kBatchBlockQubits = 10;
 constexpr size_t kWeightsCap = (size_t)256 << 20;
 
+// seconds an amplitude that tile passes compute for these gates
+double tile_arith(const GateCounts& c) { return (kTileMixFma * (c.h + c.real + c.general) + kTileDiagFma * c.diag) / kTileFmaRate; }
+
 struct BlockSet {
     std::vector<char> in;                          // per circuit: takes blocks
     std::vector<BlockStep> steps;                  // of all circuits, one after the other
@@ -332,8 +336,7 @@ struct BlockSet {
 };
 
 // Which circuits take gate blocks, and their launches.  Blocks against tile passes for the batch as a whole, by
-// the same rates as a single state's choice: tiles 3.2 FP64 multiply-adds per amplitude and mixing gate, 4 per
-// diagonal one at 0.56 T a second, 2.6 us a gate at least; a launch of blocks 5 us and 4.5 us for every tile
+// the rates of llg_cost.h, 2.6 us a gate of tile passes at least; a launch of blocks 5 us and 4.5 us for every tile
 // of the CTA that has most.  Measured, tile passes / blocks, random gates: 36 circuits of 10 to 18 qubits and 200
 // gates 1048 / 335 us; 512 of 10 to 22, 152.9 / 43.6 ms; 5 of 12 and 13 qubits and 100 gates 318 / 103 us; 16 of
 // 12 to 16 and 40 gates 312 / 73 us; 200 of 12 qubits and 200 gates, each its own CTA either way, keep 950 us of
@@ -365,7 +368,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
         }
         if (!fits) {
             // about three multiply-adds a gate
-            small_arith += 2.0 * nops * amps / 0.56e12;
+            small_arith += 2.0 * nops * amps / kTileFmaRate;
             small_longest = std::max(small_longest, 2.0e-6 * nops);
             ++alone;
             continue;
@@ -375,7 +378,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
         }
         const BlockPlan& p = planner.plan;
         if (out.steps.size() + p.steps.size() > cap) {
-            small_arith += (3.2 * p.mixing_1q + 4.0 * p.diag_1q) * amps / 0.56e12;
+            small_arith += tile_arith(p.counts) * amps;
             continue;
         }
         list.push_back({c, n, offset, (int)out.steps.size(), (int)p.steps.size()});
@@ -384,7 +387,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
             out.steps.push_back(st);
         }
         out.gates.insert(out.gates.end(), p.gates.begin(), p.gates.end());
-        arith += (3.2 * p.mixing_1q + 4.0 * p.diag_1q) * amps / 0.56e12;
+        arith += tile_arith(p.counts) * amps;
         longest = std::max(longest, 2.6e-6 * (double)p.gates.size());
     }
     if (list.empty()) return false;

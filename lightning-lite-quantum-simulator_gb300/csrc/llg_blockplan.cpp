@@ -1,5 +1,5 @@
 // llg_blockplan.cpp -- plans a gate list as dense 5-qubit blocks (llg_gateblock.cu) for 16-byte
-// states of 12 and more qubits.
+// states of 6 and more qubits.
 //
 // A block costs the same whatever it holds, so the plan wants few of them.  Runs of one-qubit gates
 // are multiplied first (g2 @ g1).  Order is kept per qubit, up to commutation in the Z basis: a
@@ -44,7 +44,87 @@ void matmul(const double* a, const double* b, double* out) {
     }
 }
 
+// what a 2x2 costs in tile passes; a run of them by the classes alone
+enum Class2x2 : uint8_t { kNone, kDiag, kMove, kH, kRealX, kRealY, kGeneral, kClasses };
+constexpr Class2x2 kMerge[kClasses][kClasses] = {
+    {kNone, kDiag, kMove, kH, kRealX, kRealY, kGeneral},
+    {kDiag, kDiag, kGeneral, kGeneral, kGeneral, kGeneral, kGeneral},
+    {kMove, kGeneral, kNone, kGeneral, kGeneral, kGeneral, kGeneral},
+    {kH, kGeneral, kGeneral, kNone, kGeneral, kGeneral, kGeneral},
+    {kRealX, kGeneral, kGeneral, kGeneral, kRealX, kGeneral, kGeneral},
+    {kRealY, kGeneral, kGeneral, kGeneral, kGeneral, kRealY, kGeneral},
+    {kGeneral, kGeneral, kGeneral, kGeneral, kGeneral, kGeneral, kGeneral},
+};
+Class2x2 class_2x2(const double* m) {
+    auto zero = [&](int k) { return m[2 * k] == 0.0 && m[2 * k + 1] == 0.0; };
+    if (zero(1) && zero(2)) return kDiag;
+    if (zero(0) && zero(3)) return kMove;
+    if (m[1] != 0.0 || m[7] != 0.0) return kGeneral;
+    if (m[3] == 0.0 && m[5] == 0.0) return m[0] == m[2] && m[0] == m[4] && m[0] == -m[6] ? kH : kRealY;
+    return m[2] == 0.0 && m[4] == 0.0 ? kRealX : kGeneral;
+}
+Class2x2 class_of(const llg_op& o) {
+    switch (o.kind) {
+        case LLG_OP_H: return kH;
+        case LLG_OP_X: return kMove;
+        case LLG_OP_RX: return kRealX;
+        case LLG_OP_RY: return kRealY;
+        case LLG_OP_RZ: return kDiag;
+        default: return class_2x2(o.m);
+    }
+}
+void add_classes(const int* count, GateCounts& c) {
+    c.diag += count[kDiag];
+    c.moves += count[kMove];
+    c.h += count[kH];
+    c.real += count[kRealX] + count[kRealY];
+    c.general += count[kGeneral];
+}
+
 }  // namespace
+
+GateCounts count_gates(int n, const llg_op* ops, int nops, const std::vector<MatrixOp>& matrices, int* two, double* partners) {
+    GateCounts c;
+    Class2x2 open[64] = {};
+    uint64_t met[64] = {};
+    int count[kClasses] = {};
+    auto close = [&](int q, uint64_t mask) {
+        ++count[open[q]];
+        open[q] = kNone;
+        met[q] |= mask;
+    };
+    *two = 0;
+    for (int i = 0; i < nops; ++i) {
+        const llg_op& o = ops[i];
+        if (o.kind == LLG_OP_CNOT || o.kind == LLG_OP_CZ) {
+            const uint64_t mask = 1ULL << o.q0 | 1ULL << o.q1;
+            close(o.q0, mask);
+            close(o.q1, mask);
+            ++*(o.kind == LLG_OP_CNOT ? &c.moves : &c.flips);
+            ++*two;
+        } else if (o.kind == LLG_OP_MCZ) {
+            for (uint64_t s = o.mask; s; s &= s - 1) close(__builtin_ctzll(s), o.mask);
+            ++c.flips;
+            ++*two;
+        } else if (o.kind == kOpMatrix) {
+            const MatrixOp& m = matrices[o.q0];
+            uint64_t mask = 0;
+            for (int j = 0; j < m.k; ++j) mask |= 1ULL << m.q[j];
+            for (int j = 0; j < m.k; ++j) close(m.q[j], mask);
+            ++(m.k <= 2 ? c.small : c.large);
+        } else {
+            open[o.q0] = kMerge[open[o.q0]][class_of(o)];
+        }
+    }
+    int pairs = 0;
+    for (int q = 0; q < n; ++q) {
+        close(q, 0);
+        pairs += met[q] ? __builtin_popcountll(met[q]) - 1 : 0;
+    }
+    add_classes(count, c);
+    *partners = (double)pairs / n;
+    return c;
+}
 
 class BlockPlanner::Impl {
 public:
@@ -334,20 +414,23 @@ private:
             g.q1 = mo.k;
             g.pad = (int)(out_.matrices.size() / 2);
             out_.matrices.insert(out_.matrices.end(), mo.m.begin(), mo.m.end());
-            ++(mo.k <= 2 ? out_.small_matrices : out_.large_matrices);
+            ++(mo.k <= 2 ? out_.counts.small : out_.counts.large);
         } else if (v.kind == 3) {
             g.q0 = local(__builtin_ctzll(v.mask));
             g.q1 = v.mat;
             g.pad = v.axis;
         } else if (v.kind == 0) {
-            if (v.weight < 1.0f) ++out_.diag_1q;
-            else ++out_.mixing_1q;
+            int count[kClasses] = {};
+            count[class_2x2(mats_[v.mat].m)] = 1;
+            add_classes(count, out_.counts);
             g.q0 = local(__builtin_ctzll(v.mask));
             std::memcpy(g.m, mats_[v.mat].m, sizeof(g.m));
         } else if (v.kind == 1) {
+            ++out_.counts.moves;
             g.q0 = local(__builtin_ctzll(v.mask & ~(1ULL << v.mat)));
             g.q1 = local(v.mat);
         } else {
+            ++out_.counts.flips;
             for (uint64_t s = v.mask; s; s &= s - 1) g.mask |= 1ULL << local(__builtin_ctzll(s));
         }
     }
@@ -439,11 +522,12 @@ bool keeps_norms(const llg_op* ops, int nops) {
     for (int i = 0; i < nops; ++i) {
         if (ops[i].kind != LLG_OP_U2) continue;
         const double* m = ops[i].m;
-        const double largest = spectral_norm_2x2(m);
-        const std::complex<double> det = std::complex<double>(m[0], m[1]) * std::complex<double>(m[6], m[7]) -
-                                         std::complex<double>(m[2], m[3]) * std::complex<double>(m[4], m[5]);
-        if (!(largest > 0.0)) return false;
-        const double off = std::max(largest - 1.0, 1.0 - std::abs(det) / largest);  // of both singular values
+        // M^+ M = [a, c; conj c, b]: its eigenvalues, the singular values' squares, are this close to 1
+        const double a = m[0] * m[0] + m[1] * m[1] + m[4] * m[4] + m[5] * m[5];
+        const double b = m[2] * m[2] + m[3] * m[3] + m[6] * m[6] + m[7] * m[7];
+        const double cr = m[0] * m[2] + m[1] * m[3] + m[4] * m[6] + m[5] * m[7];
+        const double ci = m[0] * m[3] - m[1] * m[2] + m[4] * m[7] - m[5] * m[6];
+        const double off = 0.5 * (std::max(std::fabs(a - 1.0), std::fabs(b - 1.0)) + std::fabs(cr) + std::fabs(ci));
         if (!(off <= kBlockNormLimit - 1.0)) return false;
         drift += off;
     }

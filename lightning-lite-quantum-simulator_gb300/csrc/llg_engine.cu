@@ -17,6 +17,7 @@
 
 #include "../../include/llgpu.h"
 #include "llg_common_host.h"
+#include "llg_cost.h"
 #include "llg_diag.h"
 #include "llg_diag_launch.h"
 #include "llg_internal.h"
@@ -513,74 +514,28 @@ int measure_norm(llg_state* st) {
     return LLG_OK;
 }
 
-// Microseconds that tile passes take for a gate on 6 .. 12 and more qubits, where a CTA's latency and not the arithmetic
-// counts (fits of seven circuits a size): merged gates that mix, H (cheaper in double-float), others.
-struct TileLatency {
-    double mixing, h, other;
-};
-TileLatency tile_latency(int P, int n) {
-    static const TileLatency f64[7] = {{1.15, 1.15, 0.4}, {1.35, 1.35, 0.4}, {1.4, 1.4, 0.4}, {1.6, 1.6, 0.4}, {2.45, 2.45, 0.6},
-                                      {4.0, 4.0, 0.5}, {7.0, 7.0, 0.75}};
-    static const TileLatency df64[7] = {{1.0, 1.0, 0.15}, {1.05, 1.0, 0.15}, {1.25, 1.1, 0.15}, {1.6, 1.2, 0.15}, {2.7, 1.6, 0.5},
-                                       {4.1, 2.0, 0.5}, {7.0, 3.0, 0.5}};
-    const int i = std::min(std::max(n, 6), 12) - 6;
-    return P == LLG_F64 ? f64[i] : df64[i];
+// Whether a flush whose passes the caller has left to the engine is worth the planning of blocks: by its gates' counts
+// alone, since planning that comes to nothing costs 15 to 60 us of, say, 100.  The estimates are within some 10 % on few qubits,
+// so blocks have to be that much faster there; on many, their time depends on where the targets are.  Tile passes / blocks, host included, us: 20 layers of rotations and CNOTs on 6, 8,
+// 10, 12, 16, 20 qubits 169 / 110, 241 / 159, 508 / 210, 1565 / 255, 2763 / 336, 5411 / 656; 500 H and 500 CNOTs there 575 / 488,
+// 547 / 662, 902 / 818, 2449 / 894, 2742 / 991, 5089 / 1783, in double-float 417 / 465, 384 / 614, 507 / 754, 900 / 846,
+// 1108 / 952, 1772 / 1833; 1000 CNOTs in double-float on 12 and 24 qubits 857 / 1550, 18962 / 39025.  Channels cost tile
+// passes 6 us each.
+bool worth_planning(int P, int n, const std::vector<llg_op>& q, const std::vector<MatrixOp>& matrices) {
+    int two = 0;
+    double partners = 0.0;
+    const GateCounts c = count_gates(n, q.data(), (int)q.size(), matrices, &two, &partners);
+    const double tiles = tile_seconds(P, n, c);
+    if (c.small + c.large > 0) return n >= 12 || tiles >= 45e-6;
+    const double blocks = block_seconds(P, n, likely_blocks(n, c, two, partners), 0.0) + kBlockBase + kBlockGate * (double)q.size();
+    return (n < 10 ? 1.1 : n >= 20 ? 1.05 : 1.0) * blocks < tiles + kTileBase;
 }
 
-// Which plan a flush takes when the caller has left the tile width and CTA size to the engine:
-// blocks when their passes cost less than tile passes with the same gates (judged on the blocks
-// planned so far).  Measured on this GPU, per 2^30 amplitudes: a block 8.3 (FP64) or 10.1 ms
-// (double-float), and at least 8.5 us (10 with its planning on fewer than 12 qubits, whose passes end sooner than the
-// host); a CNOT or sign-flip pass 2.6 ms.  Tile passes take 3.2 FP64 multiply-adds per amplitude for a merged one-qubit gate
-// that mixes and 4 for a diagonal one, at 0.56 T a second (double-float: 2.0 ms per 2^30 for either); no less than
-// tile_latency's; and one read and write of the state.  A channel
-// on its own is a sparse pass: 6.2 ms per 2^30 on one qubit of a density matrix, 9 on two, at least 6 us.
-// Tile passes / blocks, host included, us: 20 layers of rotations and CNOTs on 6, 8, 10, 11, 12 qubits 175 / 115, 237 /
-// 163, 498 / 231, 818 / 237, 1624 / 275; 1000 H and CNOT on 8, 10, 11, 12 547 / 899, 890 / 951, 1458 / 825, 2391 / 908.
-// h_share: of the gates that mix.
-bool blocks_pay(int P, int n, const BlockPlan& plan, double h_share) {
-    const bool f64 = P == LLG_F64;
-    const double amps = std::ldexp(1.0, n);
-    const double block = std::max(n < 12 ? 10e-6 : 8.5e-6, amps * (f64 ? 8.0e-12 : 9.6e-12));
-    const double single = 3e-6 + amps * 2.4e-12;
-    const double t_blocks = plan.blocks * block + ((double)plan.steps.size() - plan.blocks) * single + 5e-6;
-    const double arith = f64 ? (3.2 * plan.mixing_1q + 4.0 * plan.diag_1q) / 0.56e12 : 1.9e-12 * (plan.mixing_1q + plan.diag_1q);
-    const double gates = (double)plan.gates.size() - plan.small_matrices - plan.large_matrices;
-    const TileLatency l = tile_latency(P, n);
-    const double latency = 1e-6 * ((l.h * h_share + l.mixing * (1.0 - h_share)) * plan.mixing_1q + l.other * (gates - plan.mixing_1q));
-    const double t_tiles = gates > 0 ? std::max(std::max(arith * amps, latency), amps * 4.8e-12) : 0.0;
-    const double channels = plan.small_matrices * std::max(6e-6, amps * 5.8e-12) + plan.large_matrices * std::max(6e-6, amps * 8.4e-12);
-    return t_blocks < (n < 10 && channels == 0.0 ? 0.85 : 1.0) * (t_tiles + channels);  // the fits are within 15 %
-}
-
-// Whether a queue is worth the planning of blocks, by a count of its gates: planning that comes to nothing costs 10 to 60
-// us.  On fewer than 12 qubits tile passes have to take a while (without channels, which cost them 6 us each), and on
-// fewer than 10, where two-qubit gates cost them next to nothing, few gates may be of those.  H and as many CNOTs fill a block
-// with some ten gates: tile passes are faster in double-float, and on 10 qubits and fewer.
-bool worth_planning(int P, int n, const std::vector<llg_op>& q, double* h_share) {
-    double one = 0.0, two = 0.0, us = 0.0, mixing = 0.0, h = 0.0;
-    bool channels = false;
-    const TileLatency l = tile_latency(P, n);
-    for (const llg_op& o : q) {
-        if (o.kind == LLG_OP_H) {
-            us += l.h;
-            h += 1.0;
-            mixing += 1.0;
-        } else if (o.kind == LLG_OP_RX || o.kind == LLG_OP_RY || o.kind == LLG_OP_U2) {
-            us += l.mixing;
-            mixing += 1.0;
-        } else {
-            channels = channels || o.kind == kOpMatrix;
-            us += o.kind == kOpMatrix ? 6.0 : l.other;
-        }
-        if (o.kind == LLG_OP_CNOT || o.kind == LLG_OP_CZ || o.kind == LLG_OP_MCZ) two += 1.0;
-        else one += 1.0;
-    }
-    *h_share = mixing > 0.0 ? h / mixing : 0.0;
-    if (channels) return n >= 12 || us >= 45.0;
-    if ((P != LLG_F64 || n <= 10) && *h_share > 0.8 && two > 0.7 * one) return false;
-    if (n >= 12) return true;
-    return us >= (n < 9 ? 150.0 : n < 11 ? 100.0 : 80.0) && (n >= 10 || two <= 0.3 * one);
+// Whether blocks cost less than tile passes with the same gates, judged on those planned so far (on few qubits the planning,
+// which is spent by then, counts for them).
+bool blocks_pay(int P, int n, const BlockPlan& plan) {
+    const double singles = (double)plan.steps.size() - plan.blocks;
+    return block_seconds(P, n, plan.blocks, singles) < (n < 12 ? 1.05 : n < 20 ? 1.0 : 0.95) * tile_seconds(P, n, plan.counts);
 }
 
 // growth of the norm bound over a queue (2x2s that are not unitary)
@@ -623,18 +578,14 @@ int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
     if (!gate_block_eligible(st->P, st->n)) return run_tiles(st, q, mirror, mirrored);
     // amplitudes stay below 2^(limit + 10) within a flush
     const double limit = st->P == LLG_F64 ? 900.0 : 90.0;
-    double h_share = 0.0;
-    bool blocks = blocks_allowed(st) && worth_planning(st->P, st->n, q, &h_share) && has_block_plan(st->n, q.data(), (int)q.size()) &&
-                  keeps_norms(q.data(), (int)q.size());
+    bool blocks = blocks_allowed(st) && worth_planning(st->P, st->n, q, st->matrices) && keeps_norms(q.data(), (int)q.size());
     if (blocks && st->log2_norm > limit && st->log2_norm < HUGE_VAL)
         if (int rc = measure_norm(st)) return rc;
     blocks = blocks && st->log2_norm <= limit;
     if (blocks) {
         BlockPlanner planner(st->n, q.data(), (int)q.size(), false, &st->matrices);
-        // a first look on few qubits, where the planning counts
-        const bool hopeless = st->n < 12 && planner.advance(3) && !blocks_pay(st->P, st->n, planner.plan, h_share);
-        if (!hopeless) planner.advance(8);
-        bool room = !hopeless && blocks_pay(st->P, st->n, planner.plan, h_share);
+        planner.advance(st->n < 12 ? 11 : 8);
+        bool room = blocks_pay(st->P, st->n, planner.plan);
         if (room)
             if (int rc = ensure_blocks(st, q.size(), &room)) return rc;
         if (room) {

@@ -215,13 +215,25 @@ struct MatrixOp {
     int q[4];
     std::vector<double> m;  // 2 * 4^k
 };
+// Gates by what they cost in tile passes, runs of one-qubit gates merged
+struct GateCounts {
+    int h = 0;        // H
+    int real = 0;     // rotations by a real or an X-like matrix
+    int general = 0;  // other 2x2s that mix
+    int diag = 0;     // diagonal ones
+    int moves = 0;    // CNOTs and antidiagonal 2x2s
+    int flips = 0;    // sign flips
+    int small = 0, large = 0;  // dense matrices on one or two qubits, on three or four
+};
+// the counts of a list, without multiplying its runs; two: its two-qubit gates, partners: the mean number of other qubits
+// that a qubit has them with
+GateCounts count_gates(int n, const llg_op* ops, int nops, const std::vector<MatrixOp>& matrices, int* two, double* partners);
 struct BlockPlan {
     std::vector<BlockStep> steps;
     std::vector<BlockGate> gates;
     std::vector<double> matrices;  // of the kind-4 gates
     int blocks = 0;
-    int small_matrices = 0, large_matrices = 0;  // on one or two qubits, on three or four
-    int mixing_1q = 0, diag_1q = 0;  // merged one-qubit gates among `gates`, for the cost of other plans
+    GateCounts counts;  // of `gates`, for the cost of other plans
 };
 // 2x2 gates of a block have spectral norm at most this, so that its entries stay well below 2
 constexpr double kBlockNormLimit = 1.0 + 1e-6;

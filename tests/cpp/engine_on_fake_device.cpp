@@ -182,6 +182,23 @@ int second_stream(const char* kind, int from, int count) {
     return 0;
 }
 
+// The launches of one flush of the gate records in a file, from |0..0>.
+int flush(int n, int precision, const char* path) {
+    std::vector<llg_op> q;
+    if (FILE* f = std::fopen(path, "rb")) {
+        llg_op o;
+        while (std::fread(&o, sizeof(o), 1, f) == 1) q.push_back(o);
+        std::fclose(f);
+    }
+    llg_state* st = nullptr;
+    if (llg_create(n, precision, &st) || llg_apply_ops(st, q.data(), (int)q.size())) return fail("create");
+    calls.clear();
+    if (llg_flush(st)) return fail("flush");
+    std::printf("%d %d %d\n", calls["block"], calls["tile"], calls["gate"]);
+    llg_destroy(st);
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -192,6 +209,7 @@ int main(int argc, char** argv) {
     if (what == "record") rc = second_stream("event record", 1, 4);
     if (what == "wait") rc = second_stream("wait event", 1, 2);
     if (what == "block") rc = second_stream("block", 20, 20);
+    if (what == "flush" && argc == 5) return flush(std::atoi(argv[2]), std::atoi(argv[3]), argv[4]);
     if (!rc) std::printf("ok\n");
     return rc;
 }

@@ -1,14 +1,17 @@
 """The engine's host code on a recording stand-in for the device (cpp/engine_on_fake_device.cpp): what it does when a call
-fails in the middle of a flush."""
+fails in the middle of a flush, and which plan a list of gates takes."""
 from __future__ import annotations
 
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 import build_ext
+import llgpu
 from conftest import PKG, REPO
+from llgpu import OP_CNOT, OP_H, OP_RX, OP_RY, OP_RZ, OP_U2, make_ops
 
 
 @pytest.fixture(scope="module")
@@ -34,3 +37,60 @@ def run(exe, *args):
 @pytest.mark.parametrize("call", ["weights", "copy", "record", "wait", "block"])
 def test_a_failing_call_leaves_nothing_in_flight(exe, call):
     run(exe, call)
+
+
+def launches(exe, tmp_path, n, precision, ops):
+    """(blocks, tile passes, single gates) of a flush."""
+    path = str(tmp_path / "ops")
+    np.ascontiguousarray(ops, dtype=llgpu.OP_DTYPE).tofile(path)
+    r = subprocess.run([exe, "flush", str(n), str(llgpu.PRECISIONS[precision]), path], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return tuple(int(x) for x in r.stdout.split())
+
+
+def random_list(n, count, share, gate, seed=3):
+    """`count` gates, `share` of them CNOTs between random qubits, the others gate(rng, qubit)."""
+    rng = np.random.default_rng(seed)
+    recs = []
+    for _ in range(count):
+        if rng.random() < share:
+            a, b = (int(x) for x in rng.choice(n, size=2, replace=False))
+            recs.append((OP_CNOT, a, b))
+        else:
+            recs.append(gate(rng, int(rng.integers(n))))
+    return make_ops(recs)
+
+
+S = np.sqrt(0.5)
+SAME = {
+    "h": [lambda rng, q: (OP_H, q), lambda rng, q: (OP_U2, q, 0, 0.0, None, [[S, S], [S, -S]])],
+    "ry": [lambda rng, q: (OP_RY, q, 0, 0.8), lambda rng, q: (OP_U2, q, 0, 0.0, None, [[np.cos(0.4), -np.sin(0.4)], [np.sin(0.4), np.cos(0.4)]])],
+    "rx": [lambda rng, q: (OP_RX, q, 0, 0.8),
+           lambda rng, q: (OP_U2, q, 0, 0.0, None, [[np.cos(0.4), -1j * np.sin(0.4)], [-1j * np.sin(0.4), np.cos(0.4)]])],
+    "rz": [lambda rng, q: (OP_RZ, q, 0, 0.8), lambda rng, q: (OP_U2, q, 0, 0.0, None, np.diag([np.exp(-0.4j), np.exp(0.4j)]))],
+}
+
+
+@pytest.mark.parametrize("precision", ["complex128", "df64"])
+@pytest.mark.parametrize("n", [6, 8, 9, 10, 11, 12, 14])
+@pytest.mark.parametrize("gate", list(SAME))
+def test_a_gate_by_name_or_by_its_matrix(exe, tmp_path, gate, n, precision):
+    # the plan follows what the gates cost, not what they are called
+    for count, share in ((1000, 0.5), (1000, 0.25), (200, 0.25)):
+        named, matrix = (launches(exe, tmp_path, n, precision, random_list(n, count, share, g)) for g in SAME[gate])
+        assert (named[0] > 0) == (matrix[0] > 0)
+
+
+# where one form takes at most 0.8 of the other's time on the GPU, in both formats alike
+@pytest.mark.parametrize("precision", ["complex128", "df64"])
+@pytest.mark.parametrize("n", [6, 8, 10, 12, 16, 20])
+def test_the_faster_form(exe, tmp_path, n, precision):
+    layers = make_ops([r for layer in range(20) for r in
+                       [(k, q, 0, 0.3 + 0.1 * q + layer) for q in range(n) for k in (OP_RX, OP_RY, OP_RZ)] +
+                       [(OP_CNOT, q, q + 1) for q in range(layer % 2, n - 1, 2)]])
+    assert launches(exe, tmp_path, n, precision, layers)[0] > 0
+    short = make_ops([(OP_RY, q, 0, 0.4) for q in range(n)])
+    if n <= 10:
+        assert launches(exe, tmp_path, n, precision, short)[0] == 0
+        cnots = random_list(n, 1000, 1.0, None)
+        assert launches(exe, tmp_path, n, precision, cnots)[0] == 0
