@@ -1059,9 +1059,24 @@ bool plan_tiles(int n, const llg_op* ops, int nops, int tile_qubits, int P, Plan
                 case LLG_OP_CNOT: {
                     std::vector<ExecOp> tmp;
                     if (!lower_op(n, gop, PP, tmp, err)) return false;
+                    // The carried phases are of modulus 1 but for roundings, which the pushes of CNOTs in turn on two
+                    // qubits raise to Fibonacci powers (300 CNOTs between 8 qubits took 1 + 2^-53 past the format's
+                    // range): a modulus that has drifted is applied.
+                    auto shed = [&](int qb) {
+                        if (std::fabs(std::norm(ph[qb]) - 1.0) <= 0x1p-10) return;
+                        const double r = std::abs(ph[qb]);
+                        ExecOp e = blank(EX_PHASE1);
+                        e.q0 = qb;
+                        e.c[0] = pack_coef(PP, r);
+                        e.c[1] = pack_coef(PP, 0.0);
+                        emit_raw(e, -1);
+                        ph[qb] /= r;
+                    };
+                    shed(gop.q1);
                     const cd p = ph[gop.q1];
                     if (!is_one(p)) {
                         ph[gop.q0] *= p;
+                        shed(gop.q0);
                         const cd cp = 1.0 / (p * p);
                         tmp[0].flags |= OPF_PHASE;
                         tmp[0].c[0] = pack_coef(PP, cp.real());
