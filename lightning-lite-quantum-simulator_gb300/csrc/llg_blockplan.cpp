@@ -142,6 +142,17 @@ public:
         return remaining_ > 0;
     }
 
+    void mark() { marked_ = done_; }
+
+    std::vector<llg_op> rest(const llg_op* ops, int nops) const {
+        std::vector<llg_op> r;
+        for (int i = 0; i < nops; ++i) {
+            const int id = op_node_[i] < 0 ? node_of_mat_[-1 - op_node_[i]] : op_node_[i];
+            if (!marked_[id]) r.push_back(ops[i]);
+        }
+        return r;
+    }
+
 private:
     struct M8 {
         double m[8];
@@ -170,9 +181,16 @@ private:
         std::vector<char> pdiag(n_, 0);
         nodes_.reserve(nops);
         mats_.reserve(nops);
+        node_of_mat_.reserve(nops);
         seg_of_.reserve(2 * nops);
+        op_node_.resize(nops);
+        for (int q = 0; q < n_; ++q) {
+            ids_[q].reserve((size_t)nops / n_ + 8);
+            seg_start_[q].reserve((size_t)nops / n_ + 8);
+        }
         auto flush = [&](int q) {
             if (pend[q] < 0) return;
+            node_of_mat_[pend[q]] = (int)nodes_.size();
             Node v;
             v.mask = 1ULL << q;
             v.mat = pend[q];
@@ -191,6 +209,7 @@ private:
                 v.mat = occ++;
                 v.axis = op.kind == LLG_OP_RX ? 0 : (op.kind == LLG_OP_RY ? 1 : 2);
                 v.weight = v.axis == 2 ? 0.5f : 1.0f;
+                op_node_[i] = (int)nodes_.size();
                 add_node(v, v.axis == 2 ? v.mask : 0);
                 continue;
             }
@@ -201,12 +220,14 @@ private:
                 if (pend[op.q0] < 0) {
                     pend[op.q0] = (int)mats_.size();
                     mats_.push_back(g);
+                    node_of_mat_.push_back(-1);
                     pdiag[op.q0] = d;
                 } else {
                     M8& p = mats_[pend[op.q0]];
                     matmul(g.m, p.m, p.m);
                     pdiag[op.q0] = pdiag[op.q0] && d;
                 }
+                op_node_[i] = -1 - pend[op.q0];
                 continue;
             }
             if (op.kind == kOpMatrix) {
@@ -221,6 +242,7 @@ private:
                 for (int e = 0; e < d * d; ++e)
                     if (e / d != e % d) diag = diag && mo.m[2 * e] == 0.0 && mo.m[2 * e + 1] == 0.0;
                 v.weight = mo.k <= 2 ? 2.0f : 5.0f;
+                op_node_[i] = (int)nodes_.size();
                 add_node(v, diag ? v.mask : 0);
                 continue;
             }
@@ -234,6 +256,7 @@ private:
                 v.mat = op.q1;
                 z = 1ULL << op.q0;
             }
+            op_node_[i] = (int)nodes_.size();
             add_node(v, z);
         }
         for (int q = 0; q < n_; ++q) {
@@ -486,11 +509,12 @@ private:
     std::vector<M8> mats_;
     std::vector<Node> nodes_;
     std::vector<int> seg_of_;
+    std::vector<int> op_node_, node_of_mat_;  // per op: its node, or -1 less the index of its run's matrix
     std::vector<int> ids_[64], seg_start_[64];  // per qubit: its gates in order, where each segment starts
     bool last_z_[64] = {};
     int cur_[64], left_[64];  // per qubit: the current segment, its gates not done yet
     std::vector<int> stamp_, got_;
-    std::vector<char> done_;
+    std::vector<char> done_, marked_;
     Taken tried_, try_;
     int stamp_id_ = 0, remaining_ = 0, wide_ = 0;
     size_t first_ = 0;
@@ -500,6 +524,8 @@ BlockPlanner::BlockPlanner(int n, const llg_op* ops, int nops, bool params, cons
     : impl_(new Impl(n, ops, nops, params, matrices, plan)) {}
 BlockPlanner::~BlockPlanner() = default;
 bool BlockPlanner::advance(int blocks) { return impl_->advance(blocks); }
+void BlockPlanner::mark() { impl_->mark(); }
+std::vector<llg_op> BlockPlanner::rest(const llg_op* ops, int nops) const { return impl_->rest(ops, nops); }
 
 double spectral_norm_2x2(const double* m) {
     double f2 = 0.0;

@@ -381,9 +381,15 @@ int ensure_blocks(llg_state* st, size_t nops, bool* room) {
     return LLG_OK;
 }
 
-int run_block_groups(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
+GateCounts operator-(const GateCounts& a, const GateCounts& b) {
+    return {a.h - b.h, a.real - b.real, a.general - b.general, a.diag - b.diag, a.moves - b.moves, a.flips - b.flips,
+            a.small - b.small, a.large - b.large};
+}
+
+int run_block_groups(llg_state* st, BlockPlanner& planner, const std::vector<llg_op>& q, double* mirror, bool* mirrored,
+                     std::vector<llg_op>* left) {
     constexpr int kGroup = kBlockGroup;
-    const size_t wb = gate_block_weight_bytes(st->P), slots = block_slots(nops);
+    const size_t wb = gate_block_weight_bytes(st->P), slots = block_slots(q.size());
     LLG_CUDA(cudaEventSynchronize(st->ops_done), "cudaEventSynchronize");  // the staging buffer's last copies
     st->block_tc_launched = true;
     const BlockPlan& plan = planner.plan;
@@ -392,7 +398,20 @@ int run_block_groups(llg_state* st, BlockPlanner& planner, size_t nops, double* 
     std::vector<BlockStep> bs;
     bool rest = planner.advance(0);  // gates that are not planned yet
     while (from < plan.steps.size() || rest) {
-        if (from == plan.steps.size()) rest = planner.advance(kGroup);
+        if (from == plan.steps.size()) {
+            // Lists change on their way: where the next blocks would take clearly longer than tile passes, the gates that are
+            // left go there.  (Eight blocks and more: the few at a list's end hold what they hold.)
+            planner.mark();
+            const GateCounts counts = plan.counts;
+            const double blocks = plan.blocks, steps = (double)plan.steps.size();
+            rest = planner.advance(kGroup);
+            const double more = plan.blocks - blocks;
+            if (more >= 8 && block_seconds(st->P, st->n, more, (double)plan.steps.size() - steps - more) >
+                                 1.15 * tile_seconds(st->P, st->n, plan.counts - counts)) {
+                *left = planner.rest(q.data(), (int)q.size());
+                break;
+            }
+        }
         // the steps planned so far, at most kGroup blocks of them
         size_t to = from, gates_to = gates_from;
         bs.clear();
@@ -484,10 +503,11 @@ int run_block_groups(llg_state* st, BlockPlanner& planner, size_t nops, double* 
 }
 
 // A flush as dense 5-qubit blocks on the tensor cores (llg_blockplan.cpp, llg_gateblock.cu), the rest
-// of the plan made while the first blocks run.  nops: the flush's gates, for which ensure_blocks() found room.
-// mirror / mirrored: as for run_tiles.
-int run_blocks(llg_state* st, BlockPlanner& planner, size_t nops, double* mirror, bool* mirrored) {
-    const int rc = run_block_groups(st, planner, nops, mirror, mirrored);
+// of the plan made while the first blocks run.  q: the flush's gates, for which ensure_blocks() found room; left: those that
+// are to run as tile passes after the blocks.  mirror / mirrored: as for run_tiles.
+int run_blocks(llg_state* st, BlockPlanner& planner, const std::vector<llg_op>& q, double* mirror, bool* mirrored,
+               std::vector<llg_op>* left) {
+    const int rc = run_block_groups(st, planner, q, mirror, mirrored, left);
     if (rc) {
         // the streams may have parted: no upload may still read the staging buffer that the next flush fills, and no kernel
         // the weights
@@ -522,13 +542,20 @@ int measure_norm(llg_state* st) {
 // 1108 / 952, 1772 / 1833; 1000 CNOTs in double-float on 12 and 24 qubits 857 / 1550, 18962 / 39025.  Channels cost tile
 // passes 6 us each.
 bool worth_planning(int P, int n, const std::vector<llg_op>& q, const std::vector<MatrixOp>& matrices) {
-    int two = 0;
-    double partners = 0.0;
-    const GateCounts c = count_gates(n, q.data(), (int)q.size(), matrices, &two, &partners);
-    const double tiles = tile_seconds(P, n, c);
-    if (c.small + c.large > 0) return n >= 12 || tiles >= 45e-6;
-    const double blocks = block_seconds(P, n, likely_blocks(n, c, two, partners), 0.0) + kBlockBase + kBlockGate * (double)q.size();
-    return (n < 10 ? 1.1 : n >= 20 ? 1.05 : 1.0) * blocks < tiles + kTileBase;
+    // A list's first gates decide where blocks take less than half of the time there: it is looked at again on the way.
+    constexpr int kFirst = 512;
+    for (int count : {kFirst, (int)q.size()}) {
+        if (count > (int)q.size()) continue;
+        int two = 0;
+        double partners = 0.0;
+        const GateCounts c = count_gates(n, q.data(), count, matrices, &two, &partners);
+        const double tiles = tile_seconds(P, n, c);
+        if (c.small + c.large > 0 && (n >= 12 || tiles >= 45e-6)) return true;
+        const double blocks = block_seconds(P, n, likely_blocks(n, c, two, partners), 0.0) + kBlockBase + kBlockGate * (double)count;
+        if (2.0 * blocks < tiles) return true;
+        if (count == (int)q.size()) return c.small + c.large == 0 && (n < 10 ? 1.1 : n >= 20 ? 1.05 : 1.0) * blocks < tiles + kTileBase;
+    }
+    return false;
 }
 
 // Whether blocks cost less than tile passes with the same gates, judged on those planned so far (on few qubits the planning,
@@ -573,33 +600,14 @@ bool blocks_allowed(const llg_state* st) {
     return gate_block_eligible(st->P, st->n) && st->fuse_mode == LLG_FUSE_TILE && st->tile_qubits == 0 && st->tile_threads == 0;
 }
 
-// the queue as fused passes (blocks, shared-memory tiles or register tiles)
-int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = nullptr, bool* mirrored = nullptr) {
-    if (!gate_block_eligible(st->P, st->n)) return run_tiles(st, q, mirror, mirrored);
-    // amplitudes stay below 2^(limit + 10) within a flush
-    const double limit = st->P == LLG_F64 ? 900.0 : 90.0;
-    bool blocks = blocks_allowed(st) && worth_planning(st->P, st->n, q, st->matrices) && keeps_norms(q.data(), (int)q.size());
-    if (blocks && st->log2_norm > limit && st->log2_norm < HUGE_VAL)
-        if (int rc = measure_norm(st)) return rc;
-    blocks = blocks && st->log2_norm <= limit;
-    if (blocks) {
-        BlockPlanner planner(st->n, q.data(), (int)q.size(), false, &st->matrices);
-        planner.advance(st->n < 12 ? 11 : 8);
-        bool room = blocks_pay(st->P, st->n, planner.plan);
-        if (room)
-            if (int rc = ensure_blocks(st, q.size(), &room)) return rc;
-        if (room) {
-            const int rc = run_blocks(st, planner, q.size(), mirror, mirrored);
-            for (const MatrixOp& m : st->matrices) note_growth(st, m.k, m.m.data());
-            st->matrices.clear();
-            return rc;
-        }
-    }
+// gates as tile passes, channels one by one between them
+int run_unblocked(llg_state* st, const std::vector<llg_op>& q, double* mirror, bool* mirrored) {
     note_growth(st, q);
-    if (st->matrices.empty()) return run_tiles(st, q, mirror, mirrored);
-    // channels one by one, the gates between them in tile passes
     std::vector<MatrixOp> mats;
     mats.swap(st->matrices);
+    bool channels = false;
+    for (const llg_op& o : q) channels = channels || o.kind == kOpMatrix;
+    if (!channels) return run_tiles(st, q, mirror, mirrored);
     std::vector<llg_op> part;
     for (size_t i = 0; i <= q.size(); ++i) {
         if (i < q.size() && q[i].kind != kOpMatrix) {
@@ -614,6 +622,38 @@ int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
             if (int rc = apply_matrix_now(st, m.k, m.q, m.m.data())) return rc;
         }
     }
+    return LLG_OK;
+}
+
+// the queue as fused passes (blocks, shared-memory tiles or register tiles)
+int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = nullptr, bool* mirrored = nullptr) {
+    if (!gate_block_eligible(st->P, st->n)) return run_tiles(st, q, mirror, mirrored);
+    // amplitudes stay below 2^(limit + 10) within a flush
+    const double limit = st->P == LLG_F64 ? 900.0 : 90.0;
+    bool blocks = blocks_allowed(st) && worth_planning(st->P, st->n, q, st->matrices) && keeps_norms(q.data(), (int)q.size());
+    if (blocks && st->log2_norm > limit && st->log2_norm < HUGE_VAL)
+        if (int rc = measure_norm(st)) return rc;
+    blocks = blocks && st->log2_norm <= limit;
+    if (!blocks) return run_unblocked(st, q, mirror, mirrored);
+    BlockPlanner planner(st->n, q.data(), (int)q.size(), false, &st->matrices);
+    planner.advance(st->n < 12 ? 11 : 8);
+    bool room = blocks_pay(st->P, st->n, planner.plan);
+    if (room)
+        if (int rc = ensure_blocks(st, q.size(), &room)) return rc;
+    if (!room) return run_unblocked(st, q, mirror, mirrored);
+    std::vector<llg_op> left;
+    if (int rc = run_blocks(st, planner, q, mirror, mirrored, &left)) {
+        st->matrices.clear();
+        return rc;
+    }
+    // the channels that are done (each that is left notes its own)
+    std::vector<char> later(st->matrices.size(), 0);
+    for (const llg_op& o : left)
+        if (o.kind == kOpMatrix) later[o.q0] = 1;
+    for (size_t i = 0; i < st->matrices.size(); ++i)
+        if (!later[i]) note_growth(st, st->matrices[i].k, st->matrices[i].m.data());
+    if (!left.empty()) return run_unblocked(st, left, mirror, mirrored);
+    st->matrices.clear();
     return LLG_OK;
 }
 

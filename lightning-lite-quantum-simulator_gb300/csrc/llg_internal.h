@@ -255,6 +255,9 @@ public:
     BlockPlanner(int n, const llg_op* ops, int nops, bool params = false, const std::vector<MatrixOp>* matrices = nullptr);
     ~BlockPlanner();
     bool advance(int blocks);  // appends up to `blocks` blocks to `plan`; false: the list is done
+    void mark();               // takes note of the gates in the plan so far
+    // the other gates of the list (the constructor's), in their order; what the plan holds may run before them
+    std::vector<llg_op> rest(const llg_op* ops, int nops) const;
     BlockPlan plan;
 
 private:

@@ -94,3 +94,24 @@ def test_the_faster_form(exe, tmp_path, n, precision):
         assert launches(exe, tmp_path, n, precision, short)[0] == 0
         cnots = random_list(n, 1000, 1.0, None)
         assert launches(exe, tmp_path, n, precision, cnots)[0] == 0
+
+
+def changing(n, layers, cnots, seed=1):
+    """Layers of rotations and CNOTs, then CNOTs between random qubits alone."""
+    rng = np.random.default_rng(seed)
+    recs = []
+    for layer in range(layers):
+        for q in range(n):
+            recs += [(k, q, 0, float(rng.uniform(0.2, 3))) for k in (OP_RX, OP_RY, OP_RZ)]
+        recs += [(OP_CNOT, q, q + 1) for q in range(layer % 2, n - 1, 2)]
+    return make_ops(recs + [(OP_CNOT, *(int(x) for x in rng.choice(n, size=2, replace=False))) for _ in range(cnots)])
+
+
+@pytest.mark.parametrize("n,precision", [(10, "complex128"), (14, "df64"), (24, "df64")])
+def test_a_list_that_changes_on_its_way(exe, tmp_path, n, precision):
+    # the rotations as blocks, the CNOTs (5 to a block) as tile passes
+    layers, cnots = (120, 400) if n < 24 else (30, 300)
+    alone = launches(exe, tmp_path, n, precision, changing(n, layers, 0))
+    assert alone[0] > 16 and alone[1] == 0
+    both = launches(exe, tmp_path, n, precision, changing(n, layers, cnots))
+    assert alone[0] - 16 <= both[0] <= alone[0] + 16 and both[1] > 0
