@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -366,6 +367,15 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
             o.param = -1;
             if (o.kind == LLG_OP_MCZ && __builtin_popcountll(o.mask) > 5) fits = false;
         }
+        std::unique_ptr<BlockPlanner> planner;
+        if (fits) {
+            planner.reset(new BlockPlanner(n, mine.data(), nops, true));
+            while (planner->advance(64)) {
+            }
+            // a state's flush keeps off blocks for the same gates (llg_internal.h)
+            const GateCounts& g = planner->plan.counts;
+            fits = !planner->plan.fades && g.h + g.real + g.general > 0;
+        }
         if (!fits) {
             // about three multiply-adds a gate
             small_arith += 2.0 * nops * amps / kTileFmaRate;
@@ -373,10 +383,7 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
             ++alone;
             continue;
         }
-        BlockPlanner planner(n, mine.data(), nops, true);
-        while (planner.advance(64)) {
-        }
-        const BlockPlan& p = planner.plan;
+        const BlockPlan& p = planner->plan;
         if (out.steps.size() + p.steps.size() > cap) {
             small_arith += tile_arith(p.counts) * amps;
             continue;

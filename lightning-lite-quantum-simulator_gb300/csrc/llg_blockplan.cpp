@@ -48,8 +48,8 @@ void matmul(const double* a, const double* b, double* out) {
 enum Class2x2 : uint8_t { kNone, kDiag, kMove, kH, kRealX, kRealY, kGeneral, kClasses };
 constexpr Class2x2 kMerge[kClasses][kClasses] = {
     {kNone, kDiag, kMove, kH, kRealX, kRealY, kGeneral},
-    {kDiag, kDiag, kGeneral, kGeneral, kGeneral, kGeneral, kGeneral},
-    {kMove, kGeneral, kNone, kGeneral, kGeneral, kGeneral, kGeneral},
+    {kDiag, kDiag, kMove, kGeneral, kGeneral, kGeneral, kGeneral},
+    {kMove, kMove, kDiag, kGeneral, kGeneral, kGeneral, kGeneral},
     {kH, kGeneral, kGeneral, kNone, kGeneral, kGeneral, kGeneral},
     {kRealX, kGeneral, kGeneral, kGeneral, kRealX, kGeneral, kGeneral},
     {kRealY, kGeneral, kGeneral, kGeneral, kGeneral, kRealY, kGeneral},
@@ -72,6 +72,15 @@ Class2x2 class_of(const llg_op& o) {
         case LLG_OP_RZ: return kDiag;
         default: return class_2x2(o.m);
     }
+}
+// log2 of a 2x2's smallest entry where that is far below 1 (but no rounding of 0), else 0
+float small_entry(const double* m) {
+    double least = 1.0;
+    for (int k = 0; k < 4; ++k) {
+        const double n2 = m[2 * k] * m[2 * k] + m[2 * k + 1] * m[2 * k + 1];
+        if (n2 > 0x1p-100) least = std::min(least, n2);
+    }
+    return least < 0x1p-14 ? 0.5f * (float)std::log2(least) : 0.0f;
 }
 void add_classes(const int* count, GateCounts& c) {
     c.diag += count[kDiag];
@@ -446,6 +455,7 @@ private:
             int count[kClasses] = {};
             count[class_2x2(mats_[v.mat].m)] = 1;
             add_classes(count, out_.counts);
+            small_ += small_entry(mats_[v.mat].m);
             g.q0 = local(__builtin_ctzll(v.mask));
             std::memcpy(g.m, mats_[v.mat].m, sizeof(g.m));
         } else if (v.kind == 1) {
@@ -496,9 +506,11 @@ private:
         }
         st.gate_begin = (int)out_.gates.size();
         st.ngates = (int)got_.size();
+        small_ = 0.0f;
         for (int id : got_) gate(nodes_[id], to_local);
         out_.steps.push_back(st);
         ++out_.blocks;
+        out_.fades = out_.fades || small_ < -44.0f;
     }
 
     static constexpr int kSeeds = 4;
@@ -516,6 +528,7 @@ private:
     std::vector<int> stamp_, got_;
     std::vector<char> done_, marked_;
     Taken tried_, try_;
+    float small_ = 0.0f;  // of the block's gates
     int stamp_id_ = 0, remaining_ = 0, wide_ = 0;
     size_t first_ = 0;
 };

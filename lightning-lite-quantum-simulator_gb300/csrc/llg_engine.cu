@@ -406,8 +406,8 @@ int run_block_groups(llg_state* st, BlockPlanner& planner, const std::vector<llg
             const double blocks = plan.blocks, steps = (double)plan.steps.size();
             rest = planner.advance(kGroup);
             const double more = plan.blocks - blocks;
-            if (more >= 8 && block_seconds(st->P, st->n, more, (double)plan.steps.size() - steps - more) >
-                                 1.15 * tile_seconds(st->P, st->n, plan.counts - counts)) {
+            if (plan.fades || (more >= 8 && block_seconds(st->P, st->n, more, (double)plan.steps.size() - steps - more) >
+                                                1.15 * tile_seconds(st->P, st->n, plan.counts - counts))) {
                 *left = planner.rest(q.data(), (int)q.size());
                 break;
             }
@@ -540,7 +540,8 @@ int measure_norm(llg_state* st) {
 // 10, 12, 16, 20 qubits 169 / 110, 241 / 159, 508 / 210, 1565 / 255, 2763 / 336, 5411 / 656; 500 H and 500 CNOTs there 575 / 488,
 // 547 / 662, 902 / 818, 2449 / 894, 2742 / 991, 5089 / 1783, in double-float 417 / 465, 384 / 614, 507 / 754, 900 / 846,
 // 1108 / 952, 1772 / 1833; 1000 CNOTs in double-float on 12 and 24 qubits 857 / 1550, 18962 / 39025.  Channels cost tile
-// passes 6 us each.
+// passes 6 us each.  Gates that only move amplitudes, change signs or turn phases never take blocks: these would round each
+// amplitude against the largest of its group.
 bool worth_planning(int P, int n, const std::vector<llg_op>& q, const std::vector<MatrixOp>& matrices) {
     // A list's first gates decide where blocks take less than half of the time there: it is looked at again on the way.
     constexpr int kFirst = 512;
@@ -550,6 +551,7 @@ bool worth_planning(int P, int n, const std::vector<llg_op>& q, const std::vecto
         double partners = 0.0;
         const GateCounts c = count_gates(n, q.data(), count, matrices, &two, &partners);
         const double tiles = tile_seconds(P, n, c);
+        if (c.h + c.real + c.general + c.small + c.large == 0) continue;  // see below
         if (c.small + c.large > 0 && (n >= 12 || tiles >= 45e-6)) return true;
         const double blocks = block_seconds(P, n, likely_blocks(n, c, two, partners), 0.0) + kBlockBase + kBlockGate * (double)count;
         if (2.0 * blocks < tiles) return true;
@@ -561,6 +563,7 @@ bool worth_planning(int P, int n, const std::vector<llg_op>& q, const std::vecto
 // Whether blocks cost less than tile passes with the same gates, judged on those planned so far (on few qubits the planning,
 // which is spent by then, counts for them).
 bool blocks_pay(int P, int n, const BlockPlan& plan) {
+    if (plan.fades) return false;
     const double singles = (double)plan.steps.size() - plan.blocks;
     return block_seconds(P, n, plan.blocks, singles) < (n < 12 ? 1.05 : n < 20 ? 1.0 : 0.95) * tile_seconds(P, n, plan.counts);
 }

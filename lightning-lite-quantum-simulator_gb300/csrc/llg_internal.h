@@ -234,6 +234,10 @@ struct BlockPlan {
     std::vector<double> matrices;  // of the kind-4 gates
     int blocks = 0;
     GateCounts counts;  // of `gates`, for the cost of other plans
+    // A block holds its amplitudes in units of 2^-55 of the group's largest.  Rotations by small angles (or near pi) together make
+    // amplitudes that this leaves nothing of: true once the smallest entries (below 2^-7) of a block's 2x2s multiply to less
+    // than 2^-44.  Such gates are for the tile passes, where every amplitude has its own exponent.
+    bool fades = false;
 };
 // 2x2 gates of a block have spectral norm at most this, so that its entries stay well below 2
 constexpr double kBlockNormLimit = 1.0 + 1e-6;
