@@ -722,14 +722,16 @@ void ensure_blocks(llg_adjoint* h) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // sets at a time: 512 MB each for the weights and the CTAs' sums
-    constexpr size_t kCap = (size_t)512 << 20;
+    // sets at a time: 512 MB each for the weights and the CTAs' sums, but together no more than a quarter of what is free
+    size_t free_bytes = 0, all_bytes = 0;
+    if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess) cudaGetLastError();
+    const size_t cap = std::min((size_t)512 << 20, free_bytes / 8);
     const size_t steps = h->bsteps.size(), wb = gate_block_weight_bytes(LLG_F64);
-    int sets = (int)std::min<size_t>(h->max_batch, kCap / (2 * steps * wb));
+    int sets = (int)std::min<size_t>(h->max_batch, cap / (2 * steps * wb));
     size_t part = 0;
     for (int k = 1; k <= sets; ++k) {
         const size_t need = (size_t)k * cross_ctas(h->n, k, sms) * 1024 * sizeof(double2);
-        if (need > kCap) {
+        if (need > cap) {
             sets = k - 1;
             break;
         }

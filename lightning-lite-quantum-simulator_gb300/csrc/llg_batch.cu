@@ -342,7 +342,8 @@ struct BlockSet {
 // gates 1048 / 335 us; 512 of 10 to 22, 152.9 / 43.6 ms; 5 of 12 and 13 qubits and 100 gates 318 / 103 us; 16 of
 // 12 to 16 and 40 gates 312 / 73 us; 200 of 12 qubits and 200 gates, each its own CTA either way, keep 950 us of
 // tile passes.
-bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_t* off, int sms, BlockSet& out) {
+// room: bytes of device memory for the weights.
+bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_t* off, int sms, size_t room, BlockSet& out) {
     struct Circuit {
         int c, n;
         uint64_t offset;
@@ -352,10 +353,9 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
     std::vector<Circuit> list;
     out.in.assign(count, 0);
     double arith = 0.0, longest = 0.0, small_arith = 0.0, small_longest = 0.0;
-    uint64_t at = 0, total = 0;
+    uint64_t at = 0;
     int alone = 0;  // circuits of one tile that keep the queue
-    for (int c = 0; c < count; ++c) total += 1ULL << n_qubits[c];
-    const size_t cap = std::max<size_t>(kWeightsCap, total * 16) / gate_block_weight_bytes(LLG_F64);
+    const size_t cap = room / gate_block_weight_bytes(LLG_F64);
     for (int c = 0; c < count; ++c) {
         const int n = n_qubits[c], nops = (int)(off[c + 1] - off[c]);
         const uint64_t offset = at;
@@ -491,7 +491,13 @@ static int batch_build(int count, const int* n_qubits, const llg_op* ops, const 
         int dev = 0, sms = 1;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (plan_blocks(count, n_qubits, ops, op_offsets, sms, set)) {
+        // the weights: as much as the states, or 256 MB, but no more than a quarter of what those leave free
+        size_t states = 0, free_bytes = 0, all_bytes = 0;
+        for (int c = 0; c < count; ++c) states += (size_t)16 << n_qubits[c];
+        if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess) cudaGetLastError();
+        const size_t rest = free_bytes > states ? free_bytes - states : 0;
+        const size_t room = std::min(std::max(kWeightsCap, states), rest / 4);
+        if (plan_blocks(count, n_qubits, ops, op_offsets, sms, room, set)) {
             b->block_rounds = set.rounds;
             b->block_tiles = set.tiles;
             b->block_steps = (int)set.steps.size();
