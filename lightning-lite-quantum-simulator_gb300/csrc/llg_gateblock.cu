@@ -221,8 +221,9 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_s;
     // registers of fewer than 12 qubits fill a part of their one tile: the other groups are zeros that nobody stores
-    const int groups = n >= 12 ? kGroups : 1 << (n - 5);
-    const uint64_t ntiles = n >= 12 ? (1ULL << (n - 5)) / kGroups : 1;
+    constexpr bool kPart = kSplit || kMixed;  // the forms that such registers take
+    const int groups = !kPart || n >= 12 ? kGroups : 1 << (n - 5);
+    const uint64_t ntiles = !kPart || n >= 12 ? (1ULL << (n - 5)) / kGroups : 1;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
         if (tile < ntiles) {
             const auto* pb = psi + (insert0_mask(tile * kGroups + (uint64_t)g, tmask) | (h ? off(1) : 0));
 #pragma unroll
-            for (int k = 0; k < 16; ++k) a[k] = g < groups ? __ldcg(pb + off(2 * k)) : typename Elem<P>::S{};
+            for (int k = 0; k < 16; ++k) a[k] = !kPart || g < groups ? __ldcg(pb + off(2 * k)) : typename Elem<P>::S{};
         }
         int slot = 0, egb = 0;
         uint32_t phase = 1;  // of the slot's previous release: the first round needs no wait
@@ -395,7 +396,6 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                 for (int p = 0; p < 2; ++p) {
                     const int col = T::kStep * (2 * e + p);  // within each diagonal's 32 columns
                     uint32_t v[S][T::kStep];
-                    __syncwarp();  // the loads are of the whole warp: lanes part in the scaling and where a tile is partly filled
 #pragma unroll
                     for (int d = 0; d < S; ++d) {
                         const uint32_t taddr = tlane + (uint32_t)(half * T::kSetStride + 32 * d + col);
@@ -443,10 +443,10 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                             if (all_fast) {
                                 const int hi = __double2hiint(r);
                                 r = __hiloint2double(hi ? hi + (et << 20) : hi, __double2loint(r));
-                            } else if (eg == 2047) {
-                                r = __longlong_as_double(0x7FF8000000000000LL);  // an Inf or a NaN in the group
                             } else {
-                                r = scale_slow(r, et);
+                                if (eg == 2047) r = __longlong_as_double(0x7FF8000000000000LL);  // an Inf or a NaN in the group
+                                else r = scale_slow(r, et);
+                                __syncwarp();  // the lanes parted
                             }
                             if (batch.max_exp) largest = max(largest, (uint32_t)__double2hiint(r) & 0x7FFFFFFFu);
                             if (c & 1) out[c >> 1].y = r;
@@ -475,28 +475,32 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
                         }
                     }
                     meet();
-                    if (row < groups && pair32) {
+                    if (!kPart || row < groups) {
+                        if (pair32) {
 #pragma unroll
-                        for (int c = 0; c < T::kStep / 2; c += 2) {
-                            uint64_t w[4];
-                            memcpy(w, &out[c], 32);
-                            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(psi + pos + off(c)), "l"(w[0]), "l"(w[1]),
-                                         "l"(w[2]), "l"(w[3])
-                                         : "memory");
+                            for (int c = 0; c < T::kStep / 2; c += 2) {
+                                uint64_t w[4];
+                                memcpy(w, &out[c], 32);
+                                asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(psi + pos + off(c)), "l"(w[0]),
+                                             "l"(w[1]), "l"(w[2]), "l"(w[3])
+                                             : "memory");
+                            }
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < T::kStep / 2; ++c) psi[pos + off(c)] = out[c];
                         }
-                    } else if (row < groups) {
+                        if (mirror) {
 #pragma unroll
-                        for (int c = 0; c < T::kStep / 2; ++c) psi[pos + off(c)] = out[c];
-                    }
-                    if (mirror && row < groups) {
-#pragma unroll
-                        for (int c = 0; c < T::kStep / 2; ++c) {
-                            if constexpr (P == LLG_F64) mirror[pos + off(c)] = out[c];
-                            else
-                                mirror[pos + off(c)] = make_double2((double)out[c].x + (double)out[c].z,
-                                                                           (double)out[c].y + (double)out[c].w);
+                            for (int c = 0; c < T::kStep / 2; ++c) {
+                                if constexpr (P == LLG_F64) mirror[pos + off(c)] = out[c];
+                                else
+                                    mirror[pos + off(c)] = make_double2((double)out[c].x + (double)out[c].z,
+                                                                        (double)out[c].y + (double)out[c].w);
+                            }
                         }
                     }
+                    // the next tensor-memory loads are of the whole warp
+                    if (kPart && groups < kGroups) __syncwarp();
                 }
             }
         }
@@ -781,6 +785,7 @@ template <int P, bool kRows, bool kMixed = false, bool kSplit = false>
 cudaError_t launch(void* psi, int n, const BlockDesc& bd, const void* w, bool ready, int* err, cudaStream_t s, double* mirror,
                    int ctas, void* second, int sets, uint32_t* max_exp, const MixedCta* mixed = nullptr) {
     using T = Shape<P>;
+    if (!kSplit && !kMixed && n < 12) return cudaErrorInvalidValue;  // whole tiles only
     static const cudaError_t attr =
         cudaFuncSetAttribute(k_gate_block<P, kRows, kMixed, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmem);
     if (attr != cudaSuccess) return attr;
