@@ -182,14 +182,40 @@ int second_stream(const char* kind, int from, int count) {
     return 0;
 }
 
-// The launches of one flush of the gate records in a file, from |0..0>.
-int flush(int n, int precision, const char* path) {
+std::vector<llg_op> read_ops(const char* path) {
     std::vector<llg_op> q;
     if (FILE* f = std::fopen(path, "rb")) {
         llg_op o;
         while (std::fread(&o, sizeof(o), 1, f) == 1) q.push_back(o);
         std::fclose(f);
     }
+    return q;
+}
+
+// The block plan of the gate records in a file, up to `blocks` blocks, and the gates that are left then: counts, steps, gates,
+// records to another file.
+int plan(int n, int blocks, const char* path, const char* out) {
+    const std::vector<llg_op> q = read_ops(path);
+    llg::BlockPlanner p(n, q.data(), (int)q.size());
+    p.advance(blocks);
+    p.mark();
+    const size_t steps = p.plan.steps.size(), gates = p.plan.gates.size();
+    p.advance(3);  // not marked: its gates are left
+    const std::vector<llg_op> left = p.rest(q.data(), (int)q.size());
+    const long long counts[3] = {(long long)steps, (long long)gates, (long long)left.size()};
+    FILE* f = std::fopen(out, "wb");
+    if (!f) return fail("open");
+    std::fwrite(counts, sizeof(counts), 1, f);
+    std::fwrite(p.plan.steps.data(), sizeof(llg::BlockStep), steps, f);
+    std::fwrite(p.plan.gates.data(), sizeof(llg::BlockGate), gates, f);
+    std::fwrite(left.data(), sizeof(llg_op), left.size(), f);
+    std::fclose(f);
+    return 0;
+}
+
+// The launches of one flush of the gate records in a file, from |0..0>.
+int flush(int n, int precision, const char* path) {
+    const std::vector<llg_op> q = read_ops(path);
     llg_state* st = nullptr;
     if (llg_create(n, precision, &st) || llg_apply_ops(st, q.data(), (int)q.size())) return fail("create");
     calls.clear();
@@ -209,6 +235,7 @@ int main(int argc, char** argv) {
     if (what == "record") rc = second_stream("event record", 1, 4);
     if (what == "wait") rc = second_stream("wait event", 1, 2);
     if (what == "block") rc = second_stream("block", 20, 20);
+    if (what == "plan" && argc == 6) rc = plan(std::atoi(argv[2]), std::atoi(argv[3]), argv[4], argv[5]);
     if (what == "flush" && argc == 5) return flush(std::atoi(argv[2]), std::atoi(argv[3]), argv[4]);
     if (!rc) std::printf("ok\n");
     return rc;

@@ -10,6 +10,8 @@ import pytest
 
 import build_ext
 import llgpu
+import oracle
+import test_blockplan_cpu
 from conftest import PKG, REPO
 from llgpu import OP_CNOT, OP_H, OP_RX, OP_RY, OP_RZ, OP_U2, make_ops
 
@@ -115,3 +117,28 @@ def test_a_list_that_changes_on_its_way(exe, tmp_path, n, precision):
     assert alone[0] > 16 and alone[1] == 0
     both = launches(exe, tmp_path, n, precision, changing(n, layers, cnots))
     assert alone[0] - 16 <= both[0] <= alone[0] + 16 and both[1] > 0
+
+
+@pytest.mark.parametrize("blocks", [0, 1, 7, 10000])
+@pytest.mark.parametrize("n", [6, 7, 9, 11, 13])
+def test_a_plan_and_what_is_left_of_the_list(exe, tmp_path, n, blocks):
+    # registers of few qubits, whose blocks hold most of them; the plan's gates first, then the others in their order
+    for seed in range(4):
+        ops = test_blockplan_cpu._random_ops(max(n, 9), 300, 100 * n + seed)
+        ops = ops[(ops["q0"] < n) & (ops["q1"] < n) & (ops["mask"] >> np.uint64(n) == 0)][:150]
+        np.ascontiguousarray(ops, dtype=llgpu.OP_DTYPE).tofile(tmp_path / "ops")
+        run(exe, "plan", str(n), str(blocks), str(tmp_path / "ops"), str(tmp_path / "out"))
+        raw = (tmp_path / "out").read_bytes()
+        nsteps, ngates, nleft = np.frombuffer(raw, np.int64, 3)
+        steps = np.frombuffer(raw, llgpu.BLOCK_STEP_DTYPE, nsteps, 24)
+        at = 24 + steps.nbytes
+        gates = np.frombuffer(raw, llgpu.BLOCK_GATE_DTYPE, ngates, at)
+        left = np.frombuffer(raw, llgpu.OP_DTYPE, nleft, at + gates.nbytes)
+        assert steps["is_block"].sum() <= blocks and (blocks < 10000 or nleft == 0)
+        psi = np.zeros(1 << n, dtype=complex)
+        psi[0] = 1.0
+        for s in steps:
+            qubits = list(s["q"]) if s["is_block"] else list(range(n))
+            for g in gates[s["gate_begin"]:s["gate_begin"] + s["ngates"]]:
+                psi = test_blockplan_cpu._apply(psi, n, g, qubits)
+        assert np.max(np.abs(oracle.run_ops(n, left, psi) - oracle.run_ops(n, ops))) <= 1e-12
