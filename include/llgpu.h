@@ -532,8 +532,9 @@ int llg_diag_export(int n, int nterms, const int* a, const int* b, const double*
 int llg_plan_export_tables(int n, const llg_op* ops, int nops, int tile_qubits, int flags, double* tables,
                            int64_t max_doubles, int64_t* ndoubles);
 
-/* The plan of dense 5-qubit blocks that a flush of a complex128 or double-float state of 12 and more
- * qubits may take: steps in order, each either a block (gates on bits 0..4 of its index, bit b is
+/* The plan of dense 5-qubit blocks that a flush of a complex128 or double-float state may take (the engine plans
+ * registers of 6 and more qubits, this export those of 12 and more; a flush takes blocks only where all 2x2 gates are
+ * unitary and blocks are estimated to be faster): steps in order, each either a block (gates on bits 0..4 of its index, bit b is
  * qubit q[b], q increasing) or one CNOT / sign flip on global qubits.  Writes at most max_steps /
  * max_gates records and the true counts.  LLG_EINVAL when the list has no block plan. */
 typedef struct {

@@ -1218,7 +1218,7 @@ static int finish(llg_state* st, bool here = false) {
     if (!tc && !tiles) return LLG_OK;
     const bool late_products = tc && h[1], late_load = tiles && h[0];
     if (h[0] || h[1]) LLG_CUDA(cudaMemsetAsync(st->d_flags, 0, sizeof(st->h_out->flags), st->stream), "cudaMemsetAsync(flags)");
-    if (late_products) return set_error(LLG_ECUDA, "apply_matrix: a tensor-core block kernel timed out waiting for its products");
+    if (late_products) return set_error(LLG_ECUDA, "a tensor-core block kernel (gate block or apply_matrix) timed out waiting for its products");
     if (late_load) return set_error(LLG_ECUDA, "tile pass: a bulk tile load timed out");
     return LLG_OK;
 }

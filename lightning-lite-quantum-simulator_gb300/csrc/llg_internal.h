@@ -188,7 +188,7 @@ enum RegCode : int32_t {
 };
 int32_t reg_dispatch_code(const ExecOp& x);
 
-// A plan of dense 5-qubit blocks (llg_blockplan.cpp) for 16-byte states of 12 and more qubits.
+// A plan of dense 5-qubit blocks (llg_blockplan.cpp) for 16-byte states of kBlockMinQubits and more qubits.
 struct BlockGate {
     // 0: 2x2 matrix m on q0; 1: CNOT, control q0, target q1; 2: sign flip where all of `mask` is set;
     // 3 (with parameters only): rotation exp(-i theta P / 2) on q0, P = X, Y, Z for pad = 0, 1, 2, theta
