@@ -65,7 +65,10 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 static constexpr int kMaxQubits = 34;
 static constexpr size_t kQueueFlushAt = 1 << 16;
+static constexpr size_t kPinnedStage = (size_t)128 << 10;
 static constexpr uint64_t kStageAmps = 1ULL << 24;  // 256 MiB of complex128 per transfer chunk
+
+static constexpr size_t kReadoutBytes = (sizeof(llg::Readout) + 255) / 256 * 256;
 
 struct llg_state {
     int n = 0;
@@ -97,10 +100,10 @@ struct llg_state {
     bool block_tc_launched = false;
     // block plans: gates and steps (device, pinned staging) and the blocks' weights
     unsigned char* d_bplan = nullptr;
-    unsigned char* h_bplan = nullptr;
-    size_t d_bplan_cap = 0;  // of both
-    void* d_bweights = nullptr;
-    size_t d_bweights_cap = 0;
+    unsigned char* h_bplan = nullptr;   // in h_out's buffer while they are short
+    size_t d_bplan_cap = 0;             // of both
+    unsigned char* bweights = nullptr;  // of bparts groups
+    int bparts = 0;
     cudaStream_t side = nullptr;  // a group's upload and weights, under the blocks of the group before
     cudaEvent_t weights_done = nullptr, slots_free = nullptr;
     // log2 of a bound on the state's 2-norm (infinite: not known to be finite); block plans hold
@@ -114,7 +117,7 @@ struct llg_state {
     double* d_partials = nullptr;
     double* d_red = nullptr;
     unsigned* d_ticket = nullptr;
-    Readout* h_out = nullptr;  // pinned
+    Readout* h_out = nullptr;  // pinned; kPinnedStage bytes for short uploads follow it
     // the last general diagonal observable (llg_diag.h), its device copy, and a full diagonal
     DiagObsHost obs;
     void* d_obs = nullptr;
@@ -195,7 +198,7 @@ int ensure_device_buffers(llg_state* st) {
     if (!st->d_partials) {
         constexpr size_t kPart = sizeof(double) * kRedBlocks * kPartialSlots, kRed = sizeof(double) * kRedSlots;
         constexpr size_t kWords = 4 * sizeof(int);
-        if (!st->h_out) LLG_CUDA(cudaHostAlloc((void**)&st->h_out, sizeof(Readout), cudaHostAllocDefault), "cudaHostAlloc(readout)");
+        if (!st->h_out) LLG_CUDA(cudaHostAlloc((void**)&st->h_out, kReadoutBytes + kPinnedStage, cudaHostAllocDefault), "cudaHostAlloc(readout)");
         LLG_CUDA(cudaMalloc(&st->d_partials, kPart + kWords + kRed), "cudaMalloc(partials)");
         st->d_flags = reinterpret_cast<int*>(st->d_partials + kRedBlocks * kPartialSlots);
         st->d_ticket = reinterpret_cast<unsigned*>(st->d_flags + 2);
@@ -332,51 +335,57 @@ int run_tiles(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
 }
 
 constexpr int kBlockGroup = 16;   // blocks planned, uploaded and launched at a time
-constexpr int kBlockSlots = 128;  // blocks whose weights are held at once
-static_assert(kBlockSlots % kBlockGroup == 0, "a group's weights are contiguous");
+constexpr int kBlockParts = 8;    // groups whose weights are held at once
 
-size_t block_slots(size_t nops) {
-    return nops <= kBlockSlots ? (std::max<size_t>(nops, 1) + kBlockGroup - 1) / kBlockGroup * kBlockGroup : kBlockSlots;
+void free_staging(llg_state* st) {
+    if (st->d_bplan) cudaFree(st->d_bplan);
+    if (st->h_bplan && st->d_bplan_cap > kPinnedStage) cudaFreeHost(st->h_bplan);
+    st->d_bplan = st->h_bplan = nullptr;
+    st->d_bplan_cap = 0;
 }
 
-// Buffers for a flush of nops gates in blocks; *room: false where there is no memory for them (the flush then
+// Buffers for a flush of nops gates in blocks, of one group or more; *room: false where there is no memory for them (the flush then
 // takes tile passes, which need less).
-int ensure_blocks(llg_state* st, size_t nops, bool* room) {
+int ensure_blocks(llg_state* st, size_t nops, bool more, bool* room) {
     size_t mbytes = 0;
     for (const MatrixOp& m : st->matrices) mbytes += m.m.size() * sizeof(double);
-    const size_t weights = block_slots(nops) * gate_block_weight_bytes(st->P);
     // a group's upload: its blocks' steps, its gates, their matrices; every group has its own part of the buffers
     const size_t bytes = (nops / kBlockGroup + 2) * (kBlockGroup * sizeof(BlockStep) + 1024) + nops * sizeof(BlockGate) + mbytes;
-    *room = true;
     if (!st->side) {
         LLG_CUDA(cudaStreamCreateWithFlags(&st->side, cudaStreamNonBlocking), "cudaStreamCreate");
         LLG_CUDA(cudaEventCreateWithFlags(&st->weights_done, cudaEventDisableTiming), "cudaEventCreate");
         LLG_CUDA(cudaEventCreateWithFlags(&st->slots_free, cudaEventDisableTiming), "cudaEventCreate");
     }
-    if (bytes > st->d_bplan_cap || weights > st->d_bweights_cap)
-        LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
+    *room = true;
     if (bytes > st->d_bplan_cap) {
-        if (st->d_bplan) cudaFree(st->d_bplan);
-        if (st->h_bplan) cudaFreeHost(st->h_bplan);
-        st->d_bplan = st->h_bplan = nullptr;
-        st->d_bplan_cap = 0;
-        *room = cudaMalloc(&st->d_bplan, bytes) == cudaSuccess &&
-                cudaHostAlloc((void**)&st->h_bplan, bytes, cudaHostAllocDefault) == cudaSuccess;
-        if (*room) st->d_bplan_cap = bytes;
-    }
-    if (*room && weights > st->d_bweights_cap) {
-        if (st->d_bweights) cudaFree(st->d_bweights);
-        st->d_bweights = nullptr;
-        st->d_bweights_cap = 0;
-        *room = cudaMalloc(&st->d_bweights, weights) == cudaSuccess;
-        if (*room) st->d_bweights_cap = weights;
-    }
-    if (!*room) {
-        cudaGetLastError();
-        if (!st->d_bplan_cap && st->d_bplan) {
-            cudaFree(st->d_bplan);
-            st->d_bplan = nullptr;
+        LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
+        free_staging(st);
+        // short lists are staged behind the readout's words: another pinned buffer costs a state 250 us
+        const size_t cap = std::max(bytes, kPinnedStage);
+        *room = cudaMalloc(&st->d_bplan, cap) == cudaSuccess;
+        if (*room && cap > kPinnedStage) *room = cudaHostAlloc((void**)&st->h_bplan, cap, cudaHostAllocDefault) == cudaSuccess;
+        else if (*room) st->h_bplan = reinterpret_cast<unsigned char*>(st->h_out) + kReadoutBytes;
+        if (*room) {
+            st->d_bplan_cap = cap;
+        } else {
+            cudaGetLastError();
+            if (st->d_bplan) cudaFree(st->d_bplan);
+            st->d_bplan = st->h_bplan = nullptr;
         }
+    }
+    // the weights of one group, 1 MB, come from the runtime's own pool (2 us); those of several cost a state's first flush 58 with
+    // their release, and one part does where there is no room for them
+    if (*room && (st->bparts == 0 || (more && st->bparts < kBlockParts))) {
+        LLG_CUDA(cudaStreamSynchronize(st->stream), "cudaStreamSynchronize");
+        if (st->bweights) cudaFree(st->bweights);
+        st->bweights = nullptr;
+        st->bparts = 0;
+        for (int parts : {more ? kBlockParts : 1, 1}) {
+            if (st->bparts) break;
+            if (cudaMalloc(&st->bweights, parts * kBlockGroup * gate_block_weight_bytes(st->P)) == cudaSuccess) st->bparts = parts;
+            else cudaGetLastError(), st->bweights = nullptr;
+        }
+        *room = st->bparts > 0;
     }
     return LLG_OK;
 }
@@ -389,12 +398,12 @@ GateCounts operator-(const GateCounts& a, const GateCounts& b) {
 int run_block_groups(llg_state* st, BlockPlanner& planner, const std::vector<llg_op>& q, double* mirror, bool* mirrored,
                      std::vector<llg_op>* left) {
     constexpr int kGroup = kBlockGroup;
-    const size_t wb = gate_block_weight_bytes(st->P), slots = block_slots(q.size());
+    const size_t wb = gate_block_weight_bytes(st->P);
     LLG_CUDA(cudaEventSynchronize(st->ops_done), "cudaEventSynchronize");  // the staging buffer's last copies
     st->block_tc_launched = true;
     const BlockPlan& plan = planner.plan;
     size_t from = 0, gates_from = 0, off = 0;
-    int slot = 0;
+    int group = 0;
     std::vector<BlockStep> bs;
     bool rest = planner.advance(0);  // gates that are not planned yet
     while (from < plan.steps.size() || rest) {
@@ -423,8 +432,10 @@ int run_block_groups(llg_state* st, BlockPlanner& planner, const std::vector<llg
         }
         const bool last_group = !rest && to == plan.steps.size();
         int done = 0;
-        const unsigned char* w = static_cast<const unsigned char*>(st->d_bweights) + wb * slot;
+        unsigned char* w = nullptr;
         if (!bs.empty()) {
+            const int part = group++ % st->bparts;  // of the weights, in use in turn
+            w = st->bweights + (size_t)part * kGroup * wb;
             const size_t sbytes = (bs.size() * sizeof(BlockStep) + 255) / 256 * 256;
             const size_t gbytes = ((gates_to - gates_from) * sizeof(BlockGate) + 255) / 256 * 256;
             std::memcpy(st->h_bplan + off, bs.data(), bs.size() * sizeof(BlockStep));
@@ -441,9 +452,9 @@ int run_block_groups(llg_state* st, BlockPlanner& planner, const std::vector<llg
                 }
             // The first group's in the blocks' stream, the others' on one of their own, under the blocks before them: in line
             // they cost 14 us a group (1000 H and CNOT on 12 qubits 1010 -> 908 us, 20 layers on 17 qubits 397 -> 369).
-            // The buffers are free (the wait above) but for the slots that an earlier group's blocks may still read.
+            // The buffers are free (the wait above) but for the weights that an earlier group's blocks may still read.
             const cudaStream_t up = from > 0 ? st->side : st->stream;
-            if (slot == 0 && from > 0) {
+            if (part == 0 && from > 0) {
                 LLG_CUDA(cudaEventRecord(st->slots_free, st->stream), "cudaEventRecord");
                 LLG_CUDA(cudaStreamWaitEvent(st->side, st->slots_free, 0), "cudaStreamWaitEvent");
             }
@@ -452,7 +463,7 @@ int run_block_groups(llg_state* st, BlockPlanner& planner, const std::vector<llg
                      "cudaMemcpyAsync(block plan)");
             LLG_CUDA(launch_gate_block_weights(st->P, reinterpret_cast<const BlockGate*>(st->d_bplan + off + sbytes),
                                                reinterpret_cast<const BlockStep*>(st->d_bplan + off), (int)bs.size(),
-                                               static_cast<unsigned char*>(st->d_bweights) + wb * slot, up,
+                                               w, up,
                                                reinterpret_cast<const double2*>(st->d_bplan + off + sbytes + gbytes)),
                      "block weights");
             ++g_launches;
@@ -461,7 +472,6 @@ int run_block_groups(llg_state* st, BlockPlanner& planner, const std::vector<llg
                 LLG_CUDA(cudaStreamWaitEvent(st->stream, st->weights_done, 0), "cudaStreamWaitEvent");
             }
             off += (sbytes + gbytes + doubles * sizeof(double) + 255) / 256 * 256;
-            slot = (slot + kGroup) % (int)slots;
         }
         for (size_t i = from; i < to; ++i) {
             const BlockStep& p = plan.steps[i];
@@ -642,7 +652,7 @@ int run_fused(llg_state* st, const std::vector<llg_op>& q, double* mirror = null
     planner.advance(st->n < 12 ? 11 : 8);
     bool room = blocks_pay(st->P, st->n, planner.plan);
     if (room)
-        if (int rc = ensure_blocks(st, q.size(), &room)) return rc;
+        if (int rc = ensure_blocks(st, q.size(), planner.advance(0), &room)) return rc;
     if (!room) return run_unblocked(st, q, mirror, mirrored);
     std::vector<llg_op> left;
     if (int rc = run_blocks(st, planner, q, mirror, mirrored, &left)) {
@@ -807,9 +817,8 @@ int llg_destroy(llg_state* st) {
     if (st->d_block_tc) cudaFree(st->d_block_tc);
     if (st->h_block_tc) cudaFreeHost(st->h_block_tc);
     if (st->block_done) cudaEventDestroy(st->block_done);
-    if (st->d_bplan) cudaFree(st->d_bplan);
-    if (st->h_bplan) cudaFreeHost(st->h_bplan);
-    if (st->d_bweights) cudaFree(st->d_bweights);
+    free_staging(st);
+    if (st->bweights) cudaFree(st->bweights);
     if (st->weights_done) cudaEventDestroy(st->weights_done);
     if (st->slots_free) cudaEventDestroy(st->slots_free);
     if (st->side) cudaStreamDestroy(st->side);

@@ -28,6 +28,7 @@ std::map<void*, std::pair<void*, int>> recorded;
 std::map<void*, std::map<void*, int>> waited;
 size_t free_bytes = (size_t)200 << 30;
 std::map<void*, size_t> live;
+int malloc_limit = -1;                // pieces of 4 KB and more that are left (-1: any number)
 
 cudaError_t call(const char* kind, cudaError_t error = cudaErrorUnknown) {
     const int k = ++calls[kind];
@@ -50,6 +51,10 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { return *f = free_bytes, *t = (size_t)256 << 30, cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
     const cudaError_t e = call("malloc", cudaErrorMemoryAllocation);
+    if (malloc_limit >= 0 && n >= 4096 && --malloc_limit < 0) {
+        malloc_limit = 0;
+        return *p = nullptr, cudaErrorMemoryAllocation;
+    }
     if (e != cudaSuccess || n > free_bytes) return *p = nullptr, cudaErrorMemoryAllocation;
     free_bytes -= n;
     *p = std::malloc(n < 64 ? 64 : n);
@@ -225,6 +230,28 @@ int flush(int n, int precision, const char* path) {
     return 0;
 }
 
+// A long list with room for `more` pieces of memory only: the weights' parts take turns, and no work waits for room.
+int little_room(int more) {
+    llg_state* st = nullptr;
+    const std::vector<llg_op> q = layered(14, 200);  // some 400 blocks in 26 groups
+    if (llg_create(14, LLG_F64, &st) || llg_set_fusion(st, LLG_FUSE_TILE, 12)) return fail("create");
+    if (llg_apply_ops(st, q.data(), (int)q.size()) || llg_sync(st)) return fail("tile passes");  // their buffers are kept
+    if (llg_set_fusion(st, LLG_FUSE_TILE, 0) || llg_apply_ops(st, q.data(), (int)q.size())) return fail("apply");
+    calls.clear();
+    malloc_limit = more;
+    if (llg_sync(st)) return fail("flush");
+    const int first = calls["block"];
+    // one piece for the plan, one for the first group's weights
+    if ((first > 0) != (more >= 2)) return fail(more >= 2 ? "blocks had room" : "blocks had no room");
+    if (first == 0 && calls["tile"] == 0) return fail("neither form ran");
+    malloc_limit = -1;
+    if (llg_apply_ops(st, q.data(), (int)q.size()) || llg_sync(st)) return fail("the next flush");
+    if (calls["block"] <= first) return fail("blocks have room again");
+    llg_destroy(st);
+    if (!idle() || !live.empty()) return fail("memory or work left at the end of the state");
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -235,6 +262,7 @@ int main(int argc, char** argv) {
     if (what == "record") rc = second_stream("event record", 1, 4);
     if (what == "wait") rc = second_stream("wait event", 1, 2);
     if (what == "block") rc = second_stream("block", 20, 20);
+    if (what == "room" && argc == 3) rc = little_room(std::atoi(argv[2]));
     if (what == "plan" && argc == 6) rc = plan(std::atoi(argv[2]), std::atoi(argv[3]), argv[4], argv[5]);
     if (what == "flush" && argc == 5) return flush(std::atoi(argv[2]), std::atoi(argv[3]), argv[4]);
     if (!rc) std::printf("ok\n");

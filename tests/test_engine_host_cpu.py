@@ -142,3 +142,8 @@ def test_a_plan_and_what_is_left_of_the_list(exe, tmp_path, n, blocks):
             for g in gates[s["gate_begin"]:s["gate_begin"] + s["ngates"]]:
                 psi = test_blockplan_cpu._apply(psi, n, g, qubits)
         assert np.max(np.abs(oracle.run_ops(n, left, psi) - oracle.run_ops(n, ops))) <= 1e-12
+
+
+@pytest.mark.parametrize("more", [0, 1, 2, 3, 5, 8, 9, 40])
+def test_little_device_memory(exe, more):
+    run(exe, "room", str(more))
