@@ -324,9 +324,6 @@ uint64_t block_tiles(int n) { return n > 12 ? 1ULL << (n - 12) : 1; }
 constexpr int kBatchBlockQubits = 10;
 constexpr size_t kWeightsCap = (size_t)256 << 20;
 
-// seconds an amplitude that tile passes compute for these gates
-double tile_arith(const GateCounts& c) { return (kTileMixFma * (c.h + c.real + c.general) + kTileDiagFma * c.diag) / kTileFmaRate; }
-
 struct BlockSet {
     std::vector<char> in;                          // per circuit: takes blocks
     std::vector<BlockStep> steps;                  // of all circuits, one after the other
@@ -337,9 +334,11 @@ struct BlockSet {
 };
 
 // Which circuits take gate blocks, and their launches.  Blocks against tile passes for the batch as a whole, by
-// the rates of llg_cost.h, 2.6 us a gate of tile passes at least; a launch of blocks 5 us and 4.5 us for every tile
-// of the CTA that has most.  Measured, tile passes / blocks, random gates: 36 circuits of 10 to 18 qubits and 200
-// gates 1048 / 335 us; 512 of 10 to 22, 152.9 / 43.6 ms; 5 of 12 and 13 qubits and 100 gates 318 / 103 us; 16 of
+// the rates of llg_cost.h: tile passes take their arithmetic together and no less than the longest circuit's latencies; a launch
+// of blocks 5 us, 8 us for every further wave of CTAs (90, 160, 200 and 400 circuits of one tile: 13, 22, 25 and 38 us a launch)
+// and 4.5 us for every tile of the CTA that has most.  First by the gates' counts alone, since plans that come
+// to nothing made a batch's creation 10 to 20 % longer.  Measured, tile passes / blocks, random gates: 36 circuits of 10 to 18
+// qubits and 200 gates 1048 / 335 us; 512 of 10 to 22, 152.9 / 43.6 ms; 5 of 12 and 13 qubits and 100 gates 318 / 103 us; 16 of
 // 12 to 16 and 40 gates 312 / 73 us; 200 of 12 qubits and 200 gates, each its own CTA either way, keep 950 us of
 // tile passes.
 // room: bytes of device memory for the weights.
@@ -353,49 +352,70 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
     std::vector<Circuit> list;
     out.in.assign(count, 0);
     double arith = 0.0, longest = 0.0, small_arith = 0.0, small_longest = 0.0;
-    uint64_t at = 0;
-    int alone = 0;  // circuits of one tile that keep the queue
     const size_t cap = room / gate_block_weight_bytes(LLG_F64);
+    std::vector<char> fits(count, 0);
+    std::vector<double> latency(count), work(count);
+    double rounds = 0.0, tiles = 0.0;
+    const std::vector<MatrixOp> none;
+    for (int c = 0; c < count; ++c) {
+        const int n = n_qubits[c], nops = (int)(off[c + 1] - off[c]);
+        const llg_op* mine = ops + off[c];
+        int two = 0;
+        double partners = 0.0;
+        const GateCounts g = count_gates(n, mine, nops, none, &two, &partners);
+        latency[c] = tile_latency_seconds(LLG_F64, n, g);
+        work[c] = tile_arith_seconds(LLG_F64, n, g);
+        bool fit = n >= kBatchBlockQubits && nops > 0 && g.h + g.real + g.general > 0 && keeps_norms(mine, nops);
+        for (int i = 0; fit && i < nops; ++i) fit = !(mine[i].kind == LLG_OP_MCZ && __builtin_popcountll(mine[i].mask) > 5);
+        fits[c] = fit;
+        (fit ? arith : small_arith) += work[c];
+        double& most = fit ? longest : small_longest;
+        most = std::max(most, latency[c]);
+        if (fit) {
+            const double blocks = likely_blocks(n, g, two, partners);
+            rounds = std::max(rounds, blocks);
+            tiles += blocks * (double)block_tiles(n);
+        }
+    }
+    auto pays = [&](double t_blocks) {
+        return std::max(t_blocks, std::max(small_arith, small_longest)) <
+               0.9 * std::max(arith + small_arith, std::max(longest, small_longest));
+    };
+    const double waves = std::ceil((double)std::count(fits.begin(), fits.end(), 1) / sms);
+    if (rounds == 0.0 || !pays(rounds * (5e-6 + 8e-6 * (waves - 1.0)) + 4.5e-6 * (rounds + tiles / sms))) return false;
+    uint64_t at = 0;
+    int alone = 0;  // circuits that keep the queue
     for (int c = 0; c < count; ++c) {
         const int n = n_qubits[c], nops = (int)(off[c + 1] - off[c]);
         const uint64_t offset = at;
-        const double amps = std::ldexp(1.0, n);
         at += 1ULL << n;
-        std::vector<llg_op> mine(ops + off[c], ops + off[c + 1]);
-        bool fits = n >= kBatchBlockQubits && nops > 0 && has_block_plan(n, mine.data(), nops) && keeps_norms(mine.data(), nops);
-        for (llg_op& o : mine) {
-            o.param = -1;
-            if (o.kind == LLG_OP_MCZ && __builtin_popcountll(o.mask) > 5) fits = false;
-        }
+        bool fit = fits[c];
         std::unique_ptr<BlockPlanner> planner;
-        if (fits) {
+        if (fit) {
+            std::vector<llg_op> mine(ops + off[c], ops + off[c + 1]);
+            for (llg_op& o : mine) o.param = -1;
             planner.reset(new BlockPlanner(n, mine.data(), nops, true));
             while (planner->advance(64)) {
             }
             // a state's flush keeps off blocks for the same gates (llg_internal.h)
-            const GateCounts& g = planner->plan.counts;
-            fits = !planner->plan.fades && g.h + g.real + g.general > 0;
+            fit = !planner->plan.fades && out.steps.size() + planner->plan.steps.size() <= cap;
         }
-        if (!fits) {
-            // about three multiply-adds a gate
-            small_arith += 2.0 * nops * amps / kTileFmaRate;
-            small_longest = std::max(small_longest, 2.0e-6 * nops);
+        if (!fit) {
+            if (fits[c]) {
+                arith -= work[c];
+                small_arith += work[c];
+                small_longest = std::max(small_longest, latency[c]);
+            }
             ++alone;
             continue;
         }
         const BlockPlan& p = planner->plan;
-        if (out.steps.size() + p.steps.size() > cap) {
-            small_arith += tile_arith(p.counts) * amps;
-            continue;
-        }
         list.push_back({c, n, offset, (int)out.steps.size(), (int)p.steps.size()});
         for (BlockStep st : p.steps) {
             st.gate_begin += (int)out.gates.size();
             out.steps.push_back(st);
         }
         out.gates.insert(out.gates.end(), p.gates.begin(), p.gates.end());
-        arith += tile_arith(p.counts) * amps;
-        longest = std::max(longest, 2.6e-6 * (double)p.gates.size());
     }
     if (list.empty()) return false;
     // large circuits first, so that a launch does not end with one
@@ -404,11 +424,12 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
     const int budget = std::max(sms / 2, sms - std::min(alone, sms / 8));
     double t_blocks = 0.0;
     for (int r = 0;; ++r) {
-        uint64_t tiles = 0;
+        uint64_t tiles = 0, largest = 0;
         int active = 0;
         for (const Circuit& k : list)
             if (r < k.blocks) {
                 tiles += block_tiles(k.n);
+                largest = std::max(largest, block_tiles(k.n));
                 ++active;
             }
         if (!active) break;
@@ -447,11 +468,11 @@ bool plan_blocks(int count, const int* n_qubits, const llg_op* ops, const int64_
         }
         out.rounds.push_back({first, (int)out.ctas.size() - first});
         out.tiles += (int64_t)tiles;
-        t_blocks += 5e-6 + 4.5e-6 * (one_wave ? (double)per : (double)tiles / budget + per);
+        const double waves = std::ceil((double)out.rounds.back().second / sms);
+        t_blocks += 5e-6 + 8e-6 * (waves - 1.0) + 4.5e-6 * (one_wave ? (double)per : (double)tiles / budget + (double)std::min(per, largest));
     }
     for (const Circuit& k : list) out.in[k.c] = 1;
-    return std::max(t_blocks, std::max(small_arith, small_longest)) <
-           0.9 * std::max(arith + small_arith, std::max(longest, small_longest));
+    return pays(t_blocks);
 }
 
 }  // namespace

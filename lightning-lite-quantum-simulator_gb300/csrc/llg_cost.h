@@ -11,9 +11,8 @@
 
 namespace llg {
 
-// FP64 tile passes of large registers: multiply-adds a second, and an amplitude for a merged one-qubit gate that mixes and for a
-// diagonal one
-constexpr double kTileFmaRate = 0.56e12, kTileMixFma = 3.2, kTileDiagFma = 4.0;
+// FP64 tile passes of large registers: multiply-adds a second, and an amplitude for a merged one-qubit gate that mixes
+constexpr double kTileFmaRate = 0.56e12, kTileMixFma = 3.2;
 // seconds an amplitude: a pass that only moves or signs (2.6 ms per 2^30)
 constexpr double kSingleAmp = 2.4e-12;
 
@@ -37,18 +36,21 @@ inline TileGates tile_latency(int P, int n) {
 // Tile passes for these gates: their latencies (15 % more on several CTAs) and arithmetic (a CNOT between random qubits takes
 // 38 us at 2^24 amplitudes in FP64, 18.6 in double-float), at least one read and write of the state; channels are sparse
 // passes of their own, 6.2 ms per 2^30 on one qubit of a density matrix, 9 on two, at least 6 us.
-inline double tile_seconds(int P, int n, const GateCounts& c) {
-    const bool f64 = P == LLG_F64;
-    const double amps = std::ldexp(1.0, n);
+inline double tile_latency_seconds(int P, int n, const GateCounts& c) {
     const TileGates l = tile_latency(P, n);
-    const double latency = 1e-6 * (n > 12 ? 1.15 : 1.0) *
-                           (l.h * c.h + l.real * c.real + l.general * c.general + l.diag * c.diag + l.move * c.moves);
+    return 1e-6 * (n > 12 ? 1.15 : 1.0) *
+           (l.h * c.h + l.real * c.real + l.general * c.general + l.diag * c.diag + l.move * c.moves);
+}
+inline double tile_arith_seconds(int P, int n, const GateCounts& c) {
     const int mixing = c.h + c.real + c.general;
-    const double arith = amps * (f64 ? kTileMixFma / kTileFmaRate * mixing + 2.0e-12 * c.diag + 2.3e-12 * c.moves
-                                     : 2.0e-12 * mixing + 1.9e-12 * c.diag + 1.1e-12 * c.moves);
+    return std::ldexp(1.0, n) * (P == LLG_F64 ? kTileMixFma / kTileFmaRate * mixing + 2.0e-12 * c.diag + 2.3e-12 * c.moves
+                                              : 2.0e-12 * mixing + 1.9e-12 * c.diag + 1.1e-12 * c.moves);
+}
+inline double tile_seconds(int P, int n, const GateCounts& c) {
+    const double amps = std::ldexp(1.0, n), latency = tile_latency_seconds(P, n, c), arith = tile_arith_seconds(P, n, c);
     const double channels = c.small * std::max(6e-6, amps * 5.8e-12) + c.large * std::max(6e-6, amps * 8.4e-12);
-    const bool gates = mixing + c.diag + c.moves + c.flips > 0;
-    const double both = arith + latency - (f64 ? 0.0 : 0.5 * std::min(arith, latency));  // the FP32 pipe hides more
+    const bool gates = c.h + c.real + c.general + c.diag + c.moves + c.flips > 0;
+    const double both = arith + latency - (P == LLG_F64 ? 0.0 : 0.5 * std::min(arith, latency));  // the FP32 pipe hides more
     return (gates ? std::max(both, amps * 4.8e-12) : 0.0) + channels;
 }
 
