@@ -63,16 +63,9 @@ Class2x2 class_2x2(const double* m) {
     if (m[3] == 0.0 && m[5] == 0.0) return m[0] == m[2] && m[0] == m[4] && m[0] == -m[6] ? kH : kRealY;
     return m[2] == 0.0 && m[4] == 0.0 ? kRealX : kGeneral;
 }
-Class2x2 class_of(const llg_op& o) {
-    switch (o.kind) {
-        case LLG_OP_H: return kH;
-        case LLG_OP_X: return kMove;
-        case LLG_OP_RX: return kRealX;
-        case LLG_OP_RY: return kRealY;
-        case LLG_OP_RZ: return kDiag;
-        default: return class_2x2(o.m);
-    }
-}
+// of the named one-qubit gates, by kind
+constexpr Class2x2 kNamed[] = {kH, kMove, kRealX, kRealY, kDiag};
+static_assert(LLG_OP_H == 0 && LLG_OP_X == 1 && LLG_OP_RX == 2 && LLG_OP_RY == 3 && LLG_OP_RZ == 4, "kNamed's order");
 // log2 of a 2x2's smallest entry where that is far below 1 (but no rounding of 0), else 0
 float small_entry(const double* m) {
     double least = 1.0;
@@ -94,9 +87,13 @@ void add_classes(const int* count, GateCounts& c) {
 
 GateCounts count_gates(int n, const llg_op* ops, int nops, const std::vector<MatrixOp>& matrices, int* two, double* partners) {
     GateCounts c;
-    Class2x2 open[64] = {};
-    uint64_t met[64] = {};
+    Class2x2 open[64];
+    uint64_t met[64];
     int count[kClasses] = {};
+    for (int q = 0; q < n; ++q) {
+        open[q] = kNone;
+        met[q] = 0;
+    }
     auto close = [&](int q, uint64_t mask) {
         ++count[open[q]];
         open[q] = kNone;
@@ -105,7 +102,9 @@ GateCounts count_gates(int n, const llg_op* ops, int nops, const std::vector<Mat
     *two = 0;
     for (int i = 0; i < nops; ++i) {
         const llg_op& o = ops[i];
-        if (o.kind == LLG_OP_CNOT || o.kind == LLG_OP_CZ) {
+        if (o.kind <= LLG_OP_RZ) {
+            open[o.q0] = kMerge[open[o.q0]][kNamed[o.kind]];
+        } else if (o.kind == LLG_OP_CNOT || o.kind == LLG_OP_CZ) {
             const uint64_t mask = 1ULL << o.q0 | 1ULL << o.q1;
             close(o.q0, mask);
             close(o.q1, mask);
@@ -122,7 +121,7 @@ GateCounts count_gates(int n, const llg_op* ops, int nops, const std::vector<Mat
             for (int j = 0; j < m.k; ++j) close(m.q[j], mask);
             ++(m.k <= 2 ? c.small : c.large);
         } else {
-            open[o.q0] = kMerge[open[o.q0]][class_of(o)];
+            open[o.q0] = kMerge[open[o.q0]][class_2x2(o.m)];
         }
     }
     int pairs = 0;

@@ -43,11 +43,11 @@ inline double tile_latency_seconds(int P, int n, const GateCounts& c) {
 }
 inline double tile_arith_seconds(int P, int n, const GateCounts& c) {
     const int mixing = c.h + c.real + c.general;
-    return std::ldexp(1.0, n) * (P == LLG_F64 ? kTileMixFma / kTileFmaRate * mixing + 2.0e-12 * c.diag + 2.3e-12 * c.moves
+    return (double)(1ULL << n) * (P == LLG_F64 ? kTileMixFma / kTileFmaRate * mixing + 2.0e-12 * c.diag + 2.3e-12 * c.moves
                                               : 2.0e-12 * mixing + 1.9e-12 * c.diag + 1.1e-12 * c.moves);
 }
 inline double tile_seconds(int P, int n, const GateCounts& c) {
-    const double amps = std::ldexp(1.0, n), latency = tile_latency_seconds(P, n, c), arith = tile_arith_seconds(P, n, c);
+    const double amps = (double)(1ULL << n), latency = tile_latency_seconds(P, n, c), arith = tile_arith_seconds(P, n, c);
     const double channels = c.small * std::max(6e-6, amps * 5.8e-12) + c.large * std::max(6e-6, amps * 8.4e-12);
     const bool gates = c.h + c.real + c.general + c.diag + c.moves + c.flips > 0;
     const double both = arith + latency - (P == LLG_F64 ? 0.0 : 0.5 * std::min(arith, latency));  // the FP32 pipe hides more
@@ -57,7 +57,7 @@ inline double tile_seconds(int P, int n, const GateCounts& c) {
 // Blocks, and gates on their own between them: a block takes 8.2 us (7.6 on the 6 to 11 qubits of a part of a tile), and from 20
 // qubits on 5.5 us (6.6 in double-float) for every round of the SMs over its tiles of 4096 amplitudes.
 inline double block_seconds(int P, int n, double blocks, double singles) {
-    const double amps = std::ldexp(1.0, n);
+    const double amps = (double)(1ULL << n);
     const double rounds = std::ceil(amps / (4096.0 * 152.0));
     const double block = n < 12 ? 7.6e-6 : n < 20 ? 8.2e-6 : 4e-6 + rounds * (P == LLG_F64 ? 5.5e-6 : 6.6e-6);
     return blocks * block + singles * (3e-6 + amps * kSingleAmp);

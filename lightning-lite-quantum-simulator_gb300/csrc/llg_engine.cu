@@ -616,6 +616,7 @@ bool blocks_allowed(const llg_state* st) {
 // gates as tile passes, channels one by one between them
 int run_unblocked(llg_state* st, const std::vector<llg_op>& q, double* mirror, bool* mirrored) {
     note_growth(st, q);
+    if (st->matrices.empty()) return run_tiles(st, q, mirror, mirrored);
     std::vector<MatrixOp> mats;
     mats.swap(st->matrices);
     bool channels = false;
