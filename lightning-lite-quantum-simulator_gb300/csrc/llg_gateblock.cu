@@ -29,9 +29,10 @@
 //     products were bound by shared-memory reads, 48 clocks for 32 of tensor work).
 //   * 16 (FP64) or 8 epilogue warps: tcgen05.ld, recombination, stores.
 //   * one warp that prefetches into L2.
-// Measured at 26 qubits, ms per 2^30 amplitudes, targets (5, 9, 13, 17, 25) / (0, 1, 2, 3, 4): FP64 8.3 /
+// Measured at 26 qubits, ms per 2^30 amplitudes, targets (5, 9, 13, 17, 25) / (0, 1, 2, 3, 4): FP64 8.5 /
 // 12.6 (9.0k clocks per tile: the MMAs take 6.7k of them, sharing shared memory with the slicers'
-// stores; FP64 pipe 41 % busy with the conversions), double-float 10.1 / 13.0 (bound by slicing).
+// stores; FP64 pipe 43 % busy with the conversions), double-float 10.5 / 12.3 (bound by slicing); with the guards
+// of partly filled tiles 8.7 / 12.7 and 10.7 / 12.3.
 // With the lowest five qubits a warp's 32 accesses go to 32 lines.  The serial form that this replaced
 // (one set of accumulators, load - slice - multiply - recombine one after the other on 16 warps)
 // took 25k clocks per tile, 22 / 26 and 14 / 19 ms.
@@ -222,7 +223,10 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
     const uint32_t tmem = tmem_s;
     // registers of fewer than 12 qubits fill a part of their one tile: the other groups are zeros that nobody stores
     constexpr bool kPart = kSplit || kMixed;  // the forms that such registers take
-    const int groups = !kPart || n >= 12 ? kGroups : 1 << (n - 5);
+    const int present = n >= 12 ? kGroups : 1 << (n - 5), groups = kPart ? present : kGroups;
+    // (double-float's first loads ask in every form: as the compiler orders them without, targets 0 .. 4 take 13.1 ms per 2^30
+    // amplitudes instead of 12.3)
+    constexpr bool kAsk = kPart || P == LLG_DF64;
     const uint64_t ntiles = !kPart || n >= 12 ? (1ULL << (n - 5)) / kGroups : 1;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -239,7 +243,7 @@ __global__ void __launch_bounds__(Shape<P>::kThreads, 1)
         if (tile < ntiles) {
             const auto* pb = psi + (insert0_mask(tile * kGroups + (uint64_t)g, tmask) | (h ? off(1) : 0));
 #pragma unroll
-            for (int k = 0; k < 16; ++k) a[k] = !kPart || g < groups ? __ldcg(pb + off(2 * k)) : typename Elem<P>::S{};
+            for (int k = 0; k < 16; ++k) a[k] = !kAsk || g < present ? __ldcg(pb + off(2 * k)) : typename Elem<P>::S{};
         }
         int slot = 0, egb = 0;
         uint32_t phase = 1;  // of the slot's previous release: the first round needs no wait
