@@ -5,8 +5,9 @@ Workload (seeded, synthetic): a 30-qubit state from |0..0> (16 GiB of complex128
 RX, RY, RZ on every qubit (angles U[0, 2pi)) plus a CNOT brickwork on (i, i+1) with alternating
 offsets -- 1800 rotations + 290 CNOTs = 2090 gates.  One step = reset the state and run the whole
 circuit through the engine, which fuses it into dense 5-qubit blocks on the tensor cores (exact
-products of 8-bit digits, errors no larger than IEEE binary64 arithmetic's) or, where that is
-faster, into shared-memory tile passes on the FP64 pipe; complex128 amplitudes in IEEE binary64.
+products of 8-bit digits, rounded once at 2^-55 of the largest of 32 amplitudes; against the state's
+norm the errors are no larger than IEEE binary64 arithmetic's) or, where that is faster, into
+shared-memory tile passes on the FP64 pipe; complex128 amplitudes are IEEE doubles.
 
 Printed as one JSON line:
   value        gates/s over the whole job (logical, pre-fusion gates), device-timed with CUDA
@@ -595,7 +596,8 @@ def run_ours(args, rank, world, local):
                    "tile_passes": head["tile_passes"], "tile_qubits": head["tile_qubits"],
                    "precision": args.precision,
                    "arithmetic": args.precision if not is_f64(args.precision) else
-                                 "IEEE binary64 (exact 8-bit digit products on the tensor cores, 64-bit integer sums)"
+                                 "binary64 amplitudes; exact 8-bit digit products on the tensor cores, 64-bit integer "
+                                 "sums, rounded once a block at 2^-55 of the largest of 32 amplitudes"
                                  if head["gate_blocks"] else "IEEE binary64 (FP64 pipe)",
                    "fusion": head["fusion"], "autotune": head["autotune"],
                    "l2": f"inputs larger than L2 ({head['state_bytes'] / 2**30:g} GiB state), no flush needed"},
