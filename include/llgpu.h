@@ -188,7 +188,8 @@ int llg_dm_apply_op(llg_state* st, int n, const llg_op* op);
 /* KrausChannel::apply (src/Noise.cpp:174-258): rho <- sum_k K_k rho K_k^+ for nkraus operators
  * of 2^m x 2^m (m = 1 or 2; row-major, interleaved; bit j of an operator's index is
  * targets[j]), applied as one dense block sum_k K_k (x) conj(K_k) on the 2m row and column
- * qubits.  Operators must be trace preserving to 1e-10 (src/Noise.cpp:166-172). */
+ * qubits.  Operators must be trace preserving to 1e-10 (src/Noise.cpp:166-172).  On complex128 and
+ * double-float states whose passes are left to the engine the channel waits in the gate queue. */
 int llg_dm_apply_kraus(llg_state* st, int n, int nkraus, const double* kraus, int m, const int* targets);
 
 /* ---- execution and readout ---- */

@@ -66,7 +66,7 @@ Class2x2 class_2x2(const double* m) {
 // of the named one-qubit gates, by kind
 constexpr Class2x2 kNamed[] = {kH, kMove, kRealX, kRealY, kDiag};
 static_assert(LLG_OP_H == 0 && LLG_OP_X == 1 && LLG_OP_RX == 2 && LLG_OP_RY == 3 && LLG_OP_RZ == 4, "kNamed's order");
-// log2 of a 2x2's smallest entry where that is far below 1 (but no rounding of 0), else 0
+// log2 of the smallest entry of a 2x2 that mixes where that is below 2^-7, else 0 (entries below 2^-50 are roundings of 0)
 float small_entry(const double* m) {
     double least = 1.0;
     for (int k = 0; k < 4; ++k) {
@@ -451,10 +451,14 @@ private:
             g.q1 = v.mat;
             g.pad = v.axis;
         } else if (v.kind == 0) {
+            const Class2x2 cls = class_2x2(mats_[v.mat].m);
             int count[kClasses] = {};
-            count[class_2x2(mats_[v.mat].m)] = 1;
+            count[cls] = 1;
             add_classes(count, out_.counts);
-            small_ += small_entry(mats_[v.mat].m);
+            if (cls != kDiag && cls != kMove) {
+                float& most = small_[local(__builtin_ctzll(v.mask))];
+                most = std::max(most, small_entry(mats_[v.mat].m));
+            }
             g.q0 = local(__builtin_ctzll(v.mask));
             std::memcpy(g.m, mats_[v.mat].m, sizeof(g.m));
         } else if (v.kind == 1) {
@@ -505,11 +509,14 @@ private:
         }
         st.gate_begin = (int)out_.gates.size();
         st.ngates = (int)got_.size();
-        small_ = 0.0f;
+        constexpr float kUnset = -1e9f;  // no gate that mixes
+        for (int b = 0; b < 5; ++b) small_[b] = kUnset;
         for (int id : got_) gate(nodes_[id], to_local);
         out_.steps.push_back(st);
         ++out_.blocks;
-        out_.fades = out_.fades || small_ < -44.0f;
+        float bits = 0.0f;
+        for (int b = 0; b < 5; ++b) bits += small_[b] > kUnset ? small_[b] : 0.0f;
+        out_.fades = out_.fades || bits < -44.0f;
     }
 
     static constexpr int kSeeds = 4;
@@ -527,7 +534,7 @@ private:
     std::vector<int> stamp_, got_;
     std::vector<char> done_, marked_;
     Taken tried_, try_;
-    float small_ = 0.0f;  // of the block's gates
+    float small_[64] = {};  // per qubit of the block: small_entry of the gate that mixes most
     int stamp_id_ = 0, remaining_ = 0, wide_ = 0;
     size_t first_ = 0;
 };

@@ -234,9 +234,9 @@ struct BlockPlan {
     std::vector<double> matrices;  // of the kind-4 gates
     int blocks = 0;
     GateCounts counts;  // of `gates`, for the cost of other plans
-    // A block holds its amplitudes in units of 2^-55 of the group's largest.  Rotations by small angles (or near pi) together make
-    // amplitudes that this leaves nothing of: true once the smallest entries (below 2^-7) of a block's 2x2s multiply to less
-    // than 2^-44.  Such gates are for the tile passes, where every amplitude has its own exponent.
+    // A block holds its amplitudes in units of 2^-55 of the group's largest.  Rotations by small angles (or near pi) on its qubits
+    // make amplitudes that this leaves nothing of: true once the smallest entries (below 2^-7) of the 2x2s that mix most, one
+    // a qubit, multiply to less than 2^-44.  Such gates are for the tile passes, where every amplitude has its own exponent.
     bool fades = false;
 };
 // 2x2 gates of a block have spectral norm at most this, so that its entries stay well below 2

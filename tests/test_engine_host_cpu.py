@@ -147,3 +147,17 @@ def test_a_plan_and_what_is_left_of_the_list(exe, tmp_path, n, blocks):
 @pytest.mark.parametrize("more", [0, 1, 2, 3, 5, 8, 9, 40])
 def test_little_device_memory(exe, more):
     run(exe, "room", str(more))
+
+
+@pytest.mark.parametrize("n,precision", [(12, "complex128"), (16, "df64")])
+def test_small_angles(exe, tmp_path, n, precision):
+    # angles of 0.01 are in reach of a block, angles of 0.001 are not, beside qubits with strong ones they are again
+    def layers(angle, strong=False):
+        recs = []
+        for layer in range(8):
+            recs += [(OP_RY, q, 0, 1.1 if strong and q % 2 else angle) for q in range(n)] + [(OP_RZ, q, 0, 0.4) for q in range(n)]
+            recs += [(OP_CNOT, q, (q + 1) % n) for q in range(n)]
+        return make_ops(recs)
+    assert launches(exe, tmp_path, n, precision, layers(0.01))[0] > 0
+    assert launches(exe, tmp_path, n, precision, layers(0.001))[0] == 0
+    assert launches(exe, tmp_path, n, precision, layers(0.001, True))[0] > 0
