@@ -17,7 +17,7 @@
 //
 // IEEE complex128 circuits on 12 to 26 qubits run as dense 5-qubit blocks on the tensor cores where
 // that costs less (llg_gateblock.cu; the gradients of a block from one 32 x 32 matrix,
-// llg_adjblock.cu); not with checkpoints or a set CTA size.
+// llg_adjblock.cu); not with checkpoints, a set CTA size or 2x2s that are not unitary.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
