@@ -26,7 +26,10 @@ def nearly_full():
     torch.cuda.init()
     torch.cuda.synchronize()
     free, _ = torch.cuda.mem_get_info()
-    hold = torch.empty(free - 400 * MB, dtype=torch.uint8, device="cuda")
+    try:
+        hold = torch.empty(free - 400 * MB, dtype=torch.uint8, device="cuda")
+    except torch.cuda.OutOfMemoryError:
+        pytest.skip("the device's memory cannot be taken in one piece")
     yield lambda: torch.cuda.mem_get_info()[0]
     del hold
     torch.cuda.empty_cache()
